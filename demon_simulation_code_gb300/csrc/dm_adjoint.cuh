@@ -394,7 +394,9 @@ __device__ __forceinline__ void adj_pair_sums_fp32c(const AdjCloud &d, int li, b
             for (int k = 0; k < NQ; k++) s_f[k * kAsJ + e] = v[k];  // s_c[k][e/4].{x,y,z,w}[e%4]
         }
         __syncthreads();
-        if (!valid) continue;
+        // whole warps only: the lanes beyond a cloud's last particle take part
+        // in the warp votes below (their sums are not used)
+        if (!__any_sync(0xffffffffu, valid)) continue;
         for (int c = 0; c < nch; c++) {
             float4 Q[NQ];
 #pragma unroll

@@ -1,0 +1,252 @@
+// dm_fp64.cuh -- FP64 pair arithmetic for a GPU whose FP64 units run at 1/64
+// of its FP32 rate, and the culled FP64 pair + stage kernel built on it.
+//
+// An FP64 instruction of a warp occupies an SM's FP64 pipe for 16 cycles
+// however many of its lanes are active; in that time the SM issues 64 other
+// instructions.  So everything but the pair terms themselves is kept off the
+// FP64 pipe, and the pair terms always run with full warps:
+//   * which pairs are near the cutoff is found in FP32 (the conservative
+//     filter of filter_threshold), a 32 x 32 bit mask per pair of groups;
+//   * a warp collects the masks of several j groups, lays the hits out as
+//     one dense list (codes in shared memory, ordered by i), evaluates 32
+//     list entries per round, whatever i and j they belong to, and every
+//     lane then adds up its own particle's entries in list order
+//     (deterministic, no atomics);
+//   * 1/r, r and e^{-kappa r} take 13 FP64 instructions (yukawa64) instead
+//     of a square root, a division and an exponential of the math library
+//     (~70); conversions between the two precisions are integer operations.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include <cmath>
+#include <cstring>
+
+#include "dm_device.cuh"
+
+namespace dm {
+namespace cg = cooperative_groups;
+
+// 2^(k/512), k = 0..511, correctly rounded: the Taylor series of
+// exp(k ln2/512) in unevaluated double pairs (~100 bits), at compile time.
+constexpr int kExp2Bits = 9;
+constexpr int kExp2Size = 1 << kExp2Bits;
+struct Exp2Table {
+    double v[kExp2Size];
+};
+struct DD {
+    double hi, lo;
+};
+constexpr DD dd_add(DD a, DD b) {  // Knuth's TwoSum, low parts added plainly
+    const double s = a.hi + b.hi, t = s - a.hi;
+    const double e = ((a.hi - (s - t)) + (b.hi - t)) + (a.lo + b.lo);
+    const double h = s + e;
+    return {h, e - (h - s)};
+}
+constexpr DD dd_mul(DD a, DD b) {  // Dekker's product
+    const double c = 134217729.0;  // 2^27 + 1
+    const double ca = c * a.hi, cb = c * b.hi;
+    const double ah = ca - (ca - a.hi), al = a.hi - ah;
+    const double bh = cb - (cb - b.hi), bl = b.hi - bh;
+    const double p = a.hi * b.hi;
+    const double e = (((ah * bh - p) + ah * bl + al * bh) + al * bl) + (a.hi * b.lo + a.lo * b.hi);
+    const double h = p + e;
+    return {h, e - (h - p)};
+}
+constexpr Exp2Table make_exp2_table() {
+    // ln 2 as an unevaluated pair
+    const DD ln2{0.6931471805599453, 2.3190468138462996e-17};
+    // Horner's scheme in x/j, 1/j as a pair by one Newton correction of the
+    // double quotient
+    Exp2Table t{};
+    for (int k = 0; k < kExp2Size; k++) {
+        const DD x = dd_mul(ln2, DD{(double)k / kExp2Size, 0.0});
+        DD s{1.0, 0.0};
+        for (int j = 30; j >= 1; j--) {
+            const double inv = 1.0 / j;
+            const DD one = dd_mul(DD{inv, 0.0}, DD{(double)j, 0.0});
+            const DD rec{inv, -((one.hi - 1.0) + one.lo) * inv};
+            s = dd_add(DD{1.0, 0.0}, dd_mul(dd_mul(x, rec), s));
+        }
+        t.v[k] = s.hi;
+    }
+    return t;
+}
+static __device__ const Exp2Table g_exp2_table = make_exp2_table();
+
+inline Yukawa64 make_yukawa64(double kappa, double rc2) {
+    Yukawa64 K;
+    const double l_hi = 738.6598609351493, l_lo = 1.0421900155356689e-14;  // 512 log2(e)
+    K.kappa = kappa;
+    K.k_hi = -(kappa * l_hi);
+    K.k_lo = -(std::fma(kappa, l_hi, K.k_hi) + kappa * l_lo);
+    K.k_f = (float)K.k_hi;
+    uint64_t w;
+    std::memcpy(&w, &rc2, sizeof w);
+    K.rc2_word = (uint32_t)(w >> 32);
+    return K;
+}
+
+// Values of one pair at squared distance r2: y = 1/r, ex = e^{-kappa r} and
+// kappa r (formed only by callers that use it: r y kappa).
+struct Yukawa64At {
+    double y, r, ex;
+};
+
+// r2 in [2^-100, 2^100): 6 FP64 instructions for 1/r and r (a third-order
+// step from the FP32 reciprocal square root, 2^-22; e^3 < 2^-63), 7 for the
+// exponential (table of 512, degree-4 polynomial, |remainder| < 2e-18).
+// -kappa r enters as k r with k a pair, rounded once after the integer part
+// is taken off, so the exponential's error does not grow with kappa r.
+__device__ __forceinline__ Yukawa64At yukawa64(double r2, const Yukawa64 &K, const double *tab) {
+    const uint32_t lo = (uint32_t)__double2loint(r2), hi = (uint32_t)__double2hiint(r2);
+    const float rf = __uint_as_float(__funnelshift_l(lo, hi - 0x38000000u, 3));  // truncated to FP32
+    float yf;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(rf));
+    const uint32_t yb = __float_as_uint(yf);
+    const double y0 = __hiloint2double((int)((yb >> 3) + 0x38000000u), (int)(yb << 29));  // exact
+    const double t = __dmul_rn(r2, y0);
+    const double e = fma(-t, y0, 1.0);
+    const double h = __dmul_rn(e, fma(e, 0.375, 0.5));
+    Yukawa64At A;
+    A.y = fma(y0, h, y0);
+    A.r = fma(t, h, t);
+    // n = the integer nearest k r (any integer within ~0.51 of it will do)
+    const float nf = rintf((rf * yf) * K.k_f);
+    const int n = (int)nf;  // <= 0
+    const uint32_t nb = __float_as_uint(nf) & 0x7FFFFFFFu;
+    // -n as a double (n = 0 gives 2^-127: no matter)
+    const double nd = __hiloint2double((int)((nb >> 3) + 0x38000000u), (int)(nb << 29));
+    const double f = fma(A.r, K.k_lo, fma(A.r, K.k_hi, nd));
+    // (ln2/512)^m / m!
+    double p = fma(f, 1.399621994296973e-13, 4.135378350676714e-10);
+    p = fma(f, p, 9.163913992275266e-07);
+    p = fma(f, p, 0.0013538030870311431);
+    p = __dmul_rn(f, p);
+    const double T0 = tab[n & (kExp2Size - 1)];
+    const double T = __hiloint2double(__double2hiint(T0) + ((n >> kExp2Bits) << 20), __double2loint(T0));
+    A.ex = fma(T, p, T);
+    return A;
+}
+
+// Whether a pair is inside the cutoff, bit for bit as the reference decides:
+// by r2's high word away from the cutoff, else by its own operations.
+__device__ __forceinline__ bool in_cutoff64(double dx, double dy, double r2, const Yukawa64 &K) {
+    const uint32_t w = (uint32_t)__double2hiint(r2);
+    if (w + 1u < K.rc2_word) return true;  // r2 < r_c^2 (1 - 2^-21): rounding cannot matter
+    if (w > K.rc2_word + 1u) return false;
+    double r, a;
+    return ref_in_cutoff(dx, dy, K.kappa, r, a);
+}
+
+// r2 outside yukawa64's range (no cloud in SI units gets here; NaN does)
+__device__ __forceinline__ bool yukawa64_odd(double r2) {
+    return (uint32_t)__double2hiint(r2) - (923u << 20) >= (200u << 20);
+}
+__device__ __noinline__ Yukawa64At yukawa64_general(double r2, double kappa) {
+    Yukawa64At A;
+    A.r = sqrt(r2);
+    A.y = 1.0 / A.r;
+    A.ex = exp(-kappa * A.r);
+    return A;
+}
+
+// w of one pair, the force on i from j being C q_i w (dx, dy):
+// w = q_j (1 + kappa r) e^{-kappa r} / r^3 = q_j e^{-kappa r} y^2 (y + kappa)
+// (ShieldedCoulombForce.cpp:144-157); 0 outside the cutoff.
+__device__ __forceinline__ double pair_w64(double dx, double dy, double qj, const Yukawa64 &K, const double *tab) {
+    const double r2 = fma(dx, dx, __dmul_rn(dy, dy));
+    const bool in = in_cutoff64(dx, dy, r2, K);
+    Yukawa64At A;
+    if (yukawa64_odd(r2)) A = yukawa64_general(r2, K.kappa);
+    else A = yukawa64(r2, K, tab);
+    const double w = __dmul_rn(__dmul_rn(qj, A.ex), __dmul_rn(__dmul_rn(A.y, A.y), __dadd_rn(A.y, K.kappa)));
+    return in ? w : 0.0;
+}
+
+// ---------------------------------------------------------------------------
+// The hit list of one warp: masks of up to kHitGroups j groups against the
+// warp's 32 i particles, evaluated in windows of up to kHitPerLane hits of
+// every i.
+// ---------------------------------------------------------------------------
+constexpr int kHitGroups = 8;
+constexpr int kHitPerLane = 8;
+
+struct HitWarp {
+    uint32_t mask[kHitGroups][32];           // bit jl of mask[k][il]: pair (il, group k's jl)
+    int group[kHitGroups];                   // the j groups
+    float4 f[32];                            // FP32 positions of the j group being filtered
+    uint16_t code[kHitPerLane * 32];         // (k << 10) | (jl << 5) | il
+    double2 res[kHitPerLane * 32];           // the entries' results
+};
+
+// Filters j group g (FP32 positions pa, n particles) against this lane's i
+// (px2 = 2 xh_i, py2 = 2 yh_i, nu = -bound_i; nu = INFINITY: no particle) and
+// stores the lane's mask as entry k.  NaN passes: such a pair is decided in
+// FP64.  Returns the lane's number of hits.
+__device__ __forceinline__ int hit_filter(HitWarp &W, int k, int g, int self, const float4 *__restrict__ pa, int n,
+                                          float px2, float py2, float nu) {
+    const int lane = threadIdx.x & 31;
+    const int j = 32 * g + lane;
+    __syncwarp();
+    W.f[lane] = (j < n) ? pa[j] : make_float4(0.0f, 0.0f, INFINITY, 0.0f);
+    if (lane == 0) W.group[k] = g;
+    __syncwarp();
+    uint32_t m = 0u;
+#pragma unroll 8
+    for (int u = 31; u >= 0; u--) {
+        const float4 A = W.f[u];
+        const float d = fmaf(px2, -A.x, fmaf(py2, -A.y, A.z + nu));
+        m = 2u * m + (d >= 0.0f ? 0u : 1u);
+    }
+    if (nu == INFINITY) m = 0u;
+    if (g == self) m &= ~(1u << lane);  // j == i
+    const int left = n - 32 * g;
+    if (left < 32) m &= (1u << left) - 1u;
+    W.mask[k][lane] = m;
+    return __popc(m);
+}
+
+// Evaluates every hit of the first `ng` masks: eval(il, j) gives an entry's
+// result, summed per i in the order (k, jl) into (sx, sy).
+template <class Eval>
+__device__ __forceinline__ void hit_flush(HitWarp &W, int ng, double &sx, double &sy, Eval eval) {
+    const int lane = threadIdx.x & 31;
+    int k = 0;
+    uint32_t m = (ng > 0) ? W.mask[0][lane] : 0u;
+    for (;;) {
+        // this window: the lane's next hits, at most kHitPerLane
+        uint32_t left = __popc(m);
+        for (int kk = k + 1; kk < ng && left < (uint32_t)kHitPerLane; kk++) left += __popc(W.mask[kk][lane]);
+        const int c = min((int)left, kHitPerLane);
+        int off = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, off, o);
+            if (lane >= o) off += v;
+        }
+        const int total = __shfl_sync(0xffffffffu, off, 31);
+        if (total == 0) break;
+        off -= c;
+        for (int t = 0; t < c; t++) {
+            while (m == 0u) m = W.mask[++k][lane];
+            const int u = __ffs(m) - 1;
+            m &= m - 1u;
+            W.code[off + t] = (uint16_t)((k << 10) | (u << 5) | lane);
+        }
+        __syncwarp();
+        for (int t = lane; t < total; t += 32) {
+            const int code = W.code[t];
+            W.res[t] = eval(code & 31, 32 * W.group[code >> 10] + ((code >> 5) & 31));
+        }
+        __syncwarp();
+        for (int t = 0; t < c; t++) {
+            const double2 v = W.res[off + t];
+            sx = __dadd_rn(sx, v.x);
+            sy = __dadd_rn(sy, v.y);
+        }
+        __syncwarp();
+    }
+}
+
+}  // namespace dm
