@@ -32,8 +32,11 @@ namespace {
 
 std::string g_create_error;
 
-// FP64: 2 j-groups x 128 i-lanes, 2 particles per lane, 512-particle j tiles
-constexpr int kNI64 = 128, kG64 = 2, kILP64 = 2, kJT64 = 512;
+// FP64 clouds above this size are swept group by group within reach, which
+// needs the Morton order; up to it every group pair is filtered and the cloud
+// stays in whatever order it is in (at 4096 particles the filter of all 16,384
+// group pairs costs ~3 us a stage, the re-sort ~18 us a step).
+constexpr int kFp64UnsortedMax = 4096;
 constexpr int kGraphSteps = 16;
 
 }  // namespace
@@ -202,6 +205,7 @@ StageParams make_stage_params(dm_cloud *c, int stage, int mode, double dt, const
     P.rc2_hi = (float)(P.rc2 * (1.0 + 4e-6));
     P.kappa_f = (float)kappa;
     P.nkl2e = (float)(-kappa * 1.4426950408889634);
+    P.y64 = make_yukawa64(kappa, P.rc2);
     P.direct_min = direct_min_hits();
     P.near_direct_f2 = near_direct_f2();
     return P;
@@ -215,8 +219,10 @@ struct Variant {
     int precision;
     bool cluster;  // reduce through a thread-block cluster (else global partials + stage_finish)
     bool cull;     // skip j groups whose box is beyond the cutoff from the tile's (group_bounds first)
+    bool boxes;    // the stage leaves the group boxes of the buffer it writes
     int nt;        // threads per CTA
     int tile;      // particles per i tile
+    int min_j;     // j particles per block of a split at least
     size_t smem;
     const void *fn;
     cudaError_t (*launch)(const cudaLaunchConfig_t *, const StageParams &);
@@ -226,19 +232,23 @@ template <int NW, int ILP, int TC, bool CL, bool CULL>
 cudaError_t launch_fp32c(const cudaLaunchConfig_t *cfg, const StageParams &P) {
     return cudaLaunchKernelEx(cfg, pair_stage_fp32c<NW, ILP, TC, CL, CULL>, P);
 }
-template <int NI, int G, int ILP, int JT>
+template <int NW, bool CULL>
 cudaError_t launch_fp64(const cudaLaunchConfig_t *cfg, const StageParams &P) {
-    return cudaLaunchKernelEx(cfg, pair_stage_fp64<NI, G, ILP, JT>, P);
+    return cudaLaunchKernelEx(cfg, pair_group_fp64<NW, CULL>, P);
 }
 
 #define DM_FP32C_VARIANT(NW, ILP, TC, CL)                                                        \
-    {"fp32c<" #NW "," #ILP "," #TC "," #CL ">", DM_FP32C, CL, false, NW * 32, 32 * ILP,           \
+    {"fp32c<" #NW "," #ILP "," #TC "," #CL ">", DM_FP32C, CL, false, !CL, NW * 32, 32 * ILP, 64 * NW, \
      Fp32cSmem<NW, ILP, TC>::bytes, (const void *)pair_stage_fp32c<NW, ILP, TC, CL, false>,       \
      launch_fp32c<NW, ILP, TC, CL, false>}
 #define DM_FP32C_CULL_VARIANT(NW, ILP, TC, CL)                                                   \
-    {"fp32c<" #NW "," #ILP "," #TC "," #CL ",cull>", DM_FP32C, CL, true, NW * 32, 32 * ILP,      \
+    {"fp32c<" #NW "," #ILP "," #TC "," #CL ",cull>", DM_FP32C, CL, true, !CL, NW * 32, 32 * ILP, 64 * NW, \
      Fp32cSmem<NW, ILP, TC>::bytes, (const void *)pair_stage_fp32c<NW, ILP, TC, CL, true>,        \
      launch_fp32c<NW, ILP, TC, CL, true>}
+
+#define DM_FP64_VARIANT(NW, CULL, SUFFIX)                                                        \
+    {"fp64<" #NW SUFFIX ">", DM_FP64, true, CULL, true, NW * 32, 32, 32 * NW, sizeof(Group64Smem<NW>), \
+     (const void *)pair_group_fp64<NW, CULL>, launch_fp64<NW, CULL>}
 
 const Variant kVariants[] = {
     DM_FP32C_VARIANT(8, 4, 256, true),
@@ -252,13 +262,14 @@ const Variant kVariants[] = {
     DM_FP32C_CULL_VARIANT(8, 2, 256, false),
     DM_FP32C_CULL_VARIANT(4, 2, 128, false),
     DM_FP32C_CULL_VARIANT(8, 4, 256, true),
-    {"fp64<128,2,2,512>", DM_FP64, true, false, kNI64 * kG64, kNI64 * kILP64,
-     Fp64Smem<kNI64, kG64, kILP64>::bytes(kJT64),
-     (const void *)pair_stage_fp64<kNI64, kG64, kILP64, kJT64>, launch_fp64<kNI64, kG64, kILP64, kJT64>},
+    DM_FP64_VARIANT(8, false, ""),
+    DM_FP64_VARIANT(8, true, ",near"),
+    DM_FP64_VARIANT(4, true, ",near"),
+    DM_FP64_VARIANT(4, false, ""),
 };
 constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
 constexpr int kDefaultVariant32 = 0;
-constexpr int kDefaultVariant64 = kNumVariants - 1;
+constexpr int kDefaultVariant64 = kNumVariants - 1, kDefaultVariant64Cull = kNumVariants - 2;
 constexpr int kMaxSplitGlobal = 64;
 
 int ensure_kernel_attrs(dm_ctx *ctx) {
@@ -339,7 +350,8 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-int variant_groups(const Variant &k) { return k.precision == DM_FP64 ? kG64 : k.nt / 32; }
+// Whether steps and force evaluations of n particles run on the Morton order.
+bool wants_order(int n, int precision) { return precision == DM_FP32C || n > kFp64UnsortedMax; }
 
 // attr must hold 2 entries: programmatic serialization (see pdl_wait) and,
 // for cluster variants, the cluster shape.
@@ -375,7 +387,7 @@ int model_split(dm_ctx *ctx, const Variant &k, int n, int n_pad) {
     int best_s = 1;
     double best_cost = 1e300;
     for (int S = 1; S <= smax; S++) {
-        if (S > 1 && n_pad / S < 64 * variant_groups(k)) break;
+        if (S > 1 && n_pad / S < k.min_j) break;
         int slots = 0;
         if (k.cluster) {
             cudaLaunchAttribute attr[2];
@@ -428,6 +440,7 @@ int launch_variant(dm_cloud *c, int vi, int S, int stage, int mode, double dt, c
     StageParams P = make_stage_params(c, stage, mode, dt, dt_dev);
     P.split = S;
     P.partial = c->partial;
+    P.box_out = (k.boxes && mode != kModeForceOnly) ? 1 : 0;
     const int ntiles = (c->n + k.tile - 1) / k.tile;
     cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t cfg = make_cfg(ctx, k, ntiles, S, attr);
@@ -460,15 +473,13 @@ int launch_variant(dm_cloud *c, int vi, int S, int stage, int mode, double dt, c
         ctx->prof_pairs += (double)c->n * (double)(c->n - 1);
     }
     if (!k.cluster) {
-        // stage_finish also writes the group boxes of the buffer the stage writes
-        P.box_out = (mode != kModeForceOnly) ? 1 : 0;
         if (P.f.flags & ~kBasicForces)
             DM_CUDA(ctx, launch_pdl(stage_finish, dim3((c->n + 63) / 64), dim3(64), 0, ctx->stream, P));
         else  // one thread per particle and axis, one block per 32-particle group
             DM_CUDA(ctx, launch_pdl(stage_finish_axes, dim3(2 * ((c->n + 63) / 64)), dim3(64), 0, ctx->stream, P));
         ctx->launches++;
     }
-    if (mode != kModeForceOnly) c->boxes_valid[stage & 1] = !k.cluster;
+    if (mode != kModeForceOnly) c->boxes_valid[stage & 1] = k.boxes;
     return DM_OK;
 }
 
@@ -506,14 +517,15 @@ int tune_precision(dm_cloud *c, int precision) {
         if (!kVariants[c->tuned_variant[pi]].cluster) return ensure_partial(c, c->split[pi]);
         return DM_OK;
     }
-    const int defv = precision == DM_FP32C ? kDefaultVariant32 : kDefaultVariant64;
+    const bool order = wants_order(c->n, precision);
+    const int defv = precision == DM_FP32C ? kDefaultVariant32 : order ? kDefaultVariant64Cull : kDefaultVariant64;
     int best_v = defv, best_s = model_split(ctx, kVariants[defv], c->n, c->n_pad);
     if (ctx->autotune) {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         DM_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &cs));
         if (cs != cudaStreamCaptureStatusNone)
             return ctx->fail(DM_ERR_STATE, "autotuning needs an uncaptured stream (run one step first)");
-        if (c->order_dirty) {  // tune on the particle order the steps will see
+        if (order && c->order_dirty) {  // tune on the particle order the steps will see
             int rc = reorder(c);
             if (rc) return rc;
         }
@@ -524,7 +536,7 @@ int tune_precision(dm_cloud *c, int precision) {
         // and re-expands), and the best shape differs between them.
         const bool big = (double)c->n * c->n > 4e9;  // ~64k particles: keep tuning short
         int nstates = 1;
-        if (!big && c->d.rc2 > 0.0 && std::isfinite(c->d.rc2)) {
+        if (!big && !c->order_dirty && c->d.rc2 > 0.0 && std::isfinite(c->d.rc2)) {
             double v[4];  // bounding box min x, min y, max x, max y
             DM_CUDA(ctx, cudaMemcpyAsync(v, c->sort.box + 4, sizeof v, cudaMemcpyDeviceToHost, ctx->stream));
             DM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -546,7 +558,7 @@ int tune_precision(dm_cloud *c, int precision) {
         const bool verbose = ev && ev[0] && ev[0] != '0';
         for (int vi = 0; vi < kNumVariants; vi++) {
             const Variant &k = kVariants[vi];
-            if (k.precision != precision) continue;
+            if (k.precision != precision || (precision == DM_FP64 && k.cull != order)) continue;
             const int sm = model_split(ctx, k, c->n, c->n_pad);
             std::vector<int> cands = {sm};
             const int extra_c[] = {1, 2, 3, 4, 6, 8, 12, 16};
@@ -558,7 +570,7 @@ int tune_precision(dm_cloud *c, int precision) {
             std::sort(cands.begin(), cands.end());
             cands.erase(std::unique(cands.begin(), cands.end()), cands.end());
             for (int S : cands) {
-                if (S > 1 && c->n_pad / S < 64 * variant_groups(k)) continue;
+                if (S > 1 && c->n_pad / S < k.min_j) continue;
                 if (k.cluster) {
                     int nc = 0;
                     cudaLaunchAttribute attr[2];
@@ -660,8 +672,9 @@ int reorder(dm_cloud *c) {
 
 int enqueue_steps(dm_cloud *c, int nsteps, double dt, int precision) {
     for (int s = 0; s < nsteps; s++) {
-        if (c->order_dirty ||
-            (c->reorder_interval > 0 && c->host_steps % (unsigned)c->reorder_interval == 0)) {
+        if (wants_order(c->n, precision) &&
+            (c->order_dirty ||
+             (c->reorder_interval > 0 && c->host_steps % (unsigned)c->reorder_interval == 0))) {
             int rc = reorder(c);
             if (rc) return rc;
         }
@@ -683,8 +696,8 @@ int run_steps(dm_cloud *c, int nsteps, double dt, int precision) {
     }
     // the captured step sequence re-sorts at fixed positions: align the
     // host step counter and clear a pending re-sort first
-    while (nsteps > 0 && (c->order_dirty ||
-                          (c->reorder_interval > 0 && c->host_steps % kGraphSteps != 0))) {
+    while (nsteps > 0 && wants_order(c->n, precision) &&
+           (c->order_dirty || (c->reorder_interval > 0 && c->host_steps % kGraphSteps != 0))) {
         int rc = enqueue_steps(c, 1, dt, precision);
         if (rc) return rc;
         nsteps--;
@@ -693,6 +706,11 @@ int run_steps(dm_cloud *c, int nsteps, double dt, int precision) {
     const GraphKey key{precision, kGraphSteps, dt};
     auto it = c->graphs.find(key);
     if (it == c->graphs.end()) {
+        if (c->tuned_variant[precision == DM_FP32C ? 1 : 0] < 0) {  // not inside the capture
+            int rc = ensure_kernel_attrs(ctx);
+            if (!rc) rc = tune_precision(c, precision);
+            if (rc) return rc;
+        }
         cudaGraph_t g = nullptr;
         const unsigned long long saved = c->host_steps;
         const long long saved_launches = ctx->launches;
@@ -1102,7 +1120,7 @@ int dm_cloud_eval_forces_device(dm_cloud *c, int precision, double *d_fx, double
     if (precision != DM_FP64 && precision != DM_FP32C)
         return ctx->fail(DM_ERR_ARG, "bad precision %d", precision);
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
-    if (c->order_dirty) {  // spatial order first (internal only: outputs are in the caller's order)
+    if (c->order_dirty && wants_order(c->n, precision)) {  // spatial order first (internal only: outputs are in the caller's order)
         const int rc = reorder(c);
         if (rc) return rc;
     }
@@ -1286,6 +1304,7 @@ int dm_kernel_variants(char *buf, size_t len) {
 int dm_cloud_set_kernel(dm_cloud *c, const char *variant, int split) {
     if (!c || !variant) return DM_ERR_ARG;
     dm_ctx *ctx = c->ctx;
+    if (std::strcmp(variant, "fp64<128,2,2,512>") == 0) variant = "fp64<4>";  // its name in earlier versions
     int vi = -1;
     for (int v = 0; v < kNumVariants; v++)
         if (std::strcmp(kVariants[v].name, variant) == 0) vi = v;

@@ -100,6 +100,14 @@ inline int check_force_params(const ForceParams &p, const char **why) {
 
 enum StageMode : int { kModeStep = 0, kModeForceOnly = 1 };
 
+// Constants of the FP64 pair terms of one cloud (make_yukawa64).
+struct Yukawa64 {
+    double kappa;
+    double k_hi, k_lo;  // -kappa 512 log2(e) as an unevaluated pair
+    float k_f;          // the same in FP32
+    uint32_t rc2_word;  // high word of r_c^2: r^2 with a smaller one is inside the cutoff
+};
+
 // Everything a stage kernel needs, passed by value.
 struct StageParams {
     CloudDev c;
@@ -118,6 +126,7 @@ struct StageParams {
     float rc2_lo, rc2_hi; // FP32 certain-in / certain-out bounds on r^2
     float kappa_f;
     float nkl2e;          // -kappa*log2(e): e^{-kappa r} = 2^{nkl2e r}
+    Yukawa64 y64;
     // FP32C sweep: a filtered chunk whose 4 j pass the filter for at least
     // this many of the 128 (lane, j) pairs of a slot is evaluated directly
     // (all lanes, cutoff by a select) instead of through per-lane hit bits

@@ -143,7 +143,7 @@ __device__ __forceinline__ bool in_cutoff64(double dx, double dy, double r2, con
 __device__ __forceinline__ bool yukawa64_odd(double r2) {
     return (uint32_t)__double2hiint(r2) - (923u << 20) >= (200u << 20);
 }
-__device__ __noinline__ Yukawa64At yukawa64_general(double r2, double kappa) {
+static __device__ __noinline__ Yukawa64At yukawa64_general(double r2, double kappa) {
     Yukawa64At A;
     A.r = sqrt(r2);
     A.y = 1.0 / A.r;

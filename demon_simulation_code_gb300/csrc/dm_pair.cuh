@@ -28,6 +28,7 @@
 #include <type_traits>
 
 #include "dm_device.cuh"
+#include "dm_fp64.cuh"
 
 namespace dm {
 namespace cg = cooperative_groups;
@@ -748,6 +749,21 @@ __device__ __forceinline__ double finish_rank_sum(const StageParams &P, int i, i
     return __dmul_rn(pair_scale(P, i), (double)sa.hi + (double)(sa.lo - ca));
 }
 
+// The box of a 32-particle group from its lanes' FP32 positions; lane 0
+// stores it.
+__device__ __forceinline__ void store_group_box(float4 *gbox, bool live, float xh, float yh, bool store) {
+    float x0 = live ? xh : INFINITY, y0 = live ? yh : INFINITY;
+    float x1 = live ? xh : -INFINITY, y1 = live ? yh : -INFINITY;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
+        y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
+        x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
+        y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
+    }
+    if ((threadIdx.x & 31) == 0 && store) *gbox = make_float4(x0, y0, x1, y1);
+}
+
 // Completes a stage after a non-cluster pair launch when forces outside
 // kBasicForces are on (they couple the axes): one particle per thread, the
 // rank sums of both axes, then the stage epilogue.
@@ -761,37 +777,52 @@ static __global__ void __launch_bounds__(64) stage_finish(const StageParams P) {
     }
     if (P.box_out) {  // a warp is one 32-particle group: its box in the buffer just written
         const int bw = P.stage & 1;
-        float x0 = INFINITY, y0 = INFINITY, x1 = -INFINITY, y1 = -INFINITY;
-        if (i < P.c.n) {
-            const float4 A = P.c.pa[bw][i];
-            x0 = x1 = A.x;
-            y0 = y1 = A.y;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
-            y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
-            x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-            y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
-        }
-        if ((threadIdx.x & 31) == 0 && i < P.c.n_pad) P.c.gbox[bw][i >> 5] = make_float4(x0, y0, x1, y1);
+        const bool live = i < P.c.n;
+        const float4 A = live ? P.c.pa[bw][i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        store_group_box(P.c.gbox[bw] + (i >> 5), live, A.x, A.y, i < P.c.n_pad);
     }
     stage_step_advance(P);
 }
 
-// The same completion with one thread per particle and axis, for the
-// forces in kBasicForces: block = one 32-particle group, warp 0 the x and
-// warp 1 the y components.  Each axis runs exactly the operations
-// stage_epilogue runs for it, in the same order, so the results are the
-// same bits; the finish is a latency-bound chain (rank partials, FP64 at
-// GB300's FP64 rate) and this gives it twice the warps.  The two warps
-// meet once, in shared memory, for what needs both axes: the next stage's
-// packed positions, filter bound and group box.
-static __global__ void __launch_bounds__(64) stage_finish_axes(const StageParams P) {
-    pdl_wait();
-    __shared__ float s_hi[2][32], s_lo[2][32];
-    const int lane = threadIdx.x & 31, ax = threadIdx.x >> 5;
-    const int i = blockIdx.x * 32 + lane;
+// Starts bringing the operands of axes_epilogue for particle i, axis ax, into L1.
+__device__ __forceinline__ void axes_prefetch(const StageParams &P, int i, int ax) {
+    const CloudDev &c = P.c;
+    const bool fo = P.mode == kModeForceOnly;
+    const int s = fo ? 1 : P.stage;
+    const int b = fo ? P.fo_buf : (s - 1) & 1;
+    prefetch_l1((ax ? c.py[b] : c.px[b]) + i);
+    prefetch_l1(((s == 1) ? (ax ? c.vy : c.vx) : (ax ? c.vyc : c.vxc)) + i);
+    prefetch_l1(c.q + i);
+    prefetch_l1(c.m + i);
+    prefetch_l1(c.orig + i);
+    if (!fo) {
+        prefetch_l1((ax ? c.y : c.x) + i);
+        prefetch_l1((ax ? c.vy : c.vx) + i);
+        if (s >= 3) {
+            prefetch_l1(c.a23[2 * ax] + i);
+            prefetch_l1(c.a23[2 * ax + 1] + i);
+        }
+        if (s == 4) {
+            prefetch_l1(c.a1[2 * ax] + i);
+            prefetch_l1(c.a1[2 * ax + 1] + i);
+        }
+    }
+}
+
+struct AxesShared {
+    float hi[2][32], lo[2][32];
+};
+
+// The stage epilogue with one thread per particle and axis, for the forces in
+// kBasicForces: called by the first two warps of a block for one 32-particle
+// group, warp 0 the x and warp 1 the y components, fpa being the axis's pair
+// force.  Each axis runs exactly the operations stage_epilogue runs for it, in
+// the same order, so the results are the same bits; the epilogue is a
+// latency-bound chain and this gives it twice the warps.  The two warps meet
+// once, in shared memory (barrier 1, 64 threads), for what needs both axes:
+// the next stage's packed positions, filter bound and group box.
+__device__ __forceinline__ void axes_epilogue(const StageParams &P, int i, int ax, double fpa, AxesShared &S) {
+    const int lane = threadIdx.x & 31;
     const CloudDev &c = P.c;
     const bool live = i < c.n;
     const bool fo = P.mode == kModeForceOnly;
@@ -803,25 +834,6 @@ static __global__ void __launch_bounds__(64) stage_finish_axes(const StageParams
         const double *vel = (s == 1) ? (ax ? c.vy : c.vx) : (ax ? c.vyc : c.vxc);
         double *X = ax ? c.y : c.x;
         double *V = ax ? c.vy : c.vx;
-        // the operands' round trip overlaps the partials' (see stage_finish)
-        prefetch_l1(pos + i);
-        prefetch_l1(vel + i);
-        prefetch_l1(c.q + i);
-        prefetch_l1(c.m + i);
-        prefetch_l1(c.orig + i);
-        if (!fo) {
-            prefetch_l1(X + i);
-            prefetch_l1(V + i);
-            if (s >= 3) {
-                prefetch_l1(c.a23[2 * ax] + i);
-                prefetch_l1(c.a23[2 * ax + 1] + i);
-            }
-            if (s == 4) {
-                prefetch_l1(c.a1[2 * ax] + i);
-                prefetch_l1(c.a1[2 * ax + 1] + i);
-            }
-        }
-        const double fpa = finish_rank_sum(P, i, ax);
         const double xs = pos[i], vs = vel[i], q = c.q[i], m = c.m[i];
         const long long fl = P.f.flags;
         double F = 0.0;
@@ -875,179 +887,187 @@ static __global__ void __launch_bounds__(64) stage_finish_axes(const StageParams
     if (fo) return;  // uniform over the launch
     float h = 0.0f, lo = 0.0f;
     if (live) split2(na, h, lo);
-    s_hi[ax][lane] = h;
-    s_lo[ax][lane] = lo;
-    __syncthreads();
+    S.hi[ax][lane] = h;
+    S.lo[ax][lane] = lo;
+    asm volatile("bar.sync 1, 64;" ::: "memory");
     const int bw = b ^ 1;
-    const float xh = s_hi[0][lane], yh = s_hi[1][lane];
+    const float xh = S.hi[0][lane], yh = S.hi[1][lane];
     if (live) {  // write_stage_position's packed words, one float4 per warp
         const double q = c.q[i];
         if (ax == 0)
             c.pa[bw][i] = make_float4(xh, yh, fmaf(yh, yh, xh * xh), __double2float_rn(q));
         else
-            c.pb[bw][i] = make_float4(s_lo[0][lane], s_lo[1][lane], -filter_threshold(xh, yh, c.rc2), 0.0f);
+            c.pb[bw][i] = make_float4(S.lo[0][lane], S.lo[1][lane], -filter_threshold(xh, yh, c.rc2), 0.0f);
     }
-    if (P.box_out && ax == 0) {  // the group's box in the buffer just written
-        float x0 = INFINITY, y0 = INFINITY, x1 = -INFINITY, y1 = -INFINITY;
-        if (live) {
-            x0 = x1 = xh;
-            y0 = y1 = yh;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
-            y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
-            x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-            y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
-        }
-        if (lane == 0 && i < c.n_pad) c.gbox[bw][blockIdx.x] = make_float4(x0, y0, x1, y1);
+    // the group's box in the buffer just written
+    if (P.box_out && ax == 0) store_group_box(c.gbox[bw] + (i >> 5), live, xh, yh, (i & ~31) < c.n_pad);
+}
+
+// Completes a stage after a non-cluster pair launch, for the forces in
+// kBasicForces: one block of two warps per 32-particle group.
+static __global__ void __launch_bounds__(64) stage_finish_axes(const StageParams P) {
+    pdl_wait();
+    __shared__ AxesShared S;
+    const int ax = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31);
+    double fpa = 0.0;
+    if (i < P.c.n) {
+        axes_prefetch(P, i, ax);  // the operands' round trip overlaps the partials'
+        fpa = finish_rank_sum(P, i, ax);
     }
+    axes_epilogue(P, i, ax, fpa, S);
     stage_step_advance(P);
 }
 
 // ---------------------------------------------------------------------------
-// Plain FP64 kernel: same decomposition (G j-groups x NI i-lanes, cluster
-// j split, one uniform branch per j), every operation in FP64.
+// FP64 kernel: one 32-particle group of i per tile, S blocks of NW warps per
+// tile (a cluster); the j groups (CULL: those whose box is within reach of
+// the tile's) are dealt one by one to the S*NW warps, each of which filters
+// its groups in FP32 and evaluates the hits in FP64 with full warps (dm_fp64.cuh).
+// The sums meet in the cluster's first block, which runs the stage epilogue.
+//
+// Bound by the FP64 pipe on dense clouds (26 FP64 instructions per pair in
+// reach, 16 cycles each per 32 pairs), by latency on sparse ones.
 // ---------------------------------------------------------------------------
-struct alignas(32) JD {
-    double x, y, b, q;
+constexpr int kGroupList = 1024;  // j groups tested per pass of the box test
+
+template <int NW>
+struct Group64Smem {
+    HitWarp w[NW];
+    double tab[kExp2Size];
+    double ix[32], iy[32];
+    double2 acc[NW][32];
+    double2 red[32];
+    AxesShared axes;
+    int list[kGroupList];
+    int wcount[NW];
 };
 
-template <int NI, int G, int ILP>
-struct Fp64Smem {
-    static constexpr size_t part = (size_t)G * ILP * NI * sizeof(double2);
-    static constexpr size_t red = (size_t)ILP * NI * sizeof(double2);
-    static size_t bytes(int jt) { return (size_t)jt * sizeof(JD) + part + red; }
-};
-
-template <int NI, int G, int ILP, int JT>
-__global__ void __launch_bounds__(NI * G, 2) pair_stage_fp64(const StageParams P) {
+template <int NW, bool CULL>
+__global__ void __launch_bounds__(NW * 32, 20 / NW) pair_group_fp64(const StageParams P) {
     pdl_wait();
-    constexpr int NT = NI * G;
-    static_assert(NI % 32 == 0 && JT % G == 0, "shape");
+    constexpr int NT = NW * 32;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    JD *s_j = reinterpret_cast<JD *>(smem_raw);
-    double2 *s_part = reinterpret_cast<double2 *>(s_j + JT);  // [G][ILP][NI]
-    double2 *s_red = s_part + G * ILP * NI;                     // [ILP*NI]
-
+    Group64Smem<NW> &sm = *reinterpret_cast<Group64Smem<NW> *>(smem_raw);
     cg::cluster_group cl = cg::this_cluster();
-    const int S = (int)cl.num_blocks();
-    const int rank = (int)cl.block_rank();
+    const int S = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const int tile = blockIdx.x / S;
-    const int tid = threadIdx.x;
-    const int t = tid % NI, g = tid / NI;
-    const int n = P.c.n, n_pad = P.c.n_pad;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n = P.c.n;
+    const int i = tile * 32 + lane;
     const int b = (P.mode == kModeForceOnly) ? P.fo_buf : (P.stage - 1) & 1;
     const double *__restrict__ px = P.c.px[b];
     const double *__restrict__ py = P.c.py[b];
     const double *__restrict__ qa = P.c.q;
-    const double kappa = P.f.shielding;
-    const double C = P.coulomb;
-    const double rc = sqrt(P.rc2);
-
-    double xi[ILP], yi[ILP], qi[ILP], U[ILP], fx[ILP], fy[ILP];
-    int ii[ILP];
-#pragma unroll
-    for (int k = 0; k < ILP; k++) {
-        const int i = tile * NI * ILP + k * NI + t;
-        ii[k] = i;
-        fx[k] = fy[k] = 0.0;
+    const float4 *__restrict__ pa = P.c.pa[b];
+    const Yukawa64 K = P.y64;
+    const bool coul = (P.f.flags & kShieldedCoulomb) != 0;
+    if (rank == 0 && warp < 2 && i < n) axes_prefetch(P, i, warp);
+    double sx = 0.0, sy = 0.0;
+    if (coul) {
+        float px2 = 0.0f, py2 = 0.0f, nu = INFINITY;
         if (i < n) {
-            xi[k] = px[i];
-            yi[k] = py[i];
-            qi[k] = qa[i];
-            const double a2 = __dadd_rn(__dmul_rn(xi[k], xi[k]), __dmul_rn(yi[k], yi[k]));
-            const double pr = sqrt(a2) + rc;
-            U[k] = (P.rc2 - a2) + 5.684341886080802e-14 * pr * pr;
-        } else {
-            xi[k] = yi[k] = qi[k] = 0.0;
-            U[k] = -INFINITY;
-        }
-    }
-
-    const int per = ((n_pad + S - 1) / S + 63) & ~63;
-    const int j0 = rank * per;
-    const int j1 = min(n_pad, j0 + per);
-    constexpr int SUB = JT / G;
-
-    for (int jt = j0; jt < j1; jt += JT) {
-        const int cnt = min(JT, j1 - jt);
-        __syncthreads();
-        for (int e = tid; e < cnt; e += NT) {
-            const double xj = px[jt + e], yj = py[jt + e];
-            JD d;
-            d.x = xj;
-            d.y = yj;
-            d.b = __dadd_rn(__dmul_rn(xj, xj), __dmul_rn(yj, yj));
-            d.q = qa[jt + e];
-            s_j[e] = d;
-        }
-        __syncthreads();
-        const int lo = g * SUB;
-        const int hi = min(cnt, lo + SUB);
-#pragma unroll 2
-        for (int jj = lo; jj < hi; jj++) {
-            const JD d = s_j[jj];
-            double r2e[ILP];
-            bool hit = false;
-#pragma unroll
-            for (int k = 0; k < ILP; k++) {
-                r2e[k] = fma(-2.0 * xi[k], d.x, fma(-2.0 * yi[k], d.y, d.b));
-                hit |= r2e[k] < U[k];
+            const float4 A = pa[i];
+            px2 = 2.0f * A.x;
+            py2 = 2.0f * A.y;
+            nu = P.c.pb[b][i].z;
+            if (warp == 0) {
+                sm.ix[lane] = px[i];
+                sm.iy[lane] = py[i];
             }
-            if (__any_sync(0xffffffffu, hit)) {
-                const int jg = jt + jj;
+        }
+        for (int k = tid; k < kExp2Size; k += NT) sm.tab[k] = g_exp2_table.v[k];
+        __syncthreads();
+        HitWarp &W = sm.w[warp];
+        const double *tab = sm.tab;
+        auto eval = [&](int il, int j) {
+            const double dx = __dsub_rn(sm.ix[il], px[j]), dy = __dsub_rn(sm.iy[il], py[j]);
+            const double w = pair_w64(dx, dy, qa[j], K, tab);
+            return make_double2(__dmul_rn(w, dx), __dmul_rn(w, dy));
+        };
+        int nk = 0, hits = 0;
+        auto group = [&](int g) {
+            const int j = 32 * g + lane;
+            if (j < n) {
+                prefetch_l1(px + j);
+                prefetch_l1(py + j);
+                prefetch_l1(qa + j);
+            }
+            hits += hit_filter(W, nk, g, tile, pa, n, px2, py2, nu);
+            if (++nk == kHitGroups || __reduce_add_sync(0xffffffffu, hits) >= 7 * 32) {
+                __syncwarp();
+                hit_flush(W, nk, sx, sy, eval);
+                nk = hits = 0;
+            }
+        };
+        const int ngroups = (n + 31) >> 5;
+        const int NS = NW * S, me = warp * S + rank;
+        if constexpr (CULL) {
+            const float4 *__restrict__ gb = P.c.gbox[b];
+            const float4 tb = gb[tile];
+            int found = 0;
+            for (int g0 = 0; g0 < ngroups; g0 += kGroupList) {
+                // the groups of this pass within reach, in order
+                int total = 0;
+                for (int t0 = g0; t0 < min(ngroups, g0 + kGroupList); t0 += NT) {
+                    const int g = t0 + tid;
+                    const bool near = g < ngroups && boxes_near(tb, gb[g], P.rc2_hi);
+                    const uint32_t bal = __ballot_sync(0xffffffffu, near);
+                    if (lane == 0) sm.wcount[warp] = __popc(bal);
+                    __syncthreads();
+                    int off = total;
 #pragma unroll
-                for (int k = 0; k < ILP; k++) {
-                    if (r2e[k] < U[k] && jg != ii[k]) {
-                        const double dx = __dsub_rn(xi[k], d.x);
-                        const double dy = __dsub_rn(yi[k], d.y);
-                        double r, a;
-                        if (ref_in_cutoff(dx, dy, kappa, r, a)) {
-                            // C*qq*(1+a)*exp(-a)/((r*r)*r) in the reference's
-                            // block order (ShieldedCoulombForce.cpp:183-184)
-                            const double f = __ddiv_rn(
-                                __dmul_rn(__dmul_rn(__dmul_rn(C, __dmul_rn(qi[k], d.q)),
-                                                    __dadd_rn(1.0, a)),
-                                          exp(-a)),
-                                __dmul_rn(__dmul_rn(r, r), r));
-                            fx[k] = __dadd_rn(fx[k], __dmul_rn(f, dx));
-                            fy[k] = __dadd_rn(fy[k], __dmul_rn(f, dy));
-                        }
+                    for (int w = 0; w < NW; w++) {
+                        off += (w < warp) ? sm.wcount[w] : 0;
+                        total += sm.wcount[w];
                     }
+                    if (near) sm.list[off + __popc(bal & ((1u << lane) - 1u))] = g;
+                    __syncthreads();
                 }
+                for (int e = (me + NS - found % NS) % NS; e < total; e += NS) group(sm.list[e]);
+                found += total;
+                __syncthreads();  // the list is rewritten
             }
+            if (tid == 0 && rank == 0) atomicAdd(P.c.eval_pairs, 1024ull * (unsigned long long)found);
+        } else {
+            for (int g = me; g < ngroups; g += NS) group(g);
         }
+        __syncwarp();
+        hit_flush(W, nk, sx, sy, eval);
     }
-
-#pragma unroll
-    for (int k = 0; k < ILP; k++) s_part[(g * ILP + k) * NI + t] = make_double2(fx[k], fy[k]);
+    sm.acc[warp][lane] = make_double2(sx, sy);
     __syncthreads();
-    for (int e = tid; e < ILP * NI; e += NT) {
-        double sx = 0.0, sy = 0.0;
+    if (warp == 0) {
+        double fx = 0.0, fy = 0.0;
 #pragma unroll
-        for (int gg = 0; gg < G; gg++) {
-            const double2 v = s_part[gg * ILP * NI + e];
-            sx = __dadd_rn(sx, v.x);
-            sy = __dadd_rn(sy, v.y);
+        for (int w = 0; w < NW; w++) {
+            fx = __dadd_rn(fx, sm.acc[w][lane].x);
+            fy = __dadd_rn(fy, sm.acc[w][lane].y);
         }
-        s_red[e] = make_double2(sx, sy);
+        sm.red[lane] = make_double2(fx, fy);
     }
-    cl.sync();
-    for (int e = rank * NT + tid; e < NI * ILP; e += NT * S) {
-        const int i = tile * NI * ILP + e;
-        if (i < n) {
-            double sxx = 0.0, syy = 0.0;
-            for (int r = 0; r < S; r++) {
-                const double2 v = *cl.map_shared_rank(s_red + e, r);
-                sxx = __dadd_rn(sxx, v.x);
-                syy = __dadd_rn(syy, v.y);
+    if (S > 1) cl.sync();
+    else __syncthreads();
+    if (rank == 0 && warp < 2) {
+        double2 f = sm.red[lane];
+        for (int r = 1; r < S; r++) {
+            const double2 v = *cl.map_shared_rank(&sm.red[lane], r);
+            f.x = __dadd_rn(f.x, v.x);
+            f.y = __dadd_rn(f.y, v.y);
+        }
+        const double cq = (i < n) ? __dmul_rn(P.coulomb, qa[i]) : 0.0;
+        if (!(P.f.flags & ~kBasicForces)) {
+            axes_epilogue(P, i, warp, __dmul_rn(cq, warp ? f.y : f.x), sm.axes);
+        } else if (warp == 0) {
+            if (i < n) stage_epilogue(P, i, __dmul_rn(cq, f.x), __dmul_rn(cq, f.y), stage_thermal(P, i));
+            if (P.box_out) {
+                const float4 A = (i < n) ? P.c.pa[b ^ 1][i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                store_group_box(P.c.gbox[b ^ 1] + tile, i < n, A.x, A.y, true);
             }
-            stage_epilogue(P, i, sxx, syy, stage_thermal(P, i));
         }
     }
     stage_step_advance(P);
-    cl.sync();
+    if (S > 1) cl.sync();  // the other blocks' sums stay readable until here
 }
 
 }  // namespace dm
