@@ -43,20 +43,6 @@ struct alignas(16) AdjJ {
     double x, y, q, ax, ay;
 };
 
-// FP32 candidate test, conservative for the FP64 cutoff decision.  With
-// xf = fl32(x) (|xf - x| <= 2^-24 |x|) and dxf = fl32(xf_i - xf_j), the error of
-// dxf is at most 2^-24 (|x_i| + |x_j|) + 2^-24 |dxf| <= e = 2^-22 (A_i + A_t),
-// where A_i = max(|x_i|, |y_i|) and A_t bounds |x_j|, |y_j| over the j tile; the
-// error vector of (dxf, dyf) is shorter than 2e.  So every pair with true
-// r < r_c has fl32(dxf^2 + dyf^2) < (r_c + 2e)^2 (1 + 2^-20) -- the last factor
-// covers the three FP32 roundings of the square sum and of r_c itself.  The
-// exact decision is then the reference's FP64 test (ref_in_cutoff).
-__device__ __forceinline__ float adj_candidate_bound(double rc, float ai, float at) {
-    const float e = 2.384185791015625e-7f * (ai + at);  // 2^-22
-    const float r = __fadd_ru(__double2float_ru(rc), 2.0f * e);
-    return __fmul_ru(__fmul_ru(r, r), 1.0000009536743164f);  // 1 + 2^-20
-}
-
 // Pair sums of one particle: MODE 0 (sx, sy) = sum_j F_kj; MODE 1 the four
 // VJP sums (position x, position y, charge, kappa).
 struct AdjSums {
@@ -229,7 +215,7 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_kernel(
             __syncthreads();
             if (valid)
                 adj_tile_fp64<MODE>(d, sj, sf, cnt, j0, li, xi, yi, qi, axi, ayi, xfi, yfi,
-                                    adj_candidate_bound(rc, ai, __uint_as_float(s_amax)), coulomb, S);
+                                    candidate_bound(rc, ai, __uint_as_float(s_amax)), coulomb, S);
         }
     }
     if (!valid) return;
@@ -497,7 +483,7 @@ __device__ __forceinline__ void adj_pair_sums_fp64(const AdjCloud &d, int li, bo
         __syncthreads();
         if (valid)
             adj_tile_fp64<MODE>(d, sj, sf, cnt, j0, li, xi, yi, qi, axi, ayi, xfi, yfi,
-                                adj_candidate_bound(rc, ai, __uint_as_float(s_amax)), coulomb, S);
+                                candidate_bound(rc, ai, __uint_as_float(s_amax)), coulomb, S);
     }
 #pragma unroll
     for (int k = 0; k < 4; k++) out[k] = S.v[k];

@@ -89,6 +89,7 @@ struct dm_cloud {
     double coulomb = 0.0;
     double *d_fx = nullptr, *d_fy = nullptr;
     double *d_dt = nullptr;
+    double *d_diag = nullptr;    // diagnostics: [kDiagBlocks][5] partial sums, then the 5 results
     unsigned int *d_min = nullptr;
     float *d_dmin = nullptr;
     int order = 4;               // integrator: 4 = Runge_Kutta4, 2 = Runge_Kutta2
@@ -932,6 +933,7 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     const size_t nh = align256((size_t)kSortBuckets * c->sort_blocks * sizeof(uint32_t));
     const size_t ngb = align256((size_t)(c->n_pad / 32) * sizeof(float4));
     const size_t total = nd * (6 + 2 + 8 + 4 + 2 + 6) + nf4 * 4 + ngb * 2 + ni * 6 + nh + 1024 + 512 +
+                         align256(sizeof(double) * 5 * (kDiagBlocks + 1)) +
                          align256(sizeof(double) * kMomentBlocks * kMomentFields);
     cudaError_t e = cudaMalloc(&c->block, total);
     if (e != cudaSuccess) {
@@ -970,6 +972,7 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     c->sort.hist = (uint32_t *)p; p += nh;
     c->sort.box = (double *)p; p += 256;
     c->sort.moments = (double *)p; p += align256(sizeof(double) * kMomentBlocks * kMomentFields);
+    c->d_diag = (double *)p; p += align256(sizeof(double) * 5 * (kDiagBlocks + 1));
     cudaStream_t s = ctx->stream;
     const size_t bytes = (size_t)n * sizeof(double);
     e = cudaMemsetAsync(c->block, 0, total, s);
@@ -1248,21 +1251,16 @@ int dm_cloud_diagnostics(dm_cloud *c, double out[5]) {
     if (!c || !out) return DM_ERR_ARG;
     dm_ctx *ctx = c->ctx;
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
-    const int nt = 128;
-    const int blocks = (c->n + nt - 1) / nt;
-    double *partial = nullptr;
-    DM_CUDA(ctx, cudaMallocAsync((void **)&partial, sizeof(double) * 5 * blocks, ctx->stream));
-    diagnostics_partial<nt><<<blocks, nt, 0, ctx->stream>>>(c->d, c->f, c->coulomb, partial);
-    cudaError_t e = cudaGetLastError();
-    std::vector<double> h((size_t)5 * blocks);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(h.data(), partial, sizeof(double) * 5 * blocks, cudaMemcpyDeviceToHost, ctx->stream);
-    cudaFreeAsync(partial, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) return ctx->fail(DM_ERR_CUDA, "dm_cloud_diagnostics: %s", cudaGetErrorString(e));
-    for (int k = 0; k < 5; k++) out[k] = 0.0;
-    for (int b = 0; b < blocks; b++)
-        for (int k = 0; k < 5; k++) out[k] += h[(size_t)b * 5 + k];
+    const int blocks = diagnostics_blocks(c->n);
+    const double kappa = c->f.shielding, rc = (kappa > 0.0) ? 10.0 / kappa : 0.0;
+    diagnostics_partial<<<blocks, kDiagTile, 0, ctx->stream>>>(c->d, c->f, make_yukawa64(kappa, rc * rc), rc,
+                                                               c->coulomb, c->d_diag);
+    diagnostics_finish<<<1, 160, 0, ctx->stream>>>(c->d_diag, blocks, c->d_diag + 5 * kDiagBlocks);
+    DM_CUDA(ctx, cudaGetLastError());
+    ctx->launches += 2;
+    DM_CUDA(ctx, cudaMemcpyAsync(out, c->d_diag + 5 * kDiagBlocks, 5 * sizeof(double), cudaMemcpyDeviceToHost,
+                                 ctx->stream));
+    DM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return DM_OK;
 }
 

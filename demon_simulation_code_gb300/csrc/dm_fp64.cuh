@@ -249,4 +249,52 @@ __device__ __forceinline__ void hit_flush(HitWarp &W, int ng, double &sx, double
     }
 }
 
+// Calls eval(il, 32 k + jl) for every bit of the warp's masks mask[k][il],
+// k < ng, 32 hits at a time (windows of up to kHitSumPerLane hits of every
+// i); `code` is the warp's scratch.
+constexpr int kHitSumPerLane = 16;
+template <class Eval>
+__device__ __forceinline__ void hit_sum(const uint32_t (*mask)[32], int ng, uint16_t *code, Eval eval) {
+    const int lane = threadIdx.x & 31;
+    int k = 0;
+    uint32_t m = (ng > 0) ? mask[0][lane] : 0u;
+    for (;;) {
+        int left = __popc(m);
+        for (int kk = k + 1; kk < ng && left < kHitSumPerLane; kk++) left += __popc(mask[kk][lane]);
+        const int c = min(left, kHitSumPerLane);
+        int off = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, off, o);
+            if (lane >= o) off += v;
+        }
+        const int total = __shfl_sync(0xffffffffu, off, 31);
+        if (total == 0) break;
+        off -= c;
+        for (int t = 0; t < c; t++) {
+            while (m == 0u) m = mask[++k][lane];
+            const int u = __ffs(m) - 1;
+            m &= m - 1u;
+            code[off + t] = (uint16_t)((lane << 8) | (32 * k + u));
+        }
+        __syncwarp();
+        for (int t = lane; t < total; t += 32) eval(code[t] >> 8, code[t] & 255);
+        __syncwarp();
+    }
+}
+
+// FP32 candidate test, conservative for the FP64 cutoff decision.  With
+// xf = fl32(x) (|xf - x| <= 2^-24 |x|) and dxf = fl32(xf_i - xf_j), the error of
+// dxf is at most 2^-24 (|x_i| + |x_j|) + 2^-24 |dxf| <= e = 2^-22 (A_i + A_t),
+// where A_i = max(|x_i|, |y_i|) and A_t bounds |x_j|, |y_j| over the j tile; the
+// error vector of (dxf, dyf) is shorter than 2e.  So every pair with true
+// r < r_c has fl32(dxf^2 + dyf^2) < (r_c + 2e)^2 (1 + 2^-20) -- the last factor
+// covers the three FP32 roundings of the square sum and of r_c itself.  The
+// exact decision is then the reference's FP64 test (ref_in_cutoff).
+__device__ __forceinline__ float candidate_bound(double rc, float ai, float at) {
+    const float e = 2.384185791015625e-7f * (ai + at);  // 2^-22
+    const float r = __fadd_ru(__double2float_ru(rc), 2.0f * e);
+    return __fmul_ru(__fmul_ru(r, r), 1.0000009536743164f);  // 1 + 2^-20
+}
+
 }  // namespace dm

@@ -3,7 +3,7 @@
 // diagnostics and the peak-throughput probe.
 #pragma once
 
-#include "dm_device.cuh"
+#include "dm_fp64.cuh"
 
 namespace dm {
 
@@ -148,41 +148,141 @@ static __global__ void adaptive_dt(const unsigned int *min_r2_bits, double init_
 // FP64 diagnostics: per-block partial sums of kinetic energy, Yukawa
 // potential (kappa*r < 10, counted once per unordered pair), confinement
 // potential and momentum, written to partial[blockIdx.x*5 + ...] and summed
-// in block order on the host.
+// in block order by diagnostics_finish.
+//
+// The pairs (I, J >= I) of 256-particle tiles are dealt to a grid of at most
+// kDiagBlocks blocks (so the order of every sum depends on n alone).  A warp
+// filters 32 particles of tile I against tile J in FP32, from positions
+// rounded to FP32 with a bound that covers the rounding, and evaluates the
+// hits in FP64 32 at a time (dm_fp64.cuh).  Bound by the filter's issue slots
+// (~7 per 32 pairs) on sparse clouds, by the FP64 pipe on dense ones.
 // ---------------------------------------------------------------------------
-template <int NT>
-__global__ void __launch_bounds__(NT) diagnostics_partial(const CloudDev c, const ForceParams f,
-                                                          double coulomb, double *partial) {
-    __shared__ double red[5][NT];
-    const int i = blockIdx.x * NT + threadIdx.x;
+constexpr int kDiagTile = 256;
+constexpr int kDiagBlocks = 608;
+
+struct DiagSmem {
+    double x[2][kDiagTile], y[2][kDiagTile], q[2][kDiagTile];  // tiles I and J
+    float2 f[kDiagTile];                                        // tile J in FP32
+    double tab[kExp2Size];
+    uint32_t mask[kDiagTile / 32][kDiagTile / 32][32];
+    uint16_t code[kDiagTile / 32][kHitSumPerLane * 32];
+    double red[kDiagTile / 32][5];
+    unsigned int amax;
+};
+
+static __global__ void __launch_bounds__(kDiagTile) diagnostics_partial(const CloudDev c, const ForceParams f,
+                                                                        const Yukawa64 K, double rc, double coulomb,
+                                                                        double *partial) {
+    __shared__ DiagSmem sm;
+    constexpr int NG = kDiagTile / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int k = tid; k < kExp2Size; k += kDiagTile) sm.tab[k] = g_exp2_table.v[k];
     double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    if (i < c.n) {
-        const double x = c.x[i], y = c.y[i], vx = c.vx[i], vy = c.vy[i], q = c.q[i], m = c.m[i];
-        v[0] = 0.5 * m * (vx * vx + vy * vy);
-        v[3] = m * vx;
-        v[4] = m * vy;
-        if (f.flags & kConfinement) v[2] += -0.5 * q * f.confine * (x * x + y * y);
-        if (f.flags & kRectConfinement) v[2] += -0.5 * q * (f.confine_x * x * x + f.confine_y * y * y);
-        if (f.flags & kShieldedCoulomb) {
-            double pe = 0.0;
-            for (int j = 0; j < c.n; j++) {
-                if (j == i) continue;
-                const double dx = x - c.x[j], dy = y - c.y[j];
-                double r, a;
-                if (ref_in_cutoff(dx, dy, f.shielding, r, a)) pe += coulomb * q * c.q[j] * exp(-a) / r;
-            }
-            v[1] = 0.5 * pe;
+    double pe = 0.0;
+    const int nb = (c.n + kDiagTile - 1) / kDiagTile;
+    const long long total = (long long)nb * (nb + 1) / 2;
+    int have = -1, I = 0;
+    long long row = 0;  // first pair index of row I
+    for (long long p = blockIdx.x; p < total; p += gridDim.x) {
+        while (p >= row + nb - I) {
+            row += nb - I;
+            I++;
         }
-    }
-    for (int e = 0; e < 5; e++) red[e][threadIdx.x] = v[e];
-    __syncthreads();
-    for (int s = NT / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s)
-            for (int e = 0; e < 5; e++) red[e][threadIdx.x] += red[e][threadIdx.x + s];
+        const int J = I + (int)(p - row);
+        const int i = I * kDiagTile + tid, j = J * kDiagTile + tid;
+        __syncthreads();  // the previous pair's tiles are done with
+        if (I != have) {
+            have = I;
+            sm.x[0][tid] = (i < c.n) ? c.x[i] : 0.0;
+            sm.y[0][tid] = (i < c.n) ? c.y[i] : 0.0;
+            sm.q[0][tid] = (i < c.n) ? c.q[i] : 0.0;
+        }
+        if (I == J && i < c.n) {  // the tile's one-particle terms
+            const double x = c.x[i], y = c.y[i], vx = c.vx[i], vy = c.vy[i], q = c.q[i], m = c.m[i];
+            v[0] += 0.5 * m * (vx * vx + vy * vy);
+            v[3] += m * vx;
+            v[4] += m * vy;
+            if (f.flags & kConfinement) v[2] += -0.5 * q * f.confine * (x * x + y * y);
+            if (f.flags & kRectConfinement) v[2] += -0.5 * q * (f.confine_x * x * x + f.confine_y * y * y);
+        }
+        if (!(f.flags & kShieldedCoulomb)) continue;
+        float2 fj = make_float2(0.0f, 0.0f);
+        if (j < c.n) {
+            const double x = c.x[j], y = c.y[j];
+            sm.x[1][tid] = x;
+            sm.y[1][tid] = y;
+            sm.q[1][tid] = c.q[j];
+            fj = make_float2(__double2float_rn(x), __double2float_rn(y));
+        }
+        sm.f[tid] = fj;
+        if (tid == 0) sm.amax = 0u;
         __syncthreads();
+        // largest |coordinate| of the tile (NaN has the largest bits: every
+        // pair of the tile is then a candidate)
+        const uint32_t am = __reduce_max_sync(
+            0xffffffffu, max(__float_as_uint(fabsf(fj.x)), __float_as_uint(fabsf(fj.y))));
+        if (lane == 0) atomicMax(&sm.amax, am);
+        __syncthreads();
+        const float xf = __double2float_rn(sm.x[0][tid]), yf = __double2float_rn(sm.y[0][tid]);
+        const float bound =
+            candidate_bound(rc, fmaxf(fabsf(xf), fabsf(yf)), __uint_as_float(sm.amax));
+        const int left = c.n - J * kDiagTile;
+        for (int k = 0; k < NG; k++) {
+            uint32_t m = 0u;
+            if (I < J || k >= warp) {  // tile against itself: groups k >= the warp's
+#pragma unroll 8
+                for (int u = 31; u >= 0; u--) {
+                    const float2 A = sm.f[32 * k + u];
+                    const float dx = xf - A.x, dy = yf - A.y;
+                    m = 2u * m + (fmaf(dx, dx, dy * dy) >= bound ? 0u : 1u);
+                }
+                if (I == J && k == warp) m &= ~((2u << lane) - 1u);  // j > i
+                if (left < 32 * k + 32) m &= (left > 32 * k) ? (1u << (left - 32 * k)) - 1u : 0u;
+                if (i >= c.n) m = 0u;
+            }
+            sm.mask[warp][k][lane] = m;
+        }
+        __syncwarp();
+        hit_sum(sm.mask[warp], NG, sm.code[warp], [&](int il, int jl) {
+            const int a = 32 * warp + il;
+            const double dx = __dsub_rn(sm.x[0][a], sm.x[1][jl]), dy = __dsub_rn(sm.y[0][a], sm.y[1][jl]);
+            const double r2 = fma(dx, dx, __dmul_rn(dy, dy));
+            const Yukawa64At A = yukawa64_odd(r2) ? yukawa64_general(r2, K.kappa) : yukawa64(r2, K, sm.tab);
+            const double e = __dmul_rn(__dmul_rn(sm.q[0][a], sm.q[1][jl]), __dmul_rn(A.ex, A.y));
+            if (in_cutoff64(dx, dy, r2, K)) pe = __dadd_rn(pe, e);
+        });
     }
-    if (threadIdx.x == 0)
-        for (int e = 0; e < 5; e++) partial[blockIdx.x * 5 + e] = red[e][0];
+    v[1] = __dmul_rn(coulomb, pe);
+#pragma unroll
+    for (int e = 0; e < 5; e++) {
+        double t = v[e];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) sm.red[warp][e] = t;
+    }
+    __syncthreads();
+    if (tid < 5) {
+        double t = 0.0;
+        for (int w = 0; w < NG; w++) t += sm.red[w][tid];
+        partial[blockIdx.x * 5 + tid] = t;
+    }
+}
+
+// Sums the per-block partials into out[0..4]: warp e takes quantity e, lanes
+// strided over the blocks, then a butterfly.
+static __global__ void __launch_bounds__(160) diagnostics_finish(const double *partial, int nblocks, double *out) {
+    const int lane = threadIdx.x & 31, e = threadIdx.x >> 5;
+    double t = 0.0;
+    for (int b = lane; b < nblocks; b += 32) t += partial[b * 5 + e];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) out[e] = t;
+}
+
+inline int diagnostics_blocks(int n) {
+    const long long nb = (n + kDiagTile - 1) / kDiagTile;
+    const long long pairs = nb * (nb + 1) / 2;
+    return (int)(pairs < kDiagBlocks ? pairs : kDiagBlocks);
 }
 
 // ---------------------------------------------------------------------------

@@ -28,9 +28,9 @@ using namespace dm;
 
 namespace {
 
-constexpr int kDiagThreads = 128;       // same block size as dm_cloud_diagnostics
-constexpr int kMaxBlocks = 4096;        // => at most 524,288 particles per call
-constexpr int kMaxParticles = kDiagThreads * kMaxBlocks;
+constexpr int kMaxBlocks = 4096;        // rows of the scratch (kDiagBlocks of them are used)
+constexpr int kMaxParticles = 524288;   // the documented limit
+static_assert(kDiagBlocks <= kMaxBlocks, "one scratch row per block");
 
 // The scratch: one row of 5 partial sums per block.
 static __device__ __align__(256) double g_diag_scratch[kMaxBlocks * 5];
@@ -38,23 +38,6 @@ static __device__ __align__(256) double g_diag_scratch[kMaxBlocks * 5];
 // In host code g_diag_scratch names a host-side stand-in, not device memory:
 // the device address is looked up on every call, with the calling device
 // current (see scratch_for_current_device).
-
-// Sums the per-block partials into out[0..4] (one block, strided partial
-// sums then a tree): a fixed order for a given block count.
-__global__ void __launch_bounds__(256) diag_finish(const double *partial, int nblocks, double *out) {
-    __shared__ double red[5][256];
-    double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int b = threadIdx.x; b < nblocks; b += 256)
-        for (int e = 0; e < 5; e++) v[e] += partial[b * 5 + e];
-    for (int e = 0; e < 5; e++) red[e][threadIdx.x] = v[e];
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s)
-            for (int e = 0; e < 5; e++) red[e][threadIdx.x] += red[e][threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x < 5) out[threadIdx.x] = red[threadIdx.x][0];
-}
 
 // The device address of the scratch on the current device.  Looked up on
 // every call rather than cached: the lookup allocates nothing, and a cached
@@ -99,12 +82,14 @@ extern "C" int dm_diagnostics_noalloc(int n, const double *d_x, const double *d_
     c.q = const_cast<double *>(d_q);
     c.m = const_cast<double *>(d_m);
     const double coulomb = 1.0 / (4.0 * M_PI * 8.8541878E-12);
-    const int blocks = (n + kDiagThreads - 1) / kDiagThreads;
+    const double cutoff = (f.shielding > 0.0) ? 10.0 / f.shielding : 0.0;
+    const int blocks = diagnostics_blocks(n);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    diagnostics_partial<kDiagThreads><<<blocks, kDiagThreads, 0, s>>>(c, f, coulomb, scratch);
+    diagnostics_partial<<<blocks, kDiagTile, 0, s>>>(c, f, make_yukawa64(f.shielding, cutoff * cutoff), cutoff, coulomb,
+                                                     scratch);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
-        diag_finish<<<1, 256, 0, s>>>(scratch, blocks, d_out);
+        diagnostics_finish<<<1, 160, 0, s>>>(scratch, blocks, d_out);
         e = cudaGetLastError();
     }
     return e == cudaSuccess ? DM_OK : DM_ERR_CUDA;
