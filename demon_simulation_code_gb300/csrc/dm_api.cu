@@ -1971,9 +1971,14 @@ struct dm_adjoint {
     double coulomb = 0.0;
     // fused RK4 step and adjoint: one block of total-length arrays
     void *work = nullptr;
-    double *k1[4], *k23[4], *pbuf[2][4], *dk[2][4], *mu[3][4], *axd, *ayd;
-    float *axf, *ayf;
+    double *k1[4], *k23[4], *pbuf[2][4], *dk[2][4], *mu[3][4], *ax[2], *ay[2], *invm;
+    AdjSplit split[2];
+    // FP64 kernels: 32-particle groups (cloud, tile), largest clouds first, in
+    // clusters of `csize` blocks
+    int ngroups = 0, csize = 1;
+    int2 *dgroups = nullptr;
     ~dm_adjoint() {
+        if (dgroups) cudaFree(dgroups);
         if (ddesc) cudaFree(ddesc);
         if (dcloud) cudaFree(dcloud);
         if (dtile) cudaFree(dtile);
@@ -1998,20 +2003,64 @@ void adj_fill(dm_adjoint *A, const dm_force_params *params) {
         d.kappa2_f = (float)(d.kappa * d.kappa);
         kappa_log2e(d.kappa, d.kl2e_hi, d.kl2e_lo);
         d.nkl2e = (float)(-d.kappa * 1.4426950408889634);
+        d.y64 = make_yukawa64(d.kappa, d.rc2);
     }
 }
 
+// Launch of an FP64 group kernel over every 32-particle group.
+template <int NS, typename... KArgs, typename... Args>
+cudaError_t adj_launch64(dm_adjoint *A, void (*kernel)(KArgs...), Args &&...args) {
+    constexpr int smem = (int)sizeof(AdjGroupSmem<NS>);
+    cudaError_t e = cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(A->ngroups * A->csize);
+    cfg.blockDim = dim3(32 * kAdjWarps);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = A->ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = A->csize;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+cudaError_t adj_launch_prepare(dm_adjoint *A, const AdjPrepareIO &R) {
+    adj_prepare<<<A->nblocks, kAdjThreads, 0, A->ctx->stream>>>(A->ddesc, A->dcloud, A->dtile, R);
+    A->ctx->launches++;
+    return cudaGetLastError();
+}
+
+// Forces (MODE 0) or their VJP (MODE 1) alone.
 template <int MODE>
-void adj_launch(dm_adjoint *A, int precision, const double *x, const double *y, const double *vx,
-                const double *vy, const double *q, const double *m, const double *ax, const double *ay,
-                double *o0, double *o1, double *o2, double *o3, double *o4, double *o5, double *o6) {
+cudaError_t adj_launch_once(dm_adjoint *A, int precision, const AdjOnce &O) {
+    A->ctx->launches++;
+    if (precision == DM_FP32C) {
+        adjoint_kernel<MODE><<<A->nblocks, kAdjThreads, 0, A->ctx->stream>>>(A->ddesc, A->dcloud, A->dtile, O,
+                                                                             A->coulomb);
+        return cudaGetLastError();
+    }
+    // stream-ordered scratch of its own: such calls may be queued on several
+    // streams at once, and share nothing
+    AdjSplit split{};
+    const size_t n = (size_t)A->total;
     cudaStream_t st = A->ctx->stream;
-    if (precision == DM_FP32C)
-        adjoint_kernel<MODE, true><<<A->nblocks, kAdjThreads, 0, st>>>(
-            A->ddesc, A->dcloud, A->dtile, x, y, vx, vy, q, m, ax, ay, o0, o1, o2, o3, o4, o5, o6, A->coulomb);
-    else
-        adjoint_kernel<MODE, false><<<A->nblocks, kAdjThreads, 0, st>>>(
-            A->ddesc, A->dcloud, A->dtile, x, y, vx, vy, q, m, ax, ay, o0, o1, o2, o3, o4, o5, o6, A->coulomb);
+    cudaError_t e = cudaMallocAsync((void **)&split.p, n * (sizeof(float4) + sizeof(float2)), st);
+    if (e != cudaSuccess) return e;
+    split.l = (float2 *)(split.p + n);
+    AdjPrepareIO R{};
+    R.x = O.x;
+    R.y = O.y;
+    R.out = split;
+    e = adj_launch_prepare(A, R);
+    if (e == cudaSuccess)
+        e = adj_launch64<(MODE == 0 ? 2 : 4)>(A, adj_once_fp64<MODE>, (const AdjCloud *)A->ddesc,
+                                              (const int2 *)A->dgroups, O, split, A->coulomb);
+    const cudaError_t ef = cudaFreeAsync(split.p, st);
+    return e != cudaSuccess ? e : ef;
 }
 }  // namespace
 
@@ -2052,16 +2101,31 @@ int dm_adjoint_create(dm_ctx *ctx, int nclouds, const int *n, const dm_force_par
     A->total = off;
     A->nblocks = (int)bc.size();
     adj_fill(A, params);
+    std::vector<int> order(nclouds);
+    for (int c = 0; c < nclouds; c++) order[c] = c;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return n[a] > n[b]; });
+    std::vector<int2> groups;
+    for (int c : order)
+        for (int t = 0; 32 * t < n[c]; t++) groups.push_back(make_int2(c, t));
+    A->ngroups = (int)groups.size();
+    // enough blocks for four on every SM, each warp at least one j group of
+    // the largest cloud
+    A->csize = std::min({8, (4 * ctx->num_sms + A->ngroups - 1) / A->ngroups,
+                         std::max(1, (n[order[0]] + 32 * kAdjWarps - 1) / (32 * kAdjWarps))});
     cudaError_t e = cudaMalloc((void **)&A->ddesc, nclouds * sizeof(AdjCloud));
     if (e == cudaSuccess) e = cudaMalloc((void **)&A->dcloud, bc.size() * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc((void **)&A->dtile, bt.size() * sizeof(int));
     if (e == cudaSuccess) e = cudaMemcpy(A->ddesc, A->hdesc.data(), nclouds * sizeof(AdjCloud), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(A->dcloud, bc.data(), bc.size() * sizeof(int), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(A->dtile, bt.data(), bt.size() * sizeof(int), cudaMemcpyHostToDevice);
-    // scratch of the fused RK4 step and its adjoint: 38 arrays of total doubles, 2 of floats
+    if (e == cudaSuccess) e = cudaMalloc((void **)&A->dgroups, groups.size() * sizeof(int2));
+    if (e == cudaSuccess)
+        e = cudaMemcpy(A->dgroups, groups.data(), groups.size() * sizeof(int2), cudaMemcpyHostToDevice);
+    // scratch of the fused RK4 step and its adjoint: 41 arrays of total
+    // doubles, 2 of float4 and 4 of float2
     const size_t nd = align256((size_t)A->total * sizeof(double));
-    const size_t nf = align256((size_t)A->total * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&A->work, 38 * nd + 2 * nf);
+    const size_t nf4 = align256((size_t)A->total * sizeof(float4));
+    if (e == cudaSuccess) e = cudaMalloc(&A->work, (41 + 4) * nd + 2 * nf4);
     if (e == cudaSuccess) {
         char *p = (char *)A->work;
         auto take = [&]() { double *r = (double *)p; p += nd; return r; };
@@ -2073,11 +2137,17 @@ int dm_adjoint_create(dm_ctx *ctx, int nclouds, const int *n, const dm_force_par
             for (int c = 0; c < 4; c++) A->dk[b][c] = take();
         for (int b = 0; b < 3; b++)
             for (int c = 0; c < 4; c++) A->mu[b][c] = take();
-        A->axd = take();
-        A->ayd = take();
-        A->axf = (float *)p;
-        p += nf;
-        A->ayf = (float *)p;
+        for (int b = 0; b < 2; b++) {
+            A->ax[b] = take();
+            A->ay[b] = take();
+            A->split[b].l = (float2 *)take();
+            A->split[b].a = (float2 *)take();
+        }
+        A->invm = take();
+        for (int b = 0; b < 2; b++) {
+            A->split[b].p = (float4 *)p;
+            p += nf4;
+        }
     }
     if (e != cudaSuccess) {
         delete A;
@@ -2114,10 +2184,7 @@ int dm_adjoint_forces(dm_adjoint *A, int precision, const double *x, const doubl
     if (precision != DM_FP64 && precision != DM_FP32C)
         return ctx->fail(DM_ERR_ARG, "dm_adjoint_forces: unknown precision %d", precision);
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
-    adj_launch<0>(A, precision, x, y, vx, vy, q, m, nullptr, nullptr, fx, fy, fpx, fpy, nullptr, nullptr,
-                  nullptr);
-    DM_CUDA(ctx, cudaGetLastError());
-    ctx->launches++;
+    DM_CUDA(ctx, adj_launch_once<0>(A, precision, AdjOnce{x, y, vx, vy, q, m, nullptr, nullptr, {fx, fy, fpx, fpy}}));
     return DM_OK;
 }
 
@@ -2135,29 +2202,38 @@ int dm_adjoint_rk4_step(dm_adjoint *A, int precision, double dt, double *x, doub
         for (int c = 0; c < 4; c++)
             DM_CUDA(ctx, cudaMemcpyAsync(stages + c * n, base[c], n * sizeof(double), cudaMemcpyDeviceToDevice,
                                          ctx->stream));
+    AdjPrepareIO R{};
+    R.x = x;
+    R.y = y;
+    R.m = m;
+    R.out = A->split[0];
+    R.invm = A->invm;
+    DM_CUDA(ctx, adj_launch_prepare(A, R));
     for (int st = 1; st <= 4; st++) {
         AdjStepIO io{};
-        double *in[4], *nx[4];
+        double *in[4];
         for (int c = 0; c < 4; c++) {
             in[c] = (st == 1) ? base[c] : stages ? stages + (4 * (st - 1) + c) * n : A->pbuf[st & 1][c];
-            nx[c] = (st == 4) ? nullptr : stages ? stages + (4 * st + c) * n : A->pbuf[(st + 1) & 1][c];
+            io.next[c] = (st == 4) ? nullptr : stages ? stages + (4 * st + c) * n : A->pbuf[(st + 1) & 1][c];
+            io.s[c] = base[c];
             io.k1[c] = A->k1[c];
             io.k23[c] = A->k23[c];
         }
         io.x = in[0]; io.y = in[1]; io.vx = in[2]; io.vy = in[3];
-        io.sx = x; io.sy = y; io.svx = vx; io.svy = vy;
-        io.nx = nx[0]; io.ny = nx[1]; io.nvx = nx[2]; io.nvy = nx[3];
+        io.in = A->split[(st - 1) & 1];
+        io.out = A->split[st & 1];
         io.q = q;
         io.m = m;
+        io.invm = A->invm;
         io.dt = dt;
         io.stage = st;
-        if (precision == DM_FP32C)
-            adj_step_forces<true><<<A->nblocks, kAdjThreads, 0, ctx->stream>>>(A->ddesc, A->dcloud, A->dtile, io,
-                                                                              A->coulomb);
-        else
-            adj_step_forces<false><<<A->nblocks, kAdjThreads, 0, ctx->stream>>>(A->ddesc, A->dcloud, A->dtile, io,
-                                                                               A->coulomb);
-        DM_CUDA(ctx, cudaGetLastError());
+        if (precision == DM_FP32C) {
+            adj_step_fp32c<<<A->nblocks, kAdjThreads, 0, ctx->stream>>>(A->ddesc, A->dcloud, A->dtile, io, A->coulomb);
+            DM_CUDA(ctx, cudaGetLastError());
+        } else {
+            DM_CUDA(ctx, adj_launch64<2>(A, adj_step_fp64, (const AdjCloud *)A->ddesc, (const int2 *)A->dgroups, io,
+                                         A->coulomb));
+        }
         ctx->launches++;
     }
     return DM_OK;
@@ -2174,18 +2250,40 @@ int dm_adjoint_rk4_step_vjp(dm_adjoint *A, int precision, double dt, const doubl
     if (!std::isfinite(dt)) return ctx->fail(DM_ERR_ARG, "dm_adjoint_rk4_step_vjp: dt must be finite");
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
     const size_t n = (size_t)A->total;
+    double *lam[4] = {lx, ly, lvx, lvy};
+    AdjPrepareIO R{};
+    R.x = stages + 12 * n;
+    R.y = stages + 13 * n;
+    R.m = m;
+    R.out = A->split[0];
+    R.invm = A->invm;
+    R.ax = A->ax[0];
+    R.ay = A->ay[0];
+    R.dt = dt;
+    for (int c = 0; c < 4; c++) {
+        R.lam[c] = lam[c];
+        R.dk[c] = A->dk[1][c];
+    }
+    DM_CUDA(ctx, adj_launch_prepare(A, R));
     for (int st = 4; st >= 1; st--) {
         AdjVjpIO V{};
         V.x = stages + (4 * (st - 1) + 0) * n;
         V.y = stages + (4 * (st - 1) + 1) * n;
-        V.vx = stages + (4 * (st - 1) + 2) * n;
-        V.vy = stages + (4 * (st - 1) + 3) * n;
-        // dk_3 in dk[0], dk_2 in dk[1], dk_1 in dk[0]; dk_4 = lam / 6
-        const int rd = (st == 3 || st == 1) ? 0 : 1, wr = (st == 4 || st == 2) ? 0 : 1;
-        double *lam[4] = {lx, ly, lvx, lvy};
+        if (st > 1) {
+            V.xn = stages + (4 * (st - 2) + 0) * n;
+            V.yn = stages + (4 * (st - 2) + 1) * n;
+        }
+        const int rd = (st == 3 || st == 1) ? 1 : 0, wr = rd ^ 1;  // split positions and force adjoints
+        V.in = A->split[rd];
+        V.out = A->split[wr];
+        V.ax = A->ax[rd];
+        V.ay = A->ay[rd];
+        V.axn = A->ax[wr];
+        V.ayn = A->ay[wr];
+        // dk_4 in dk[1], dk_3 in dk[0], dk_2 in dk[1], dk_1 in dk[0]
         for (int c = 0; c < 4; c++) {
-            V.dk[c] = A->dk[rd][c];
-            V.dkn[c] = A->dk[wr][c];
+            V.dk[c] = A->dk[rd ^ 1][c];
+            V.dkn[c] = A->dk[wr ^ 1][c];
             V.lam[c] = lam[c];
             for (int b = 0; b < 3; b++) V.mu[b][c] = A->mu[b][c];
         }
@@ -2194,19 +2292,17 @@ int dm_adjoint_rk4_step_vjp(dm_adjoint *A, int precision, double dt, const doubl
         V.gkc = gkc;
         V.q = q;
         V.m = m;
+        V.invm = A->invm;
         V.dt = dt;
         V.stage = st;
-        adj_force_adjoint<<<(A->total + 255) / 256, 256, 0, ctx->stream>>>(V, A->total, A->axf, A->ayf, A->axd,
-                                                                         A->ayd);
-        DM_CUDA(ctx, cudaGetLastError());
-        if (precision == DM_FP32C)
-            adj_step_vjp<true><<<A->nblocks, kAdjThreads, 0, ctx->stream>>>(A->ddesc, A->dcloud, A->dtile, V, A->axf,
-                                                                           A->ayf, A->axd, A->ayd, A->coulomb);
-        else
-            adj_step_vjp<false><<<A->nblocks, kAdjThreads, 0, ctx->stream>>>(A->ddesc, A->dcloud, A->dtile, V, A->axf,
-                                                                            A->ayf, A->axd, A->ayd, A->coulomb);
-        DM_CUDA(ctx, cudaGetLastError());
-        ctx->launches += 2;
+        if (precision == DM_FP32C) {
+            adj_vjp_fp32c<<<A->nblocks, kAdjThreads, 0, ctx->stream>>>(A->ddesc, A->dcloud, A->dtile, V, A->coulomb);
+            DM_CUDA(ctx, cudaGetLastError());
+        } else {
+            DM_CUDA(ctx, adj_launch64<4>(A, adj_vjp_fp64, (const AdjCloud *)A->ddesc, (const int2 *)A->dgroups, V,
+                                         A->coulomb));
+        }
+        ctx->launches++;
     }
     return DM_OK;
 }
@@ -2221,9 +2317,8 @@ int dm_adjoint_vjp(dm_adjoint *A, int precision, const double *x, const double *
     if (precision != DM_FP64 && precision != DM_FP32C)
         return ctx->fail(DM_ERR_ARG, "dm_adjoint_vjp: unknown precision %d", precision);
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
-    adj_launch<1>(A, precision, x, y, vx, vy, q, m, ax, ay, gx, gy, gvx, gvy, gq, gkappa, gkc);
-    DM_CUDA(ctx, cudaGetLastError());
-    ctx->launches++;
+    DM_CUDA(ctx, adj_launch_once<1>(A, precision,
+                                    AdjOnce{x, y, vx, vy, q, m, ax, ay, {gx, gy, gvx, gvy, gq, gkappa, gkc}}));
     return DM_OK;
 }
 

@@ -933,7 +933,7 @@ constexpr int kGroupList = 1024;  // j groups tested per pass of the box test
 
 template <int NW>
 struct Group64Smem {
-    HitWarp w[NW];
+    HitWarp<2> w[NW];
     double tab[kExp2Size];
     double ix[32], iy[32];
     double2 acc[NW][32];
@@ -963,7 +963,7 @@ __global__ void __launch_bounds__(NW * 32, 20 / NW) pair_group_fp64(const StageP
     const Yukawa64 K = P.y64;
     const bool coul = (P.f.flags & kShieldedCoulomb) != 0;
     if (rank == 0 && warp < 2 && i < n) axes_prefetch(P, i, warp);
-    double sx = 0.0, sy = 0.0;
+    double sum[2] = {0.0, 0.0};
     if (coul) {
         float px2 = 0.0f, py2 = 0.0f, nu = INFINITY;
         if (i < n) {
@@ -978,12 +978,12 @@ __global__ void __launch_bounds__(NW * 32, 20 / NW) pair_group_fp64(const StageP
         }
         for (int k = tid; k < kExp2Size; k += NT) sm.tab[k] = g_exp2_table.v[k];
         __syncthreads();
-        HitWarp &W = sm.w[warp];
+        HitWarp<2> &W = sm.w[warp];
         const double *tab = sm.tab;
         auto eval = [&](int il, int j) {
             const double dx = __dsub_rn(sm.ix[il], px[j]), dy = __dsub_rn(sm.iy[il], py[j]);
             const double w = pair_w64(dx, dy, qa[j], K, tab);
-            return make_double2(__dmul_rn(w, dx), __dmul_rn(w, dy));
+            return HitResult<2>{__dmul_rn(w, dx), __dmul_rn(w, dy)};
         };
         int nk = 0, hits = 0;
         auto group = [&](int g) {
@@ -996,7 +996,7 @@ __global__ void __launch_bounds__(NW * 32, 20 / NW) pair_group_fp64(const StageP
             hits += hit_filter(W, nk, g, tile, pa, n, px2, py2, nu);
             if (++nk == kHitGroups || __reduce_add_sync(0xffffffffu, hits) >= 7 * 32) {
                 __syncwarp();
-                hit_flush(W, nk, sx, sy, eval);
+                hit_flush(W, nk, sum, eval);
                 nk = hits = 0;
             }
         };
@@ -1033,9 +1033,9 @@ __global__ void __launch_bounds__(NW * 32, 20 / NW) pair_group_fp64(const StageP
             for (int g = me; g < ngroups; g += NS) group(g);
         }
         __syncwarp();
-        hit_flush(W, nk, sx, sy, eval);
+        hit_flush(W, nk, sum, eval);
     }
-    sm.acc[warp][lane] = make_double2(sx, sy);
+    sm.acc[warp][lane] = make_double2(sum[0], sum[1]);
     __syncthreads();
     if (warp == 0) {
         double fx = 0.0, fy = 0.0;
