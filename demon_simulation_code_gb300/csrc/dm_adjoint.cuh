@@ -31,6 +31,7 @@ struct AdjCloud {
     double kappa, confine, confine_x, confine_y, gamma;
     double rc2;
     float rc2_lo, rc2_hi;  // FP32 certain-in / certain-out bounds on r^2
+    float rc2_up;          // rc2 rounded up
     float kappa_f, kappa2_f;
     float kl2e_hi, kl2e_lo;  // kappa*log2(e) as a float pair (SFU exponential)
     float nkl2e;             // -kappa*log2(e): e^{-kappa r} = 2^{nkl2e r} (packed pair terms)
@@ -260,13 +261,11 @@ struct AdjVjpIO {
     int stage;
 };
 
-constexpr double kThird = 1.0 / 3.0, kSixth = 1.0 / 6.0;
-
-__device__ __forceinline__ void adj_store_split(const AdjSplit &o, int i, double x, double y, double rc2) {
+__device__ __forceinline__ void adj_store_split(const AdjSplit &o, int i, double x, double y, float rc2_up) {
     float xh, xl, yh, yl;
     split2(x, xh, xl);
     split2(y, yh, yl);
-    o.p[i] = make_float4(xh, yh, fmaf(yh, yh, xh * xh), -filter_threshold(xh, yh, rc2));
+    o.p[i] = make_float4(xh, yh, fmaf(yh, yh, xh * xh), -filter_threshold(xh, yh, rc2_up));
     o.l[i] = make_float2(xl, yl);
 }
 
@@ -289,7 +288,7 @@ static __global__ void __launch_bounds__(kAdjThreads) adj_prepare(const AdjCloud
     const int li = tile_of_block[blockIdx.x] * kAdjThreads + threadIdx.x;
     if (li >= d.n) return;
     const int i = d.off + li;
-    adj_store_split(R.out, i, R.x[i], R.y[i], d.rc2);
+    adj_store_split(R.out, i, R.x[i], R.y[i], d.rc2_up);
     if (!R.invm) return;
     const double m = R.m[i], inv = __drcp_rn(m);
     R.invm[i] = inv;
@@ -593,7 +592,7 @@ static __global__ void __launch_bounds__(kAdjThreads) adj_step_fp32c(const AdjCl
     const double nx = adj_step_component(d, io, i, 0, 0.0), ny = adj_step_component(d, io, i, 1, 0.0);
     adj_step_component(d, io, i, 2, px);
     adj_step_component(d, io, i, 3, py);
-    if (io.stage < 4) adj_store_split(io.out, i, nx, ny, d.rc2);
+    if (io.stage < 4) adj_store_split(io.out, i, nx, ny, d.rc2_up);
 }
 
 // Backward stage, FP32C (one thread per particle).
@@ -624,7 +623,7 @@ static __global__ void __launch_bounds__(kAdjThreads) adj_vjp_fp32c(const AdjClo
         V.axn[i] = ax;
         V.ayn[i] = ay;
         V.out.a[i] = make_float2((float)ax, (float)ay);
-        adj_store_split(V.out, i, V.xn[i], V.yn[i], d.rc2);
+        adj_store_split(V.out, i, V.xn[i], V.yn[i], d.rc2_up);
     }
 }
 
@@ -642,7 +641,7 @@ constexpr int kAdjWarps = 4;
 
 template <int NS>
 struct AdjGroupSmem {
-    HitWarp<NS> w[kAdjWarps];
+    HitWarp<HitResult<NS>> w[kAdjWarps];
     double tab[kExp2Size];
     double ix[32], iy[32], iax[32], iay[32];
     double acc[kAdjWarps][NS][32];
@@ -720,7 +719,7 @@ __device__ __forceinline__ void adj_group_sums(const AdjCloud &d, int tile, cons
         }
         for (int k = tid; k < kExp2Size; k += 32 * kAdjWarps) sm.tab[k] = g_exp2_table.v[k];
         __syncthreads();
-        HitWarp<NS> &W = sm.w[warp];
+        HitWarp<HitResult<NS>> &W = sm.w[warp];
         const double *tab = sm.tab;
         const Yukawa64 K = d.y64;
         auto eval = [&](int il, int j) {
@@ -810,7 +809,7 @@ static __global__ void __launch_bounds__(32 * kAdjWarps) adj_step_fp64(const Adj
             if (warp < 2) sm.xch[warp][lane] = v;
         }
         __syncthreads();
-        if (valid && warp == 0 && io.stage < 4) adj_store_split(io.out, i, sm.xch[0][lane], sm.xch[1][lane], d.rc2);
+        if (valid && warp == 0 && io.stage < 4) adj_store_split(io.out, i, sm.xch[0][lane], sm.xch[1][lane], d.rc2_up);
     }
     if (cl.num_blocks() > 1) cl.sync();  // the other blocks' sums stay readable until here
 }
@@ -832,7 +831,7 @@ static __global__ void __launch_bounds__(32 * kAdjWarps) adj_vjp_fp64(const AdjC
         const double dkn = adj_vjp_component(d, V, i, warp, S);
         if (V.stage > 1) {
             if (warp >= 2) (warp == 2 ? V.axn : V.ayn)[i] = adj_next_force_adjoint(V, i, dkn);
-            else if (warp == 0) adj_store_split(V.out, i, V.xn[i], V.yn[i], d.rc2);
+            else if (warp == 0) adj_store_split(V.out, i, V.xn[i], V.yn[i], d.rc2_up);
         }
     }
     if (cl.num_blocks() > 1) cl.sync();

@@ -73,9 +73,11 @@ struct GraphKey {
     int precision;
     int nsteps;
     double dt;
+    int slot;  // step counter / force time slot current at the first step
     bool operator<(const GraphKey &o) const {
         if (precision != o.precision) return precision < o.precision;
         if (nsteps != o.nsteps) return nsteps < o.nsteps;
+        if (slot != o.slot) return slot < o.slot;
         return dt < o.dt;
     }
 };
@@ -94,11 +96,14 @@ struct dm_cloud {
     float *d_dmin = nullptr;
     int order = 4;               // integrator: 4 = Runge_Kutta4, 2 = Runge_Kutta2
     int eval_thermal_stage = 1;  // substep of the thermal kicks in force-only evaluations
-    int fo_buf = 0;              // stage buffer force-only launches read (the autotuner's dense copy: 1)
-    bool boxes_valid[2] = {false, false};  // group boxes (culling) match stage buffer b
+    bool boxes_valid[4] = {false, false, false, false};  // group boxes (culling) match position set b
+    bool supers_valid[2] = {false, false};  // super group boxes match sets 2 p, 2 p + 1
+    bool mid_valid = false;      // position set 1 is the midpoint for time step mid_dt
+    double mid_dt = 0.0;
+    int slot = 0;                // current step counter / force time slot (RK2 steps alternate it)
     int split[2] = {0, 0};  // cluster size per precision (0 = not chosen yet)
     int tuned_variant[2] = {-1, -1};  // per precision: index into kVariants
-    float2 *partial = nullptr;         // [partial_cap][2][n_pad] non-cluster partial sums (per rank, axis)
+    float2 *partial = nullptr;         // [2 partial_cap][2][n_pad] non-cluster partial sums (per set and rank, axis)
     int partial_cap = 0;
     SortScratch sort{};
     int sort_blocks = 0;
@@ -112,6 +117,12 @@ struct dm_cloud {
     void drop_graphs() {
         for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
         graphs.clear();
+    }
+    // the state (set 0) was rewritten: what was derived from it is stale;
+    // boxes: set 0's group boxes were rewritten with it
+    void state_changed(bool boxes) {
+        boxes_valid[0] = boxes;
+        boxes_valid[1] = mid_valid = supers_valid[0] = false;
     }
     ~dm_cloud() {
         if (partial) cudaFree(partial);
@@ -149,6 +160,19 @@ int check_device_errors(dm_ctx *ctx, dm_cloud *c) {
     return device_error_status(ctx, c, h);
 }
 
+// The autotuners' weights of a candidate's time on the cloud as it is and on
+// its dense copy: a confined cloud passes through its focus in about one step
+// of four to seven.  (With equal weights the dense copy, five times as slow,
+// decided alone: the batch of 256 clouds took a variant 0.7% better in the sum
+// and 29% slower on the clouds at rest.)
+constexpr float kTuneWeight[2] = {3.0f, 1.0f};
+
+// DM_TUNE_VERBOSE: the autotuners' timings of every candidate on stderr.
+bool tune_verbose() {
+    const char *e = getenv("DM_TUNE_VERBOSE");
+    return e && e[0] && e[0] != '0';
+}
+
 // The FP32C sweep's threshold for evaluating a filtered chunk directly
 // (StageParams::direct_min): at least this many of a slot's 128 (lane, j)
 // pairs passed the filter.  DM_DIRECT_MIN_HITS overrides it (1..129; 129
@@ -184,15 +208,21 @@ void kappa_log2e(double kappa, float &hi, float &lo) {
     lo = (float)(k - (double)hi);
 }
 
-StageParams make_stage_params(dm_cloud *c, int stage, int mode, double dt, const double *dt_dev) {
+// The parameters of pass 0 or 1 of a step, or (mode kModeForceOnly) of one
+// force evaluation at position set buf, evaluated nsets times.
+StageParams make_stage_params(dm_cloud *c, int pass, int mode, double dt, const double *dt_dev, int buf = 0,
+                              int nsets = 1) {
     StageParams P{};
     P.c = c->d;
     P.f = c->f;
-    P.stage = stage;
+    P.pass = pass;
     P.order = c->order;
     P.mode = mode;
-    P.therm_stage = (mode == kModeForceOnly) ? c->eval_thermal_stage : stage;
-    P.fo_buf = (mode == kModeForceOnly) ? c->fo_buf : 0;
+    P.nsets = (mode == kModeForceOnly) ? nsets : 2;
+    P.buf[0] = (mode == kModeForceOnly) ? buf : 2 * pass;
+    P.buf[1] = (mode == kModeForceOnly) ? buf : 2 * pass + 1;
+    P.slot = c->slot;
+    P.therm_stage = c->eval_thermal_stage;
     P.dt = dt;
     P.dt_dev = dt_dev;
     P.coulomb = c->coulomb;
@@ -220,11 +250,10 @@ struct Variant {
     int precision;
     bool cluster;  // reduce through a thread-block cluster (else global partials + stage_finish)
     bool cull;     // skip j groups whose box is beyond the cutoff from the tile's (group_bounds first)
-    bool boxes;    // the stage leaves the group boxes of the buffer it writes
-    int nt;        // threads per CTA
+    int nt;        // threads per CTA (cluster variants: and position set)
     int tile;      // particles per i tile
     int min_j;     // j particles per block of a split at least
-    size_t smem;
+    size_t smem;   // cluster variants: for both position sets
     const void *fn;
     cudaError_t (*launch)(const cudaLaunchConfig_t *, const StageParams &);
 };
@@ -239,16 +268,16 @@ cudaError_t launch_fp64(const cudaLaunchConfig_t *cfg, const StageParams &P) {
 }
 
 #define DM_FP32C_VARIANT(NW, ILP, TC, CL)                                                        \
-    {"fp32c<" #NW "," #ILP "," #TC "," #CL ">", DM_FP32C, CL, false, !CL, NW * 32, 32 * ILP, 64 * NW, \
-     Fp32cSmem<NW, ILP, TC>::bytes, (const void *)pair_stage_fp32c<NW, ILP, TC, CL, false>,       \
+    {"fp32c<" #NW "," #ILP "," #TC "," #CL ">", DM_FP32C, CL, false, NW * 32, 32 * ILP, 64 * NW, \
+     (CL ? 2 : 1) * Fp32cSmem<NW, ILP, TC>::bytes, (const void *)pair_stage_fp32c<NW, ILP, TC, CL, false>,       \
      launch_fp32c<NW, ILP, TC, CL, false>}
 #define DM_FP32C_CULL_VARIANT(NW, ILP, TC, CL)                                                   \
-    {"fp32c<" #NW "," #ILP "," #TC "," #CL ",cull>", DM_FP32C, CL, true, !CL, NW * 32, 32 * ILP, 64 * NW, \
-     Fp32cSmem<NW, ILP, TC>::bytes, (const void *)pair_stage_fp32c<NW, ILP, TC, CL, true>,        \
+    {"fp32c<" #NW "," #ILP "," #TC "," #CL ",cull>", DM_FP32C, CL, true, NW * 32, 32 * ILP, 64 * NW, \
+     (CL ? 2 : 1) * Fp32cSmem<NW, ILP, TC>::bytes, (const void *)pair_stage_fp32c<NW, ILP, TC, CL, true>,        \
      launch_fp32c<NW, ILP, TC, CL, true>}
 
 #define DM_FP64_VARIANT(NW, CULL, SUFFIX)                                                        \
-    {"fp64<" #NW SUFFIX ">", DM_FP64, true, CULL, true, NW * 32, 32, 32 * NW, sizeof(Group64Smem<NW>), \
+    {"fp64<" #NW SUFFIX ">", DM_FP64, true, CULL, NW * 32, 32, 32 * NW, sizeof(Group64Smem<NW>), \
      (const void *)pair_group_fp64<NW, CULL>, launch_fp64<NW, CULL>}
 
 const Variant kVariants[] = {
@@ -272,6 +301,8 @@ constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
 constexpr int kDefaultVariant32 = 0;
 constexpr int kDefaultVariant64 = kNumVariants - 1, kDefaultVariant64Cull = kNumVariants - 2;
 constexpr int kMaxSplitGlobal = 64;
+constexpr int kMaxSplitCluster = 16;
+constexpr int kSuperMin = 1024;      // 32-particle groups from which super group boxes are kept
 
 int ensure_kernel_attrs(dm_ctx *ctx) {
     static bool done[64] = {false};
@@ -356,10 +387,10 @@ bool wants_order(int n, int precision) { return precision == DM_FP32C || n > kFp
 
 // attr must hold 2 entries: programmatic serialization (see pdl_wait) and,
 // for cluster variants, the cluster shape.
-cudaLaunchConfig_t make_cfg(dm_ctx *ctx, const Variant &k, int ntiles, int S, cudaLaunchAttribute *attr) {
+cudaLaunchConfig_t make_cfg(dm_ctx *ctx, const Variant &k, int ntiles, int S, int nsets, cudaLaunchAttribute *attr) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ntiles * S, 1, 1);
-    cfg.blockDim = dim3(k.nt, 1, 1);
+    cfg.gridDim = dim3(ntiles * S * (k.cluster ? 1 : nsets), 1, 1);
+    cfg.blockDim = dim3(k.nt * (k.cluster ? nsets : 1), 1, 1);
     cfg.dynamicSmemBytes = k.smem;
     cfg.stream = ctx->stream;
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -384,7 +415,7 @@ cudaLaunchConfig_t make_cfg(dm_ctx *ctx, const Variant &k, int ntiles, int S, cu
 // more co-resident CTAs hide latency better.
 int model_split(dm_ctx *ctx, const Variant &k, int n, int n_pad) {
     const int ntiles = (n + k.tile - 1) / k.tile;
-    const int smax = k.cluster ? 16 : kMaxSplitGlobal;
+    const int smax = k.cluster ? kMaxSplitCluster : kMaxSplitGlobal;
     int best_s = 1;
     double best_cost = 1e300;
     for (int S = 1; S <= smax; S++) {
@@ -392,7 +423,7 @@ int model_split(dm_ctx *ctx, const Variant &k, int n, int n_pad) {
         int slots = 0;
         if (k.cluster) {
             cudaLaunchAttribute attr[2];
-            cudaLaunchConfig_t cfg = make_cfg(ctx, k, ntiles, S, attr);
+            cudaLaunchConfig_t cfg = make_cfg(ctx, k, ntiles, S, 2, attr);
             if (cudaOccupancyMaxActiveClusters(&slots, k.fn, &cfg) != cudaSuccess) {
                 cudaGetLastError();
                 continue;
@@ -403,12 +434,12 @@ int model_split(dm_ctx *ctx, const Variant &k, int n, int n_pad) {
                 cudaGetLastError();
                 continue;
             }
-            slots = per_sm * ctx->num_sms / S;  // co-resident "tiles"
+            slots = per_sm * ctx->num_sms / (2 * S);  // co-resident tiles (both position sets)
         }
         if (slots <= 0) continue;
         double cost = 0.0;
         for (int left = ntiles; left > 0; left -= slots) {
-            const int in_wave = std::min(left, slots) * S;
+            const int in_wave = std::min(left, slots) * S * (k.cluster ? 1 : 2);
             cost += (double)((in_wave + ctx->num_sms - 1) / ctx->num_sms) / S;
         }
         if (cost <= best_cost * 1.02) {
@@ -426,7 +457,7 @@ int ensure_partial(dm_cloud *c, int S) {
     if (c->partial) cudaFree(c->partial);
     c->partial = nullptr;
     c->partial_cap = 0;
-    cudaError_t e = cudaMalloc((void **)&c->partial, (size_t)S * 2 * c->n_pad * sizeof(float2));
+    cudaError_t e = cudaMalloc((void **)&c->partial, (size_t)S * 4 * c->n_pad * sizeof(float2));
     if (e != cudaSuccess)
         return ctx->fail(DM_ERR_NOMEM, "partial-sum buffer (%d x %d): %s", S, c->n_pad, cudaGetErrorString(e));
     c->partial_cap = S;
@@ -434,22 +465,32 @@ int ensure_partial(dm_cloud *c, int S) {
     return DM_OK;
 }
 
-// One stage: the pair kernel (+ stage_finish for non-cluster variants).
-int launch_variant(dm_cloud *c, int vi, int S, int stage, int mode, double dt, const double *dt_dev) {
+// One pass: the pair kernel (+ stage_finish for non-cluster variants), after
+// the group boxes that it needs and lacks.
+int launch_variant(dm_cloud *c, int vi, int S, StageParams P) {
     dm_ctx *ctx = c->ctx;
     const Variant &k = kVariants[vi];
-    StageParams P = make_stage_params(c, stage, mode, dt, dt_dev);
     P.split = S;
     P.partial = c->partial;
-    P.box_out = (k.boxes && mode != kModeForceOnly) ? 1 : 0;
-    const int ntiles = (c->n + k.tile - 1) / k.tile;
+    const int ngroups = (c->n + 31) / 32;
     cudaLaunchAttribute attr[2];
-    cudaLaunchConfig_t cfg = make_cfg(ctx, k, ntiles, S, attr);
-    const int br = (mode == kModeForceOnly) ? c->fo_buf : (stage - 1) & 1;  // buffer read
-    if (k.cull && !c->boxes_valid[br]) {  // boxes of the buffer this stage reads
-        DM_CUDA(ctx, launch_pdl(group_bounds, dim3((c->n_pad + 255) / 256), dim3(256), 0, ctx->stream, c->d, br));
-        ctx->launches++;
-        c->boxes_valid[br] = true;
+    cudaLaunchConfig_t cfg = make_cfg(ctx, k, (c->n + k.tile - 1) / k.tile, S, P.nsets, attr);
+    if (k.cull) {
+        for (int e = 0; e < P.nsets; e++) {
+            const int b = P.buf[e];
+            if (c->boxes_valid[b]) continue;
+            DM_CUDA(ctx, launch_pdl(group_bounds, dim3((c->n_pad + 255) / 256), dim3(256), 0, ctx->stream, c->d, b));
+            ctx->launches++;
+            c->boxes_valid[b] = true;
+            c->supers_valid[b / 2] = false;
+        }
+        if (c->d.gsuper[0] && !c->supers_valid[P.buf[0] / 2]) {
+            const int nsuper = (ngroups + 31) / 32;
+            DM_CUDA(ctx, launch_pdl(super_bounds, dim3((2 * nsuper + 7) / 8), dim3(256), 0, ctx->stream, c->d,
+                                    P.buf[0] & 2, ngroups));
+            ctx->launches++;
+            c->supers_valid[P.buf[0] / 2] = true;
+        }
     }
     // profiling (dm_ctx_profile_enable): CUDA events around the pair launch
     // alone (a cluster variant's launch includes its epilogue)
@@ -471,36 +512,64 @@ int launch_variant(dm_cloud *c, int vi, int S, int stage, int mode, double dt, c
     if (ctx->prof) {
         DM_CUDA(ctx, cudaEventRecord(e1, ctx->stream));
         ctx->prof_launches++;
-        ctx->prof_pairs += (double)c->n * (double)(c->n - 1);
+        ctx->prof_pairs += (double)P.nsets * (double)c->n * (double)(c->n - 1);
     }
     if (!k.cluster) {
-        if (P.f.flags & ~kBasicForces)
-            DM_CUDA(ctx, launch_pdl(stage_finish, dim3((c->n + 63) / 64), dim3(64), 0, ctx->stream, P));
-        else  // one thread per particle and axis, one block per 32-particle group
-            DM_CUDA(ctx, launch_pdl(stage_finish_axes, dim3(2 * ((c->n + 63) / 64)), dim3(64), 0, ctx->stream, P));
+        DM_CUDA(ctx, launch_pdl(stage_finish, dim3(ngroups), dim3(128), 0, ctx->stream, P));
         ctx->launches++;
     }
-    if (mode != kModeForceOnly) c->boxes_valid[stage & 1] = k.boxes;
+    if (P.mode == kModeForceOnly) return DM_OK;
+    // the epilogue leaves two position sets with their boxes
+    const int ob = (P.pass == 0) ? 2 : 0;
+    c->boxes_valid[ob] = c->boxes_valid[ob + 1] = true;
+    c->supers_valid[ob / 2] = false;
+    if (P.order == 2) {
+        DM_CUDA(ctx, launch_pdl(adopt_sets, dim3((c->n + 255) / 256), dim3(256), 0, ctx->stream, c->d, ngroups));
+        ctx->launches++;
+        c->boxes_valid[0] = c->boxes_valid[1] = true;
+        c->supers_valid[0] = false;
+    }
+    if (P.order == 2 || P.pass == 1) {  // the step is done: set 1 is the next step's midpoint for the same dt
+        c->mid_valid = P.dt_dev == nullptr;
+        c->mid_dt = P.dt;
+        if (P.order == 2) c->slot ^= 1;
+    }
     return DM_OK;
 }
 
 int tune_precision(dm_cloud *c, int precision);
-int reorder(dm_cloud *c);
+int reorder(dm_cloud *c, double dt = 0.0, bool mid = false);
 
-// One launch of the fused pair + stage kernel(s) with the cloud's tuned
-// variant and split.
-int launch_stage(dm_cloud *c, int precision, int stage, int mode, double dt, const double *dt_dev) {
-    dm_ctx *ctx = c->ctx;
-    int rc = ensure_kernel_attrs(ctx);
+int ensure_tuned(dm_cloud *c, int precision) {
+    const int rc = ensure_kernel_attrs(c->ctx);
     if (rc) return rc;
+    return (c->tuned_variant[precision == DM_FP32C ? 1 : 0] < 0) ? tune_precision(c, precision) : DM_OK;
+}
+
+// One pass (or force evaluation) with the cloud's tuned variant and split.
+int launch_tuned(dm_cloud *c, int precision, const StageParams &P) {
     const int pi = precision == DM_FP32C ? 1 : 0;
-    if (c->tuned_variant[pi] < 0) {
-        rc = tune_precision(c, precision);
-        if (rc) return rc;
+    return launch_variant(c, c->tuned_variant[pi], c->split[pi], P);
+}
+
+// The passes of one step from set 0 (and set 1, if it is the midpoint for
+// this dt; dt_dev: the adaptive dt, never).
+int launch_step(dm_cloud *c, int precision, double dt, const double *dt_dev) {
+    dm_ctx *ctx = c->ctx;
+    int rc = ensure_tuned(c, precision);  // may use set 1
+    if (rc) return rc;
+    if (dt_dev || !c->mid_valid || c->mid_dt != dt) {
+        DM_CUDA(ctx, launch_pdl(prepare_midpoint, dim3((c->n + 255) / 256), dim3(256), 0, ctx->stream, c->d, dt,
+                                dt_dev));
+        ctx->launches++;
+        c->boxes_valid[1] = true;
+        c->supers_valid[0] = false;
+        c->mid_valid = dt_dev == nullptr;
+        c->mid_dt = dt;
     }
-    const int vi = c->tuned_variant[pi];
-    const int S = c->split[pi];
-    return launch_variant(c, vi, S, stage, mode, dt, dt_dev);
+    for (int pass = 0; pass < c->order / 2 && !rc; pass++)
+        rc = launch_tuned(c, precision, make_stage_params(c, pass, kModeStep, dt, dt_dev));
+    return rc;
 }
 
 // Autotuner: times every variant of this precision over a set of splits on
@@ -537,14 +606,17 @@ int tune_precision(dm_cloud *c, int precision) {
         // and re-expands), and the best shape differs between them.
         const bool big = (double)c->n * c->n > 4e9;  // ~64k particles: keep tuning short
         int nstates = 1;
-        if (!big && !c->order_dirty && c->d.rc2 > 0.0 && std::isfinite(c->d.rc2)) {
+        // FP64: the cloud as it is decides -- dense copies are FP64-pipe bound
+        // whatever the split (within 16% of each other at 16,384 particles,
+        // where the cloud at rest takes 45 to 250 us).
+        if (!big && precision == DM_FP32C && !c->order_dirty && c->d.rc2 > 0.0 && std::isfinite(c->d.rc2)) {
             double v[4];  // bounding box min x, min y, max x, max y
             DM_CUDA(ctx, cudaMemcpyAsync(v, c->sort.box + 4, sizeof v, cudaMemcpyDeviceToHost, ctx->stream));
             DM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             const double half = 0.5 * std::max(v[2] - v[0], v[3] - v[1]);
             const double lam = 1.8 * std::sqrt(c->d.rc2) / half;
             if (std::isfinite(half) && half > 0.0 && lam < 0.9) {
-                c->boxes_valid[1] = false;
+                c->boxes_valid[1] = c->mid_valid = c->supers_valid[0] = false;
                 tune_compress<<<(c->n + 255) / 256, 256, 0, ctx->stream>>>(c->d, 0.5 * (v[0] + v[2]),
                                                                             0.5 * (v[1] + v[3]), lam);
                 DM_CUDA(ctx, cudaGetLastError());
@@ -555,15 +627,22 @@ int tune_precision(dm_cloud *c, int precision) {
         DM_CUDA(ctx, cudaEventCreate(&a));
         DM_CUDA(ctx, cudaEventCreate(&b));
         float best_ms = 1e30f;
-        const char *ev = getenv("DM_TUNE_VERBOSE");  // per-candidate timings on stderr
-        const bool verbose = ev && ev[0] && ev[0] != '0';
-        for (int vi = 0; vi < kNumVariants; vi++) {
+        const bool verbose = tune_verbose();
+        // culling variants first: most of the others are dropped after one
+        // launch (a candidate whose first launch alone costs more than 1.3
+        // times the best total is not timed further)
+        std::vector<int> candidates;
+        for (const bool cull : {true, false})
+            for (int vi = 0; vi < kNumVariants; vi++)
+                if (kVariants[vi].cull == cull) candidates.push_back(vi);
+        for (const int vi : candidates) {
             const Variant &k = kVariants[vi];
             if (k.precision != precision || (precision == DM_FP64 && k.cull != order)) continue;
             const int sm = model_split(ctx, k, c->n, c->n_pad);
             std::vector<int> cands = {sm};
-            const int extra_c[] = {1, 2, 3, 4, 6, 8, 12, 16};
-            const int extra_g[] = {1, 2, 4, 8, 12, 16, 24, 32, 48, 64};
+            if (big && !k.cluster && k.cull) cands = {1, 2, 4};
+            const int extra_c[] = {1, 2, 3, 4, 6, 8, 16};
+            const int extra_g[] = {1, 2, 3, 4, 5, 6, 8, 12, 16, 24, 32};
             if (!big) {
                 if (k.cluster) cands.insert(cands.end(), std::begin(extra_c), std::end(extra_c));
                 else cands.insert(cands.end(), std::begin(extra_g), std::end(extra_g));
@@ -575,7 +654,7 @@ int tune_precision(dm_cloud *c, int precision) {
                 if (k.cluster) {
                     int nc = 0;
                     cudaLaunchAttribute attr[2];
-                    cudaLaunchConfig_t cfg = make_cfg(ctx, k, (c->n + k.tile - 1) / k.tile, S, attr);
+                    cudaLaunchConfig_t cfg = make_cfg(ctx, k, (c->n + k.tile - 1) / k.tile, S, 2, attr);
                     if (cudaOccupancyMaxActiveClusters(&nc, k.fn, &cfg) != cudaSuccess || nc <= 0) {
                         cudaGetLastError();
                         continue;
@@ -586,21 +665,22 @@ int tune_precision(dm_cloud *c, int precision) {
                 }
                 const int reps = big ? 1 : 3;
                 float ms = 0.0f, ms_state[2] = {0.0f, 0.0f};
-                for (int st = 0; st < nstates; st++) {
-                    c->fo_buf = st;
-                    int rc = launch_variant(c, vi, S, 1, kModeForceOnly, 0.0, nullptr);  // warm-up
-                    if (!rc) rc = cudaEventRecord(a, ctx->stream) == cudaSuccess ? DM_OK : DM_ERR_CUDA;
-                    for (int r = 0; r < reps && !rc; r++) rc = launch_variant(c, vi, S, 1, kModeForceOnly, 0.0, nullptr);
-                    if (!rc) rc = cudaEventRecord(b, ctx->stream) == cudaSuccess ? DM_OK : DM_ERR_CUDA;
-                    if (!rc) rc = cudaEventSynchronize(b) == cudaSuccess ? DM_OK : DM_ERR_CUDA;
-                    c->fo_buf = 0;
-                    if (rc) return rc == DM_ERR_CUDA ? ctx->fail(rc, "autotuner timing failed") : rc;
-                    float one = 0.0f;
-                    DM_CUDA(ctx, cudaEventElapsedTime(&one, a, b));
-                    ms += one;
-                    ms_state[st] = one / reps;
+                for (int st = 0; st < nstates && ms < 1.3f * best_ms; st++) {
+                    // both sets on the same buffer: a pass's work
+                    const StageParams P = make_stage_params(c, 0, kModeForceOnly, 0.0, nullptr, st, 2);
+                    for (int runs : {1, reps}) {  // one launch, then the timed ones
+                        int rc = cudaEventRecord(a, ctx->stream) == cudaSuccess ? DM_OK : DM_ERR_CUDA;
+                        for (int r = 0; r < runs && !rc; r++) rc = launch_variant(c, vi, S, P);
+                        if (!rc) rc = cudaEventRecord(b, ctx->stream) == cudaSuccess ? DM_OK : DM_ERR_CUDA;
+                        if (!rc) rc = cudaEventSynchronize(b) == cudaSuccess ? DM_OK : DM_ERR_CUDA;
+                        if (rc) return rc == DM_ERR_CUDA ? ctx->fail(rc, "autotuner timing failed") : rc;
+                        float one = 0.0f;
+                        DM_CUDA(ctx, cudaEventElapsedTime(&one, a, b));
+                        ms_state[st] = one / runs;
+                        if (ms + kTuneWeight[st] * ms_state[st] >= 1.3f * best_ms) break;
+                    }
+                    ms += kTuneWeight[st] * ms_state[st];
                 }
-                ms /= reps;
                 if (verbose)
                     fprintf(stderr, "dm autotune n=%d %s split %d: %.4f ms (state) %.4f ms (dense copy)\n", c->n,
                             k.name, S, ms_state[0], ms_state[1]);
@@ -621,8 +701,9 @@ int tune_precision(dm_cloud *c, int precision) {
     return DM_OK;
 }
 
-// Puts the cloud in Morton order (dm_sort.cuh); graph-capturable.
-int reorder(dm_cloud *c) {
+// Puts the cloud in Morton order (dm_sort.cuh); graph-capturable.  mid: the
+// next step's time step is dt (the small clouds' sort leaves its midpoint too).
+int reorder(dm_cloud *c, double dt, bool mid) {
     dm_ctx *ctx = c->ctx;
     cudaStream_t s = ctx->stream;
     const int n = c->n;
@@ -636,13 +717,14 @@ int reorder(dm_cloud *c) {
         const float4 *pa0 = c->d.pa[0];
         if (ctx->sort_ctas == 16) {
             const cudaLaunchConfig_t cfg = sort_cluster_cfg<16>(s, attr);
-            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<16>, pa0, c->d, z));
+            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<16>, pa0, c->d, z, dt, mid));
         } else {
             const cudaLaunchConfig_t cfg = sort_cluster_cfg<8>(s, attr);
-            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<8>, pa0, c->d, z));
+            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<8>, pa0, c->d, z, dt, mid));
         }
-        c->boxes_valid[0] = true;  // written by sort_cluster
-        c->boxes_valid[1] = false;
+        c->state_changed(true);
+        c->boxes_valid[1] = c->mid_valid = mid;
+        c->mid_dt = dt;
         DM_CUDA(ctx, cudaGetLastError());
         ctx->launches += 1;
         c->order_dirty = false;
@@ -664,25 +746,27 @@ int reorder(dm_cloud *c) {
     permute_gather<<<grid, 256, 0, s>>>(c->d, z.vals[cur], z);
     permute_commit<<<grid, 256, 0, s>>>(c->d, z);
     init_positions<<<(c->n_pad + 255) / 256, 256, 0, s>>>(c->d);
-    c->boxes_valid[0] = c->boxes_valid[1] = false;
+    c->state_changed(false);
     DM_CUDA(ctx, cudaGetLastError());
     ctx->launches += 3;
     c->order_dirty = false;
     return DM_OK;
 }
 
+// The re-sort at the start of a step, where one is due.
+int reorder_if_due(dm_cloud *c, int precision, double dt, bool mid) {
+    if (!wants_order(c->n, precision)) return DM_OK;
+    if (c->order_dirty || (c->reorder_interval > 0 && c->host_steps % (unsigned)c->reorder_interval == 0))
+        return reorder(c, dt, mid);
+    return DM_OK;
+}
+
 int enqueue_steps(dm_cloud *c, int nsteps, double dt, int precision) {
     for (int s = 0; s < nsteps; s++) {
-        if (wants_order(c->n, precision) &&
-            (c->order_dirty ||
-             (c->reorder_interval > 0 && c->host_steps % (unsigned)c->reorder_interval == 0))) {
-            int rc = reorder(c);
-            if (rc) return rc;
-        }
-        for (int st = 1; st <= c->order; st++) {
-            int rc = launch_stage(c, precision, st, kModeStep, dt, nullptr);
-            if (rc) return rc;
-        }
+        int rc = reorder_if_due(c, precision, dt, true);
+        if (rc) return rc;
+        rc = launch_step(c, precision, dt, nullptr);
+        if (rc) return rc;
         c->host_steps++;
     }
     return DM_OK;
@@ -704,14 +788,19 @@ int run_steps(dm_cloud *c, int nsteps, double dt, int precision) {
         nsteps--;
     }
     if (nsteps < kGraphSteps) return enqueue_steps(c, nsteps, dt, precision);
-    const GraphKey key{precision, kGraphSteps, dt};
+    // the captured steps start from a midpoint left by the step before (or by
+    // the re-sort that begins them): make it so, outside the capture
+    int rc0 = ensure_tuned(c, precision);
+    if (rc0) return rc0;
+    const bool sorts = wants_order(c->n, precision) && c->reorder_interval > 0 && c->n <= kSmallSortMax;
+    if (!sorts && !(c->mid_valid && c->mid_dt == dt)) {
+        rc0 = enqueue_steps(c, 1, dt, precision);
+        if (rc0) return rc0;
+        return run_steps(c, nsteps - 1, dt, precision);
+    }
+    const GraphKey key{precision, kGraphSteps, dt, c->slot};
     auto it = c->graphs.find(key);
     if (it == c->graphs.end()) {
-        if (c->tuned_variant[precision == DM_FP32C ? 1 : 0] < 0) {  // not inside the capture
-            int rc = ensure_kernel_attrs(ctx);
-            if (!rc) rc = tune_precision(c, precision);
-            if (rc) return rc;
-        }
         cudaGraph_t g = nullptr;
         const unsigned long long saved = c->host_steps;
         const long long saved_launches = ctx->launches;
@@ -737,6 +826,10 @@ int run_steps(dm_cloud *c, int nsteps, double dt, int precision) {
         DM_CUDA(ctx, cudaGraphLaunch(it->second, ctx->stream));
         c->host_steps += kGraphSteps;
         ctx->launches += c->graph_launches;
+        c->mid_valid = true;  // the replayed steps leave every position set's boxes and the midpoint
+        c->mid_dt = dt;
+        for (bool &v : c->boxes_valid) v = true;
+        c->supers_valid[0] = false;
     }
     return enqueue_steps(c, nsteps - reps * kGraphSteps, dt, precision);
 }
@@ -926,13 +1019,15 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     c->coulomb = 1.0 / (4.0 * M_PI * 8.8541878E-12);
     c->d.coulomb = c->coulomb;
     c->d.rc2 = (10.0 / 2e4) * (10.0 / 2e4);  // default kappa until set_forces
+    c->d.rc2_up = round_up_f32(c->d.rc2);
     const size_t nd = align256((size_t)c->n_pad * sizeof(double));
     const size_t nf4 = align256((size_t)c->n_pad * sizeof(float4));
     const size_t ni = align256((size_t)c->n_pad * sizeof(int));
     c->sort_blocks = (n + kSortPerBlock - 1) / kSortPerBlock;
     const size_t nh = align256((size_t)kSortBuckets * c->sort_blocks * sizeof(uint32_t));
     const size_t ngb = align256((size_t)(c->n_pad / 32) * sizeof(float4));
-    const size_t total = nd * (6 + 2 + 8 + 4 + 2 + 6) + nf4 * 4 + ngb * 2 + ni * 6 + nh + 1024 + 512 +
+    const size_t nsp = align256((size_t)(c->n_pad / 1024 + 1) * sizeof(float4));
+    const size_t total = nd * (6 + 5 + 6 + 2 + 6) + nf4 * 8 + (ngb + nsp) * 4 + ni * 6 + nh + 1024 + 512 +
                          align256(sizeof(double) * 5 * (kDiagBlocks + 1)) +
                          align256(sizeof(double) * kMomentBlocks * kMomentFields);
     cudaError_t e = cudaMalloc(&c->block, total);
@@ -947,14 +1042,19 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     c->d.n_pad = c->n_pad;
     c->d.x = takeD(); c->d.y = takeD(); c->d.vx = takeD(); c->d.vy = takeD();
     c->d.q = takeD(); c->d.m = takeD();
-    c->d.vxc = takeD(); c->d.vyc = takeD();
-    for (int k = 0; k < 4; k++) c->d.a1[k] = takeD();
-    for (int k = 0; k < 4; k++) c->d.a23[k] = takeD();
-    for (int b = 0; b < 2; b++) { c->d.px[b] = takeD(); c->d.py[b] = takeD(); }
+    for (int k = 0; k < 2; k++) { c->d.k1[k] = takeD(); c->d.k2[k] = takeD(); }
+    c->d.invm = takeD();
+    c->d.px[0] = c->d.x;  // position set 0 is the state
+    c->d.py[0] = c->d.y;
+    for (int b = 1; b < 4; b++) { c->d.px[b] = takeD(); c->d.py[b] = takeD(); }
     c->d_fx = takeD();
     c->d_fy = takeD();
-    for (int b = 0; b < 2; b++) { c->d.pa[b] = takeF4(); c->d.pb[b] = takeF4(); }
-    for (int b = 0; b < 2; b++) { c->d.gbox[b] = (float4 *)p; p += ngb; }
+    for (int b = 0; b < 4; b++) { c->d.pa[b] = takeF4(); c->d.pb[b] = takeF4(); }
+    for (int b = 0; b < 4; b++) { c->d.gbox[b] = (float4 *)p; p += ngb; }
+    for (int b = 0; b < 4; b++) {
+        c->d.gsuper[b] = (c->n_pad / 32 >= kSuperMin) ? (float4 *)p : nullptr;
+        p += nsp;
+    }
     c->d.eval_pairs = (unsigned long long *)p; p += 256;
     c->d.step_ctr = (unsigned long long *)p; p += 256;
     c->d.time = (double *)(c->d.step_ctr + 4);  // same 256-byte slot, bytes 32-47
@@ -985,7 +1085,6 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     if (e == cudaSuccess) {
         set_identity<<<(n + 255) / 256, 256, 0, s>>>(c->d.orig, n);
         init_positions<<<(c->n_pad + 255) / 256, 256, 0, s>>>(c->d);
-        c->boxes_valid[0] = c->boxes_valid[1] = false;
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -1025,7 +1124,7 @@ int dm_cloud_upload(dm_cloud *c, const double *x, const double *y, const double 
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
     const size_t bytes = (size_t)c->n * sizeof(double);
     // caller order -> staging -> the cloud's current internal order (charges,
-    // masses and the order stay; stage buffer 0 and its boxes are rewritten)
+    // masses and the order stay; position set 0 and its boxes are rewritten)
     double **st = c->sort.stage;
     const void *dv[4] = {device_view(x), device_view(y), device_view(vx), device_view(vy)};
     if (dv[0] && dv[1] && dv[2] && dv[3]) {
@@ -1041,8 +1140,7 @@ int dm_cloud_upload(dm_cloud *c, const double *x, const double *y, const double 
         DM_CUDA(ctx, cudaMemcpyAsync(st[3], vy, bytes, cudaMemcpyHostToDevice, ctx->stream));
     }
     upload_internal_order<<<(c->n_pad + 255) / 256, 256, 0, ctx->stream>>>(c->d, c->sort);
-    c->boxes_valid[0] = true;
-    c->boxes_valid[1] = false;
+    c->state_changed(true);
     DM_CUDA(ctx, cudaGetLastError());
     ctx->launches += 1;
     c->order_dirty = true;  // the uploaded positions may be far from the old order
@@ -1091,9 +1189,9 @@ int dm_cloud_set_charge_mass(dm_cloud *c, const double *q, const double *m) {
     if (m) DM_CUDA(ctx, cudaMemcpyAsync(st[5], m, bytes, cudaMemcpyHostToDevice, ctx->stream));
     gather_from_caller<<<(c->n + 255) / 256, 256, 0, ctx->stream>>>(
         c->d.orig, c->n, q ? st[4] : nullptr, m ? st[5] : nullptr, c->d.q, c->d.m);
-    // the float charge copy lives in the stage buffers: refresh buffer 0
+    // the float charge copy lives in the position sets: refresh set 0
     init_positions<<<(c->n_pad + 255) / 256, 256, 0, ctx->stream>>>(c->d);
-    c->boxes_valid[0] = c->boxes_valid[1] = false;
+    c->state_changed(false);
     DM_CUDA(ctx, cudaGetLastError());
     return DM_OK;
 }
@@ -1108,11 +1206,12 @@ int dm_cloud_set_forces(dm_cloud *c, const dm_force_params *p) {
         return ctx->fail(st, "dm_cloud_set_forces: %s (flags 0x%llx)", why, (unsigned long long)p->flags);
     c->f = fp;
     c->d.rc2 = (p->shielding > 0.0) ? (10.0 / p->shielding) * (10.0 / p->shielding) : 0.0;
+    c->d.rc2_up = round_up_f32(c->d.rc2);
     c->drop_graphs();
-    // the stage buffers carry a per-particle filter bound that depends on kappa
+    // the position sets carry a per-particle filter bound that depends on kappa
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
     init_positions<<<(c->n_pad + 255) / 256, 256, 0, ctx->stream>>>(c->d);
-    c->boxes_valid[0] = c->boxes_valid[1] = false;
+    c->state_changed(false);
     DM_CUDA(ctx, cudaGetLastError());
     return DM_OK;
 }
@@ -1127,7 +1226,8 @@ int dm_cloud_eval_forces_device(dm_cloud *c, int precision, double *d_fx, double
         const int rc = reorder(c);
         if (rc) return rc;
     }
-    int rc = launch_stage(c, precision, 1, kModeForceOnly, 0.0, nullptr);
+    int rc = ensure_tuned(c, precision);
+    if (!rc) rc = launch_tuned(c, precision, make_stage_params(c, 0, kModeForceOnly, 0.0, nullptr));
     if (rc) return rc;
     const size_t bytes = (size_t)c->n * sizeof(double);
     if (d_fx && d_fx != c->d_fx) DM_CUDA(ctx, cudaMemcpyAsync(d_fx, c->d_fx, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
@@ -1232,12 +1332,12 @@ int dm_cloud_move_particles(dm_cloud *c, double end_time, double dt, int precisi
     } else {
         while (t < end_time) {
             double step_dt = 0.0;
-            int rc = dm_cloud_modify_timestep(c, dt, nullptr, &step_dt);
+            int rc = reorder_if_due(c, precision, 0.0, false);
+            if (!rc) rc = dm_cloud_modify_timestep(c, dt, nullptr, &step_dt);
             if (rc) return rc;
-            for (int st = 1; st <= c->order; st++) {
-                rc = launch_stage(c, precision, st, kModeStep, 0.0, c->d_dt);
-                if (rc) return rc;
-            }
+            rc = launch_step(c, precision, 0.0, c->d_dt);
+            if (rc) return rc;
+            c->host_steps++;
             t += step_dt;
             count++;
         }
@@ -1276,13 +1376,9 @@ int dm_cloud_autotune(dm_cloud *c, int precision, char *variant, size_t len, int
     dm_ctx *ctx = c->ctx;
     if (precision != DM_FP64 && precision != DM_FP32C) return ctx->fail(DM_ERR_ARG, "bad precision %d", precision);
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
-    int rc = ensure_kernel_attrs(ctx);
+    const int rc = ensure_tuned(c, precision);
     if (rc) return rc;
     const int pi = precision == DM_FP32C ? 1 : 0;
-    if (c->tuned_variant[pi] < 0) {
-        rc = tune_precision(c, precision);
-        if (rc) return rc;
-    }
     if (variant && len) snprintf(variant, len, "%s", kVariants[c->tuned_variant[pi]].name);
     if (split) *split = c->split[pi];
     return DM_OK;
@@ -1308,7 +1404,7 @@ int dm_cloud_set_kernel(dm_cloud *c, const char *variant, int split) {
         if (std::strcmp(kVariants[v].name, variant) == 0) vi = v;
     if (vi < 0) return ctx->fail(DM_ERR_ARG, "unknown kernel variant '%s'", variant);
     const Variant &k = kVariants[vi];
-    const int smax = k.cluster ? 16 : kMaxSplitGlobal;
+    const int smax = k.cluster ? kMaxSplitCluster : kMaxSplitGlobal;
     if (split < 0 || split > smax) return ctx->fail(DM_ERR_ARG, "split %d outside [0, %d]", split, smax);
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
     int rc = ensure_kernel_attrs(ctx);
@@ -1317,7 +1413,7 @@ int dm_cloud_set_kernel(dm_cloud *c, const char *variant, int split) {
     if (k.cluster) {
         int nc = 0;
         cudaLaunchAttribute attr[2];
-        cudaLaunchConfig_t cfg = make_cfg(ctx, k, (c->n + k.tile - 1) / k.tile, split, attr);
+        cudaLaunchConfig_t cfg = make_cfg(ctx, k, (c->n + k.tile - 1) / k.tile, split, 2, attr);
         if (cudaOccupancyMaxActiveClusters(&nc, k.fn, &cfg) != cudaSuccess || nc <= 0) {
             cudaGetLastError();
             return ctx->fail(DM_ERR_UNSUPPORTED, "cluster of %d CTAs of %s cannot be scheduled", split, k.name);
@@ -1374,7 +1470,7 @@ int dm_cloud_get_time(dm_cloud *c, double *t) {
     dm_ctx *ctx = c->ctx;
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
     double v = 0.0;
-    DM_CUDA(ctx, cudaMemcpyAsync(&v, c->d.time, sizeof(v), cudaMemcpyDeviceToHost, ctx->stream));
+    DM_CUDA(ctx, cudaMemcpyAsync(&v, c->d.time + c->slot, sizeof(v), cudaMemcpyDeviceToHost, ctx->stream));
     DM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     *t = v;
     return DM_OK;
@@ -1385,7 +1481,7 @@ int dm_cloud_get_step_counter(dm_cloud *c, uint64_t *step) {
     dm_ctx *ctx = c->ctx;
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
     unsigned long long v = 0;
-    DM_CUDA(ctx, cudaMemcpyAsync(&v, c->d.step_ctr, sizeof(v), cudaMemcpyDeviceToHost, ctx->stream));
+    DM_CUDA(ctx, cudaMemcpyAsync(&v, c->d.step_ctr + c->slot, sizeof(v), cudaMemcpyDeviceToHost, ctx->stream));
     DM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     *step = v;
     return DM_OK;
@@ -1405,14 +1501,13 @@ struct BatchVariant {
     int nt, tile;
     size_t smem;
     const void *fn;
-    cudaError_t (*launch)(dim3, dim3, size_t, cudaStream_t, const StageParams &, const BatchCloud *,
-                          const int2 *, int, unsigned int *);
+    cudaError_t (*launch)(const cudaLaunchConfig_t *, const StageParams &, const BatchCloud *, const int2 *);
 };
 
 template <int NW, int ILP, int TC, bool CULL>
-cudaError_t launch_batch(dim3 g, dim3 b, size_t smem, cudaStream_t s, const StageParams &P,
-                         const BatchCloud *desc, const int2 *items, int nitems, unsigned int *ctr) {
-    return launch_pdl(batch_stage_fp32c<NW, ILP, TC, CULL>, g, b, smem, s, P, desc, items, nitems, ctr);
+cudaError_t launch_batch(const cudaLaunchConfig_t *cfg, const StageParams &P, const BatchCloud *desc,
+                         const int2 *items) {
+    return cudaLaunchKernelEx(cfg, batch_stage_fp32c<NW, ILP, TC, CULL>, P, desc, items);
 }
 
 #define DM_BATCH_VARIANT(NW, ILP, TC, CULL, SUFFIX)                                                \
@@ -1442,15 +1537,14 @@ struct dm_batch {
     std::vector<int> hn;
     BatchCloud *ddesc = nullptr;
     int *dseg = nullptr;
-    unsigned int *dcounter = nullptr;  // [4] work-item counters, one per stage
     int2 *ditems[kNumBatchVariants] = {nullptr};
     int nitems[kNumBatchVariants] = {0};
-    int grid[kNumBatchVariants] = {0};
     double *dbox = nullptr;  // [nclouds][8] key box and bounding box (batch_boxes)
     SortScratch sort{};
     int sort_blocks = 0;
     int mbits = 24;
     double *d_fx = nullptr, *d_fy = nullptr;
+    float2 *partial = nullptr;  // [2 sets][2 axes][total_pad] pair sums of a pass
     int ngroups = 0;            // 32-particle groups over all clouds
     int *dgseg = nullptr;       // [ngroups] cloud of each group
     int variant = -1;
@@ -1458,6 +1552,10 @@ struct dm_batch {
     int max_n = 0;             // largest cloud
     int order = 4;  // integrator: 4 = Runge_Kutta4, 2 = Runge_Kutta2
     bool order_dirty = true;
+    bool boxes_valid[4] = {false, false, false, false};  // as dm_cloud's
+    bool mid_valid = false;
+    double mid_dt = 0.0;
+    int slot = 0;
     unsigned long long host_steps = 0;
     std::map<GraphKey, cudaGraphExec_t> graphs;
     cudaStream_t graph_stream = nullptr;
@@ -1476,50 +1574,85 @@ struct dm_batch {
 
 namespace {
 
-int batch_launch_stage(dm_batch *B, int stage, int mode, double dt, int fo_buf = 0) {
+// One pass of every cloud; mode kModeForceOnly: the forces at position set
+// buf, evaluated nsets times.
+int batch_launch_pass(dm_batch *B, int pass, int mode, double dt, int buf = 0, int nsets = 1) {
     dm_ctx *ctx = B->ctx;
     const BatchVariant &k = kBatchVariants[B->variant];
     StageParams P{};
     P.c = B->d;
-    P.stage = stage;
+    P.pass = pass;
     P.order = B->order;
     P.mode = mode;
-    P.therm_stage = (mode == kModeForceOnly) ? 1 : stage;
-    P.fo_buf = (mode == kModeForceOnly) ? fo_buf : 0;
+    P.nsets = (mode == kModeForceOnly) ? nsets : 2;
+    P.buf[0] = (mode == kModeForceOnly) ? buf : 2 * pass;
+    P.buf[1] = (mode == kModeForceOnly) ? buf : 2 * pass + 1;
+    P.slot = B->slot;
+    P.therm_stage = 1;
     P.dt = dt;
     P.coulomb = B->d.coulomb;
     P.fx_out = B->d_fx;
     P.fy_out = B->d_fy;
     P.direct_min = direct_min_hits();
     P.near_direct_f2 = near_direct_f2();
-    const int slot = (mode == kModeForceOnly) ? 0 : stage - 1;
-    if (k.cull) {  // group boxes of the buffer this stage reads
-        const int br = (mode == kModeForceOnly) ? fo_buf : (stage - 1) & 1;
-        DM_CUDA(ctx, launch_pdl(batch_group_bounds, dim3((B->ngroups * 32 + 255) / 256), dim3(256), 0, ctx->stream,
-                                B->d, (const BatchCloud *)B->ddesc, (const int *)B->dgseg, B->ngroups, br));
+    if (k.cull)
+        for (int e = 0; e < P.nsets; e++) {
+            const int b = P.buf[e];
+            if (B->boxes_valid[b]) continue;
+            DM_CUDA(ctx, launch_pdl(batch_group_bounds, dim3((B->ngroups * 32 + 255) / 256), dim3(256), 0, ctx->stream,
+                                    B->d, (const BatchCloud *)B->ddesc, (const int *)B->dgseg, B->ngroups, b));
+            ctx->launches++;
+            B->boxes_valid[b] = true;
+        }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(B->nitems[B->variant] * P.nsets);
+    cfg.blockDim = dim3(k.nt);
+    cfg.dynamicSmemBytes = k.smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    P.split = 1;
+    P.partial = B->partial;
+    DM_CUDA(ctx, k.launch(&cfg, P, B->ddesc, B->ditems[B->variant]));
+    DM_CUDA(ctx, launch_pdl(batch_finish, dim3(B->ngroups), dim3(64), 0, ctx->stream, P, (const BatchCloud *)B->ddesc,
+                            (const int *)B->dgseg));
+    ctx->launches += 2;
+    if (mode == kModeForceOnly) return DM_OK;
+    const int ob = (pass == 0) ? 2 : 0;
+    B->boxes_valid[ob] = B->boxes_valid[ob + 1] = true;
+    if (P.order == 2) {
+        DM_CUDA(ctx, launch_pdl(adopt_sets, dim3((B->total + 255) / 256), dim3(256), 0, ctx->stream, B->d,
+                                B->ngroups));
         ctx->launches++;
+        B->boxes_valid[0] = B->boxes_valid[1] = true;
     }
-    DM_CUDA(ctx, k.launch(dim3(B->grid[B->variant]), dim3(k.nt), k.smem, ctx->stream, P, B->ddesc,
-                          B->ditems[B->variant], B->nitems[B->variant], B->dcounter + slot));
-    ctx->launches++;
+    if (P.order == 2 || pass == 1) {
+        B->mid_valid = true;
+        B->mid_dt = dt;
+        if (P.order == 2) B->slot ^= 1;
+    }
     return DM_OK;
 }
 
-int batch_reorder(dm_batch *B) {
+// Puts every cloud in Morton order; mid: as reorder's.
+int batch_reorder(dm_batch *B, double dt = 0.0, bool mid = false) {
     dm_ctx *ctx = B->ctx;
     cudaStream_t s = ctx->stream;
     const int n = B->total;
     const int grid = (n + 255) / 256;
     SortScratch &z = B->sort;
-    if (B->max_n <= kBatchSortMax) {  // one block per cloud sorts and gathers; two more commit
+    if (B->max_n <= kBatchSortMax) {  // one block per cloud sorts it in place
         DM_CUDA(ctx, cudaFuncSetAttribute(batch_sort_clouds, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)kBatchSortSmem));
         DM_CUDA(ctx, launch_pdl(batch_sort_clouds, dim3(B->nclouds), dim3(kBatchSortThreads), kBatchSortSmem, s,
-                                B->d, (const BatchCloud *)B->ddesc, B->dbox, z));
-        DM_CUDA(ctx, launch_pdl(permute_commit, dim3(grid), dim3(256), 0, s, B->d, z));
-        DM_CUDA(ctx, launch_pdl(batch_init_positions, dim3((B->total_pad + 255) / 256), dim3(256), 0, s, B->d,
-                                (const BatchCloud *)B->ddesc, (const int *)B->dseg));
-        ctx->launches += 3;
+                                B->d, (const BatchCloud *)B->ddesc, B->dbox, dt, mid));
+        ctx->launches++;
+        B->boxes_valid[0] = true;
+        B->boxes_valid[1] = B->mid_valid = mid;
+        B->mid_dt = dt;
         B->order_dirty = false;
         return DM_OK;
     }
@@ -1541,6 +1674,7 @@ int batch_reorder(dm_batch *B) {
     batch_init_positions<<<(B->total_pad + 255) / 256, 256, 0, s>>>(B->d, B->ddesc, B->dseg);
     DM_CUDA(ctx, cudaGetLastError());
     ctx->launches += 5 + 3 * passes;
+    B->boxes_valid[0] = B->boxes_valid[1] = B->mid_valid = false;
     B->order_dirty = false;
     return DM_OK;
 }
@@ -1549,12 +1683,19 @@ int batch_enqueue_steps(dm_batch *B, int nsteps, double dt) {
     dm_ctx *ctx = B->ctx;
     for (int s = 0; s < nsteps; s++) {
         if (B->order_dirty || (B->reorder_interval > 0 && B->host_steps % (unsigned)B->reorder_interval == 0)) {
-            int rc = batch_reorder(B);
+            int rc = batch_reorder(B, dt, true);
             if (rc) return rc;
         }
-        DM_CUDA(ctx, cudaMemsetAsync(B->dcounter, 0, 4 * sizeof(unsigned int), ctx->stream));
-        for (int st = 1; st <= B->order; st++) {
-            int rc = batch_launch_stage(B, st, kModeStep, dt);
+        if (!B->mid_valid || B->mid_dt != dt) {
+            DM_CUDA(ctx, launch_pdl(batch_midpoint, dim3((B->total + 255) / 256), dim3(256), 0, ctx->stream, B->d,
+                                    (const BatchCloud *)B->ddesc, (const int *)B->dseg, dt));
+            ctx->launches++;
+            B->boxes_valid[1] = false;
+            B->mid_valid = true;
+            B->mid_dt = dt;
+        }
+        for (int pass = 0; pass < B->order / 2; pass++) {
+            int rc = batch_launch_pass(B, pass, kModeStep, dt);
             if (rc) return rc;
         }
         B->host_steps++;
@@ -1568,9 +1709,6 @@ int batch_tune(dm_batch *B) {
     for (int v = 0; v < kNumBatchVariants; v++) {
         const BatchVariant &k = kBatchVariants[v];
         DM_CUDA(ctx, cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem));
-        int per_sm = 0;
-        DM_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, k.nt, k.smem));
-        B->grid[v] = std::max(1, per_sm) * ctx->num_sms;
         // work items (cloud, tile), largest clouds first
         std::vector<int2> items;
         std::vector<int> order(B->nclouds);
@@ -1595,23 +1733,25 @@ int batch_tune(dm_batch *B) {
         // two states, as for one cloud: the batch as it is (buffer 0) and
         // every cloud squeezed to ~30% in-cutoff pairs (buffer 1)
         batch_tune_compress<<<(B->total + 255) / 256, 256, 0, ctx->stream>>>(B->d, B->ddesc, B->dseg, B->dbox);
+        B->boxes_valid[1] = B->mid_valid = false;
         DM_CUDA(ctx, cudaGetLastError());
         cudaEvent_t a, b;
         DM_CUDA(ctx, cudaEventCreate(&a));
         DM_CUDA(ctx, cudaEventCreate(&b));
         float best_ms = 1e30f;
-        for (int v = 0; v < kNumBatchVariants; v++) {
+        std::vector<int> candidates;  // culling variants first (see tune_precision)
+        for (const bool cull : {true, false})
+            for (int v = 0; v < kNumBatchVariants; v++)
+                if (kBatchVariants[v].cull == cull) candidates.push_back(v);
+        for (const int v : candidates) {
             B->variant = v;
-            float total = 0.0f;
-            for (int st = 0; st < 2; st++) {
-                DM_CUDA(ctx, cudaMemsetAsync(B->dcounter, 0, sizeof(unsigned int), ctx->stream));
-                rc = batch_launch_stage(B, 1, kModeForceOnly, 0.0, st);  // warm-up
-                if (rc) return rc;
+            float total = 0.0f, ms_state[2] = {0.0f, 0.0f};
+            for (int st = 0; st < 2 && total < 1.3f * best_ms; st++) {
                 float one = 1e30f;
                 for (int r = 0; r < 3; r++) {  // best of three
-                    DM_CUDA(ctx, cudaMemsetAsync(B->dcounter, 0, sizeof(unsigned int), ctx->stream));
+                    if (total + kTuneWeight[st] * std::min(one, 1e6f) * (r > 0) >= 1.3f * best_ms) break;
                     DM_CUDA(ctx, cudaEventRecord(a, ctx->stream));
-                    rc = batch_launch_stage(B, 1, kModeForceOnly, 0.0, st);
+                    rc = batch_launch_pass(B, 0, kModeForceOnly, 0.0, st, 2);
                     if (rc) return rc;
                     DM_CUDA(ctx, cudaEventRecord(b, ctx->stream));
                     DM_CUDA(ctx, cudaEventSynchronize(b));
@@ -1619,8 +1759,12 @@ int batch_tune(dm_batch *B) {
                     DM_CUDA(ctx, cudaEventElapsedTime(&ms, a, b));
                     one = std::min(one, ms);
                 }
-                total += one;
+                total += kTuneWeight[st] * one;
+                ms_state[st] = one;
             }
+            if (tune_verbose())
+                fprintf(stderr, "dm autotune batch %s: %.4f ms (state) %.4f ms (dense copy)\n", kBatchVariants[v].name,
+                        ms_state[0], ms_state[1]);
             if (total < best_ms) {
                 best_ms = total;
                 best = v;
@@ -1677,7 +1821,7 @@ int dm_batch_create(dm_ctx *ctx, int nclouds, const int *n, const double *x, con
     const size_t nh = align256((size_t)kSortBuckets * B->sort_blocks * sizeof(uint32_t));
     const size_t ndesc = align256((size_t)nclouds * sizeof(BatchCloud));
     const size_t nbb = align256((size_t)nclouds * 8 * sizeof(double));
-    const size_t bytes_total = nd * (6 + 2 + 8 + 4 + 2 + 6) + nf4 * 4 + ni * 7 + nh + ndesc + nbb + 1024;
+    const size_t bytes_total = nd * (6 + 5 + 6 + 2 + 6) + nf4 * 8 + ni * 7 + nh + ndesc + nbb + 1024;
     cudaError_t e = cudaMalloc(&B->block, bytes_total);
     if (e != cudaSuccess) {
         delete B;
@@ -1692,14 +1836,15 @@ int dm_batch_create(dm_ctx *ctx, int nclouds, const int *n, const double *x, con
     d.n_pad = np;
     d.coulomb = coulomb;
     d.x = takeD(); d.y = takeD(); d.vx = takeD(); d.vy = takeD(); d.q = takeD(); d.m = takeD();
-    d.vxc = takeD(); d.vyc = takeD();
-    for (int k = 0; k < 4; k++) d.a1[k] = takeD();
-    for (int k = 0; k < 4; k++) d.a23[k] = takeD();
-    for (int b = 0; b < 2; b++) { d.px[b] = takeD(); d.py[b] = takeD(); }
+    for (int k = 0; k < 2; k++) { d.k1[k] = takeD(); d.k2[k] = takeD(); }
+    d.invm = takeD();
+    d.px[0] = d.x;  // position set 0 is the state
+    d.py[0] = d.y;
+    for (int b = 1; b < 4; b++) { d.px[b] = takeD(); d.py[b] = takeD(); }
     B->d_fx = takeD();
     B->d_fy = takeD();
     for (int k = 0; k < 6; k++) B->sort.stage[k] = takeD();
-    for (int b = 0; b < 2; b++) { d.pa[b] = takeF4(); d.pb[b] = takeF4(); }
+    for (int b = 0; b < 4; b++) { d.pa[b] = takeF4(); d.pb[b] = takeF4(); }
     d.orig = takeI();
     B->dseg = takeI();
     B->sort.keys[0] = (uint32_t *)takeI();
@@ -1713,7 +1858,6 @@ int dm_batch_create(dm_ctx *ctx, int nclouds, const int *n, const double *x, con
     d.step_ctr = (unsigned long long *)p; p += 256;
     d.time = (double *)(d.step_ctr + 4);  // same 256-byte slot, bytes 32-47
     d.err = (int *)p; p += 256;
-    B->dcounter = (unsigned int *)p; p += 256;
     // host descriptors
     B->hdesc.resize(nclouds);
     std::vector<int> seg((size_t)B->total), orig((size_t)B->total), gseg;
@@ -1728,6 +1872,7 @@ int dm_batch_create(dm_ctx *ctx, int nclouds, const int *n, const double *x, con
         std::memcpy(&bc.f, &params[c], sizeof(ForceParams));
         const double kappa = params[c].shielding;
         bc.rc2 = (kappa > 0.0) ? (10.0 / kappa) * (10.0 / kappa) : 0.0;
+        bc.rc2_up = round_up_f32(bc.rc2);
         bc.rc2_lo = (float)(bc.rc2 * (1.0 - 4e-6));
         bc.rc2_hi = (float)(bc.rc2 * (1.0 + 4e-6));
         bc.kappa_f = (float)kappa;
@@ -1740,10 +1885,12 @@ int dm_batch_create(dm_ctx *ctx, int nclouds, const int *n, const double *x, con
     }
     cudaStream_t s = ctx->stream;
     // group boxes (culling kernels), the group -> cloud map, the swept-pair counter
-    for (int b = 0; b < 2 && e == cudaSuccess; b++) {
+    for (int b = 0; b < 4 && e == cudaSuccess; b++) {
         e = cudaMalloc((void **)&d.gbox[b], (size_t)B->ngroups * sizeof(float4));
         if (e == cudaSuccess) B->extra.push_back(d.gbox[b]);
     }
+    if (e == cudaSuccess) e = cudaMalloc((void **)&B->partial, (size_t)4 * np * sizeof(float2));
+    if (e == cudaSuccess) B->extra.push_back(B->partial);
     if (e == cudaSuccess) e = cudaMalloc((void **)&B->dgseg, gseg.size() * sizeof(int));
     if (e == cudaSuccess) B->extra.push_back(B->dgseg);
     if (e == cudaSuccess) e = cudaMalloc((void **)&d.eval_pairs, sizeof(unsigned long long));
@@ -1807,7 +1954,12 @@ int dm_batch_step(dm_batch *B, int nsteps, double dt, int precision) {
         nsteps--;
     }
     if (nsteps < kGraphSteps) return batch_enqueue_steps(B, nsteps, dt);
-    const GraphKey key{DM_FP32C, kGraphSteps, dt};
+    const bool sorts = B->reorder_interval > 0 && B->max_n <= kBatchSortMax;
+    if (!sorts && !(B->mid_valid && B->mid_dt == dt)) {  // the captured steps start from a midpoint (see run_steps)
+        int rc = batch_enqueue_steps(B, 1, dt);
+        return rc ? rc : dm_batch_step(B, nsteps - 1, dt, precision);
+    }
+    const GraphKey key{DM_FP32C, kGraphSteps, dt, B->slot};
     auto it = B->graphs.find(key);
     static long long graph_launches_cache = 0;
     if (it == B->graphs.end()) {
@@ -1836,6 +1988,9 @@ int dm_batch_step(dm_batch *B, int nsteps, double dt, int precision) {
         DM_CUDA(ctx, cudaGraphLaunch(it->second, ctx->stream));
         B->host_steps += kGraphSteps;
         ctx->launches += graph_launches_cache;
+        B->mid_valid = true;
+        B->mid_dt = dt;
+        for (bool &v : B->boxes_valid) v = true;
     }
     return batch_enqueue_steps(B, nsteps - reps * kGraphSteps, dt);
 }
@@ -1846,8 +2001,7 @@ int dm_batch_eval_forces(dm_batch *B, int precision, double *fx, double *fy) {
     if (precision != DM_FP32C)
         return ctx->fail(DM_ERR_UNSUPPORTED, "batched clouds run the FP32C kernel");
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
-    DM_CUDA(ctx, cudaMemsetAsync(B->dcounter, 0, sizeof(unsigned int), ctx->stream));
-    int rc = batch_launch_stage(B, 1, kModeForceOnly, 0.0);
+    int rc = batch_launch_pass(B, 0, kModeForceOnly, 0.0);
     if (rc) return rc;
     const size_t bt = (size_t)B->total * sizeof(double);
     DM_CUDA(ctx, cudaMemcpyAsync(fx, B->d_fx, bt, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1916,7 +2070,7 @@ int dm_batch_info(dm_batch *B, char *variant, size_t len, int *nitems, int *grid
     if (!B) return DM_ERR_ARG;
     if (variant && len) snprintf(variant, len, "%s", kBatchVariants[B->variant].name);
     if (nitems) *nitems = B->nitems[B->variant];
-    if (grid) *grid = B->grid[B->variant];
+    if (grid) *grid = 2 * B->nitems[B->variant];  // a block per position set
     return DM_OK;
 }
 
@@ -1942,7 +2096,7 @@ int dm_batch_get_time(dm_batch *B, double *t) {
     dm_ctx *ctx = B->ctx;
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
     double v = 0.0;
-    DM_CUDA(ctx, cudaMemcpyAsync(&v, B->d.time, sizeof(v), cudaMemcpyDeviceToHost, ctx->stream));
+    DM_CUDA(ctx, cudaMemcpyAsync(&v, B->d.time + B->slot, sizeof(v), cudaMemcpyDeviceToHost, ctx->stream));
     DM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     *t = v;
     return DM_OK;
@@ -1997,6 +2151,7 @@ void adj_fill(dm_adjoint *A, const dm_force_params *params) {
         d.confine_y = params[c].confine_y;
         d.gamma = params[c].gamma;
         d.rc2 = (d.kappa > 0.0) ? (10.0 / d.kappa) * (10.0 / d.kappa) : 0.0;
+        d.rc2_up = round_up_f32(d.rc2);
         d.rc2_lo = (float)(d.rc2 * (1.0 - 4e-6));
         d.rc2_hi = (float)(d.rc2 * (1.0 + 4e-6));
         d.kappa_f = (float)d.kappa;

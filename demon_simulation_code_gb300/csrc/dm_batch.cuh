@@ -3,13 +3,17 @@
 // The clouds are concatenated (caller order: cloud 0's particles, then cloud
 // 1's, ...) into one set of device arrays with no per-cloud padding; each
 // cloud keeps its own force parameters (kappa, charge, confinement, ...).
-// A stage is ONE persistent launch: every CTA repeatedly takes the next work
-// item -- (cloud, i-tile) -- from a global counter and runs the same FP32C
-// sweep as the single-cloud kernel over that cloud's j, then the stage
-// epilogue for the tile's particles.  Items are ordered by cost (largest
-// clouds first), so the dynamic hand-out is a longest-processing-time
-// schedule; since an item is computed entirely by one CTA, the result does
-// not depend on which CTA takes it (deterministic, no atomics on forces).
+// The pair forces of a pass (two RK stages, see dm_device.cuh) are ONE launch:
+// a work item is a (cloud, i-tile, position set), taken by one block that runs
+// the same FP32C sweep as the single-cloud kernel over that cloud's j and
+// leaves the tile's sums in global memory; batch_finish then runs the epilogue
+// of every 32-particle group.  (In one launch, the blocks' epilogues -- chains
+// of FP64 operations on two of a block's warps -- kept the registers and
+// shared memory of the sweep occupied while they ran.)  Items are ordered by
+// cost (largest clouds first) and blocks start in that order as SMs free up, a
+// longest-processing-time schedule; an item is computed entirely by one
+// block, so the result does not depend on where it runs (deterministic, no
+// atomics on forces).
 #pragma once
 
 #include "dm_pair.cuh"
@@ -23,70 +27,87 @@ struct BatchCloud {
     int goff;       // first of the cloud's 32-particle groups in the batch's group boxes
     ForceParams f;
     double rc2;
-    float rc2_lo, rc2_hi, kappa_f;
+    float rc2_lo, rc2_hi, rc2_up, kappa_f;
     float nkl2e;    // -kappa*log2(e)
 };
 
-// A StageParams view of one cloud: pointers offset to the cloud's particles.
-__device__ __forceinline__ void batch_view(StageParams &V, const StageParams &P0, const BatchCloud &d) {
-    V = P0;
-    const int o = d.off;
-    CloudDev &c = V.c;
-    c.x += o; c.y += o; c.vx += o; c.vy += o; c.q += o; c.m += o;
-    c.vxc += o; c.vyc += o;
-    for (int k = 0; k < 4; k++) { c.a1[k] += o; c.a23[k] += o; }
-    for (int b = 0; b < 2; b++) {
-        c.px[b] += o; c.py[b] += o; c.pa[b] += o; c.pb[b] += o;
-        c.gbox[b] += d.goff;  // group boxes numbered within the cloud
+// The StageParams of one cloud in shared memory: a copy of the batch's with
+// pointers offset to the cloud's particles.  Every thread of the block.
+__device__ __forceinline__ void batch_view(StageParams &V, const StageParams &P0, const BatchCloud *desc) {
+    static_assert(sizeof(StageParams) % 4 == 0, "copied by words");
+    for (int k = threadIdx.x; k < (int)(sizeof(StageParams) / 4); k += blockDim.x)
+        reinterpret_cast<uint32_t *>(&V)[k] = reinterpret_cast<const uint32_t *>(&P0)[k];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int o = desc->off, n = desc->n, goff = desc->goff;
+        CloudDev &c = V.c;
+        c.x += o; c.y += o; c.vx += o; c.vy += o; c.q += o; c.m += o;
+        for (int k = 0; k < 2; k++) { c.k1[k] += o; c.k2[k] += o; }
+        c.invm += o;
+        for (int b = 0; b < 4; b++) {
+            c.px[b] += o; c.py[b] += o; c.pa[b] += o; c.pb[b] += o;
+            c.gbox[b] += goff;  // group boxes numbered within the cloud
+        }
+        c.orig += o;  // values stay global caller indices (thermal counter, outputs)
+        c.n = n;
+        c.n_pad = n;
+        c.rc2 = desc->rc2;
+        c.rc2_up = desc->rc2_up;
+        V.rc2 = desc->rc2;
+        V.rc2_lo = desc->rc2_lo;
+        V.rc2_hi = desc->rc2_hi;
+        V.kappa_f = desc->kappa_f;
+        V.nkl2e = desc->nkl2e;
     }
-    c.orig += o;  // values stay global caller indices (thermal counter, outputs)
-    c.n = d.n;
-    c.n_pad = d.n;
-    c.rc2 = d.rc2;
-    V.f = d.f;
-    V.rc2 = d.rc2;
-    V.rc2_lo = d.rc2_lo;
-    V.rc2_hi = d.rc2_hi;
-    V.kappa_f = d.kappa_f;
-    V.nkl2e = d.nkl2e;
+    for (int k = threadIdx.x; k < (int)(sizeof(ForceParams) / 4); k += blockDim.x)
+        reinterpret_cast<uint32_t *>(&V.f)[k] = reinterpret_cast<const uint32_t *>(&desc->f)[k];
+    __syncthreads();
 }
 
 template <int NW, int ILP, int TC, bool CULL = false>
-__global__ void __launch_bounds__(NW * 32, (24 / NW > 0 ? 24 / NW : 1))
-    batch_stage_fp32c(const StageParams P0, const BatchCloud *__restrict__ desc,
-                      const int2 *__restrict__ items, int nitems, unsigned int *counter) {
+__global__ void __launch_bounds__(NW * 32, fp32c_min_blocks<NW, ILP>())
+    batch_stage_fp32c(const StageParams P0, const BatchCloud *__restrict__ desc, const int2 *__restrict__ items) {
     constexpr int TILE = 32 * ILP;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ StageParams sV;
-    __shared__ int s_item;
-    float4 *s_red = reinterpret_cast<float4 *>(smem_raw) + Fp32cSmem<NW, ILP, TC>::red_offset;
-    const int tid = threadIdx.x;
+    const float4 *s_red = reinterpret_cast<const float4 *>(smem_raw) + Fp32cSmem<NW, ILP, TC>::red_offset;
     pdl_wait();
-    for (;;) {
-        if (tid == 0) s_item = (int)atomicAdd(counter, 1u);
-        __syncthreads();
-        const int it = s_item;
-        if (it >= nitems) break;
-        const int2 w = items[it];
-        if (tid == 0) batch_view(sV, P0, desc[w.x]);
-        __syncthreads();
-        const int tile = w.y;
-        fp32c_sweep<NW, ILP, TC, CULL>(sV, tile, 0, 1, smem_raw);
-        if (tid < TILE) {
-            const int i = tile * TILE + tid;
-            if (i < sV.c.n) {
-                const float4 v = s_red[tid];
-                const double cq = pair_scale(sV, i);
-                stage_epilogue(sV, i, __dmul_rn(cq, (double)v.x - (double)v.z),
-                               __dmul_rn(cq, (double)v.y - (double)v.w), stage_thermal(sV, i));
-            }
-        }
-        __syncthreads();  // before the next item reuses shared memory
+    const int set = blockIdx.x % P0.nsets;
+    const int2 w = items[blockIdx.x / P0.nsets];
+    batch_view(sV, P0, desc + w.x);
+    fp32c_sweep<NW, ILP, TC, CULL>(sV, sV.buf[set], w.y, 0, 1, threadIdx.x, [] { __syncthreads(); }, smem_raw);
+    const int first = (int)(sV.c.x - P0.c.x) + w.y * TILE, n = min(TILE, sV.c.n - w.y * TILE);
+    for (int e = threadIdx.x; e < n; e += NW * 32) {
+        const float4 v = s_red[e];
+        P0.partial[(size_t)(2 * set) * P0.c.n_pad + first + e] = make_float2(v.x, v.z);
+        P0.partial[(size_t)(2 * set + 1) * P0.c.n_pad + first + e] = make_float2(v.y, v.w);
     }
-    stage_step_advance(P0);
 }
 
-// Box of every cloud's 32-particle groups in stage buffer b (one warp per
+// The pass's epilogue for every 32-particle group of every cloud (group w is
+// of cloud gseg[w]): one block of two warps each.
+static __global__ void __launch_bounds__(64) batch_finish(const StageParams P, const BatchCloud *__restrict__ desc,
+                                                          const int *__restrict__ gseg) {
+    __shared__ EpilogueShared S;
+    pdl_wait();
+    const int lane = threadIdx.x & 31, ax = threadIdx.x >> 5;
+    const BatchCloud &d = desc[gseg[blockIdx.x]];
+    const int li = 32 * ((int)blockIdx.x - d.goff) + lane, i = d.off + li;
+    const bool live = li < d.n;
+    const bool both = (d.f.flags & ~kBasicForces) != 0;  // else a warp needs its own axis only
+    double2 f[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+    if (live) {
+        epilogue_prefetch(P, i, ax);
+        for (int e = 0; e < P.nsets; e++) {
+            if (both || ax == 0) f[e].x = finish_rank_sum(P, i, e, 0);
+            if (both || ax == 1) f[e].y = finish_rank_sum(P, i, e, 1);
+        }
+    }
+    pass_epilogue(P, EpilogueCloud{d.f, d.rc2_up, live, (int)blockIdx.x}, i, ax, kBarEpilogue, f[0], f[1], S);
+    pass_step_advance(P);
+}
+
+// Box of every cloud's 32-particle groups in position set b (one warp per
 // group; gseg[w] is group w's cloud; a cloud's last group may be partial).
 static __global__ void batch_group_bounds(CloudDev c, const BatchCloud *__restrict__ desc,
                                           const int *__restrict__ gseg, int ngroups, int b) {
@@ -94,22 +115,22 @@ static __global__ void batch_group_bounds(CloudDev c, const BatchCloud *__restri
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= ngroups) return;  // whole warp
-    const BatchCloud d = desc[gseg[w]];
+    const BatchCloud &d = desc[gseg[w]];
     const int li = 32 * (w - d.goff) + lane;
-    float x0 = INFINITY, y0 = INFINITY, x1 = -INFINITY, y1 = -INFINITY;
-    if (li < d.n) {
-        const float4 A = c.pa[b][d.off + li];
-        x0 = x1 = A.x;
-        y0 = y1 = A.y;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
-        y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
-        x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-        y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
-    }
-    if (lane == 0) c.gbox[b][w] = make_float4(x0, y0, x1, y1);
+    const float4 A = (li < d.n) ? c.pa[b][d.off + li] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    store_group_box(c.gbox[b] + w, li < d.n, A.x, A.y, true);
+}
+
+// Position set 1 (the step's midpoint) of every cloud, when the step before
+// did not leave it for this dt.
+static __global__ void batch_midpoint(CloudDev c, const BatchCloud *__restrict__ desc, const int *__restrict__ seg,
+                                      double dt) {
+    pdl_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= c.n) return;
+    CloudDev v = c;
+    v.rc2_up = desc[seg[i]].rc2_up;
+    write_midpoint(v, i, c.x[i], c.y[i], c.vx[i], c.vy[i], dt);
 }
 
 // --- per-cloud Morton order ------------------------------------------------
@@ -151,14 +172,16 @@ static __global__ void batch_keys(const double *__restrict__ x, const double *__
 // ---------------------------------------------------------------------------
 // Per-cloud sort for batches whose clouds all hold at most kBatchSortMax
 // particles: block b sorts cloud b on its own -- key box, 24-bit Morton keys,
-// three stable 8-bit LSD passes in shared memory -- and gathers the cloud's
-// state in the new order into the staging arrays (permute_commit copies it
-// back).  One launch replaces the batch-wide path (per-cloud boxes, keys with
-// the cloud index in the high bits, four radix passes over every particle of
-// every cloud, gather: fifteen dependent launches).  As in sort_cluster the
-// key box and keys are FP32 functions of the positions' hi parts (stage
-// buffer 0), lanes with equal digits are found by match_digit8, and the
-// element order (warp, round, lane) makes every pass stable.
+// three stable 8-bit LSD passes in shared memory -- gathers the cloud's state
+// in the new order into registers and, after a block barrier (the block holds
+// the whole cloud), rewrites the cloud's arrays in place with position sets 0
+// and 1 and their group boxes.  One launch replaces the batch-wide path
+// (per-cloud boxes, keys with the cloud index in the high bits, four radix
+// passes over every particle of every cloud, gather: fifteen dependent
+// launches).  As in sort_cluster the key box and keys are FP32 functions of
+// the positions' hi parts (set 0), lanes with equal digits are found by
+// match_digit8, and the element order (warp, round, lane) makes every pass
+// stable.
 // ---------------------------------------------------------------------------
 constexpr int kBatchSortMax = 4096;
 constexpr int kBatchSortThreads = 1024;
@@ -179,7 +202,7 @@ constexpr size_t kBatchSortSmem = sizeof(BatchSortSmem);
 // box_out[8 * cloud]: key box x0, y0, extent, 0, bounding box min x, min y,
 // max x, max y (as batch_boxes writes them; the batch autotuner reads it).
 static __global__ void __launch_bounds__(kBatchSortThreads, 1)
-    batch_sort_clouds(CloudDev c, const BatchCloud *__restrict__ desc, double *box_out, SortScratch z) {
+    batch_sort_clouds(CloudDev c, const BatchCloud *__restrict__ desc, double *box_out, double dt, bool mid) {
     pdl_wait();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     BatchSortSmem &S = *reinterpret_cast<BatchSortSmem *>(smem_raw);
@@ -327,31 +350,45 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
         }
         src[k] = off + o;
     }
-    const double *__restrict__ in[6] = {c.x, c.y, c.vx, c.vy, c.q, c.m};
+    const double *in[6] = {c.x, c.y, c.vx, c.vy, c.q, c.m};
     double val[6][kBatchSortRounds];
     int ov[kBatchSortRounds];
 #pragma unroll
     for (int k = 0; k < kBatchSortRounds; k++) {
         const bool ok = k * kBatchSortThreads + tid < n;
 #pragma unroll
-        for (int a = 0; a < 6; a++) val[a][k] = ok ? __ldg(in[a] + src[k]) : 0.0;
-        ov[k] = ok ? __ldg(c.orig + src[k]) : 0;
+        for (int a = 0; a < 6; a++) val[a][k] = ok ? in[a][src[k]] : 0.0;
+        ov[k] = ok ? c.orig[src[k]] : 0;
     }
+    __syncthreads();  // every source is in registers: the cloud is rewritten in place
+    CloudDev v = c;
+    v.rc2_up = d.rc2_up;
 #pragma unroll
     for (int k = 0; k < kBatchSortRounds; k++) {
-        const int li = k * kBatchSortThreads + tid;
+        const int li = k * kBatchSortThreads + tid, s = off + li;  // a warp holds 32 consecutive slots
+        float2 h[2] = {};
         if (li < n) {
-#pragma unroll
-            for (int a = 0; a < 6; a++) z.stage[a][off + li] = val[a][k];
-            z.orig_stage[off + li] = ov[k];
+            c.vx[s] = val[2][k];
+            c.vy[s] = val[3][k];
+            c.q[s] = val[4][k];
+            c.m[s] = val[5][k];
+            c.orig[s] = ov[k];
+            write_stage_position(v, 0, s, val[0][k], val[1][k]);  // set 0 is the state: x, y
+            h[0] = make_float2(__double2float_rn(val[0][k]), __double2float_rn(val[1][k]));
+            if (mid) {
+                write_midpoint(v, s, val[0][k], val[1][k], val[2][k], val[3][k], dt);
+                const float4 A = c.pa[1][s];
+                h[1] = make_float2(A.x, A.y);
+            }
         }
+        store_group_box(c.gbox[0] + d.goff + (li >> 5), li < n, h[0].x, h[0].y, (li & ~31) < n);
+        if (mid) store_group_box(c.gbox[1] + d.goff + (li >> 5), li < n, h[1].x, h[1].y, (li & ~31) < n);
     }
 }
 
 // For the batch autotuner: every cloud squeezed about its own box centre
 // so that ~30% of its pairs are inside its cutoff (clouds already that dense
-// are copied as they are), written as stage buffer 1 (nothing live there
-// between steps).
+// are copied as they are), written as position set 1.
 static __global__ void batch_tune_compress(CloudDev c, const BatchCloud *__restrict__ desc,
                                            const int *__restrict__ seg, const double *__restrict__ box) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -364,27 +401,22 @@ static __global__ void batch_tune_compress(CloudDev c, const BatchCloud *__restr
     if (!(isfinite(lam) && lam > 0.0 && lam < 1.0)) lam = 1.0;
     const double cx = 0.5 * (x0 + x1), cy = 0.5 * (y0 + y1);
     CloudDev v = c;
-    v.rc2 = desc[sg].rc2;
+    v.rc2_up = desc[sg].rc2_up;
     write_stage_position(v, 1, i, cx + lam * (c.x[i] - cx), cy + lam * (c.y[i] - cy));
 }
 
-// Stage buffer 0 from the base positions, with each particle's own cloud's
-// filter bound.
+// Position set 0 from the state, with each particle's own cloud's filter
+// bound, and the padding.
 static __global__ void batch_init_positions(CloudDev c, const BatchCloud *__restrict__ desc,
                                             const int *__restrict__ seg) {
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < c.n) {
         CloudDev v = c;
-        v.rc2 = desc[seg[i]].rc2;
+        v.rc2_up = desc[seg[i]].rc2_up;
         write_stage_position(v, 0, i, c.x[i], c.y[i]);
     } else if (i < c.n_pad) {
-        for (int b = 0; b < 2; b++) {
-            c.px[b][i] = (double)kPadPosition;
-            c.py[b][i] = (double)kPadPosition;
-            c.pa[b][i] = make_float4(kPadPosition, kPadPosition, kPadPosition * kPadPosition, 0.0f);
-            c.pb[b][i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
+        write_padding(c, i);
     }
 }
 

@@ -139,16 +139,6 @@ __device__ __forceinline__ bool in_cutoff64(double dx, double dy, double r2, con
     return ref_in_cutoff(dx, dy, K.kappa, r, a);
 }
 
-// a / b correctly rounded, given rb = 1/b correctly rounded: one residual
-// correction of a rb (Markstein), 3 FP64 instructions instead of the ~9 of a
-// division.  Zero, tiny, huge and non-finite values take the division itself.
-__device__ __forceinline__ double div_by(double a, double b, double rb) {
-    const double q = __dmul_rn(a, rb);
-    const uint32_t ea = ((uint32_t)__double2hiint(a) >> 20) & 0x7FFu, eq = ((uint32_t)__double2hiint(q) >> 20) & 0x7FFu;
-    if (ea - 256u >= 1536u || eq - 256u >= 1536u) return __ddiv_rn(a, b);
-    return fma(fma(-b, q, a), rb, q);
-}
-
 // r2 outside yukawa64's range (no cloud in SI units gets here; NaN does)
 __device__ __forceinline__ bool yukawa64_odd(double r2) {
     return (uint32_t)__double2hiint(r2) - (923u << 20) >= (200u << 20);
@@ -187,35 +177,48 @@ struct HitResult {
     double v[NS];
 };
 
-template <int NS>  // NS sums per i
-struct HitWarp {
-    HitResult<NS> res[kHitPerLane * 32];     // the entries' results
-    float4 f[32];                            // FP32 positions of the j group being filtered
-    uint32_t mask[kHitGroups][32];           // bit jl of mask[k][il]: pair (il, group k's jl)
-    int group[kHitGroups];                   // the j groups
-    uint16_t code[kHitPerLane * 32];         // (k << 10) | (jl << 5) | il
+template <class Result>
+struct alignas(16) HitWarp {
+    Result res[kHitPerLane * 32];     // the entries' results
+    float fx[32], fy[32], fb[32];     // the j group being filtered: xh, yh, -|p|^2
+    uint32_t mask[kHitGroups][32];    // bit jl of mask[k][il]: pair (il, group k's jl)
+    int group[kHitGroups];            // the j groups
+    uint16_t code[kHitPerLane * 32];  // (k << 10) | (jl << 5) | il
 };
 
 // Filters j group g (FP32 positions pa, n particles) against this lane's i
 // (px2 = 2 xh_i, py2 = 2 yh_i, nu = -bound_i; nu = INFINITY: no particle) and
-// stores the lane's mask as entry k.  NaN passes: such a pair is decided in
-// FP64.  Returns the lane's number of hits.
-template <int NS>
-__device__ __forceinline__ int hit_filter(HitWarp<NS> &W, int k, int g, int self, const float4 *__restrict__ pa, int n,
-                                          float px2, float py2, float nu) {
+// stores the lane's mask as entry k.  A pair is out if bound_i - |p_j|^2 + 2
+// p_i.p_j is negative (two j per packed instruction, 3 instructions per pair);
+// NaN passes: such a pair is decided later.  Returns the lane's number of hits.
+template <class Result>
+__device__ __forceinline__ int hit_filter(HitWarp<Result> &W, int k, int g, int self, const float4 *__restrict__ pa,
+                                          int n, float px2, float py2, float nu) {
     const int lane = threadIdx.x & 31;
     const int j = 32 * g + lane;
+    const float4 A = (j < n) ? pa[j] : make_float4(0.0f, 0.0f, INFINITY, 0.0f);
     __syncwarp();
-    W.f[lane] = (j < n) ? pa[j] : make_float4(0.0f, 0.0f, INFINITY, 0.0f);
+    W.fx[lane] = A.x;
+    W.fy[lane] = A.y;
+    W.fb[lane] = -A.z;
     if (lane == 0) W.group[k] = g;
     __syncwarp();
+    const float2 p2 = make_float2(px2, px2), q2 = make_float2(py2, py2), nb = make_float2(-nu, -nu);
     uint32_t m = 0u;
-#pragma unroll 8
-    for (int u = 31; u >= 0; u--) {
-        const float4 A = W.f[u];
-        const float d = fmaf(px2, -A.x, fmaf(py2, -A.y, A.z + nu));
-        m = 2u * m + (d >= 0.0f ? 0u : 1u);
+#pragma unroll
+    for (int c = 7; c >= 0; c--) {
+        const float4 X = reinterpret_cast<const float4 *>(W.fx)[c], Y = reinterpret_cast<const float4 *>(W.fy)[c],
+                     B = reinterpret_cast<const float4 *>(W.fb)[c];
+        const float2 t01 = __ffma2_rn(p2, make_float2(X.x, X.y),
+                                      __ffma2_rn(q2, make_float2(Y.x, Y.y), __fadd2_rn(make_float2(B.x, B.y), nb)));
+        const float2 t23 = __ffma2_rn(p2, make_float2(X.z, X.w),
+                                      __ffma2_rn(q2, make_float2(Y.z, Y.w), __fadd2_rn(make_float2(B.z, B.w), nb)));
+        m = __funnelshift_l(__float_as_uint(t23.y), m, 1);
+        m = __funnelshift_l(__float_as_uint(t23.x), m, 1);
+        m = __funnelshift_l(__float_as_uint(t01.y), m, 1);
+        m = __funnelshift_l(__float_as_uint(t01.x), m, 1);
     }
+    m = ~m;
     if (nu == INFINITY) m = 0u;
     if (g == self) m &= ~(1u << lane);  // j == i
     const int left = n - 32 * g;
@@ -224,15 +227,16 @@ __device__ __forceinline__ int hit_filter(HitWarp<NS> &W, int k, int g, int self
     return __popc(m);
 }
 
-// Evaluates every hit of the first `ng` masks: eval(il, j) gives an entry's
-// result, summed per i in the order (k, jl) into sum[NS].
-template <int NS, class Eval>
-__device__ __forceinline__ void hit_flush(HitWarp<NS> &W, int ng, double (&sum)[NS], Eval eval) {
+// Lays every hit of the first `ng` masks out in windows of up to kHitPerLane
+// hits of every i: work(total) runs on the window's entries (code[0 ..
+// total-1], ordered by i), then collect(off, c) on every lane with the range of
+// its own i's entries, in the order (k, jl).
+template <class Result, class Work, class Collect>
+__device__ __forceinline__ void hit_windows(HitWarp<Result> &W, int ng, Work work, Collect collect) {
     const int lane = threadIdx.x & 31;
     int k = 0;
     uint32_t m = (ng > 0) ? W.mask[0][lane] : 0u;
     for (;;) {
-        // this window: the lane's next hits, at most kHitPerLane
         int left = __popc(m);
         for (int kk = k + 1; kk < ng && left < kHitPerLane; kk++) left += __popc(W.mask[kk][lane]);
         const int c = min(left, kHitPerLane);
@@ -252,17 +256,30 @@ __device__ __forceinline__ void hit_flush(HitWarp<NS> &W, int ng, double (&sum)[
             W.code[off + t] = (uint16_t)((k << 10) | (u << 5) | lane);
         }
         __syncwarp();
-        for (int t = lane; t < total; t += 32) {
-            const int code = W.code[t];
-            W.res[t] = eval(code & 31, 32 * W.group[code >> 10] + ((code >> 5) & 31));
-        }
+        work(total);
         __syncwarp();
-        for (int t = 0; t < c; t++) {
-#pragma unroll
-            for (int e = 0; e < NS; e++) sum[e] = __dadd_rn(sum[e], W.res[off + t].v[e]);
-        }
+        collect(off, c);
         __syncwarp();
     }
+}
+
+// FP64: eval(il, j) gives an entry's result, summed per i into sum[NS].
+template <int NS, class Eval>
+__device__ __forceinline__ void hit_flush(HitWarp<HitResult<NS>> &W, int ng, double (&sum)[NS], Eval eval) {
+    hit_windows(
+        W, ng,
+        [&](int total) {
+            for (int t = threadIdx.x & 31; t < total; t += 32) {
+                const int code = W.code[t];
+                W.res[t] = eval(code & 31, 32 * W.group[code >> 10] + ((code >> 5) & 31));
+            }
+        },
+        [&](int off, int c) {
+            for (int t = 0; t < c; t++) {
+#pragma unroll
+                for (int e = 0; e < NS; e++) sum[e] = __dadd_rn(sum[e], W.res[off + t].v[e]);
+            }
+        });
 }
 
 // Calls eval(il, 32 k + jl) for every bit of the warp's masks mask[k][il],

@@ -7,41 +7,89 @@
 
 namespace dm {
 
-// Writes stage buffer 0 (FP64 and two-float copies) from the base
-// positions, and the padding particles of both buffers.
+// Writes position set 0 (two-float copies and filter bounds) from the state,
+// and the padding particles of every set.
 static __global__ void init_positions(CloudDev c) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n_pad) return;
     if (i < c.n) {
         write_stage_position(c, 0, i, c.x[i], c.y[i]);
     } else {
-        for (int b = 0; b < 2; b++) {
-            c.px[b][i] = (double)kPadPosition;
-            c.py[b][i] = (double)kPadPosition;
-            c.pa[b][i] = make_float4(kPadPosition, kPadPosition, kPadPosition * kPadPosition, 0.0f);
-            c.pb[b][i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
+        write_padding(c, i);
         c.q[i] = 0.0;
         c.m[i] = 1.0;
     }
 }
 
-// For the autotuner: the positions squeezed about (cx, cy) by lam, written
-// as stage buffer 1 (which holds nothing live between steps), so kernels can
-// be timed on a denser copy of the cloud without touching its state.
-// Both force time slots = t (see stage_time()).
+// Position set 1 (x2 = x + dt v/2) and its group boxes from the state, when
+// the step before did not leave them for this dt (one warp per group).
+static __global__ void prepare_midpoint(CloudDev c, double dt, const double *dt_dev) {
+    pdl_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if ((i & ~31) >= c.n) return;  // whole warp
+    float xh = 0.0f, yh = 0.0f;
+    if (i < c.n) {
+        write_midpoint(c, i, c.x[i], c.y[i], c.vx[i], c.vy[i], dt_dev ? *dt_dev : dt);
+        const float4 A = c.pa[1][i];
+        xh = A.x;
+        yh = A.y;
+    }
+    store_group_box(c.gbox[1] + (i >> 5), i < c.n, xh, yh, true);
+}
+
+// After an RK2 step: its results, left in sets 2 and 3 because other blocks
+// were still reading sets 0 and 1, become sets 0 (the state) and 1.
+static __global__ void adopt_sets(CloudDev c, int ngroups) {
+    pdl_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
+    for (int b = 0; b < 2; b++) {
+        if (i < c.n) {
+            c.px[b][i] = c.px[b + 2][i];
+            c.py[b][i] = c.py[b + 2][i];
+            c.pa[b][i] = c.pa[b + 2][i];
+            c.pb[b][i] = c.pb[b + 2][i];
+        }
+        if (i < ngroups) c.gbox[b][i] = c.gbox[b + 2][i];
+    }
+}
+
+// Boxes of every 32 consecutive groups of sets b and b + 1 (large clouds): one
+// warp per super group and set.
+static __global__ void super_bounds(CloudDev c, int b, int ngroups) {
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const int nsuper = (ngroups + 31) >> 5;
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= 2 * nsuper) return;  // whole warp
+    const int e = w / nsuper, s = w % nsuper, g = 32 * s + lane;
+    float4 v = (g < ngroups) ? c.gbox[b + e][g] : make_float4(INFINITY, INFINITY, -INFINITY, -INFINITY);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        v.x = fminf(v.x, __shfl_xor_sync(0xffffffffu, v.x, o));
+        v.y = fminf(v.y, __shfl_xor_sync(0xffffffffu, v.y, o));
+        v.z = fmaxf(v.z, __shfl_xor_sync(0xffffffffu, v.z, o));
+        v.w = fmaxf(v.w, __shfl_xor_sync(0xffffffffu, v.w, o));
+    }
+    if (lane == 0) c.gsuper[b + e][s] = v;
+}
+
+// Force time slots = t (see stage_time()).
 static __global__ void set_time_slots(double *time, double t) {
     time[0] = t;
     time[1] = t;
 }
 
+// For the autotuner: the positions squeezed about (cx, cy) by lam, written
+// as position set 1, so kernels can be timed on a denser copy of the cloud
+// without touching its state.
 static __global__ void tune_compress(CloudDev c, double cx, double cy, double lam) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < c.n) write_stage_position(c, 1, i, cx + lam * (c.x[i] - cx), cy + lam * (c.y[i] - cy));
 }
 
 // Bounding box of each 32-particle group's FP32 positions (hi parts) in
-// stage buffer b, for the culling pair kernels: one warp per group; padding
+// position set b, for the culling pair kernels: one warp per group; padding
 // particles are left out, so an all-padding group gets an empty box.
 static __global__ void group_bounds(CloudDev c, int b) {
     pdl_wait();
@@ -49,20 +97,8 @@ static __global__ void group_bounds(CloudDev c, int b) {
     const int lane = threadIdx.x & 31;
     const int i = 32 * g + lane;
     if (32 * g >= c.n_pad) return;  // whole warp
-    float x0 = INFINITY, y0 = INFINITY, x1 = -INFINITY, y1 = -INFINITY;
-    if (i < c.n) {
-        const float4 A = c.pa[b][i];
-        x0 = x1 = A.x;
-        y0 = y1 = A.y;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
-        y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
-        x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-        y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
-    }
-    if (lane == 0) c.gbox[b][g] = make_float4(x0, y0, x1, y1);
+    const float4 A = (i < c.n) ? c.pa[b][i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    store_group_box(c.gbox[b] + g, i < c.n, A.x, A.y, true);
 }
 
 // ---------------------------------------------------------------------------

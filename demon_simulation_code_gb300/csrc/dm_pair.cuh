@@ -2,17 +2,18 @@
 // RK4 stage epilogue fused in, for sm_103a.
 //
 // Replaces ShieldedCoulombForce::force1..4 (ShieldedCoulombForce.cpp:37-237)
-// plus, in the epilogue, the per-particle forces, CacheOperator and the RK4
+// plus, in the epilogue, the per-particle forces, CacheOperator and the RK
 // stage/combine loops (see dm_device.cuh).
 //
-// Work decomposition (owner computes, no atomics on forces):
-//   * an i-tile of 32*ILP particles belongs to S CTAs (a thread-block
-//     cluster, or S plain blocks whose partial sums stage_finish adds); lane
-//     l of every warp of those CTAs owns particles i = tile*32*ILP + k*32 + l,
-//     k < ILP (the lane's i "slots"), kept in registers;
+// Work decomposition (owner computes, no atomics on forces), for each of the
+// pass's position sets (dm_device.cuh):
+//   * an i-tile of 32*ILP particles belongs to S CTAs (with the other set's S
+//     CTAs a thread-block cluster, or plain blocks whose partial sums
+//     stage_finish adds); lane l of every warp of those CTAs owns particles i
+//     = tile*32*ILP + k*32 + l, k < ILP (the lane's i "slots"), in registers;
 //   * rank r of the S sweeps every S-th chunk of 4 j (or, culling, every
-//     S-th 32-particle j group within reach of the tile), staging them in
-//     shared memory; the CTA's warps deal the staged chunks round-robin;
+//     S-th of the 32-particle j groups within reach of the tile), staging them
+//     in shared memory; the CTA's warps deal the staged chunks round-robin;
 //   * pairs of groups that may hold a pair within the cutoff are first
 //     filtered with the expanded distance |p_j|^2 - 2 p_i.p_j against a per-i
 //     bound (two j per packed FMA) -- the GPU form of the reference's early
@@ -20,7 +21,7 @@
 //     entirely within the cutoff skip the filter;
 //   * the pair terms are evaluated two j at a time in packed f32x2
 //     arithmetic (pair2_terms); the per-particle sums are compensated and the
-//     stage epilogue runs once per particle in FP64.
+//     pass's epilogue runs once per particle in FP64.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -150,47 +151,6 @@ __device__ __forceinline__ float border_pair(const StageParams &P, int b, const 
     return (q * ex) * ((y * y) * (y + P.kappa_f));
 }
 
-struct PairTuning {
-    int nt, ilp, jt, s;
-};
-
-// ---------------------------------------------------------------------------
-// FP32-compensated kernel.
-//
-// A CTA of NW warps shares one i tile of 32*ILP particles (lane l, slot k ->
-// i = tile*32*ILP + k*32 + l).  Each staged j chunk (4 j) goes to one warp;
-// its pairs are classified:
-//   * groups entirely within the cutoff of the tile (box test): evaluated
-//     directly, every lane on the same j from shared-memory broadcasts, two
-//     j per packed instruction, no filter and no cutoff test;
-//   * other groups within reach: the packed filter on all 4 j and every
-//     slot, one warp vote per chunk; where it fired, per slot, the number
-//     of (lane, j) pairs that passed decides (a warp reduction): at least
-//     P.direct_min of the 128 -> the chunk is evaluated directly for that
-//     slot with the cutoff taken by a select; fewer -> each lane records its
-//     own passing j as hit bits (4 per chunk, 8 chunks per 32-bit word) and
-//     later evaluates them two at a time.
-// Each lane accumulates only into its own sums (plain f32x2 sums over a few
-// chunks, then Kahan), so the result is deterministic and needs no atomics.
-// The sums leave out C q_i (applied in FP64 once per particle).
-// ---------------------------------------------------------------------------
-template <int NW, int ILP, int TC>
-struct Fp32cSmem {
-    // j tile: TC 4-j chunks, each field of the 4 j in one 16-byte word
-    // (-xh, -yh, |p|^2, -xl, -yl, q, j): two consecutive j of a field load
-    // straight into the register pair a packed instruction takes
-    static constexpr size_t tile = (size_t)TC * 7 * sizeof(float4);
-    static constexpr size_t cold = (size_t)ILP * 32 * sizeof(float4);
-    static constexpr size_t acc = (size_t)NW * ILP * 32 * sizeof(float4);
-    static constexpr size_t red = (size_t)ILP * 32 * sizeof(float4);
-    // culling: near, inside and mostly-inside group lists (NT each) and
-    // their per-warp counts
-    static constexpr size_t glist = 3 * ((size_t)NW * 32 * sizeof(int) + NW * sizeof(int));
-    static constexpr size_t bytes = tile + cold + acc + red + glist;
-    // s_red, in float4 units from the start of shared memory
-    static constexpr size_t red_offset = (tile + cold + acc) / sizeof(float4);
-};
-
 // Conservative FP32 test: can any point of box a come within the cutoff of
 // any point of box b?  Boxes are (x0, y0, x1, y1) of FP32 hi parts; the true
 // positions lie within an ulp of them and the box arithmetic rounds, so the
@@ -221,14 +181,180 @@ __device__ __forceinline__ bool boxes_inside(const float4 &a, const float4 &b, f
     return fmaf(dx, dx, dy * dy) < 0.999f * rc2_lo;
 }
 
+// Barrier `id` of `threads` threads of the block.  The blocks that sweep a
+// tile's two position sets hold one half of NW warps per set; each half goes
+// through its sweep on its own.
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+constexpr int kBarSet = 1;       // + set: the set's half of the block
+constexpr int kBarEpilogue = 3;  // + pair: two warps
+
+// ---------------------------------------------------------------------------
+// The j groups within reach of an i tile, by class.  Groups are tested by
+// their boxes, 32 consecutive groups (a super group) per warp at a time; in
+// large clouds super groups out of reach are skipped whole by their own boxes
+// (Morton order keeps both compact), so a tile of a 262,144-particle cloud
+// tests 256 + 32 per super group in reach instead of 8192.  The lists keep
+// the groups' order.
+// ---------------------------------------------------------------------------
+constexpr int kSuperCap = 256;  // super groups considered at a time
+
+template <int NW, int NCLASS>
+struct NearLists {
+    static constexpr int rounds = 16 / NW > 0 ? 16 / NW : 1;  // tests of a warp per batch
+    static constexpr int cap = 32 * NW * rounds;              // groups of a batch
+    int list[cap];  // the classes one after the other
+    int super[kSuperCap];
+    int count[NCLASS][NW];
+};
+
+// Lists the groups within reach batch by batch and calls use(first, total) for
+// every batch that has any (every thread of the NW warps, `tid` its index
+// among them): class k's groups are L.list[first[k] .. first[k] + total[k] - 1].
+// classify(g, box) is the class of a group within reach.  Of every `stride`
+// groups only the `offset`-th is considered (the ranks of a j split share the
+// tests); gs: super group boxes (stride 1), or nullptr.
+//
+// A warp tests its part of a batch on its own and keeps the classes in one
+// register per lane; the warps meet twice to lay the lists out.
+template <int NW, int NCLASS, class Sync, class Classify, class Use>
+__device__ __forceinline__ void for_near_groups(NearLists<NW, NCLASS> &L, const float4 *__restrict__ gb,
+                                                const float4 *__restrict__ gs, int ngroups, int offset, int stride,
+                                                const float4 &tb, float rc2_hi, int tid, Sync sync, Classify classify,
+                                                Use use) {
+    constexpr int NR = NearLists<NW, NCLASS>::rounds;
+    const int lane = tid & 31, warp = tid >> 5;
+    const uint32_t below = (1u << lane) - 1u;
+    const int ncand = (ngroups - offset + stride - 1) / stride;  // candidate t is group t*stride + offset
+    const int nsuper = (ncand + 31) >> 5;
+    for (int s0 = 0; s0 < nsuper; s0 += kSuperCap) {
+        int ns = min(kSuperCap, nsuper - s0);
+        if (gs) {  // the super groups within reach, in order
+            const int all = ns;
+            ns = 0;
+            for (int t0 = 0; t0 < all; t0 += 32 * NW) {
+                const int t = t0 + tid;
+                const bool near = t < all && boxes_near(tb, gs[s0 + t], rc2_hi);
+                const uint32_t bal = __ballot_sync(0xffffffffu, near);
+                if (lane == 0) L.count[0][warp] = __popc(bal);
+                sync();
+                int off = ns;
+#pragma unroll
+                for (int w = 0; w < NW; w++) {
+                    off += (w < warp) ? L.count[0][w] : 0;
+                    ns += L.count[0][w];
+                }
+                if (near) L.super[off + __popc(bal & below)] = s0 + t;
+                sync();
+            }
+        }
+        auto group_of = [&](int e) { return (32 * (gs ? L.super[e] : s0 + e) + lane) * stride + offset; };
+        for (int e0 = 0; e0 < ns; e0 += NW * NR) {
+            for (int u = 1; u < NR; u++) {  // one round trip to L2 (~900 cycles) for the batch's boxes
+                const int e = e0 + u * NW + warp, g = (e < ns) ? group_of(e) : ngroups;
+                if (g < ngroups) prefetch_l1(gb + g);
+            }
+            uint32_t cls = 0u;  // 2 bits per round: class + 1, 0 = out of reach
+            static_assert(NR <= 16 && NCLASS <= 3, "classes fit a register");
+            int cnt[NCLASS];  // of this warp
+#pragma unroll
+            for (int k = 0; k < NCLASS; k++) cnt[k] = 0;
+            for (int u = 0; u < NR; u++) {
+                const int e = e0 + u * NW + warp;
+                if (e >= ns) break;
+                const int g = group_of(e);
+                const float4 box = (g < ngroups) ? gb[g] : make_float4(INFINITY, INFINITY, -INFINITY, -INFINITY);
+                const bool near = g < ngroups && boxes_near(tb, box, rc2_hi);
+                if (!__any_sync(0xffffffffu, near)) continue;
+                const uint32_t c = near ? (uint32_t)classify(g, box) + 1u : 0u;
+                cls |= c << (2 * u);
+#pragma unroll
+                for (int k = 0; k < NCLASS; k++) cnt[k] += __popc(__ballot_sync(0xffffffffu, c == k + 1u));
+            }
+            if (lane == 0)
+#pragma unroll
+                for (int k = 0; k < NCLASS; k++) L.count[k][warp] = cnt[k];
+            sync();
+            int first[NCLASS], total[NCLASS], off[NCLASS], at = 0;
+#pragma unroll
+            for (int k = 0; k < NCLASS; k++) {
+                first[k] = off[k] = at;
+#pragma unroll
+                for (int w = 0; w < NW; w++) {
+                    off[k] += (w < warp) ? L.count[k][w] : 0;
+                    at += L.count[k][w];
+                }
+                total[k] = at - first[k];
+            }
+            if (at == 0) {
+                sync();  // the counts are rewritten
+                continue;
+            }
+            for (int u = 0; u < NR; u++) {
+                const int e = e0 + u * NW + warp;
+                const uint32_t c = (cls >> (2 * u)) & 3u;
+                if (!__any_sync(0xffffffffu, c != 0u)) continue;
+                const int g = group_of(e);
+#pragma unroll
+                for (int k = 0; k < NCLASS; k++) {
+                    const uint32_t bal = __ballot_sync(0xffffffffu, c == k + 1u);
+                    if (c == k + 1u) L.list[off[k] + __popc(bal & below)] = g;
+                    off[k] += __popc(bal);
+                }
+            }
+            sync();
+            use(first, total);
+            sync();
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FP32-compensated kernel.
+//
+// A CTA of NW warps shares one i tile of 32*ILP particles (lane l, slot k ->
+// i = tile*32*ILP + k*32 + l).  Each staged j chunk (4 j) goes to one warp;
+// its pairs are classified:
+//   * groups entirely within the cutoff of the tile (box test): evaluated
+//     directly, every lane on the same j from shared-memory broadcasts, two
+//     j per packed instruction, no filter and no cutoff test;
+//   * other groups within reach: the packed filter on all 4 j and every
+//     slot, each lane recording its own passing j as hit bits (a funnel shift
+//     of the sign per pair; 8 chunks per 32-bit word); per word and slot the
+//     number of (lane, j) pairs that passed decides (a warp reduction): at
+//     least 8 P.direct_min of the 1024 -> the 8 chunks are evaluated directly
+//     for that slot with the cutoff taken by a select; fewer -> each lane
+//     evaluates its hits of the whole staged tile two at a time.
+// Each lane accumulates only into its own sums (plain f32x2 sums over a few
+// chunks, then Kahan), so the result is deterministic and needs no atomics.
+// The sums leave out C q_i (applied in FP64 once per particle).
+// ---------------------------------------------------------------------------
+template <int NW, int ILP, int TC>
+struct Fp32cSmem {
+    // j tile: TC 4-j chunks, each field of the 4 j in one 16-byte word
+    // (-xh, -yh, |p|^2, -xl, -yl, q, j): two consecutive j of a field load
+    // straight into the register pair a packed instruction takes
+    static constexpr size_t tile = (size_t)TC * 7 * sizeof(float4);
+    static constexpr size_t cold = (size_t)ILP * 32 * sizeof(float4);
+    static constexpr size_t acc = (size_t)NW * ILP * 32 * sizeof(float4);
+    static constexpr size_t red = (size_t)ILP * 32 * sizeof(float4);
+    // culling: near, inside and mostly-inside group lists
+    static constexpr size_t glist = sizeof(NearLists<NW, 3>);
+    static constexpr size_t bytes = tile + cold + acc + red + glist;
+    // s_red, in float4 units from the start of shared memory
+    static constexpr size_t red_offset = (tile + cold + acc) / sizeof(float4);
+};
+
 // The FP32C sweep of one i tile against rank `rank` of S of the j chunks:
-// i-side setup, the classified j loop, and the combine of the NW warps'
+// of position set buffer b: i-side setup, the classified j loop, and the combine of the NW warps'
 // Kahan sums into s_red[TILE] = (sx, sy, cx, cy) (force / (C q_i) = s - c).
-// Ends with the block synchronised.  `P` may live in shared memory (batched
+// By NW warps (`tid` the thread's index among them, sync() their barrier); ends
+// with them synchronised.  `P` may live in shared memory (batched
 // kernel).  Particles are those of P.c (n = P.c.n); j at or beyond n read as
 // padding, so a cloud needs no padding of its own.
-template <int NW, int ILP, int TC, bool CULL = false>
-__device__ __forceinline__ void fp32c_sweep(const StageParams &P, int tile, int rank, int S,
+template <int NW, int ILP, int TC, bool CULL, class Sync>
+__device__ __forceinline__ void fp32c_sweep(const StageParams &P, int b, int tile, int rank, int S, int tid, Sync sync,
                                             unsigned char *smem_raw) {
     constexpr int NT = NW * 32;
     constexpr int TILE = 32 * ILP;  // particles per i tile
@@ -243,13 +369,9 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int tile, int 
     float4 *s_cold = reinterpret_cast<float4 *>(s_j4 + TC);  // [ILP][32] (xl, yl, -, i)
     float4 *s_acc = s_cold + ILP * 32;                     // [NW][ILP][32]
     float4 *s_red = s_acc + NW * ILP * 32;                 // [TILE]
-    int *s_glist = reinterpret_cast<int *>(s_red + TILE);  // [NT] surviving groups
-    int *s_wcount = s_glist + NT;                          // [NW]
 
-    const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const int n = P.c.n;
-    const int b = (P.mode == kModeForceOnly) ? P.fo_buf : (P.stage - 1) & 1;
     const float4 *__restrict__ pa = P.c.pa[b];
     const float4 *__restrict__ pb = P.c.pb[b];
     float4 *my_acc = s_acc + warp * ILP * 32;
@@ -292,64 +414,74 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int tile, int 
         return PairI{dup2(xh), dup2(yh), dup2(c4.x), dup2(c4.y)};
     };
 
-    // Filter hits are recorded per lane: bit 4*g + u of hits[k] is the pair
-    // (slot k's i, j = 4*(cbase + g*NW) + u of the staged tile), for the
-    // last (up to 8) chunks this warp swept.  The flush evaluates every
-    // lane's own hits two at a time, slot by slot.
-    uint32_t hits[ILP];
-#pragma unroll
-    for (int k = 0; k < ILP; k++) hits[k] = 0u;
+    // Filter hits are recorded per lane, one word per 8 chunks this warp swept:
+    // bit 31 - (4 g + u) of word w of slot k is the pair (slot k's i, j = 4 (warp
+    // + (8 w + g) NW) + u of the staged tile).  A tile holds at most kWords
+    // words of a warp's chunks; they are evaluated together, every lane its own
+    // hits two at a time, so a lane with few hits in one stretch of j makes up
+    // for it in another (0.5 hits per lane and word on a calm cloud: word by
+    // word, five of six lanes were idle).
+    constexpr int kWords = (TC / NW + 7) / 8;
     const float *s_xf = reinterpret_cast<const float *>(s_x4);
     const float *s_yf = reinterpret_cast<const float *>(s_y4);
     const float *s_xlf = reinterpret_cast<const float *>(s_xl4);
     const float *s_ylf = reinterpret_cast<const float *>(s_yl4);
     const float *s_qf = reinterpret_cast<const float *>(s_q4);
     const int *s_jf = reinterpret_cast<const int *>(s_j4);
-    auto flush_hits = [&](int cbase) {
-#pragma unroll 1
-        for (int k = 0; k < ILP; k++) {
-            uint32_t m = hits[0];
+    auto flush_hits = [&](int k, uint32_t (&m)[kWords]) {
+        int ii;
+        const PairI I = slot_i(k, ii);
+        float4 acc = my_acc[k * 32 + lane];
+        // the next hit's index into the tile's j; words in order
+        auto next = [&]() {
+            int w = 0;
+            uint32_t v = m[0];
 #pragma unroll
-            for (int t = 1; t < ILP; t++) m = (k == t) ? hits[t] : m;
-            if (!__any_sync(0xffffffffu, m != 0u)) continue;
-            int ii;
-            const PairI I = slot_i(k, ii);
-            float4 acc = my_acc[k * 32 + lane];
-            const int jbase = 4 * cbase;  // j of bit 0
-            while (m) {
-                // two hits per packed evaluation; a missing second one
-                // repeats the first with q = 0 (a finite, zero term)
-                const int e0 = __ffs(m) - 1;
-                m &= m - 1u;
-                const int e1 = m ? __ffs(m) - 1 : e0;
-                const float q1 = m ? 1.0f : 0.0f;
-                m &= m - 1u;
-                const int j0 = jbase + (e0 >> 2) * (4 * NW) + (e0 & 3);  // index into the tile's j
-                const int j1 = jbase + (e1 >> 2) * (4 * NW) + (e1 & 3);
-                float2 dx, dy, r2, w;
-                pair2_terms(I, make_float2(s_xf[j0], s_xf[j1]), make_float2(s_yf[j0], s_yf[j1]),
-                            make_float2(s_xlf[j0], s_xlf[j1]), make_float2(s_ylf[j0], s_ylf[j1]),
-                            make_float2(s_qf[j0], s_qf[j1] * q1), kap, nkl2e, dx, dy, r2, w);
-                const int g0 = s_jf[j0], g1 = s_jf[j1];
-                // certainly inside: r2 < rc2_lo; borderline pairs decided exactly
-                w.x = (r2.x < rc2_lo && g0 != ii) ? w.x : 0.0f;
-                w.y = (r2.y < rc2_lo && g1 != ii && q1 != 0.0f) ? w.y : 0.0f;
-                if (!(r2.x < rc2_lo) && r2.x < rc2_hi) {
-                    float bx, by;
-                    w.x = border_pair(P, b, I, ii, s_xf[j0], s_yf[j0], s_xlf[j0], s_ylf[j0], s_qf[j0], g0, bx, by);
+            for (int t = 1; t < kWords; t++)
+                if (v == 0u) {
+                    v = m[t];
+                    w = t;
                 }
-                if (q1 != 0.0f && !(r2.y < rc2_lo) && r2.y < rc2_hi) {
-                    float bx, by;
-                    w.y = border_pair(P, b, I, ii, s_xf[j1], s_yf[j1], s_xlf[j1], s_ylf[j1], s_qf[j1], g1, bx, by);
-                }
-                const float2 fx = mul2(w, dx), fy = mul2(w, dy);
-                kahan_add(acc.x, acc.z, fx.x + fx.y);
-                kahan_add(acc.y, acc.w, fy.x + fy.y);
+            const int pos = __clz(v);
+            v &= ~(0x80000000u >> pos);
+#pragma unroll
+            for (int t = 0; t < kWords; t++) m[t] = (t == w) ? v : m[t];
+            return 4 * (warp + (8 * w + (pos >> 2)) * NW) + (pos & 3);
+        };
+        auto any = [&]() {
+            uint32_t v = 0u;
+#pragma unroll
+            for (int t = 0; t < kWords; t++) v |= m[t];
+            return v != 0u;
+        };
+        while (any()) {
+            // two hits per packed evaluation; a missing second one repeats
+            // the first with q = 0 (a finite, zero term)
+            const int j0 = next();
+            const bool two = any();
+            const int j1 = two ? next() : j0;
+            const float q1 = two ? 1.0f : 0.0f;
+            float2 dx, dy, r2, w;
+            pair2_terms(I, make_float2(s_xf[j0], s_xf[j1]), make_float2(s_yf[j0], s_yf[j1]),
+                        make_float2(s_xlf[j0], s_xlf[j1]), make_float2(s_ylf[j0], s_ylf[j1]),
+                        make_float2(s_qf[j0], s_qf[j1] * q1), kap, nkl2e, dx, dy, r2, w);
+            const int g0 = s_jf[j0], g1 = s_jf[j1];
+            // certainly inside: r2 < rc2_lo; borderline pairs decided exactly
+            w.x = (r2.x < rc2_lo && g0 != ii) ? w.x : 0.0f;
+            w.y = (r2.y < rc2_lo && g1 != ii && two) ? w.y : 0.0f;
+            if (!(r2.x < rc2_lo) && r2.x < rc2_hi) {
+                float bx, by;
+                w.x = border_pair(P, b, I, ii, s_xf[j0], s_yf[j0], s_xlf[j0], s_ylf[j0], s_qf[j0], g0, bx, by);
             }
-            my_acc[k * 32 + lane] = acc;
+            if (two && !(r2.y < rc2_lo) && r2.y < rc2_hi) {
+                float bx, by;
+                w.y = border_pair(P, b, I, ii, s_xf[j1], s_yf[j1], s_xlf[j1], s_ylf[j1], s_qf[j1], g1, bx, by);
+            }
+            const float2 fx = mul2(w, dx), fy = mul2(w, dy);
+            kahan_add(acc.x, acc.z, fx.x + fx.y);
+            kahan_add(acc.y, acc.w, fy.x + fy.y);
         }
-#pragma unroll
-        for (int k = 0; k < ILP; k++) hits[k] = 0u;
+        my_acc[k * 32 + lane] = acc;
     };
 
     // Chunk c of the staged tile against slot k (runtime k), every lane on
@@ -412,7 +544,7 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int tile, int 
     constexpr bool DENSE = MODE == 1;
     for (int q0 = 0; q0 < count; q0 += TC) {
         const int tcn = min(TC, count - q0);
-        __syncthreads();
+        sync();
         for (int e = tid; e < tcn; e += NT) {
             const int jb = 4 * chunk_of(q0 + e);  // first j of the chunk
             float xs[4], ys[4], bs[4];
@@ -443,7 +575,7 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int tile, int 
             s_y4[e] = make_float4(ys[0], ys[1], ys[2], ys[3]);
             s_b4[e] = make_float4(bs[0], bs[1], bs[2], bs[3]);
         }
-        __syncthreads();
+        sync();
         if constexpr (DENSE) {
             // every pair of these groups is inside the cutoff (and j != i):
             // no filter, no select; each lane evaluates its own i against the
@@ -496,60 +628,65 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int tile, int 
                 for (int k = 0; k < ILP; k++) direct_chunk(c, k);
             }
         } else {
-        // one flush site: the loop runs one step past the tile's last chunk
-        int nb = 0, cbase = warp;  // chunks recorded in hits, chunk of bit group 0
-        bool any_hit = false;      // warp-uniform
-        for (int c = warp;; c += NW) {
-            const bool live = c < tcn;  // warp-uniform
-            if (live) {
-                const float4 X = s_x4[c], Y = s_y4[c], Bq = s_b4[c];
-                const float2 X01 = make_float2(X.x, X.y), X23 = make_float2(X.z, X.w);
-                const float2 Y01 = make_float2(Y.x, Y.y), Y23 = make_float2(Y.z, Y.w);
-                const float2 B01 = make_float2(Bq.x, Bq.y), B23 = make_float2(Bq.z, Bq.w);
-                // d = |p_j|^2 - 2 p_i.p_j - bound_i: pair (i, j) passes iff d < 0
-                float2 d01[ILP], d23[ILP];
-                uint32_t sgn = 0u;
+            uint32_t hits[ILP][kWords];
 #pragma unroll
-                for (int k = 0; k < ILP; k++) {
-                    d01[k] = fma2(px2[k], X01, fma2(py2[k], Y01, add2(B01, nu2[k])));
-                    d23[k] = fma2(px2[k], X23, fma2(py2[k], Y23, add2(B23, nu2[k])));
-                    sgn |= __float_as_uint(d01[k].x) | __float_as_uint(d01[k].y) | __float_as_uint(d23[k].x) |
-                           __float_as_uint(d23[k].y);
+            for (int w = 0; w < kWords; w++) {
+                uint32_t m[ILP];
+#pragma unroll
+                for (int k = 0; k < ILP; k++) m[k] = 0u;
+                const int c0 = warp + 8 * w * NW, gn = min(8, (tcn - c0 + NW - 1) / NW);  // this word's chunks
+                if (gn <= 0) {  // warp-uniform: the tile is done
+#pragma unroll
+                    for (int k = 0; k < ILP; k++) hits[k][w] = 0u;
+                    continue;
                 }
-                if (__any_sync(0xffffffffu, (int)sgn < 0)) {
-                    // per slot: enough passing (lane, j) pairs -> the whole
-                    // chunk directly; else this lane's hits as bits
-                    uint32_t direct = 0u;
+#pragma unroll 2
+                for (int g = 0; g < gn; g++) {
+                    const int c = c0 + g * NW;
+                    const float4 X = s_x4[c], Y = s_y4[c], Bq = s_b4[c];
+                    const float2 X01 = make_float2(X.x, X.y), X23 = make_float2(X.z, X.w);
+                    const float2 Y01 = make_float2(Y.x, Y.y), Y23 = make_float2(Y.z, Y.w);
+                    const float2 B01 = make_float2(Bq.x, Bq.y), B23 = make_float2(Bq.z, Bq.w);
+                    // d = |p_j|^2 - 2 p_i.p_j - bound_i: pair (i, j) passes iff d < 0
 #pragma unroll
                     for (int k = 0; k < ILP; k++) {
-                        const uint32_t bits = (__float_as_uint(d01[k].x) >> 31) |
-                                              ((__float_as_uint(d01[k].y) >> 30) & 2u) |
-                                              ((__float_as_uint(d23[k].x) >> 29) & 4u) |
-                                              ((__float_as_uint(d23[k].y) >> 28) & 8u);
-                        const bool dir = (int)__reduce_add_sync(0xffffffffu, __popc(bits)) >= P.direct_min;
-                        direct |= (dir ? 1u : 0u) << k;
-                        hits[k] |= dir ? 0u : bits << (4 * nb);
+                        const float2 d01 = fma2(px2[k], X01, fma2(py2[k], Y01, add2(B01, nu2[k])));
+                        const float2 d23 = fma2(px2[k], X23, fma2(py2[k], Y23, add2(B23, nu2[k])));
+                        m[k] = __funnelshift_l(__float_as_uint(d01.x), m[k], 1);
+                        m[k] = __funnelshift_l(__float_as_uint(d01.y), m[k], 1);
+                        m[k] = __funnelshift_l(__float_as_uint(d23.x), m[k], 1);
+                        m[k] = __funnelshift_l(__float_as_uint(d23.y), m[k], 1);
                     }
-#pragma unroll 1
-                    for (int k = 0; k < ILP; k++)
-                        if ((direct >> k) & 1u) direct_chunk(c, k);
-                    any_hit = true;
                 }
-                nb++;
+                // enough passing (lane, j) pairs: the word's chunks directly
+#pragma unroll
+                for (int k = 0; k < ILP; k++) {
+                    if (gn < 8) m[k] <<= 32 - 4 * gn;
+                    if ((int)__reduce_add_sync(0xffffffffu, __popc(m[k])) >= 8 * P.direct_min) {
+#pragma unroll 1
+                        for (int g = 0; g < gn; g++) direct_chunk(c0 + g * NW, k);
+                        m[k] = 0u;
+                    }
+                    hits[k][w] = m[k];
+                }
             }
-            if (!live || nb == 8) {  // bits full, or the tile is done: its j are overwritten next
-                if (any_hit) flush_hits(cbase);
-                any_hit = false;
-                nb = 0;
-                cbase = c + NW;
-                if (!live) break;
+#pragma unroll 1
+            for (int k = 0; k < ILP; k++) {
+                uint32_t m[kWords], v = 0u;
+#pragma unroll
+                for (int w = 0; w < kWords; w++) {
+                    m[w] = hits[0][w];
+#pragma unroll
+                    for (int t = 1; t < ILP; t++) m[w] = (k == t) ? hits[t][w] : m[w];
+                    v |= m[w];
+                }
+                if (__any_sync(0xffffffffu, v != 0u)) flush_hits(k, m);
             }
-        }
         }
     }
     };
 
-    __syncthreads();  // s_cold complete
+    sync();  // s_cold complete
     if constexpr (!CULL) {
         // chunks dealt round-robin: chunk c belongs to rank c % S, so every
         // rank (and every warp) samples the whole cloud evenly
@@ -557,10 +694,11 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int tile, int 
         const int my_nch = (nch_all - rank + S - 1) / S;  // chunks of this rank
         sweep(my_nch, [&](int q) { return q * S + rank; }, std::integral_constant<int, 0>{});
     } else {
-        // 32-particle groups dealt round-robin to ranks; a group whose box is
-        // beyond the cutoff from the tile's box is skipped whole (it holds no
-        // pair the reference counts).  The survivors keep their order.
+        // the 32-particle groups whose box is within the cutoff of the tile's
+        // box (the others hold no pair the reference counts), dealt
+        // round-robin to the ranks, class by class
         const float4 *__restrict__ gb = P.c.gbox[b];
+        NearLists<NW, 3> &L = *reinterpret_cast<NearLists<NW, 3> *>(s_red + TILE);
         const int ngroups = (n + 31) >> 5;
         float4 tb = gb[tile * ILP];
 #pragma unroll
@@ -570,65 +708,37 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int tile, int 
                 tb = make_float4(fminf(tb.x, v.x), fminf(tb.y, v.y), fmaxf(tb.z, v.z), fmaxf(tb.w, v.w));
             }
         }
-        const int my_ng = (ngroups - rank + S - 1) / S;
         unsigned long long swept = 0ull;
-        int *s_glist2 = s_wcount + NW;   // [NT] groups entirely inside the cutoff
-        int *s_wcount2 = s_glist2 + NT;  // [NW]
-        int *s_glist3 = s_wcount2 + NW;  // [NT] groups mostly inside it
-        int *s_wcount3 = s_glist3 + NT;  // [NW]
         const float rc2_mostly = P.rc2_lo * P.near_direct_f2;  // 0: no such class
-        for (int t0 = 0; t0 < my_ng; t0 += NT) {
-            const int t = t0 + tid;
-            const int g = t * S + rank;
-            bool near = false, inside = false, mostly = false;
-            if (t < my_ng) {
-                const float4 gbox = gb[g];
-                near = boxes_near(tb, gbox, P.rc2_hi);
+        const float4 *gs = P.c.gsuper[b];
+        // the ranks share the tests (rank r takes every S-th group), or, with
+        // super groups, the groups found
+        const int deal = gs ? S : 1, mine_of = gs ? rank : 0;
+        for_near_groups(
+            L, gb, gs, ngroups, gs ? 0 : rank, gs ? 1 : S, tb, P.rc2_hi, tid, sync,
+            [&](int g, const float4 &gbox) {
                 // the tile's own groups hold the pairs j == i: not "inside"
-                inside = near && g / ILP != tile && boxes_inside(tb, gbox, P.rc2_lo);
+                if (g / ILP != tile && boxes_inside(tb, gbox, P.rc2_lo)) return 1;
                 // farthest separation within sqrt(near_direct_f2) r_c: most
                 // pairs pass the filter, so it is skipped
-                mostly = near && !inside && rc2_mostly > 0.0f && boxes_inside(tb, gbox, rc2_mostly);
-            }
-            const uint32_t bal = __ballot_sync(0xffffffffu, near && !inside && !mostly);
-            const uint32_t bal2 = __ballot_sync(0xffffffffu, inside);
-            const uint32_t bal3 = __ballot_sync(0xffffffffu, mostly);
-            if (lane == 0) {
-                s_wcount[warp] = __popc(bal);
-                s_wcount2[warp] = __popc(bal2);
-                s_wcount3[warp] = __popc(bal3);
-            }
-            __syncthreads();
-            int off = 0, total = 0, off2 = 0, total2 = 0, off3 = 0, total3 = 0;
-#pragma unroll
-            for (int w = 0; w < NW; w++) {
-                const int cw = s_wcount[w], cw2 = s_wcount2[w], cw3 = s_wcount3[w];
-                off += (w < warp) ? cw : 0;
-                off2 += (w < warp) ? cw2 : 0;
-                off3 += (w < warp) ? cw3 : 0;
-                total += cw;
-                total2 += cw2;
-                total3 += cw3;
-            }
-            const uint32_t below = (1u << lane) - 1u;
-            if (near && !inside && !mostly) s_glist[off + __popc(bal & below)] = g;
-            if (inside) s_glist2[off2 + __popc(bal2 & below)] = g;
-            if (mostly) s_glist3[off3 + __popc(bal3 & below)] = g;
-            sweep(8 * total, [&](int q) { return 8 * s_glist[q >> 3] + (q & 7); }, std::integral_constant<int, 0>{});
-            sweep(8 * total2, [&](int q) { return 8 * s_glist2[q >> 3] + (q & 7); },
-                  std::integral_constant<int, 1>{});
-            sweep(8 * total3, [&](int q) { return 8 * s_glist3[q >> 3] + (q & 7); },
-                  std::integral_constant<int, 2>{});
-            swept += (unsigned long long)(total + total2 + total3);
-            __syncthreads();  // the lists and counts are reused by the next batch
-        }
-        if (tid == 0 && swept) atomicAdd(P.c.eval_pairs, swept * 32ull * (unsigned long long)TILE);
+                return (rc2_mostly > 0.0f && boxes_inside(tb, gbox, rc2_mostly)) ? 2 : 0;
+            },
+            [&](const int (&first)[3], const int (&total)[3]) {
+                auto mine = [&](int t) { return 8 * ((t - mine_of + deal - 1) / deal); };  // this rank's chunks of t groups
+                auto chunk_of = [&](int k, int q) { return 8 * L.list[first[k] + (q >> 3) * deal + mine_of] + (q & 7); };
+                sweep(mine(total[0]), [&](int q) { return chunk_of(0, q); }, std::integral_constant<int, 0>{});
+                sweep(mine(total[1]), [&](int q) { return chunk_of(1, q); }, std::integral_constant<int, 1>{});
+                sweep(mine(total[2]), [&](int q) { return chunk_of(2, q); }, std::integral_constant<int, 2>{});
+                swept += (unsigned long long)(total[0] + total[1] + total[2]);
+            });
+        if (tid == 0 && (rank == 0 || !gs) && swept)
+            atomicAdd(P.c.eval_pairs, swept * 32ull * (unsigned long long)TILE);
     }
 
     // combine the NW warps in fixed order with a compensated FP32 sum (each
     // warp's Kahan pair (s, c) stands for s - c); FP64 comes later, once per
     // particle (FP64 runs at 1/64 of the FP32 rate here)
-    __syncthreads();
+    sync();
     for (int e = tid; e < TILE; e += NT) {
         float sx = 0.0f, cx = 0.0f, sy = 0.0f, cy = 0.0f;
 #pragma unroll
@@ -641,82 +751,372 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int tile, int 
         }
         s_red[e] = make_float4(sx, sy, cx, cy);
     }
-    __syncthreads();
+    sync();
 }
 
-// C q_i in FP64: the factor the FP32C sweeps leave out of their sums.
+// C q_i in FP64: the factor the sweeps leave out of their sums.
 __device__ __forceinline__ double pair_scale(const StageParams &P, int i) {
     return __dmul_rn(P.coulomb, P.c.q[i]);
 }
 
-// CL = true: the S ranks of a tile form a thread-block cluster, combine
-// through distributed shared memory and run the stage epilogue in the same
-// launch.  CL = false: plain blocks; each writes its partial sums to global
-// memory and stage_finish (below) completes the stage.
+// ---------------------------------------------------------------------------
+// The epilogue of a pass for one 32-particle group, by two warps.
+// ---------------------------------------------------------------------------
+
+struct EpilogueShared {
+    union {
+        struct {
+            float hi[2][2][32], lo[2][2][32];  // [set][axis][particle]
+        };
+        PositionTerms terms[2][32];  // [set][particle]
+    };
+};
+
+// What the epilogue needs to know of a particle's cloud (a batch holds many).
+struct EpilogueCloud {
+    const ForceParams &f;
+    float rc2_up;
+    bool live;  // the lane holds a particle
+    int group;  // its 32-particle group among the cloud's (batch's) boxes
+};
+
+// Starts bringing the operands of pass_epilogue for particle i, axis ax, into L1.
+__device__ __forceinline__ void epilogue_prefetch(const StageParams &P, int i, int ax) {
+    const CloudDev &c = P.c;
+    prefetch_l1((ax ? c.y : c.x) + i);
+    prefetch_l1((ax ? c.vy : c.vx) + i);
+    prefetch_l1(c.q + i);
+    prefetch_l1(c.m + i);
+    prefetch_l1(c.orig + i);
+    if (P.mode == kModeForceOnly) return;
+    if (P.pass == 0) {
+        prefetch_l1((ax ? c.py : c.px)[1] + i);
+    } else {
+        prefetch_l1((ax ? c.py : c.px)[2] + i);
+        prefetch_l1((ax ? c.py : c.px)[3] + i);
+        prefetch_l1(c.k1[ax] + i);
+        prefetch_l1(c.k2[ax] + i);
+        prefetch_l1(c.invm + i);
+    }
+}
+
+// 1/m of particle i: computed by a step's first pass, which leaves it for the second.
+__device__ __forceinline__ double pass_reciprocal(const StageParams &P, int i, double m, bool store) {
+    if (P.pass == 1) return P.c.invm[i];
+    const double inv = __drcp_rn(m);
+    if (store && P.order == 4) P.c.invm[i] = inv;
+    return inv;
+}
+
+// One axis of particle i's part of the pass, the total force at set e and
+// axis velocity v given by force(e, x, v): the new positions of both sets
+// (out[0], out[1]), stored but for their packed words; returns whether the
+// positions are finite.
+template <class Force>
+__device__ __forceinline__ bool advance_axis(const StageParams &P, int i, int ax, double inv, double (&out)[2],
+                                             Force force) {
+    const CloudDev &c = P.c;
+    double *X = ax ? c.y : c.x, *V = ax ? c.vy : c.vx;
+    double *const *p = ax ? c.py : c.px;
+    const double dt = stage_dt(P), m = c.m[i];
+    const double x = X[i], v = V[i];
+    auto increment = [&](double F) { return div_by(__dmul_rn(dt, F), m, inv); };
+    bool fine = true;
+    double k1, k2, v2;
+    if (P.pass == 0) {
+        const double x2 = p[1][i];
+        k1 = increment(force(0, x, v));
+        v2 = half_step(v, k1);
+        k2 = increment(force(1, x2, v2));
+        fine = isfinite(x2);
+    } else {
+        k1 = c.k1[ax][i];
+        k2 = c.k2[ax][i];
+        v2 = half_step(v, k1);
+    }
+    const double l2 = __dmul_rn(dt, v2);
+    if (P.order == 2) {  // x += l2, V += k2; the positions go to sets 2 and 3 (see adopt_sets)
+        const double vn = __dadd_rn(v, k2);
+        out[0] = __dadd_rn(x, l2);
+        out[1] = half_step(out[0], __dmul_rn(dt, vn));
+        V[i] = vn;
+        p[2][i] = out[0];
+        p[3][i] = out[1];
+        return fine && isfinite(out[0]);
+    }
+    const double v3 = half_step(v, k2), l3 = __dmul_rn(dt, v3);
+    if (P.pass == 0) {
+        c.k1[ax][i] = k1;
+        c.k2[ax][i] = k2;
+        out[0] = half_step(x, l2);
+        out[1] = __dadd_rn(x, l3);
+        p[2][i] = out[0];
+        p[3][i] = out[1];
+        return fine && isfinite(out[0]) && isfinite(out[1]);
+    }
+    const double k3 = increment(force(0, p[2][i], v3));
+    const double v4 = __dadd_rn(v, k3);
+    const double k4 = increment(force(1, p[3][i], v4));
+    const double xn = rk4_sum(x, __dmul_rn(dt, v), l2, l3, __dmul_rn(dt, v4));
+    const double vn = rk4_sum(v, k1, k2, k3, k4);
+    X[i] = xn;
+    V[i] = vn;
+    out[0] = xn;
+    out[1] = half_step(xn, __dmul_rn(dt, vn));  // the next step's x2, for the same dt
+    p[1][i] = out[1];
+    return isfinite(xn);
+}
+
+// The pass's epilogue for one 32-particle group: lane = particle i, `half` =
+// 0 or 1, the calling warp of the two (they meet at named barrier `bar`);
+// fs0, fs1 the pair forces (x, y) at the two sets, C q_i included.  Sums the
+// forces, advances the particles, writes the next pass's position sets and
+// their group boxes (force-only: the forces, in the caller's order).
+//
+// With the forces of kBasicForces each warp takes one axis (the epilogue is a
+// chain of dependent FP64 operations at 64 cycles each; two axes are two
+// chains).  The other forces couple the axes: the warps compute the terms of
+// the position sets, one each, and warp 0 advances both axes.
+__device__ __forceinline__ void pass_epilogue(const StageParams &P, const EpilogueCloud &E, int i, int half, int bar,
+                                              double2 fs0, double2 fs1, EpilogueShared &S) {
+    const int lane = threadIdx.x & 31;
+    const CloudDev &c = P.c;
+    const ForceParams &f = E.f;
+    const bool live = E.live;
+    const bool fo = P.mode == kModeForceOnly;
+    const bool basic = !(f.flags & ~kBasicForces);
+    auto meet = [&] { bar_sync(bar, 64); };
+    const int ob = (P.pass == 0) ? 2 : 0;  // first buffer written
+    if (basic) {
+        const int ax = half;
+        double out[2] = {0.0, 0.0};
+        if (live) {
+            const double q = c.q[i], m = c.m[i];
+            auto force = [&](int e, double x, double v) {
+                double therm = 0.0;
+                if (f.flags & kThermal) {
+                    const double2 t = stage_thermal(P, f, i, e);
+                    therm = ax ? t.y : t.x;
+                }
+                const double2 fp = e ? fs1 : fs0;
+                return axis_force(f, ax, x, v, q, m, ax ? fp.y : fp.x, therm);
+            };
+            if (fo) {
+                const int b = P.buf[0];
+                (ax ? P.fy_out : P.fx_out)[c.orig[i]] = force(0, (ax ? c.py : c.px)[b][i], (ax ? c.vy : c.vx)[i]);
+            } else if (!advance_axis(P, i, ax, pass_reciprocal(P, i, m, ax == 0), out, force)) {
+                atomicOr(c.err, 1);
+            }
+        }
+        if (fo) return;  // uniform over the launch
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            float h = 0.0f, lo = 0.0f;
+            if (live) split2(out[e], h, lo);
+            S.hi[e][ax][lane] = h;
+            S.lo[e][ax][lane] = lo;
+        }
+        meet();
+        // write_stage_position's packed words and the group's box, one set per warp
+        const int e = half;
+        const float xh = S.hi[e][0][lane], yh = S.hi[e][1][lane];
+        if (live) {
+            c.pa[ob + e][i] = make_float4(xh, yh, fmaf(yh, yh, xh * xh), c.pa[P.buf[0]][i].w);
+            c.pb[ob + e][i] = make_float4(S.lo[e][0][lane], S.lo[e][1][lane], -filter_threshold(xh, yh, E.rc2_up), 0.0f);
+        }
+        store_group_box(c.gbox[ob + e] + E.group, live, xh, yh, true);
+        return;
+    }
+    // the terms of set `half`
+    if (live && (half == 0 || P.nsets > 1)) {
+        const int b = P.buf[half];
+        S.terms[half][lane] = position_terms(f, c.px[b][i], c.py[b][i], c.q[i],
+                                             (f.flags & kDriving) ? stage_time(P, half) : 0.0);
+    }
+    meet();
+    if (half != 0) return;
+    const double q = live ? c.q[i] : 0.0, m = live ? c.m[i] : 1.0;
+    if (fo) {
+        if (live) {
+            const int b = P.buf[0];
+            const ParticleAt s{c.px[b][i], c.py[b][i], c.vx[i], c.vy[i], q, m};
+            double Fx, Fy;
+            total_force(P, f, i, 0, s, S.terms[0][lane], fs0.x, fs0.y, Fx, Fy);
+            P.fx_out[c.orig[i]] = Fx;
+            P.fy_out[c.orig[i]] = Fy;
+        }
+        return;
+    }
+    float h[2][2] = {};
+    if (live) {
+        // the axes in step: stage by stage, both components
+        const double dt = stage_dt(P), inv = pass_reciprocal(P, i, m, true);
+        const double x = c.x[i], y = c.y[i], vx = c.vx[i], vy = c.vy[i];
+        const int b1 = P.buf[1], b0 = P.buf[0];
+        auto increments = [&](int e, double vxs, double vys, double &kx, double &ky) {
+            const int b = e ? b1 : b0;
+            const double2 fp = e ? fs1 : fs0;
+            const ParticleAt s{c.px[b][i], c.py[b][i], vxs, vys, q, m};
+            double Fx, Fy;
+            total_force(P, f, i, e, s, S.terms[e][lane], fp.x, fp.y, Fx, Fy);
+            kx = div_by(__dmul_rn(dt, Fx), m, inv);
+            ky = div_by(__dmul_rn(dt, Fy), m, inv);
+        };
+        double k1x, k1y, k2x, k2y, n0x, n0y, n1x, n1y;
+        if (P.pass == 0) {
+            increments(0, vx, vy, k1x, k1y);
+            increments(1, half_step(vx, k1x), half_step(vy, k1y), k2x, k2y);
+        } else {
+            k1x = c.k1[0][i]; k1y = c.k1[1][i];
+            k2x = c.k2[0][i]; k2y = c.k2[1][i];
+        }
+        const double l2x = __dmul_rn(dt, half_step(vx, k1x)), l2y = __dmul_rn(dt, half_step(vy, k1y));
+        double vnx = vx, vny = vy;
+        bool fine = true;
+        if (P.order == 2) {
+            n0x = __dadd_rn(x, l2x);
+            n0y = __dadd_rn(y, l2y);
+            vnx = __dadd_rn(vx, k2x);
+            vny = __dadd_rn(vy, k2y);
+            fine = isfinite(c.px[1][i]) && isfinite(c.py[1][i]);
+        } else {
+            const double v3x = half_step(vx, k2x), v3y = half_step(vy, k2y);
+            const double l3x = __dmul_rn(dt, v3x), l3y = __dmul_rn(dt, v3y);
+            if (P.pass == 0) {
+                c.k1[0][i] = k1x; c.k1[1][i] = k1y;
+                c.k2[0][i] = k2x; c.k2[1][i] = k2y;
+                n0x = half_step(x, l2x);
+                n0y = half_step(y, l2y);
+                n1x = __dadd_rn(x, l3x);
+                n1y = __dadd_rn(y, l3y);
+                fine = isfinite(c.px[1][i]) && isfinite(c.py[1][i]) && isfinite(n1x) && isfinite(n1y);
+            } else {
+                double k3x, k3y, k4x, k4y;
+                increments(0, v3x, v3y, k3x, k3y);
+                const double v4x = __dadd_rn(vx, k3x), v4y = __dadd_rn(vy, k3y);
+                increments(1, v4x, v4y, k4x, k4y);
+                n0x = rk4_sum(x, __dmul_rn(dt, vx), l2x, l3x, __dmul_rn(dt, v4x));
+                n0y = rk4_sum(y, __dmul_rn(dt, vy), l2y, l3y, __dmul_rn(dt, v4y));
+                vnx = rk4_sum(vx, k1x, k2x, k3x, k4x);
+                vny = rk4_sum(vy, k1y, k2y, k3y, k4y);
+            }
+        }
+        if (P.order == 2 || P.pass == 1) {  // the step ends (set 0 is the state: x, y)
+            c.vx[i] = vnx;
+            c.vy[i] = vny;
+            n1x = half_step(n0x, __dmul_rn(dt, vnx));
+            n1y = half_step(n0y, __dmul_rn(dt, vny));
+        }
+        write_stage_position(c, ob, i, n0x, n0y, E.rc2_up);
+        write_stage_position(c, ob + 1, i, n1x, n1y, E.rc2_up);
+        if (!(fine && isfinite(n0x) && isfinite(n0y))) atomicOr(c.err, 1);
+        h[0][0] = __double2float_rn(n0x);
+        h[0][1] = __double2float_rn(n0y);
+        h[1][0] = __double2float_rn(n1x);
+        h[1][1] = __double2float_rn(n1y);
+    }
+#pragma unroll
+    for (int e = 0; e < 2; e++) store_group_box(c.gbox[ob + e] + E.group, live, h[e][0], h[e][1], true);
+}
+
+// ---------------------------------------------------------------------------
+// FP32C pair kernel.
+//
+// CL = true: a block holds NW warps per position set of the launch, the S
+// ranks of a tile form a thread-block cluster, combine through distributed
+// shared memory and run the epilogue in the same launch.  CL = false: plain
+// blocks of NW warps for one set; each writes its partial sums to global
+// memory and stage_finish (below) completes the pass.
 // Occupancy: with two i slots per lane the kernel is bounded to 64
 // registers, so 32 warps per SM are resident (more latency hidden in the
 // sparse phases, where a block is short and bound by dependent loads and
 // barriers); four slots need more registers and stay at 24 warps.
+// ---------------------------------------------------------------------------
 template <int NW, int ILP>
 constexpr int fp32c_min_blocks() {
     return (ILP <= 2 ? 32 : 24) / NW > 0 ? (ILP <= 2 ? 32 : 24) / NW : 1;
 }
 
+// The epilogue of a tile: pairs of warps of the first block take its groups
+// in turn, adding the S ranks' sums (s_red of each set, `stride` float4 apart)
+// in order.  The first pair is the tile's number modulo the pairs: warp w
+// issues on scheduler w mod 4, and each scheduler has an FP64 unit of its own.
+template <int ILP>
+__device__ __forceinline__ void tile_epilogue(const StageParams &P, float4 *s_red, int stride, int tile, int S,
+                                              EpilogueShared *shared) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int npairs = blockDim.x >> 6, pair = ((warp >> 1) + tile) % npairs;
+    const bool both = (P.f.flags & ~kBasicForces) != 0;  // else a warp needs its own axis only
+#pragma unroll 1
+    for (int g = pair; g < ILP; g += npairs) {
+        const int e = g * 32 + lane, i = tile * 32 * ILP + e;
+        double2 f[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+        const double cq = (i < P.c.n) ? pair_scale(P, i) : 0.0;
+        for (int set = 0; set < P.nsets; set++) {
+            float4 *mine = s_red + set * stride + e;
+            float4 v = *mine;
+            TwoFloatSum sx, sy;
+            sx.add(v.x);
+            sy.add(v.y);
+            float cx = v.z, cy = v.w;
+            for (int r = 1; r < S; r++) {
+                v = *cg::this_cluster().map_shared_rank(mine, r);
+                sx.add(v.x);
+                sy.add(v.y);
+                cx += v.z;
+                cy += v.w;
+            }
+            if (both || (warp & 1) == 0) f[set].x = __dmul_rn(cq, widen(sx.hi) + widen(sx.lo - cx));
+            if (both || (warp & 1) == 1) f[set].y = __dmul_rn(cq, widen(sy.hi) + widen(sy.lo - cy));
+        }
+        pass_epilogue(P, EpilogueCloud{P.f, P.c.rc2_up, i < P.c.n, i >> 5}, i, warp & 1, kBarEpilogue + (warp >> 1), f[0],
+                      f[1], shared[g]);
+    }
+}
+
 template <int NW, int ILP, int TC, bool CL, bool CULL = false>
-__global__ void __launch_bounds__(NW * 32, fp32c_min_blocks<NW, ILP>())
+__global__ void __launch_bounds__((CL ? 2 : 1) * NW * 32, fp32c_min_blocks<(CL ? 2 : 1) * NW, ILP>())
     pair_stage_fp32c(const StageParams P) {
     pdl_wait();
     constexpr int TILE = 32 * ILP;
+    constexpr int kBytes = (int)Fp32cSmem<NW, ILP, TC>::bytes;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int S = CL ? (int)cg::this_cluster().num_blocks() : P.split;
-    const int rank = CL ? (int)cg::this_cluster().block_rank() : (int)(blockIdx.x % P.split);
-    const int tile = blockIdx.x / S;
-    const int tid = threadIdx.x;
-    const int n = P.c.n, n_pad = P.c.n_pad;
-    fp32c_sweep<NW, ILP, TC, CULL>(P, tile, rank, S, smem_raw);
     float4 *s_red = reinterpret_cast<float4 *>(smem_raw) + Fp32cSmem<NW, ILP, TC>::red_offset;
+    const int n = P.c.n, n_pad = P.c.n_pad;
     if constexpr (!CL) {
+        const int S = P.split, r = (int)(blockIdx.x % (S * P.nsets)), set = r / S, rank = r % S;
+        const int tile = blockIdx.x / (S * P.nsets), tid = threadIdx.x;
+        fp32c_sweep<NW, ILP, TC, CULL>(P, P.buf[set], tile, rank, S, tid, [] { __syncthreads(); }, smem_raw);
         for (int e = tid; e < TILE; e += NW * 32)
             if (tile * TILE + e < n) {
                 const float4 v = s_red[e];
-                P.partial[(size_t)(2 * rank) * n_pad + tile * TILE + e] = make_float2(v.x, v.z);
-                P.partial[(size_t)(2 * rank + 1) * n_pad + tile * TILE + e] = make_float2(v.y, v.w);
+                P.partial[(size_t)(2 * r) * n_pad + tile * TILE + e] = make_float2(v.x, v.z);
+                P.partial[(size_t)(2 * r + 1) * n_pad + tile * TILE + e] = make_float2(v.y, v.w);
             }
     } else {
-        // finalise particles [rank*fchunk, (rank+1)*fchunk) of the tile in
-        // whole warps: an FP64 warp instruction costs the same with 1 or 32
-        // active lanes, so the FP64 epilogue runs on as few warps as possible
-        cg::cluster_group cl = cg::this_cluster();
-        const int fchunk = max(32, (TILE + S - 1) / S);
-        cl.sync();
-        if (tid < fchunk) {
-            const int e = rank * fchunk + tid;
-            if (e < TILE && tile * TILE + e < n) {
-                const int i = tile * TILE + e;
-                double fx = 0.0, fy = 0.0;
-                for (int r = 0; r < S; r++) {
-                    const float4 v = *cl.map_shared_rank(s_red + e, r);
-                    fx += (double)v.x - (double)v.z;
-                    fy += (double)v.y - (double)v.w;
-                }
-                const double cq = pair_scale(P, i);
-                stage_epilogue(P, i, __dmul_rn(cq, fx), __dmul_rn(cq, fy), stage_thermal(P, i));
-            }
-        }
-        stage_step_advance(P);
-        cl.sync();
+        static_assert(sizeof(EpilogueShared) * ILP <= Fp32cSmem<NW, ILP, TC>::tile, "epilogue over the j tile");
+        const int S = (int)cg::this_cluster().num_blocks(), rank = (int)cg::this_cluster().block_rank();
+        const int tile = blockIdx.x / S, set = threadIdx.x / (NW * 32), tid = threadIdx.x % (NW * 32);
+        fp32c_sweep<NW, ILP, TC, CULL>(P, P.buf[set], tile, rank, S, tid, [&] { bar_sync(kBarSet + set, NW * 32); },
+                                       smem_raw + set * kBytes);
+        if (S > 1) cg::this_cluster().sync();
+        else __syncthreads();
+        if (rank == 0)
+            tile_epilogue<ILP>(P, s_red, kBytes / 16, tile, S, reinterpret_cast<EpilogueShared *>(smem_raw));
+        pass_step_advance(P);
+        if (S > 1) cg::this_cluster().sync();  // the other blocks' sums stay readable until here
     }
 }
 
 // Sum over the j split's ranks, in rank order, of one axis's partials
-// (s, c) of particle i (each stands for s - c): the s exactly as an
+// (s, c) of particle i at set e (each stands for s - c): the s exactly as an
 // unevaluated float pair (TwoSum), the small c plainly, FP64 once -- FP64
 // runs at ~1/64 of the FP32 rate here and an FP64 sum over the ranks
 // dominated the finish.  Times C q_i (left out of the sweeps), in FP64.
-__device__ __forceinline__ double finish_rank_sum(const StageParams &P, int i, int axis) {
+__device__ __forceinline__ double finish_rank_sum(const StageParams &P, int i, int e, int axis) {
     TwoFloatSum sa;
     float ca = 0.0f;
-    const float2 *p = P.partial + (size_t)axis * P.c.n_pad + i;
+    const float2 *p = P.partial + (size_t)(2 * e * P.split + axis) * P.c.n_pad + i;
     const size_t stride = 2 * (size_t)P.c.n_pad;
     int r = 0;
     for (; r + 16 <= P.split; r += 16) {  // 16 loads in flight, summed in rank order
@@ -746,243 +1146,107 @@ __device__ __forceinline__ double finish_rank_sum(const StageParams &P, int i, i
     }
     // the two small corrections combined in FP32 (their rounding is ~2^-24
     // of ~2^-24 of the sum): two FP64 operations fewer per particle and axis
-    return __dmul_rn(pair_scale(P, i), (double)sa.hi + (double)(sa.lo - ca));
+    return __dmul_rn(pair_scale(P, i), widen(sa.hi) + widen(sa.lo - ca));
 }
 
-// The box of a 32-particle group from its lanes' FP32 positions; lane 0
-// stores it.
-__device__ __forceinline__ void store_group_box(float4 *gbox, bool live, float xh, float yh, bool store) {
-    float x0 = live ? xh : INFINITY, y0 = live ? yh : INFINITY;
-    float x1 = live ? xh : -INFINITY, y1 = live ? yh : -INFINITY;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
-        y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
-        x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-        y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
-    }
-    if ((threadIdx.x & 31) == 0 && store) *gbox = make_float4(x0, y0, x1, y1);
-}
-
-// Completes a stage after a non-cluster pair launch when forces outside
-// kBasicForces are on (they couple the axes): one particle per thread, the
-// rank sums of both axes, then the stage epilogue.
-static __global__ void __launch_bounds__(64) stage_finish(const StageParams P) {
+// Completes a pass after a non-cluster pair launch: one block per
+// 32-particle group, warp w < 2 nsets sums set w/2, axis w%2 over the ranks,
+// then the first two warps run the epilogue.
+static __global__ void __launch_bounds__(128) stage_finish(const StageParams P) {
     pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ EpilogueShared S;
+    __shared__ double s_f[2][2][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
     if (i < P.c.n) {
-        const double fx = finish_rank_sum(P, i, 0);
-        const double fy = finish_rank_sum(P, i, 1);
-        stage_epilogue(P, i, fx, fy, stage_thermal(P, i));
+        if (warp < 2) epilogue_prefetch(P, i, warp);  // the operands' round trip overlaps the partials'
+        if (warp < 2 * P.nsets) s_f[warp >> 1][warp & 1][lane] = finish_rank_sum(P, i, warp >> 1, warp & 1);
     }
-    if (P.box_out) {  // a warp is one 32-particle group: its box in the buffer just written
-        const int bw = P.stage & 1;
-        const bool live = i < P.c.n;
-        const float4 A = live ? P.c.pa[bw][i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        store_group_box(P.c.gbox[bw] + (i >> 5), live, A.x, A.y, i < P.c.n_pad);
-    }
-    stage_step_advance(P);
-}
-
-// Starts bringing the operands of axes_epilogue for particle i, axis ax, into L1.
-__device__ __forceinline__ void axes_prefetch(const StageParams &P, int i, int ax) {
-    const CloudDev &c = P.c;
-    const bool fo = P.mode == kModeForceOnly;
-    const int s = fo ? 1 : P.stage;
-    const int b = fo ? P.fo_buf : (s - 1) & 1;
-    prefetch_l1((ax ? c.py[b] : c.px[b]) + i);
-    prefetch_l1(((s == 1) ? (ax ? c.vy : c.vx) : (ax ? c.vyc : c.vxc)) + i);
-    prefetch_l1(c.q + i);
-    prefetch_l1(c.m + i);
-    prefetch_l1(c.orig + i);
-    if (!fo) {
-        prefetch_l1((ax ? c.y : c.x) + i);
-        prefetch_l1((ax ? c.vy : c.vx) + i);
-        if (s >= 3) {
-            prefetch_l1(c.a23[2 * ax] + i);
-            prefetch_l1(c.a23[2 * ax + 1] + i);
-        }
-        if (s == 4) {
-            prefetch_l1(c.a1[2 * ax] + i);
-            prefetch_l1(c.a1[2 * ax + 1] + i);
-        }
-    }
-}
-
-struct AxesShared {
-    float hi[2][32], lo[2][32];
-};
-
-// The stage epilogue with one thread per particle and axis, for the forces in
-// kBasicForces: called by the first two warps of a block for one 32-particle
-// group, warp 0 the x and warp 1 the y components, fpa being the axis's pair
-// force.  Each axis runs exactly the operations stage_epilogue runs for it, in
-// the same order, so the results are the same bits; the epilogue is a
-// latency-bound chain and this gives it twice the warps.  The two warps meet
-// once, in shared memory (barrier 1, 64 threads), for what needs both axes:
-// the next stage's packed positions, filter bound and group box.
-__device__ __forceinline__ void axes_epilogue(const StageParams &P, int i, int ax, double fpa, AxesShared &S) {
-    const int lane = threadIdx.x & 31;
-    const CloudDev &c = P.c;
-    const bool live = i < c.n;
-    const bool fo = P.mode == kModeForceOnly;
-    const int s = fo ? 1 : P.stage;
-    const int b = fo ? P.fo_buf : (s - 1) & 1;
-    double na = 0.0;  // this axis's coordinate at the next stage
-    if (live) {
-        const double *pos = ax ? c.py[b] : c.px[b];
-        const double *vel = (s == 1) ? (ax ? c.vy : c.vx) : (ax ? c.vyc : c.vxc);
-        double *X = ax ? c.y : c.x;
-        double *V = ax ? c.vy : c.vx;
-        const double xs = pos[i], vs = vel[i], q = c.q[i], m = c.m[i];
-        const long long fl = P.f.flags;
-        double F = 0.0;
-        if (fl & kConfinement) F = __dadd_rn(F, __dmul_rn(__dmul_rn(q, P.f.confine), xs));
-        if (fl & kDrag) F = __dadd_rn(F, __dmul_rn(__dmul_rn(m, -P.f.gamma), vs));
-        if (fl & kRectConfinement)
-            F = __dadd_rn(F, __dmul_rn(__dmul_rn(q, ax ? P.f.confine_y : P.f.confine_x), xs));
-        if (fl & kShieldedCoulomb) F = __dadd_rn(F, fpa);
-        if (fl & kThermal) {
-            const double2 t = stage_thermal(P, i);
-            F = __dadd_rn(F, ax ? t.y : t.x);
-        }
-        if (fo) {
-            (ax ? P.fy_out : P.fx_out)[c.orig[i]] = F;
-        } else {
-            const double dt = stage_dt(P);
-            const double k = __ddiv_rn(__dmul_rn(dt, F), m);
-            const double l = __dmul_rn(dt, vs);
-            const double x = X[i], v = V[i];
-            const bool last = (s == P.order);
-            double nv = 0.0;
-            if (last && s == 2) {  // Runge_Kutta2: x += l2, V += k2
-                na = __dadd_rn(x, l);
-                V[i] = __dadd_rn(v, k);
-                X[i] = na;
-            } else if (s == 1 || s == 2) {
-                double *const *acc = (s == 1) ? c.a1 : c.a23;
-                acc[2 * ax][i] = k;
-                acc[2 * ax + 1][i] = l;
-                na = __dadd_rn(__dmul_rn(0.5, l), x);
-                nv = __dadd_rn(__dmul_rn(0.5, k), v);
-            } else if (s == 3) {
-                c.a23[2 * ax][i] = __dadd_rn(c.a23[2 * ax][i], k);
-                c.a23[2 * ax + 1][i] = __dadd_rn(c.a23[2 * ax + 1][i], l);
-                na = __dadd_rn(x, l);
-                nv = __dadd_rn(v, k);
-            } else {
-                const double dv =
-                    __ddiv_rn(__dadd_rn(c.a1[2 * ax][i], __dadd_rn(__dmul_rn(c.a23[2 * ax][i], 2.0), k)), 6.0);
-                const double d =
-                    __ddiv_rn(__dadd_rn(c.a1[2 * ax + 1][i], __dadd_rn(__dmul_rn(c.a23[2 * ax + 1][i], 2.0), l)), 6.0);
-                na = __dadd_rn(x, d);
-                V[i] = __dadd_rn(v, dv);
-                X[i] = na;
-            }
-            (ax ? c.py : c.px)[b ^ 1][i] = na;
-            if (!last) (ax ? c.vyc : c.vxc)[i] = nv;
-            if (!isfinite(na)) atomicOr(c.err, 1);
-        }
-    }
-    if (fo) return;  // uniform over the launch
-    float h = 0.0f, lo = 0.0f;
-    if (live) split2(na, h, lo);
-    S.hi[ax][lane] = h;
-    S.lo[ax][lane] = lo;
-    asm volatile("bar.sync 1, 64;" ::: "memory");
-    const int bw = b ^ 1;
-    const float xh = S.hi[0][lane], yh = S.hi[1][lane];
-    if (live) {  // write_stage_position's packed words, one float4 per warp
-        const double q = c.q[i];
-        if (ax == 0)
-            c.pa[bw][i] = make_float4(xh, yh, fmaf(yh, yh, xh * xh), __double2float_rn(q));
-        else
-            c.pb[bw][i] = make_float4(S.lo[0][lane], S.lo[1][lane], -filter_threshold(xh, yh, c.rc2), 0.0f);
-    }
-    // the group's box in the buffer just written
-    if (P.box_out && ax == 0) store_group_box(c.gbox[bw] + (i >> 5), live, xh, yh, (i & ~31) < c.n_pad);
-}
-
-// Completes a stage after a non-cluster pair launch, for the forces in
-// kBasicForces: one block of two warps per 32-particle group.
-static __global__ void __launch_bounds__(64) stage_finish_axes(const StageParams P) {
-    pdl_wait();
-    __shared__ AxesShared S;
-    const int ax = threadIdx.x >> 5;
-    const int i = blockIdx.x * 32 + (threadIdx.x & 31);
-    double fpa = 0.0;
-    if (i < P.c.n) {
-        axes_prefetch(P, i, ax);  // the operands' round trip overlaps the partials'
-        fpa = finish_rank_sum(P, i, ax);
-    }
-    axes_epilogue(P, i, ax, fpa, S);
-    stage_step_advance(P);
+    __syncthreads();
+    if (warp < 2)
+        pass_epilogue(P, EpilogueCloud{P.f, P.c.rc2_up, i < P.c.n, i >> 5}, i, warp, kBarEpilogue, make_double2(s_f[0][0][lane], s_f[0][1][lane]),
+                      make_double2(s_f[1][0][lane], s_f[1][1][lane]), S);
+    pass_step_advance(P);
 }
 
 // ---------------------------------------------------------------------------
-// FP64 kernel: one 32-particle group of i per tile, S blocks of NW warps per
-// tile (a cluster); the j groups (CULL: those whose box is within reach of
-// the tile's) are dealt one by one to the S*NW warps, each of which filters
-// its groups in FP32 and evaluates the hits in FP64 with full warps (dm_fp64.cuh).
-// The sums meet in the cluster's first block, which runs the stage epilogue.
+// FP64 kernel: one 32-particle group of i per tile, S blocks per tile (a
+// cluster), each with NW warps per position set; the j groups (CULL: those
+// whose box is within reach of the tile's) are dealt one by one to the S*NW
+// warps of a set, each of which filters its groups in FP32 and evaluates the
+// hits in FP64 with full warps (dm_fp64.cuh).  The sums meet in the cluster's
+// first block, which runs the epilogue.
 //
 // Bound by the FP64 pipe on dense clouds (26 FP64 instructions per pair in
-// reach, 16 cycles each per 32 pairs), by latency on sparse ones.
+// reach, 64 cycles of a scheduler's FP64 unit per 32 pairs each), by latency
+// on sparse ones.
 // ---------------------------------------------------------------------------
-constexpr int kGroupList = 1024;  // j groups tested per pass of the box test
-
 template <int NW>
-struct Group64Smem {
-    HitWarp<2> w[NW];
-    double tab[kExp2Size];
+struct Group64Set {  // one position set's half of the block
+    HitWarp<HitResult<2>> w[NW];
     double ix[32], iy[32];
     double2 acc[NW][32];
     double2 red[32];
-    AxesShared axes;
-    int list[kGroupList];
-    int wcount[NW];
+    NearLists<NW, 1> near;
+};
+template <int NW>
+struct Group64Smem {
+    Group64Set<NW> set[2];
+    double tab[kExp2Size];
+    EpilogueShared epi;
 };
 
 template <int NW, bool CULL>
-__global__ void __launch_bounds__(NW * 32, 20 / NW) pair_group_fp64(const StageParams P) {
+__global__ void __launch_bounds__(2 * NW * 32, 10 / NW) pair_group_fp64(const StageParams P) {
     pdl_wait();
     constexpr int NT = NW * 32;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    Group64Smem<NW> &sm = *reinterpret_cast<Group64Smem<NW> *>(smem_raw);
+    Group64Smem<NW> &sh = *reinterpret_cast<Group64Smem<NW> *>(smem_raw);
     cg::cluster_group cl = cg::this_cluster();
     const int S = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const int tile = blockIdx.x / S;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int set = threadIdx.x / NT, tid = threadIdx.x % NT, lane = tid & 31, warp = tid >> 5;
+    Group64Set<NW> &sm = sh.set[set];
     const int n = P.c.n;
     const int i = tile * 32 + lane;
-    const int b = (P.mode == kModeForceOnly) ? P.fo_buf : (P.stage - 1) & 1;
+    const int b = P.buf[set];
     const double *__restrict__ px = P.c.px[b];
     const double *__restrict__ py = P.c.py[b];
     const double *__restrict__ qa = P.c.q;
     const float4 *__restrict__ pa = P.c.pa[b];
     const Yukawa64 K = P.y64;
     const bool coul = (P.f.flags & kShieldedCoulomb) != 0;
-    if (rank == 0 && warp < 2 && i < n) axes_prefetch(P, i, warp);
+    // the warps that run the epilogue: see tile_epilogue
+    const int npairs = blockDim.x >> 6, wib = threadIdx.x >> 5;
+    const bool mine = rank == 0 && ((wib >> 1) + tile) % npairs == 0;
     double sum[2] = {0.0, 0.0};
     if (coul) {
-        float px2 = 0.0f, py2 = 0.0f, nu = INFINITY;
+        // every load of the prologue in flight at once
+        float4 A = make_float4(0.0f, 0.0f, 0.0f, 0.0f), B = make_float4(0.0f, 0.0f, INFINITY, 0.0f);
+        double xi = 0.0, yi = 0.0, tab[kExp2Size / NT];
         if (i < n) {
-            const float4 A = pa[i];
-            px2 = 2.0f * A.x;
-            py2 = 2.0f * A.y;
-            nu = P.c.pb[b][i].z;
-            if (warp == 0) {
-                sm.ix[lane] = px[i];
-                sm.iy[lane] = py[i];
-            }
+            A = pa[i];
+            B = P.c.pb[b][i];
+            xi = px[i];
+            yi = py[i];
+            if (mine) epilogue_prefetch(P, i, wib & 1);
         }
-        for (int k = tid; k < kExp2Size; k += NT) sm.tab[k] = g_exp2_table.v[k];
+        if (set == 0)
+#pragma unroll
+            for (int k = 0; k < kExp2Size / NT; k++) tab[k] = g_exp2_table.v[k * NT + tid];
+        if (warp == 0) {
+            sm.ix[lane] = xi;
+            sm.iy[lane] = yi;
+        }
+        if (set == 0)
+#pragma unroll
+            for (int k = 0; k < kExp2Size / NT; k++) sh.tab[k * NT + tid] = tab[k];
+        const float px2 = 2.0f * A.x, py2 = 2.0f * A.y, nu = B.z;
         __syncthreads();
-        HitWarp<2> &W = sm.w[warp];
-        const double *tab = sm.tab;
+        HitWarp<HitResult<2>> &W = sm.w[warp];
         auto eval = [&](int il, int j) {
             const double dx = __dsub_rn(sm.ix[il], px[j]), dy = __dsub_rn(sm.iy[il], py[j]);
-            const double w = pair_w64(dx, dy, qa[j], K, tab);
+            const double w = pair_w64(dx, dy, qa[j], K, sh.tab);
             return HitResult<2>{__dmul_rn(w, dx), __dmul_rn(w, dy)};
         };
         int nk = 0, hits = 0;
@@ -1003,31 +1267,15 @@ __global__ void __launch_bounds__(NW * 32, 20 / NW) pair_group_fp64(const StageP
         const int ngroups = (n + 31) >> 5;
         const int NS = NW * S, me = warp * S + rank;
         if constexpr (CULL) {
-            const float4 *__restrict__ gb = P.c.gbox[b];
-            const float4 tb = gb[tile];
+            const float4 tb = P.c.gbox[b][tile];
             int found = 0;
-            for (int g0 = 0; g0 < ngroups; g0 += kGroupList) {
-                // the groups of this pass within reach, in order
-                int total = 0;
-                for (int t0 = g0; t0 < min(ngroups, g0 + kGroupList); t0 += NT) {
-                    const int g = t0 + tid;
-                    const bool near = g < ngroups && boxes_near(tb, gb[g], P.rc2_hi);
-                    const uint32_t bal = __ballot_sync(0xffffffffu, near);
-                    if (lane == 0) sm.wcount[warp] = __popc(bal);
-                    __syncthreads();
-                    int off = total;
-#pragma unroll
-                    for (int w = 0; w < NW; w++) {
-                        off += (w < warp) ? sm.wcount[w] : 0;
-                        total += sm.wcount[w];
-                    }
-                    if (near) sm.list[off + __popc(bal & ((1u << lane) - 1u))] = g;
-                    __syncthreads();
-                }
-                for (int e = (me + NS - found % NS) % NS; e < total; e += NS) group(sm.list[e]);
-                found += total;
-                __syncthreads();  // the list is rewritten
-            }
+            for_near_groups(
+                sm.near, P.c.gbox[b], P.c.gsuper[b], ngroups, 0, 1, tb, P.rc2_hi, tid,
+                [&] { bar_sync(kBarSet + set, NT); }, [](int, const float4 &) { return 0; },
+                [&](const int (&)[1], const int (&total)[1]) {
+                    for (int e = (me + NS - found % NS) % NS; e < total[0]; e += NS) group(sm.near.list[e]);
+                    found += total[0];
+                });
             if (tid == 0 && rank == 0) atomicAdd(P.c.eval_pairs, 1024ull * (unsigned long long)found);
         } else {
             for (int g = me; g < ngroups; g += NS) group(g);
@@ -1036,37 +1284,38 @@ __global__ void __launch_bounds__(NW * 32, 20 / NW) pair_group_fp64(const StageP
         hit_flush(W, nk, sum, eval);
     }
     sm.acc[warp][lane] = make_double2(sum[0], sum[1]);
-    __syncthreads();
-    if (warp == 0) {
-        double fx = 0.0, fy = 0.0;
+    if (S > 1) {  // each block's sums, for the first block to read
+        bar_sync(kBarSet + set, NT);
+        if (warp == 0) {
+            double2 t = sm.acc[0][lane];
 #pragma unroll
-        for (int w = 0; w < NW; w++) {
-            fx = __dadd_rn(fx, sm.acc[w][lane].x);
-            fy = __dadd_rn(fy, sm.acc[w][lane].y);
+            for (int w = 1; w < NW; w++) t = make_double2(__dadd_rn(t.x, sm.acc[w][lane].x), __dadd_rn(t.y, sm.acc[w][lane].y));
+            sm.red[lane] = t;
         }
-        sm.red[lane] = make_double2(fx, fy);
+        cl.sync();
+    } else {
+        __syncthreads();
     }
-    if (S > 1) cl.sync();
-    else __syncthreads();
-    if (rank == 0 && warp < 2) {
-        double2 f = sm.red[lane];
-        for (int r = 1; r < S; r++) {
-            const double2 v = *cl.map_shared_rank(&sm.red[lane], r);
-            f.x = __dadd_rn(f.x, v.x);
-            f.y = __dadd_rn(f.y, v.y);
-        }
+    if (mine) {
+        const bool basic = !(P.f.flags & ~kBasicForces);
+        const int ax = wib & 1;
         const double cq = (i < n) ? __dmul_rn(P.coulomb, qa[i]) : 0.0;
-        if (!(P.f.flags & ~kBasicForces)) {
-            axes_epilogue(P, i, warp, __dmul_rn(cq, warp ? f.y : f.x), sm.axes);
-        } else if (warp == 0) {
-            if (i < n) stage_epilogue(P, i, __dmul_rn(cq, f.x), __dmul_rn(cq, f.y), stage_thermal(P, i));
-            if (P.box_out) {
-                const float4 A = (i < n) ? P.c.pa[b ^ 1][i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                store_group_box(P.c.gbox[b ^ 1] + tile, i < n, A.x, A.y, true);
+        double2 f[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+        for (int e = 0; e < P.nsets; e++) {
+            // one axis per warp where the axes are independent
+            double2 t = make_double2(0.0, 0.0);
+            const int terms = (S > 1) ? S : NW;
+            for (int k = 0; k < terms; k++) {
+                const double2 v = (S > 1) ? *cl.map_shared_rank(&sh.set[e].red[lane], k) : sh.set[e].acc[k][lane];
+                if (!basic || ax == 0) t.x = __dadd_rn(t.x, v.x);
+                if (!basic || ax == 1) t.y = __dadd_rn(t.y, v.y);
             }
+            if (!basic || ax == 0) f[e].x = __dmul_rn(cq, t.x);
+            if (!basic || ax == 1) f[e].y = __dmul_rn(cq, t.y);
         }
+        pass_epilogue(P, EpilogueCloud{P.f, P.c.rc2_up, i < n, tile}, i, ax, kBarEpilogue, f[0], f[1], sh.epi);
     }
-    stage_step_advance(P);
+    pass_step_advance(P);
     if (S > 1) cl.sync();  // the other blocks' sums stay readable until here
 }
 

@@ -360,13 +360,14 @@ __device__ __forceinline__ void moments_f32_merge(float *v, const float *o) {
     v[8] = fmaxf(v[8], o[8]);
 }
 
-// pa0: the FP32 hi parts of the current positions (stage buffer 0 holds them
+// pa0: the FP32 hi parts of the current positions (position set 0 holds them
 // at every step boundary).  The cloud's x, y, vx, vy, q, m and orig end up in
-// the new order, with stage buffer 0 and the group boxes rewritten.
+// the new order, with position set 0, set 1 for time step dt (if mid) and
+// their group boxes rewritten.
 // Launched as one cluster of CTAS blocks.
 template <int CTAS>
 static __global__ void __launch_bounds__(kSortClusterThreads, 1)
-    sort_cluster(const float4 *__restrict__ pa0, CloudDev c, SortScratch z) {
+    sort_cluster(const float4 *__restrict__ pa0, CloudDev c, SortScratch z, double dt, bool mid) {
     constexpr int kSortClusterCtas = CTAS;
     constexpr int kSortClusterPer = SortClusterShape<CTAS>::per;
     constexpr int kSortClusterRounds = SortClusterShape<CTAS>::rounds;
@@ -566,43 +567,34 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
     // Every block of the cluster holds its sources in registers, and the
     // cluster barrier orders those loads before any block's stores.  The
     // cluster covers every slot of the cloud, so the cloud's arrays are
-    // rewritten in place in the new order, with stage buffer 0 (the first
-    // stage's inputs), the padding slots and the 32-particle group boxes.
+    // rewritten in place in the new order, with position sets 0 and 1 (the
+    // next pass's inputs), the padding slots and the 32-particle group boxes.
     cl.sync();
 #pragma unroll
     for (int k = 0; k < kSortClusterRounds; k++) {
         const int s = e0 + k * kSortClusterThreads + tid;  // a warp holds 32 consecutive slots
-        float x0 = INFINITY, y0 = INFINITY, x1 = -INFINITY, y1 = -INFINITY;
+        float2 h[2] = {};
         if (s < n) {
             const double x = val[0][k], y = val[1][k];
-            c.x[s] = x;
-            c.y[s] = y;
             c.vx[s] = val[2][k];
             c.vy[s] = val[3][k];
             c.q[s] = val[4][k];
             c.m[s] = val[5][k];
             c.orig[s] = ov[k];
-            write_stage_position(c, 0, s, x, y);
-            x0 = x1 = __double2float_rn(x);  // the hi parts write_stage_position stored
-            y0 = y1 = __double2float_rn(y);
-        } else if (s < c.n_pad) {
-            for (int b = 0; b < 2; b++) {
-                c.px[b][s] = (double)kPadPosition;
-                c.py[b][s] = (double)kPadPosition;
-                c.pa[b][s] = make_float4(kPadPosition, kPadPosition, kPadPosition * kPadPosition, 0.0f);
-                c.pb[b][s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            write_stage_position(c, 0, s, x, y);  // set 0 is the state: x, y
+            h[0] = make_float2(__double2float_rn(x), __double2float_rn(y));
+            if (mid) {
+                write_midpoint(c, s, x, y, val[2][k], val[3][k], dt);
+                const float4 A = c.pa[1][s];
+                h[1] = make_float2(A.x, A.y);
             }
+        } else if (s < c.n_pad) {
+            write_padding(c, s);
             c.q[s] = 0.0;
             c.m[s] = 1.0;
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
-            y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
-            x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-            y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
-        }
-        if (lane == 0 && s < c.n_pad) c.gbox[0][s >> 5] = make_float4(x0, y0, x1, y1);
+        store_group_box(c.gbox[0] + (s >> 5), s < n, h[0].x, h[0].y, (s & ~31) < c.n_pad);
+        if (mid) store_group_box(c.gbox[1] + (s >> 5), s < n, h[1].x, h[1].y, (s & ~31) < c.n_pad);
     }
 }
 
@@ -636,33 +628,24 @@ static __global__ void permute_commit(CloudDev c, SortScratch z) {
 }
 
 // An upload in the caller's order (staging arrays 0..3: x, y, vx, vy) put
-// straight into the cloud's current internal order, with stage buffer 0 and
+// straight into the cloud's current internal order, with position set 0 and
 // the boxes of its 32-particle groups: charges, masses and the order itself
 // stay where they are (the next re-sort starts from them).
 static __global__ void upload_internal_order(CloudDev c, SortScratch z) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= c.n_pad) return;  // whole warps: n_pad is a multiple of 64
-    float x0 = INFINITY, y0 = INFINITY, x1 = -INFINITY, y1 = -INFINITY;
+    float xh = 0.0f, yh = 0.0f;
     if (s < c.n) {
         const int o = c.orig[s];
         const double x = z.stage[0][o], y = z.stage[1][o];
-        c.x[s] = x;
-        c.y[s] = y;
         c.vx[s] = z.stage[2][o];
         c.vy[s] = z.stage[3][o];
-        write_stage_position(c, 0, s, x, y);
+        write_stage_position(c, 0, s, x, y);  // set 0 is the state: x, y
         const float4 A = c.pa[0][s];
-        x0 = x1 = A.x;
-        y0 = y1 = A.y;
+        xh = A.x;
+        yh = A.y;
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, off));
-        y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, off));
-        x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, off));
-        y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, off));
-    }
-    if ((threadIdx.x & 31) == 0) c.gbox[0][s >> 5] = make_float4(x0, y0, x1, y1);
+    store_group_box(c.gbox[0] + (s >> 5), s < c.n, xh, yh, true);
 }
 
 static __global__ void set_identity(int *orig, int n) {
