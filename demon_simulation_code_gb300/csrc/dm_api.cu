@@ -538,7 +538,7 @@ int launch_variant(dm_cloud *c, int vi, int S, StageParams P) {
 }
 
 int tune_precision(dm_cloud *c, int precision);
-int reorder(dm_cloud *c, double dt = 0.0, bool mid = false);
+int reorder(dm_cloud *c, double dt = 0.0, bool mid = false, bool force = true);
 
 int ensure_tuned(dm_cloud *c, int precision) {
     const int rc = ensure_kernel_attrs(c->ctx);
@@ -703,7 +703,8 @@ int tune_precision(dm_cloud *c, int precision) {
 
 // Puts the cloud in Morton order (dm_sort.cuh); graph-capturable.  mid: the
 // next step's time step is dt (the small clouds' sort leaves its midpoint too).
-int reorder(dm_cloud *c, double dt, bool mid) {
+// Without `force` a small cloud whose order is still good stays as it is.
+int reorder(dm_cloud *c, double dt, bool mid, bool force) {
     dm_ctx *ctx = c->ctx;
     cudaStream_t s = ctx->stream;
     const int n = c->n;
@@ -715,12 +716,14 @@ int reorder(dm_cloud *c, double dt, bool mid) {
         if (rc) return rc;
         cudaLaunchAttribute attr[2];
         const float4 *pa0 = c->d.pa[0];
+        const bool mid_ready = c->mid_valid && c->mid_dt == dt && c->boxes_valid[1];
+        force = force || !c->boxes_valid[0];
         if (ctx->sort_ctas == 16) {
             const cudaLaunchConfig_t cfg = sort_cluster_cfg<16>(s, attr);
-            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<16>, pa0, c->d, z, dt, mid));
+            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<16>, pa0, c->d, z, dt, mid, mid_ready, force));
         } else {
             const cudaLaunchConfig_t cfg = sort_cluster_cfg<8>(s, attr);
-            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<8>, pa0, c->d, z, dt, mid));
+            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<8>, pa0, c->d, z, dt, mid, mid_ready, force));
         }
         c->state_changed(true);
         c->boxes_valid[1] = c->mid_valid = mid;
@@ -757,7 +760,8 @@ int reorder(dm_cloud *c, double dt, bool mid) {
 int reorder_if_due(dm_cloud *c, int precision, double dt, bool mid) {
     if (!wants_order(c->n, precision)) return DM_OK;
     if (c->order_dirty || (c->reorder_interval > 0 && c->host_steps % (unsigned)c->reorder_interval == 0))
-        return reorder(c, dt, mid);
+        return reorder(c, dt, mid,
+                       c->order_dirty || c->reorder_interval != 1 || c->host_steps % (unsigned)kOrderKeep == 0);
     return DM_OK;
 }
 
@@ -1070,7 +1074,7 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     c->sort.orig_stage = takeI();
     for (int k = 0; k < 6; k++) c->sort.stage[k] = takeD();
     c->sort.hist = (uint32_t *)p; p += nh;
-    c->sort.box = (double *)p; p += 256;
+    c->sort.box = (double *)p; c->sort.cost = (float *)(p + 64); p += 256;
     c->sort.moments = (double *)p; p += align256(sizeof(double) * kMomentBlocks * kMomentFields);
     c->d_diag = (double *)p; p += align256(sizeof(double) * 5 * (kDiagBlocks + 1));
     cudaStream_t s = ctx->stream;
@@ -1637,8 +1641,8 @@ int batch_launch_pass(dm_batch *B, int pass, int mode, double dt, int buf = 0, i
     return DM_OK;
 }
 
-// Puts every cloud in Morton order; mid: as reorder's.
-int batch_reorder(dm_batch *B, double dt = 0.0, bool mid = false) {
+// Puts every cloud in Morton order; mid, force: as reorder's.
+int batch_reorder(dm_batch *B, double dt = 0.0, bool mid = false, bool force = true) {
     dm_ctx *ctx = B->ctx;
     cudaStream_t s = ctx->stream;
     const int n = B->total;
@@ -1648,7 +1652,8 @@ int batch_reorder(dm_batch *B, double dt = 0.0, bool mid = false) {
         DM_CUDA(ctx, cudaFuncSetAttribute(batch_sort_clouds, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)kBatchSortSmem));
         DM_CUDA(ctx, launch_pdl(batch_sort_clouds, dim3(B->nclouds), dim3(kBatchSortThreads), kBatchSortSmem, s,
-                                B->d, (const BatchCloud *)B->ddesc, B->dbox, dt, mid));
+                                B->d, (const BatchCloud *)B->ddesc, B->dbox, dt, mid,
+                                B->mid_valid && B->mid_dt == dt && B->boxes_valid[1], force || !B->boxes_valid[0]));
         ctx->launches++;
         B->boxes_valid[0] = true;
         B->boxes_valid[1] = B->mid_valid = mid;
@@ -1683,7 +1688,9 @@ int batch_enqueue_steps(dm_batch *B, int nsteps, double dt) {
     dm_ctx *ctx = B->ctx;
     for (int s = 0; s < nsteps; s++) {
         if (B->order_dirty || (B->reorder_interval > 0 && B->host_steps % (unsigned)B->reorder_interval == 0)) {
-            int rc = batch_reorder(B, dt, true);
+            int rc = batch_reorder(B, dt, true,
+                                   B->order_dirty || B->reorder_interval != 1 ||
+                                       B->host_steps % (unsigned)kOrderKeep == 0);
             if (rc) return rc;
         }
         if (!B->mid_valid || B->mid_dt != dt) {

@@ -199,10 +199,14 @@ struct BatchSortSmem {
 };
 constexpr size_t kBatchSortSmem = sizeof(BatchSortSmem);
 
-// box_out[8 * cloud]: key box x0, y0, extent, 0, bounding box min x, min y,
-// max x, max y (as batch_boxes writes them; the batch autotuner reads it).
+// box_out[8 * cloud]: key box x0, y0, extent, order_cost of the sorted cloud,
+// bounding box min x, min y, max x, max y (as batch_boxes writes them; the
+// batch autotuner reads it).  Without `force` a cloud in good order (see
+// kOrderKeep) is left as it is; if `mid` and not `mid_ready` its set 1 is
+// written.
 static __global__ void __launch_bounds__(kBatchSortThreads, 1)
-    batch_sort_clouds(CloudDev c, const BatchCloud *__restrict__ desc, double *box_out, double dt, bool mid) {
+    batch_sort_clouds(CloudDev c, const BatchCloud *__restrict__ desc, double *box_out, double dt, bool mid,
+                      bool mid_ready, bool force) {
     pdl_wait();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     BatchSortSmem &S = *reinterpret_cast<BatchSortSmem *>(smem_raw);
@@ -210,6 +214,23 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
     const BatchCloud d = desc[blockIdx.x];
     const int off = d.off, n = d.n;
     const float4 *__restrict__ pa0 = c.pa[0] + off;
+    const float rc = sqrtf(d.rc2_up);
+
+    if (!force) {
+        const float now = (tid < (n + 31) / 32) ? order_cost(c.gbox[0][d.goff + tid], rc) : 0.0f;
+        const float was = (lane == 0) ? (float)box_out[8 * blockIdx.x + 3] : 0.0f;
+        if (block_order_kept<kBatchSortWarps>(now, was, S.wmom)) {
+            if (mid && !mid_ready) {
+                CloudDev v = c;
+                v.rc2_up = d.rc2_up;
+                for (int k = 0; k < kBatchSortRounds; k++) {
+                    const int li = k * kBatchSortThreads + tid;
+                    write_midpoint_group(v, off + li, li < n, c.gbox[1] + d.goff + (li >> 5), (li & ~31) < n, dt);
+                }
+            }
+            return;
+        }
+    }
 
     float4 pos[kBatchSortRounds];
 #pragma unroll
@@ -256,7 +277,6 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
             bo[0] = S.box[0];
             bo[1] = S.box[1];
             bo[2] = S.box[2];
-            bo[3] = 0.0;
             for (int k = 0; k < 4; k++) bo[4 + k] = (v[0] > 0.0f) ? (double)v[5 + k] : 0.0;
         }
         __syncthreads();
@@ -363,6 +383,7 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
     __syncthreads();  // every source is in registers: the cloud is rewritten in place
     CloudDev v = c;
     v.rc2_up = d.rc2_up;
+    float cost = 0.0f;
 #pragma unroll
     for (int k = 0; k < kBatchSortRounds; k++) {
         const int li = k * kBatchSortThreads + tid, s = off + li;  // a warp holds 32 consecutive slots
@@ -381,8 +402,16 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
                 h[1] = make_float2(A.x, A.y);
             }
         }
-        store_group_box(c.gbox[0] + d.goff + (li >> 5), li < n, h[0].x, h[0].y, (li & ~31) < n);
+        const float4 box =
+            store_group_box(c.gbox[0] + d.goff + (li >> 5), li < n, h[0].x, h[0].y, (li & ~31) < n);
         if (mid) store_group_box(c.gbox[1] + d.goff + (li >> 5), li < n, h[1].x, h[1].y, (li & ~31) < n);
+        cost += order_cost(box, rc);
+    }
+    if (lane == 0) S.wmom[warp][0] = cost;
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < kBatchSortWarps; w++) cost += S.wmom[w][0];
+        box_out[8 * blockIdx.x + 3] = cost;
     }
 }
 

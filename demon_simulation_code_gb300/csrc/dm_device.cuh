@@ -399,8 +399,8 @@ __device__ __forceinline__ void write_midpoint(const CloudDev &c, int i, double 
 }
 
 // The box of a 32-particle group from its lanes' FP32 positions; lane 0
-// stores it.
-__device__ __forceinline__ void store_group_box(float4 *gbox, bool live, float xh, float yh, bool store) {
+// stores it, every lane returns it.
+__device__ __forceinline__ float4 store_group_box(float4 *gbox, bool live, float xh, float yh, bool store) {
     float x0 = live ? xh : INFINITY, y0 = live ? yh : INFINITY;
     float x1 = live ? xh : -INFINITY, y1 = live ? yh : -INFINITY;
 #pragma unroll
@@ -411,6 +411,7 @@ __device__ __forceinline__ void store_group_box(float4 *gbox, bool live, float x
         y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
     }
     if ((threadIdx.x & 31) == 0 && store) *gbox = make_float4(x0, y0, x1, y1);
+    return make_float4(x0, y0, x1, y1);
 }
 
 // A padding particle in every position set.

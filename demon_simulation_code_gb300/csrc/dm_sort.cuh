@@ -36,12 +36,31 @@ constexpr int kSortBits = 24;
 constexpr int kSortDigitBits = 8;  // 24-bit keys: 3 passes
 constexpr int kSortBuckets = 1 << kSortDigitBits;
 
+// A one-launch sort that is due but not required (same trajectory since a sort
+// or an upload, at most kOrderKeep steps ago) leaves a cloud alone whose order
+// is still good: the area within the cutoff of its 32-particle groups' boxes,
+// which decides how many groups a tile of the sweep has to filter, has grown
+// by less than kOrderSlack since the sort.  The check costs 3 us of a 22-26 us
+// sort (one cluster, latency bound): 4095 particles, 10 RK2 steps 594 -> 437
+// us, 16,384 and 4 RK4 steps 415 -> 345 us, 3 steps through a focus 1396 ->
+// 1358 us, 256 clouds and 16 steps 12.94 -> 12.6 ms.  A required sort at least
+// every kOrderKeep steps, so that a cloud that shrinks while its order decays
+// is put right too.
+constexpr int kOrderKeep = 8;
+constexpr float kOrderSlack = 1.1f;
+
+// A group's share of that area: its box grown by half a cutoff on each side.
+__device__ __forceinline__ float order_cost(const float4 &b, float rc) {
+    return (b.z >= b.x) ? (b.z - b.x + rc) * (b.w - b.y + rc) : 0.0f;
+}
+
 constexpr int kMomentBlocks = 64;  // fixed partition of the moment reduction
 constexpr int kMomentFields = 9;   // count, sum dx, sum dy, sum dx^2, sum dy^2, min x, min y, max x, max y
 
 struct SortScratch {
     double *moments;           // [kMomentBlocks][kMomentFields] per-block partials
     double *box;               // [8]: key box x0, y0, extent; -; bounding box min x, min y, max x, max y
+    float *cost;               // [16]: order_cost of the last one-launch sort, per block
     uint32_t *keys[2];
     int *vals[2];
     uint32_t *hist;            // [kSortBuckets * nblocks]
@@ -360,14 +379,45 @@ __device__ __forceinline__ void moments_f32_merge(float *v, const float *o) {
     v[8] = fmaxf(v[8], o[8]);
 }
 
+// Whether the block's threads' costs `now` together stay within kOrderSlack of
+// the warp's lanes' `was` (the same in every warp).  Every thread of the block;
+// scratch: a row per warp.
+template <int WARPS, int FIELDS>
+__device__ __forceinline__ bool block_order_kept(float now, float was, float (&scratch)[WARPS][FIELDS]) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        now += __shfl_xor_sync(0xffffffffu, now, o);
+        was += __shfl_xor_sync(0xffffffffu, was, o);
+    }
+    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5][0] = now;
+    __syncthreads();
+    float sum = 0.0f;
+    for (int w = 0; w < WARPS; w++) sum += scratch[w][0];
+    __syncthreads();  // scratch is reused
+    return sum <= kOrderSlack * was;  // false for NaN
+}
+
+// Position set 1 (see write_midpoint) of slot s and its group's box; whole warps.
+__device__ __forceinline__ void write_midpoint_group(const CloudDev &c, int s, bool live, float4 *gbox, bool store,
+                                                     double dt) {
+    float4 A = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (live) {
+        write_midpoint(c, s, c.x[s], c.y[s], c.vx[s], c.vy[s], dt);
+        A = c.pa[1][s];
+    }
+    store_group_box(gbox, live, A.x, A.y, store);
+}
+
 // pa0: the FP32 hi parts of the current positions (position set 0 holds them
 // at every step boundary).  The cloud's x, y, vx, vy, q, m and orig end up in
 // the new order, with position set 0, set 1 for time step dt (if mid) and
-// their group boxes rewritten.
-// Launched as one cluster of CTAS blocks.
+// their group boxes rewritten.  Without `force` a cloud in good order (see
+// kOrderKeep) is left as it is; if `mid` and not `mid_ready` its set 1 is
+// written.  Launched as one cluster of CTAS blocks.
 template <int CTAS>
 static __global__ void __launch_bounds__(kSortClusterThreads, 1)
-    sort_cluster(const float4 *__restrict__ pa0, CloudDev c, SortScratch z, double dt, bool mid) {
+    sort_cluster(const float4 *__restrict__ pa0, CloudDev c, SortScratch z, double dt, bool mid, bool mid_ready,
+                 bool force) {
     constexpr int kSortClusterCtas = CTAS;
     constexpr int kSortClusterPer = SortClusterShape<CTAS>::per;
     constexpr int kSortClusterRounds = SortClusterShape<CTAS>::rounds;
@@ -379,6 +429,21 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = c.n;
     const int e0 = r * kSortClusterPer;
+    const float rc = sqrtf(c.rc2_up);
+
+    if (!force) {  // every block comes to the same decision, from the same sums
+        float now = 0.0f;
+        for (int g = tid; g < (n + 31) / 32; g += kSortClusterThreads) now += order_cost(c.gbox[0][g], rc);
+        float was = (lane < kSortClusterCtas) ? z.cost[lane] : 0.0f;
+        if (block_order_kept<kSortClusterWarps>(now, was, S.wmom)) {
+            if (mid && !mid_ready)
+                for (int k = 0; k < kSortClusterRounds; k++) {
+                    const int s = e0 + k * kSortClusterThreads + tid;
+                    write_midpoint_group(c, s, s < n, c.gbox[1] + (s >> 5), (s & ~31) < c.n_pad, dt);
+                }
+            return;
+        }
+    }
 
     // this block's positions, loaded once (moments, then keys)
     float4 pos[kSortClusterRounds];
@@ -570,6 +635,7 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
     // rewritten in place in the new order, with position sets 0 and 1 (the
     // next pass's inputs), the padding slots and the 32-particle group boxes.
     cl.sync();
+    float cost = 0.0f;
 #pragma unroll
     for (int k = 0; k < kSortClusterRounds; k++) {
         const int s = e0 + k * kSortClusterThreads + tid;  // a warp holds 32 consecutive slots
@@ -593,8 +659,16 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
             c.q[s] = 0.0;
             c.m[s] = 1.0;
         }
-        store_group_box(c.gbox[0] + (s >> 5), s < n, h[0].x, h[0].y, (s & ~31) < c.n_pad);
+        const float4 box = store_group_box(c.gbox[0] + (s >> 5), s < n, h[0].x, h[0].y, (s & ~31) < c.n_pad);
         if (mid) store_group_box(c.gbox[1] + (s >> 5), s < n, h[1].x, h[1].y, (s & ~31) < c.n_pad);
+        cost += order_cost(box, rc);
+    }
+    if (lane == 0) S.wmom[warp][0] = cost;
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < kSortClusterWarps; w++) cost += S.wmom[w][0];
+        z.cost[r] = cost;
+        if (r + kSortClusterCtas < 16) z.cost[r + kSortClusterCtas] = 0.0f;
     }
 }
 

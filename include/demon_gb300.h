@@ -263,7 +263,9 @@ int dm_cloud_set_kernel(dm_cloud *cloud, const char *variant, int split);
  * array crossing this ABI is in the caller's order).  The cloud is re-sorted
  * every `steps` RK4 steps (0 = only after an upload; otherwise a power of
  * two <= 16).  Default: every step (clouds of up to 16384 particles are
- * sorted by one thread-block cluster in one launch).  No reference
+ * sorted by one thread-block cluster in one launch, which seven steps of
+ * eight first looks whether the order is still good and then leaves it).
+ * FP64 steps of up to 4096 particles run on the caller's order.  No reference
  * counterpart. */
 int dm_cloud_set_reorder_interval(dm_cloud *cloud, int steps);
 
