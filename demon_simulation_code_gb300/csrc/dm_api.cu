@@ -701,9 +701,31 @@ int tune_precision(dm_cloud *c, int precision) {
     return DM_OK;
 }
 
+// The radix passes over `bits` of z.keys[0] / z.vals[0] (`first`: the first
+// digit's histogram is there); *cur: the buffer that holds the result.
+int radix_passes(dm_ctx *ctx, const SortScratch &z, int n, int nblocks, int bits, bool first, const int *keep,
+                 int *cur) {
+    cudaStream_t s = ctx->stream;
+    *cur = 0;
+    for (int shift = 0; shift < bits; shift += kSortDigitBits) {
+        if (shift > 0 || !first) {
+            DM_CUDA(ctx, launch_pdl(radix_hist, dim3(nblocks), dim3(kSortThreads), 0, s,
+                                    (const uint32_t *)z.keys[*cur], n, shift, z.hist, keep));
+            ctx->launches++;
+        }
+        DM_CUDA(ctx, launch_pdl(radix_scan, dim3(kSortBuckets), dim3(256), 0, s, z.hist, nblocks, keep));
+        DM_CUDA(ctx, launch_pdl(radix_scatter, dim3(nblocks), dim3(kSortThreads), 0, s,
+                                (const uint32_t *)z.keys[*cur], (const int *)z.vals[*cur], z.keys[*cur ^ 1],
+                                z.vals[*cur ^ 1], n, shift, (const uint32_t *)z.hist, keep));
+        ctx->launches += 2;
+        *cur ^= 1;
+    }
+    return DM_OK;
+}
+
 // Puts the cloud in Morton order (dm_sort.cuh); graph-capturable.  mid: the
-// next step's time step is dt (the small clouds' sort leaves its midpoint too).
-// Without `force` a small cloud whose order is still good stays as it is.
+// next step's time step is dt: the sort leaves its midpoint too.  Without
+// `force` a cloud whose order is still good stays as it is.
 int reorder(dm_cloud *c, double dt, bool mid, bool force) {
     dm_ctx *ctx = c->ctx;
     cudaStream_t s = ctx->stream;
@@ -732,26 +754,26 @@ int reorder(dm_cloud *c, double dt, bool mid, bool force) {
         ctx->launches += 1;
         c->order_dirty = false;
         return DM_OK;
-    } else {
-        const int mblocks = std::min(grid, kMomentBlocks);
-        sort_moments<<<mblocks, 256, 0, s>>>(c->d.x, c->d.y, n, z.moments);
-        sort_box<<<1, 32, 0, s>>>(z.moments, mblocks, c->d.x, c->d.y, z.box);
-        sort_keys<<<grid, 256, 0, s>>>(c->d.x, c->d.y, n, z.box, z.keys[0], z.vals[0]);
-        for (int shift = 0; shift < kSortBits; shift += kSortDigitBits) {
-            radix_hist<<<c->sort_blocks, kSortThreads, 0, s>>>(z.keys[cur], n, shift, z.hist);
-            radix_scan<<<1, 1024, 0, s>>>(z.hist, kSortBuckets * c->sort_blocks);
-            radix_scatter<<<c->sort_blocks, kSortThreads, 0, s>>>(z.keys[cur], z.vals[cur], z.keys[cur ^ 1],
-                                                                   z.vals[cur ^ 1], n, shift, z.hist);
-            cur ^= 1;
-        }
-        ctx->launches += 3 + 3 * (kSortBits / kSortDigitBits);
     }
-    permute_gather<<<grid, 256, 0, s>>>(c->d, z.vals[cur], z);
-    permute_commit<<<grid, 256, 0, s>>>(c->d, z);
-    init_positions<<<(c->n_pad + 255) / 256, 256, 0, s>>>(c->d);
-    c->state_changed(false);
-    DM_CUDA(ctx, cudaGetLastError());
-    ctx->launches += 3;
+    const int nb = c->sort_blocks, cblocks = (c->n_pad + 255) / 256;
+    const int mblocks = std::min(nb, kMomentBlocks);
+    const float4 *pa0 = c->d.pa[0];
+    const bool mid_ready = c->mid_valid && c->mid_dt == dt && c->boxes_valid[1];
+    const int *keep = (force || !c->boxes_valid[0]) ? nullptr : z.keep;
+    if (keep) {
+        DM_CUDA(ctx, launch_pdl(order_check, dim3(1), dim3(1024), 0, s, c->d, z, cblocks));
+        ctx->launches++;
+    }
+    DM_CUDA(ctx, launch_pdl(sort_moments, dim3(mblocks), dim3(256), 0, s, pa0, n, z.moments, keep));
+    DM_CUDA(ctx, launch_pdl(sort_keys, dim3(nb), dim3(kSortThreads), 0, s, pa0, n, mblocks, z, keep));
+    int rc = radix_passes(ctx, z, n, nb, kSortBits, true, keep, &cur);
+    if (rc) return rc;
+    DM_CUDA(ctx, launch_pdl(permute_gather, dim3(grid), dim3(256), 0, s, c->d, (const int *)z.vals[cur], z, keep));
+    DM_CUDA(ctx, launch_pdl(permute_commit, dim3(cblocks), dim3(256), 0, s, c->d, z, dt, mid, mid_ready, keep));
+    c->state_changed(true);
+    c->boxes_valid[1] = c->mid_valid = mid;
+    c->mid_dt = dt;
+    ctx->launches += 4;
     c->order_dirty = false;
     return DM_OK;
 }
@@ -796,7 +818,7 @@ int run_steps(dm_cloud *c, int nsteps, double dt, int precision) {
     // the re-sort that begins them): make it so, outside the capture
     int rc0 = ensure_tuned(c, precision);
     if (rc0) return rc0;
-    const bool sorts = wants_order(c->n, precision) && c->reorder_interval > 0 && c->n <= kSmallSortMax;
+    const bool sorts = wants_order(c->n, precision) && c->reorder_interval > 0;
     if (!sorts && !(c->mid_valid && c->mid_dt == dt)) {
         rc0 = enqueue_steps(c, 1, dt, precision);
         if (rc0) return rc0;
@@ -1028,12 +1050,13 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     const size_t nf4 = align256((size_t)c->n_pad * sizeof(float4));
     const size_t ni = align256((size_t)c->n_pad * sizeof(int));
     c->sort_blocks = (n + kSortPerBlock - 1) / kSortPerBlock;
-    const size_t nh = align256((size_t)kSortBuckets * c->sort_blocks * sizeof(uint32_t));
+    const size_t nh = align256((size_t)kSortBuckets * (c->sort_blocks + 1) * sizeof(uint32_t));
+    const size_t nco = align256((size_t)((c->n_pad + 255) / 256 + 16) * sizeof(float));
     const size_t ngb = align256((size_t)(c->n_pad / 32) * sizeof(float4));
     const size_t nsp = align256((size_t)(c->n_pad / 1024 + 1) * sizeof(float4));
-    const size_t total = nd * (6 + 5 + 6 + 2 + 6) + nf4 * 8 + (ngb + nsp) * 4 + ni * 6 + nh + 1024 + 512 +
+    const size_t total = nd * (6 + 5 + 6 + 2 + 6) + nf4 * 8 + (ngb + nsp) * 4 + ni * 6 + nh + nco + 1024 + 512 +
                          align256(sizeof(double) * 5 * (kDiagBlocks + 1)) +
-                         align256(sizeof(double) * kMomentBlocks * kMomentFields);
+                         align256(sizeof(float) * kMomentBlocks * kMomentFields);
     cudaError_t e = cudaMalloc(&c->block, total);
     if (e != cudaSuccess) {
         delete c;
@@ -1074,8 +1097,9 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     c->sort.orig_stage = takeI();
     for (int k = 0; k < 6; k++) c->sort.stage[k] = takeD();
     c->sort.hist = (uint32_t *)p; p += nh;
-    c->sort.box = (double *)p; c->sort.cost = (float *)(p + 64); p += 256;
-    c->sort.moments = (double *)p; p += align256(sizeof(double) * kMomentBlocks * kMomentFields);
+    c->sort.box = (double *)p; c->sort.keep = (int *)(p + 64); p += 256;
+    c->sort.cost = (float *)p; p += nco;
+    c->sort.moments = (float *)p; p += align256(sizeof(float) * kMomentBlocks * kMomentFields);
     c->d_diag = (double *)p; p += align256(sizeof(double) * 5 * (kDiagBlocks + 1));
     cudaStream_t s = ctx->stream;
     const size_t bytes = (size_t)n * sizeof(double);
@@ -1663,22 +1687,16 @@ int batch_reorder(dm_batch *B, double dt = 0.0, bool mid = false, bool force = t
     }
     batch_boxes<<<B->nclouds, 256, 0, s>>>(B->d.x, B->d.y, B->ddesc, B->dbox);
     batch_keys<<<grid, 256, 0, s>>>(B->d.x, B->d.y, n, B->dseg, B->dbox, B->mbits, z.keys[0], z.vals[0]);
-    int cur = 0;
-    int passes = 0;
     const int bits = B->mbits + 32 - __builtin_clz((unsigned)std::max(B->nclouds - 1, 1));
-    for (int shift = 0; shift < bits; shift += kSortDigitBits) {
-        radix_hist<<<B->sort_blocks, kSortThreads, 0, s>>>(z.keys[cur], n, shift, z.hist);
-        radix_scan<<<1, 1024, 0, s>>>(z.hist, kSortBuckets * B->sort_blocks);
-        radix_scatter<<<B->sort_blocks, kSortThreads, 0, s>>>(z.keys[cur], z.vals[cur], z.keys[cur ^ 1],
-                                                               z.vals[cur ^ 1], n, shift, z.hist);
-        cur ^= 1;
-        passes++;
-    }
-    permute_gather<<<grid, 256, 0, s>>>(B->d, z.vals[cur], z);
-    permute_commit<<<grid, 256, 0, s>>>(B->d, z);
-    batch_init_positions<<<(B->total_pad + 255) / 256, 256, 0, s>>>(B->d, B->ddesc, B->dseg);
     DM_CUDA(ctx, cudaGetLastError());
-    ctx->launches += 5 + 3 * passes;
+    int cur = 0;
+    int rc = radix_passes(ctx, z, n, B->sort_blocks, bits, false, nullptr, &cur);
+    if (rc) return rc;
+    DM_CUDA(ctx, launch_pdl(permute_gather, dim3(grid), dim3(256), 0, s, B->d, (const int *)z.vals[cur], z,
+                            (const int *)nullptr));
+    DM_CUDA(ctx, launch_pdl(batch_commit, dim3((B->total_pad + 255) / 256), dim3(256), 0, s, B->d,
+                            (const BatchCloud *)B->ddesc, (const int *)B->dseg, z));
+    ctx->launches += 4;
     B->boxes_valid[0] = B->boxes_valid[1] = B->mid_valid = false;
     B->order_dirty = false;
     return DM_OK;
@@ -1825,7 +1843,7 @@ int dm_batch_create(dm_ctx *ctx, int nclouds, const int *n, const double *x, con
     const size_t nf4 = align256((size_t)np * sizeof(float4));
     const size_t ni = align256((size_t)np * sizeof(int));
     B->sort_blocks = (B->total + kSortPerBlock - 1) / kSortPerBlock;
-    const size_t nh = align256((size_t)kSortBuckets * B->sort_blocks * sizeof(uint32_t));
+    const size_t nh = align256((size_t)kSortBuckets * (B->sort_blocks + 1) * sizeof(uint32_t));
     const size_t ndesc = align256((size_t)nclouds * sizeof(BatchCloud));
     const size_t nbb = align256((size_t)nclouds * 8 * sizeof(double));
     const size_t bytes_total = nd * (6 + 5 + 6 + 2 + 6) + nf4 * 8 + ni * 7 + nh + ndesc + nbb + 1024;

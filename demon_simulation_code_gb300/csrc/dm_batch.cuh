@@ -218,7 +218,7 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
 
     if (!force) {
         const float now = (tid < (n + 31) / 32) ? order_cost(c.gbox[0][d.goff + tid], rc) : 0.0f;
-        const float was = (lane == 0) ? (float)box_out[8 * blockIdx.x + 3] : 0.0f;
+        const float was = (tid == 0) ? (float)box_out[8 * blockIdx.x + 3] : 0.0f;
         if (block_order_kept<kBatchSortWarps>(now, was, S.wmom)) {
             if (mid && !mid_ready) {
                 CloudDev v = c;
@@ -244,35 +244,9 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
         float v[kMomentFields] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, INFINITY, INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int k = 0; k < kBatchSortRounds; k++) moments_f32_add(v, pos[k], ox, oy);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            float w[kMomentFields];
-#pragma unroll
-            for (int k = 0; k < kMomentFields; k++) w[k] = __shfl_xor_sync(0xffffffffu, v[k], o);
-            moments_f32_merge(v, w);
-        }
-        if (lane == 0)
-            for (int k = 0; k < kMomentFields; k++) S.wmom[warp][k] = v[k];
-        __syncthreads();
+        moments_f32_block<kBatchSortWarps>(v, S.wmom);
         if (tid == 0) {
-            for (int w = 1; w < kBatchSortWarps; w++) moments_f32_merge(v, S.wmom[w]);
-            float lo[2] = {0.0f, 0.0f}, hi[2] = {0.0f, 0.0f};
-            if (v[0] > 0.0f) {
-                const float org[2] = {ox, oy};
-                for (int a = 0; a < 2; a++) {
-                    const float mean = v[1 + a] / v[0];
-                    const float sd = sqrtf(fmaxf(v[3 + a] / v[0] - mean * mean, 0.0f));
-                    lo[a] = fmaxf(v[5 + a], org[a] + mean - 4.0f * sd);
-                    hi[a] = fminf(v[7 + a], org[a] + mean + 4.0f * sd);
-                    if (!(lo[a] <= hi[a])) {
-                        lo[a] = v[5 + a];
-                        hi[a] = v[7 + a];
-                    }
-                }
-            }
-            S.box[0] = lo[0];
-            S.box[1] = lo[1];
-            S.box[2] = fmaxf(hi[0] - lo[0], hi[1] - lo[1]);
+            key_box_f32(v, ox, oy, S.box);
             double *bo = box_out + 8 * blockIdx.x;
             bo[0] = S.box[0];
             bo[1] = S.box[1];
@@ -281,22 +255,11 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
         }
         __syncthreads();
     }
-    {
-        const float x0 = S.box[0], y0 = S.box[1], ext = S.box[2];
-        const float scale = (ext > 0.0f && isfinite(ext)) ? 4095.0f / ext : 0.0f;
 #pragma unroll
-        for (int k = 0; k < kBatchSortRounds; k++) {
-            const int li = k * kBatchSortThreads + tid;
-            uint32_t key = 0u;
-            if (li < n) {
-                const float fx = (pos[k].x - x0) * scale, fy = (pos[k].y - y0) * scale;
-                const uint32_t qx = (fx > 0.0f) ? (uint32_t)fminf(fx, 4095.0f) : 0u;  // NaN: 0
-                const uint32_t qy = (fy > 0.0f) ? (uint32_t)fminf(fy, 4095.0f) : 0u;
-                key = spread_bits12(qx) | (spread_bits12(qy) << 1);
-            }
-            S.keys[0][li] = key;
-            S.slot[0][li] = (uint16_t)li;
-        }
+    for (int k = 0; k < kBatchSortRounds; k++) {
+        const int li = k * kBatchSortThreads + tid;
+        S.keys[0][li] = (li < n) ? morton_key_f32(pos[k].x, pos[k].y, S.box) : 0u;
+        S.slot[0][li] = (uint16_t)li;
     }
     __syncthreads();
 
@@ -432,6 +395,26 @@ static __global__ void batch_tune_compress(CloudDev c, const BatchCloud *__restr
     CloudDev v = c;
     v.rc2_up = desc[sg].rc2_up;
     write_stage_position(v, 1, i, cx + lam * (c.x[i] - cx), cy + lam * (c.y[i] - cy));
+}
+
+// After permute_gather: the state in its new order, with position set 0 (each
+// particle's own cloud's filter bound) and the padding.
+static __global__ void batch_commit(CloudDev c, const BatchCloud *__restrict__ desc, const int *__restrict__ seg,
+                                    SortScratch z) {
+    pdl_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < c.n) {
+        c.vx[i] = z.stage[2][i];
+        c.vy[i] = z.stage[3][i];
+        c.q[i] = z.stage[4][i];
+        c.m[i] = z.stage[5][i];
+        c.orig[i] = z.orig_stage[i];
+        CloudDev v = c;
+        v.rc2_up = desc[seg[i]].rc2_up;
+        write_stage_position(v, 0, i, z.stage[0][i], z.stage[1][i]);
+    } else if (i < c.n_pad) {
+        write_padding(c, i);
+    }
 }
 
 // Position set 0 from the state, with each particle's own cloud's filter

@@ -11,8 +11,8 @@
 // pair pattern, all of which are defined on the caller's order).
 //
 // Sort: 24-bit Morton keys (12 bits per axis) and a deterministic, stable
-// LSD radix sort with 8-bit digits (per-block digit histograms, one scan,
-// stable scatter ranked by a ballot-based digit match).  No atomics decide any
+// LSD radix sort with 8-bit digits (per-block digit histograms, a scan per
+// digit, stable scatter ranked by a ballot-based digit match).  No atomics decide any
 // order; the result depends only on the positions.
 //
 // The key box is the bounding box clipped to mean +- 4 standard deviations
@@ -54,16 +54,17 @@ __device__ __forceinline__ float order_cost(const float4 &b, float rc) {
     return (b.z >= b.x) ? (b.z - b.x + rc) * (b.w - b.y + rc) : 0.0f;
 }
 
-constexpr int kMomentBlocks = 64;  // fixed partition of the moment reduction
+constexpr int kMomentBlocks = 128;  // fixed partition of the moment reduction
 constexpr int kMomentFields = 9;   // count, sum dx, sum dy, sum dx^2, sum dy^2, min x, min y, max x, max y
 
 struct SortScratch {
-    double *moments;           // [kMomentBlocks][kMomentFields] per-block partials
+    float *moments;            // [kMomentBlocks][kMomentFields] per-block partials
     double *box;               // [8]: key box x0, y0, extent; -; bounding box min x, min y, max x, max y
-    float *cost;               // [16]: order_cost of the last one-launch sort, per block
+    float *cost;               // order_cost of the cloud as last sorted, per block of the kernel that wrote it
+    int *keep;                 // set by order_check: the order is still good
     uint32_t *keys[2];
     int *vals[2];
-    uint32_t *hist;            // [kSortBuckets * nblocks]
+    uint32_t *hist;            // [kSortBuckets * nblocks], then [kSortBuckets] totals
     double *stage[6];          // gather staging for x, y, vx, vy, q, m
     int *orig_stage;
 };
@@ -157,23 +158,64 @@ __device__ __forceinline__ void moments_to_box(const Moments &m, double ox, doub
 
 __device__ __forceinline__ double finite_or_zero(double v) { return isfinite(v) ? v : 0.0; }
 
-// Per-block moments of one cloud's positions (origin: its first particle).
-static __global__ void __launch_bounds__(256) sort_moments(const double *__restrict__ x,
-                                                           const double *__restrict__ y, int n, double *part) {
-    const double ox = finite_or_zero(x[0]), oy = finite_or_zero(y[0]);
-    const Moments m = block_moments(x, y, blockIdx.x * blockDim.x, n, gridDim.x * blockDim.x, ox, oy);
-    if (threadIdx.x == 0)
-        for (int k = 0; k < kMomentFields; k++) part[blockIdx.x * kMomentFields + k] = m.v[k];
+__device__ __forceinline__ void moments_f32_add(float *v, float4 a, float ox, float oy) {
+    if (!(isfinite(a.x) && isfinite(a.y))) return;
+    const float dx = a.x - ox, dy = a.y - oy;
+    v[0] += 1.0f;
+    v[1] += dx;
+    v[2] += dy;
+    v[3] = fmaf(dx, dx, v[3]);
+    v[4] = fmaf(dy, dy, v[4]);
+    v[5] = fminf(v[5], a.x);
+    v[6] = fminf(v[6], a.y);
+    v[7] = fmaxf(v[7], a.x);
+    v[8] = fmaxf(v[8], a.y);
 }
 
-// One warp: the per-block moments summed in fixed order, then the key box.
-static __global__ void sort_box(const double *__restrict__ part, int nparts, const double *__restrict__ x,
-                                const double *__restrict__ y, double *box) {
-    Moments m;
-    m.clear();
-    for (int b = (int)threadIdx.x; b < nparts; b += 32) m.merge(part + b * kMomentFields);
-    m.warp_reduce();
-    if (threadIdx.x == 0) moments_to_box(m, finite_or_zero(x[0]), finite_or_zero(y[0]), box);
+__device__ __forceinline__ void moments_f32_merge(float *v, const float *o) {
+    for (int k = 0; k < 5; k++) v[k] += o[k];
+    v[5] = fminf(v[5], o[5]);
+    v[6] = fminf(v[6], o[6]);
+    v[7] = fmaxf(v[7], o[7]);
+    v[8] = fmaxf(v[8], o[8]);
+}
+
+// The block's moments of its threads' v; valid in thread 0.  scratch: a row per warp.
+template <int WARPS, int FIELDS>
+__device__ __forceinline__ void moments_f32_block(float (&v)[kMomentFields], float (&scratch)[WARPS][FIELDS]) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        float w[kMomentFields];
+#pragma unroll
+        for (int k = 0; k < kMomentFields; k++) w[k] = __shfl_xor_sync(0xffffffffu, v[k], o);
+        moments_f32_merge(v, w);
+    }
+    if ((threadIdx.x & 31) == 0)
+        for (int k = 0; k < kMomentFields; k++) scratch[threadIdx.x >> 5][k] = v[k];
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < WARPS; w++) moments_f32_merge(v, scratch[w]);
+}
+
+// Key box of FP32 moments about the origin (ox, oy), as moments_to_box: x0, y0, extent.
+__device__ __forceinline__ void key_box_f32(const float *v, float ox, float oy, float *box) {
+    float lo[2] = {0.0f, 0.0f}, hi[2] = {0.0f, 0.0f};
+    if (v[0] > 0.0f) {
+        const float org[2] = {ox, oy};
+        for (int a = 0; a < 2; a++) {
+            const float mean = v[1 + a] / v[0];
+            const float sd = sqrtf(fmaxf(v[3 + a] / v[0] - mean * mean, 0.0f));
+            lo[a] = fmaxf(v[5 + a], org[a] + mean - 4.0f * sd);
+            hi[a] = fminf(v[7 + a], org[a] + mean + 4.0f * sd);
+            if (!(lo[a] <= hi[a])) {
+                lo[a] = v[5 + a];
+                hi[a] = v[7 + a];
+            }
+        }
+    }
+    box[0] = lo[0];
+    box[1] = lo[1];
+    box[2] = fmaxf(hi[0] - lo[0], hi[1] - lo[1]);
 }
 
 // Spreads the low 12 bits of v to the even bit positions.
@@ -201,85 +243,208 @@ __device__ __forceinline__ uint32_t match_digit8(uint32_t d, bool valid) {
     return m;
 }
 
-static __global__ void sort_keys(const double *__restrict__ x, const double *__restrict__ y, int n,
-                                 const double *__restrict__ box, uint32_t *keys, int *vals) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double x0 = box[0], y0 = box[1], ext = box[2];
-    const double scale = (ext > 0.0 && isfinite(ext)) ? 4095.0 / ext : 0.0;
-    const double fx = (x[i] - x0) * scale, fy = (y[i] - y0) * scale;
-    const uint32_t qx = (fx > 0.0) ? (uint32_t)fmin(fx, 4095.0) : 0u;
-    const uint32_t qy = (fy > 0.0) ? (uint32_t)fmin(fy, 4095.0) : 0u;
-    keys[i] = spread_bits12(qx) | (spread_bits12(qy) << 1);
-    vals[i] = i;
+// 24-bit Morton key of position (x, y) in a key box.
+__device__ __forceinline__ uint32_t morton_key_f32(float x, float y, const float *box) {
+    const float ext = box[2];
+    const float scale = (ext > 0.0f && isfinite(ext)) ? 4095.0f / ext : 0.0f;
+    const float fx = (x - box[0]) * scale, fy = (y - box[1]) * scale;
+    const uint32_t qx = (fx > 0.0f) ? (uint32_t)fminf(fx, 4095.0f) : 0u;  // NaN: 0
+    const uint32_t qy = (fy > 0.0f) ? (uint32_t)fminf(fy, 4095.0f) : 0u;
+    return spread_bits12(qx) | (spread_bits12(qy) << 1);
+}
+
+// Whether the block's threads' costs `now` together are within kOrderSlack of
+// their `was`.  Every thread of the block; scratch: a row per warp.
+template <int WARPS, int FIELDS>
+__device__ __forceinline__ bool block_order_kept(float now, float was, float (&scratch)[WARPS][FIELDS]) {
+    static_assert(FIELDS >= 2, "two sums");
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        now += __shfl_xor_sync(0xffffffffu, now, o);
+        was += __shfl_xor_sync(0xffffffffu, was, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        scratch[threadIdx.x >> 5][0] = now;
+        scratch[threadIdx.x >> 5][1] = was;
+    }
+    __syncthreads();
+    now = was = 0.0f;
+    for (int w = 0; w < WARPS; w++) {
+        now += scratch[w][0];
+        was += scratch[w][1];
+    }
+    __syncthreads();  // scratch is reused
+    return now <= kOrderSlack * was;  // false for NaN
+}
+
+// Position set 1 (see write_midpoint) of slot s and its group's box; whole warps.
+__device__ __forceinline__ void write_midpoint_group(const CloudDev &c, int s, bool live, float4 *gbox, bool store,
+                                                     double dt) {
+    float4 A = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (live) {
+        write_midpoint(c, s, c.x[s], c.y[s], c.vx[s], c.vy[s], dt);
+        A = c.pa[1][s];
+    }
+    store_group_box(gbox, live, A.x, A.y, store);
+}
+
+// ---------------------------------------------------------------------------
+// The sort of clouds larger than one cluster holds: order_check, sort_moments,
+// sort_keys (with the first digit's histogram), per 8-bit digit radix_scan and
+// radix_scatter (and radix_hist before the next), permute_gather and
+// permute_commit.  Where order_check found the order still good the others
+// return at once (`keep`; null: always sort).  Bound by launch latency and by
+// a pass over the keys each (262,144 particles: ~60 us sorted, 17 us kept;
+// with FP64 moments and keys, one block scanning all the counts and separate
+// position and midpoint launches it took 150 us, every step).  The key box and
+// the keys are FP32 functions of the positions' hi parts, as in sort_cluster.
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ bool order_is_kept(const int *keep) { return keep && *keep; }
+
+// One block: whether the cloud's order is still good.
+static __global__ void __launch_bounds__(1024) order_check(CloudDev c, SortScratch z, int ncost) {
+    pdl_wait();
+    __shared__ float s[32][2];
+    const float rc = sqrtf(c.rc2_up);
+    float now = 0.0f, was = 0.0f;
+    for (int g = threadIdx.x; g < (c.n + 31) / 32; g += 1024) now += order_cost(c.gbox[0][g], rc);
+    for (int b = threadIdx.x; b < ncost; b += 1024) was += z.cost[b];
+    const bool kept = block_order_kept<32>(now, was, s);
+    if (threadIdx.x == 0) *z.keep = kept;
+}
+
+// Per-block moments of the cloud's positions (origin: its first particle).
+static __global__ void __launch_bounds__(256) sort_moments(const float4 *__restrict__ pa0, int n, float *part,
+                                                           const int *keep) {
+    pdl_wait();
+    if (order_is_kept(keep)) return;
+    __shared__ float s[8][kMomentFields];
+    const float4 p0 = pa0[0];
+    const float ox = isfinite(p0.x) ? p0.x : 0.0f, oy = isfinite(p0.y) ? p0.y : 0.0f;
+    float v[kMomentFields] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, INFINITY, INFINITY, -INFINITY, -INFINITY};
+#pragma unroll 4
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) moments_f32_add(v, pa0[i], ox, oy);
+    moments_f32_block<8>(v, s);
+    if (threadIdx.x == 0)
+        for (int k = 0; k < kMomentFields; k++) part[blockIdx.x * kMomentFields + k] = v[k];
+}
+
+// The key box from the nparts blocks' moments (every block the same; block 0
+// stores it), the keys of the block's kSortPerBlock particles and their first
+// digit's histogram.
+static __global__ void __launch_bounds__(kSortThreads) sort_keys(const float4 *__restrict__ pa0, int n, int nparts,
+                                                                 SortScratch z, const int *keep) {
+    pdl_wait();
+    if (order_is_kept(keep)) return;
+    __shared__ float box[3];
+    __shared__ uint32_t h[kSortBuckets];
+    h[threadIdx.x] = 0u;
+    if (threadIdx.x < 32) {
+        float v[kMomentFields] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, INFINITY, INFINITY, -INFINITY, -INFINITY};
+        for (int b = threadIdx.x; b < nparts; b += 32) moments_f32_merge(v, z.moments + b * kMomentFields);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            float w[kMomentFields];
+#pragma unroll
+            for (int k = 0; k < kMomentFields; k++) w[k] = __shfl_xor_sync(0xffffffffu, v[k], o);
+            moments_f32_merge(v, w);
+        }
+        if (threadIdx.x == 0) {
+            const float4 p0 = pa0[0];
+            key_box_f32(v, isfinite(p0.x) ? p0.x : 0.0f, isfinite(p0.y) ? p0.y : 0.0f, box);
+            if (blockIdx.x == 0) {
+                for (int k = 0; k < 3; k++) z.box[k] = box[k];
+                z.box[3] = 0.0;
+                for (int k = 0; k < 4; k++) z.box[4 + k] = (v[0] > 0.0f) ? (double)v[5 + k] : 0.0;
+            }
+        }
+    }
+    __syncthreads();
+    for (int k = 0; k < 4; k++) {
+        const int e = blockIdx.x * kSortPerBlock + k * kSortThreads + threadIdx.x;
+        if (e >= n) continue;
+        const float4 p = pa0[e];
+        const uint32_t key = morton_key_f32(p.x, p.y, box);
+        z.keys[0][e] = key;
+        z.vals[0][e] = e;
+        atomicAdd(&h[key & (kSortBuckets - 1)], 1u);
+    }
+    __syncthreads();
+    z.hist[threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
 }
 
 static __global__ void __launch_bounds__(kSortThreads) radix_hist(const uint32_t *__restrict__ keys, int n,
-                                                                  int shift, uint32_t *hist) {
+                                                                  int shift, uint32_t *hist, const int *keep) {
+    pdl_wait();
+    if (order_is_kept(keep)) return;
     __shared__ uint32_t h[kSortBuckets];
-    if (threadIdx.x < kSortBuckets) h[threadIdx.x] = 0u;
+    h[threadIdx.x] = 0u;
     __syncthreads();
     for (int k = 0; k < 4; k++) {
         const int e = blockIdx.x * kSortPerBlock + k * kSortThreads + threadIdx.x;
         if (e < n) atomicAdd(&h[(keys[e] >> shift) & (kSortBuckets - 1)], 1u);
     }
     __syncthreads();
-    if (threadIdx.x < kSortBuckets) hist[threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
+    hist[threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
 }
 
-// Exclusive scan of len entries in one block of 1024 threads.  Warp w owns
-// the w-th of 32 consecutive segments and reads it 32 entries at a time
-// (lane l takes entry 32 r + l of the segment, so every load is one
-// coalesced row): first the segment's total, then, after a scan of the 32
-// totals, the segment again, row by row, each row scanned by shuffles on top
-// of the carried prefix.  (A thread per contiguous run of entries made every
-// warp load touch 32 cache lines: 110 us for the 65,536 entries of a
-// 262,144-particle sort.)
-static __global__ void __launch_bounds__(1024) radix_scan(uint32_t *hist, int len) {
-    __shared__ uint32_t wsum[32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int seg = (len + 31) / 32;
-    const int lo = min(len, warp * seg), hi = min(len, lo + seg);
-    uint32_t s = 0;
-    for (int e = lo + lane; e < hi; e += 32) s += hist[e];
-    s = __reduce_add_sync(0xffffffffu, s);
-    if (lane == 0) wsum[warp] = s;
-    __syncthreads();
-    if (warp == 0) {  // exclusive prefix of the 32 segment totals
-        const uint32_t v = wsum[lane];
-        uint32_t inc = v;
+// Exclusive prefix over the block of 256 threads; total: the block's sum.
+__device__ __forceinline__ uint32_t block_exclusive_256(uint32_t v, uint32_t &total) {
+    __shared__ uint32_t ws[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t inc = v;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, inc, off);
-            if (lane >= off) inc += t;
-        }
-        wsum[lane] = inc - v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) ws[warp] = inc;
+    __syncthreads();
+    uint32_t before = 0u;
+    total = 0u;
+    for (int w = 0; w < 8; w++) {
+        before += (w < warp) ? ws[w] : 0u;
+        total += ws[w];
     }
     __syncthreads();
-    uint32_t carry = wsum[warp];
-    for (int r = lo; r < hi; r += 32) {
-        const int e = r + lane;
-        const uint32_t v = (e < hi) ? hist[e] : 0u;
-        uint32_t inc = v;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, inc, off);
-            if (lane >= off) inc += t;
-        }
-        if (e < hi) hist[e] = carry + inc - v;
-        carry += __shfl_sync(0xffffffffu, inc, 31);
+    return before + inc - v;
+}
+
+// Block d: the exclusive prefix of digit d's nblocks counts, in place, and
+// their total (hist[kSortBuckets * nblocks + d]).  The digits' own bases are
+// formed by radix_scatter's blocks.  (One block over all the counts took 21 us
+// for the 65,536 of a 262,144-particle sort.)
+static __global__ void __launch_bounds__(256) radix_scan(uint32_t *hist, int nblocks, const int *keep) {
+    pdl_wait();
+    if (order_is_kept(keep)) return;
+    uint32_t *row = hist + (size_t)blockIdx.x * nblocks, carry = 0u;
+    for (int b0 = 0; b0 < nblocks; b0 += 256) {
+        const int b = b0 + threadIdx.x;
+        uint32_t total;
+        const uint32_t pre = block_exclusive_256((b < nblocks) ? row[b] : 0u, total);
+        if (b < nblocks) row[b] = carry + pre;
+        carry += total;
     }
+    if (threadIdx.x == 0) hist[(size_t)kSortBuckets * nblocks + blockIdx.x] = carry;
 }
 
 // Stable scatter: elements are ranked in index order (chunk, warp, lane).
 static __global__ void __launch_bounds__(kSortThreads) radix_scatter(
     const uint32_t *__restrict__ kin, const int *__restrict__ vin, uint32_t *kout, int *vout, int n,
-    int shift, const uint32_t *__restrict__ hist) {
+    int shift, const uint32_t *__restrict__ hist, const int *keep) {
+    pdl_wait();
+    if (order_is_kept(keep)) return;
     constexpr int NWARP = kSortThreads / 32;
+    static_assert(kSortThreads == kSortBuckets, "a thread per digit");
     __shared__ uint32_t base[kSortBuckets];
     __shared__ uint32_t wcnt[NWARP][kSortBuckets];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x < kSortBuckets) base[threadIdx.x] = hist[threadIdx.x * gridDim.x + blockIdx.x];
+    {
+        uint32_t all;
+        const uint32_t first = block_exclusive_256(hist[(size_t)kSortBuckets * gridDim.x + threadIdx.x], all);
+        base[threadIdx.x] = first + hist[(size_t)threadIdx.x * gridDim.x + blockIdx.x];
+    }
     for (int k = 0; k < 4; k++) {
         for (int e = threadIdx.x; e < NWARP * kSortBuckets; e += kSortThreads) (&wcnt[0][0])[e] = 0u;
         __syncthreads();
@@ -298,11 +463,9 @@ static __global__ void __launch_bounds__(kSortThreads) radix_scatter(
             vout[pos] = vin[e];
         }
         __syncthreads();
-        if (threadIdx.x < kSortBuckets) {
-            uint32_t add = 0;
-            for (int w = 0; w < NWARP; w++) add += wcnt[w][threadIdx.x];
-            base[threadIdx.x] += add;
-        }
+        uint32_t add = 0;
+        for (int w = 0; w < NWARP; w++) add += wcnt[w][threadIdx.x];
+        base[threadIdx.x] += add;
         __syncthreads();
     }
 }
@@ -357,57 +520,6 @@ struct SortClusterSmem {
 template <int CTAS>
 constexpr size_t sort_cluster_smem() { return sizeof(SortClusterSmem<CTAS>); }
 
-__device__ __forceinline__ void moments_f32_add(float *v, float4 a, float ox, float oy) {
-    if (!(isfinite(a.x) && isfinite(a.y))) return;
-    const float dx = a.x - ox, dy = a.y - oy;
-    v[0] += 1.0f;
-    v[1] += dx;
-    v[2] += dy;
-    v[3] = fmaf(dx, dx, v[3]);
-    v[4] = fmaf(dy, dy, v[4]);
-    v[5] = fminf(v[5], a.x);
-    v[6] = fminf(v[6], a.y);
-    v[7] = fmaxf(v[7], a.x);
-    v[8] = fmaxf(v[8], a.y);
-}
-
-__device__ __forceinline__ void moments_f32_merge(float *v, const float *o) {
-    for (int k = 0; k < 5; k++) v[k] += o[k];
-    v[5] = fminf(v[5], o[5]);
-    v[6] = fminf(v[6], o[6]);
-    v[7] = fmaxf(v[7], o[7]);
-    v[8] = fmaxf(v[8], o[8]);
-}
-
-// Whether the block's threads' costs `now` together stay within kOrderSlack of
-// the warp's lanes' `was` (the same in every warp).  Every thread of the block;
-// scratch: a row per warp.
-template <int WARPS, int FIELDS>
-__device__ __forceinline__ bool block_order_kept(float now, float was, float (&scratch)[WARPS][FIELDS]) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        now += __shfl_xor_sync(0xffffffffu, now, o);
-        was += __shfl_xor_sync(0xffffffffu, was, o);
-    }
-    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5][0] = now;
-    __syncthreads();
-    float sum = 0.0f;
-    for (int w = 0; w < WARPS; w++) sum += scratch[w][0];
-    __syncthreads();  // scratch is reused
-    return sum <= kOrderSlack * was;  // false for NaN
-}
-
-// Position set 1 (see write_midpoint) of slot s and its group's box; whole warps.
-__device__ __forceinline__ void write_midpoint_group(const CloudDev &c, int s, bool live, float4 *gbox, bool store,
-                                                     double dt) {
-    float4 A = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (live) {
-        write_midpoint(c, s, c.x[s], c.y[s], c.vx[s], c.vy[s], dt);
-        A = c.pa[1][s];
-    }
-    store_group_box(gbox, live, A.x, A.y, store);
-}
-
 // pa0: the FP32 hi parts of the current positions (position set 0 holds them
 // at every step boundary).  The cloud's x, y, vx, vy, q, m and orig end up in
 // the new order, with position set 0, set 1 for time step dt (if mid) and
@@ -434,7 +546,7 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
     if (!force) {  // every block comes to the same decision, from the same sums
         float now = 0.0f;
         for (int g = tid; g < (n + 31) / 32; g += kSortClusterThreads) now += order_cost(c.gbox[0][g], rc);
-        float was = (lane < kSortClusterCtas) ? z.cost[lane] : 0.0f;
+        const float was = (tid < kSortClusterCtas) ? z.cost[tid] : 0.0f;
         if (block_order_kept<kSortClusterWarps>(now, was, S.wmom)) {
             if (mid && !mid_ready)
                 for (int k = 0; k < kSortClusterRounds; k++) {
@@ -461,20 +573,9 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
         float v[kMomentFields] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, INFINITY, INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int k = 0; k < kSortClusterRounds; k++) moments_f32_add(v, pos[k], ox, oy);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            float o[kMomentFields];
-#pragma unroll
-            for (int k = 0; k < kMomentFields; k++) o[k] = __shfl_xor_sync(0xffffffffu, v[k], off);
-            moments_f32_merge(v, o);
-        }
-        if (lane == 0)
-            for (int k = 0; k < kMomentFields; k++) S.wmom[warp][k] = v[k];
-        __syncthreads();
-        if (tid == 0) {
-            for (int w = 1; w < kSortClusterWarps; w++) moments_f32_merge(v, S.wmom[w]);
+        moments_f32_block<kSortClusterWarps>(v, S.wmom);
+        if (tid == 0)
             for (int k = 0; k < kMomentFields; k++) S.mom[k] = v[k];
-        }
     }
     cl.sync();
     if (warp == 0) {
@@ -490,24 +591,7 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
             moments_f32_merge(v, o);
         }
         if (lane == 0) {
-            // bounding box clipped to mean +- 4 sd per axis
-            float lo[2] = {0.0f, 0.0f}, hi[2] = {0.0f, 0.0f};
-            if (v[0] > 0.0f) {
-                const float org[2] = {ox, oy};
-                for (int a = 0; a < 2; a++) {
-                    const float mean = v[1 + a] / v[0];
-                    const float sd = sqrtf(fmaxf(v[3 + a] / v[0] - mean * mean, 0.0f));
-                    lo[a] = fmaxf(v[5 + a], org[a] + mean - 4.0f * sd);
-                    hi[a] = fminf(v[7 + a], org[a] + mean + 4.0f * sd);
-                    if (!(lo[a] <= hi[a])) {
-                        lo[a] = v[5 + a];
-                        hi[a] = v[7 + a];
-                    }
-                }
-            }
-            S.box[0] = lo[0];
-            S.box[1] = lo[1];
-            S.box[2] = fmaxf(hi[0] - lo[0], hi[1] - lo[1]);
+            key_box_f32(v, ox, oy, S.box);
             if (r == 0) {  // the key box and the bounding box, as the multi-kernel path writes them
                 z.box[0] = S.box[0];
                 z.box[1] = S.box[1];
@@ -518,22 +602,11 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
         }
     }
     __syncthreads();
-    {
-        const float x0 = S.box[0], y0 = S.box[1], ext = S.box[2];
-        const float scale = (ext > 0.0f && isfinite(ext)) ? 4095.0f / ext : 0.0f;
 #pragma unroll
-        for (int k = 0; k < kSortClusterRounds; k++) {
-            const int li = k * kSortClusterThreads + tid, e = e0 + li;
-            uint32_t key = 0u;
-            if (e < n) {
-                const float fx = (pos[k].x - x0) * scale, fy = (pos[k].y - y0) * scale;
-                const uint32_t qx = (fx > 0.0f) ? (uint32_t)fminf(fx, 4095.0f) : 0u;  // NaN: 0
-                const uint32_t qy = (fy > 0.0f) ? (uint32_t)fminf(fy, 4095.0f) : 0u;
-                key = spread_bits12(qx) | (spread_bits12(qy) << 1);
-            }
-            S.keys[0][li] = key;
-            S.slot[0][li] = (uint16_t)e;
-        }
+    for (int k = 0; k < kSortClusterRounds; k++) {
+        const int li = k * kSortClusterThreads + tid, e = e0 + li;
+        S.keys[0][li] = (e < n) ? morton_key_f32(pos[k].x, pos[k].y, S.box) : 0u;
+        S.slot[0][li] = (uint16_t)e;
     }
     __syncthreads();
 
@@ -668,12 +741,13 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
     if (tid == 0) {
         for (int w = 1; w < kSortClusterWarps; w++) cost += S.wmom[w][0];
         z.cost[r] = cost;
-        if (r + kSortClusterCtas < 16) z.cost[r + kSortClusterCtas] = 0.0f;
     }
 }
 
 // new slot s takes old slot perm[s]: gather into staging ...
-static __global__ void permute_gather(CloudDev c, const int *__restrict__ perm, SortScratch z) {
+static __global__ void permute_gather(CloudDev c, const int *__restrict__ perm, SortScratch z, const int *keep) {
+    pdl_wait();
+    if (order_is_kept(keep)) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= c.n) return;
     const int o = perm[s];
@@ -687,18 +761,43 @@ static __global__ void permute_gather(CloudDev c, const int *__restrict__ perm, 
 }
 
 // ... and copy back (the cloud's array addresses never change, so captured
-// CUDA graphs stay valid)
-static __global__ void permute_commit(CloudDev c, SortScratch z) {
+// CUDA graphs stay valid), with position set 0, set 1 for time step dt (if
+// mid), the padding and the group boxes.  Blocks of 256.
+static __global__ void __launch_bounds__(256) permute_commit(CloudDev c, SortScratch z, double dt, bool mid,
+                                                             bool mid_ready, const int *keep) {
     pdl_wait();
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= c.n) return;
-    c.x[s] = z.stage[0][s];
-    c.y[s] = z.stage[1][s];
-    c.vx[s] = z.stage[2][s];
-    c.vy[s] = z.stage[3][s];
-    c.q[s] = z.stage[4][s];
-    c.m[s] = z.stage[5][s];
-    c.orig[s] = z.orig_stage[s];
+    __shared__ float s_cost[8];
+    const int s = blockIdx.x * 256 + threadIdx.x;  // n_pad: whole warps
+    const bool live = s < c.n, store = s < c.n_pad;
+    if (!order_is_kept(keep)) {
+        float xh = 0.0f, yh = 0.0f;
+        if (live) {
+            c.vx[s] = z.stage[2][s];
+            c.vy[s] = z.stage[3][s];
+            c.q[s] = z.stage[4][s];
+            c.m[s] = z.stage[5][s];
+            c.orig[s] = z.orig_stage[s];
+            write_stage_position(c, 0, s, z.stage[0][s], z.stage[1][s]);  // set 0 is the state: x, y
+            const float4 A = c.pa[0][s];
+            xh = A.x;
+            yh = A.y;
+        } else if (store) {
+            write_padding(c, s);
+            c.q[s] = 0.0;
+            c.m[s] = 1.0;
+        }
+        const float4 box = store_group_box(c.gbox[0] + (s >> 5), live, xh, yh, store);
+        if ((threadIdx.x & 31) == 0) s_cost[threadIdx.x >> 5] = order_cost(box, sqrtf(c.rc2_up));
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float cost = 0.0f;
+            for (int w = 0; w < 8; w++) cost += s_cost[w];
+            z.cost[blockIdx.x] = cost;
+        }
+    } else if (mid_ready) {
+        return;
+    }
+    if (mid) write_midpoint_group(c, s, live, c.gbox[1] + (s >> 5), store, dt);
 }
 
 // An upload in the caller's order (staging arrays 0..3: x, y, vx, vy) put

@@ -31,7 +31,7 @@ def oracle_run(oracle_lib, c0):
 
 
 @pytest.mark.parametrize("speed", [1e-6, 5.0])
-@pytest.mark.parametrize("n", [1, 33, 1025, 16384])
+@pytest.mark.parametrize("n", [1, 33, 1025, 16384, 16385, 70001])
 def test_cloud_trajectory_with_skipped_sorts(gpu_ctx, oracle_lib, n, speed):
     c0 = free_cloud(n, 40 + n, speed)
     c = DeviceCloud.from_cloud(gpu_ctx, c0)
