@@ -113,8 +113,9 @@ enum StageMode : int { kModeStep = 0, kModeForceOnly = 1 };
 // Constants of the FP64 pair terms of one cloud (make_yukawa64).
 struct Yukawa64 {
     double kappa;
-    double k_hi, k_lo;  // -kappa 512 log2(e) as an unevaluated pair
+    double k_hi;        // -kappa 512 log2(e)
     float k_f;          // the same in FP32
+    float k_lo;         // what k_hi lacks, times ln2/512
     uint32_t rc2_word;  // high word of r_c^2: r^2 with a smaller one is inside the cutoff
 };
 
@@ -160,6 +161,19 @@ struct StageParams {
 __device__ __forceinline__ double widen(float v) {
     const uint32_t b = __float_as_uint(v), e = (b >> 23) & 0xFFu;
     if (e - 1u >= 254u) return (double)v;
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+
+// A double rounded toward zero to FP32, by integer operations; 0 below 2^-126.
+// |v| < 2^128.
+__device__ __forceinline__ float narrow(double v) {
+    const uint32_t h = (uint32_t)__double2hiint(v), m = h & 0x7FFFFFFFu;
+    const uint32_t b = __funnelshift_l((uint32_t)__double2loint(v), m - 0x38000000u, 3);
+    return __uint_as_float((h & 0x80000000u) | (m < 0x38100000u ? 0u : b));
+}
+// widen for a normal number or one too small to matter (zero gives 2^-127).
+__device__ __forceinline__ double widen_normal(float v) {
+    const uint32_t b = __float_as_uint(v);
     return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u)), (int)(b << 29));
 }
 

@@ -1177,7 +1177,7 @@ static __global__ void __launch_bounds__(128) stage_finish(const StageParams P) 
 // hits in FP64 with full warps (dm_fp64.cuh).  The sums meet in the cluster's
 // first block, which runs the epilogue.
 //
-// Bound by the FP64 pipe on dense clouds (26 FP64 instructions per pair in
+// Bound by the FP64 pipe on dense clouds (22 FP64 instructions per pair in
 // reach, 64 cycles of a scheduler's FP64 unit per 32 pairs each), by latency
 // on sparse ones.
 // ---------------------------------------------------------------------------
