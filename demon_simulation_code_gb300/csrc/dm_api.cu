@@ -515,7 +515,10 @@ int launch_variant(dm_cloud *c, int vi, int S, StageParams P) {
         ctx->prof_pairs += (double)P.nsets * (double)c->n * (double)(c->n - 1);
     }
     if (!k.cluster) {
-        DM_CUDA(ctx, launch_pdl(stage_finish, dim3(ngroups), dim3(128), 0, ctx->stream, P));
+        if (P.f.flags & ~kBasicForces)
+            DM_CUDA(ctx, launch_pdl(stage_finish<true>, dim3(ngroups), dim3(64 * kTermParts), 0, ctx->stream, P));
+        else
+            DM_CUDA(ctx, launch_pdl(stage_finish<false>, dim3(ngroups), dim3(128), 0, ctx->stream, P));
         ctx->launches++;
     }
     if (P.mode == kModeForceOnly) return DM_OK;

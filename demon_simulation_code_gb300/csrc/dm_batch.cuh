@@ -94,14 +94,10 @@ static __global__ void __launch_bounds__(64) batch_finish(const StageParams P, c
     const BatchCloud &d = desc[gseg[blockIdx.x]];
     const int li = 32 * ((int)blockIdx.x - d.goff) + lane, i = d.off + li;
     const bool live = li < d.n;
-    const bool both = (d.f.flags & ~kBasicForces) != 0;  // else a warp needs its own axis only
-    double2 f[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+    double f[2] = {0.0, 0.0};
     if (live) {
         epilogue_prefetch(P, i, ax);
-        for (int e = 0; e < P.nsets; e++) {
-            if (both || ax == 0) f[e].x = finish_rank_sum(P, i, e, 0);
-            if (both || ax == 1) f[e].y = finish_rank_sum(P, i, e, 1);
-        }
+        for (int e = 0; e < P.nsets; e++) f[e] = finish_rank_sum(P, i, e, ax);
     }
     pass_epilogue(P, EpilogueCloud{d.f, d.rc2_up, live, (int)blockIdx.x}, i, ax, kBarEpilogue, f[0], f[1], S);
     pass_step_advance(P);
@@ -356,6 +352,7 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
             c.vy[s] = val[3][k];
             c.q[s] = val[4][k];
             c.m[s] = val[5][k];
+            c.invm[s] = __drcp_rn(val[5][k]);
             c.orig[s] = ov[k];
             write_stage_position(v, 0, s, val[0][k], val[1][k]);  // set 0 is the state: x, y
             h[0] = make_float2(__double2float_rn(val[0][k]), __double2float_rn(val[1][k]));
@@ -408,6 +405,7 @@ static __global__ void batch_commit(CloudDev c, const BatchCloud *__restrict__ d
         c.vy[i] = z.stage[3][i];
         c.q[i] = z.stage[4][i];
         c.m[i] = z.stage[5][i];
+        c.invm[i] = __drcp_rn(z.stage[5][i]);
         c.orig[i] = z.orig_stage[i];
         CloudDev v = c;
         v.rc2_up = desc[seg[i]].rc2_up;
@@ -418,7 +416,7 @@ static __global__ void batch_commit(CloudDev c, const BatchCloud *__restrict__ d
 }
 
 // Position set 0 from the state, with each particle's own cloud's filter
-// bound, and the padding.
+// bound, 1/m, and the padding.
 static __global__ void batch_init_positions(CloudDev c, const BatchCloud *__restrict__ desc,
                                             const int *__restrict__ seg) {
     pdl_wait();
@@ -427,6 +425,7 @@ static __global__ void batch_init_positions(CloudDev c, const BatchCloud *__rest
         CloudDev v = c;
         v.rc2_up = desc[seg[i]].rc2_up;
         write_stage_position(v, 0, i, c.x[i], c.y[i]);
+        c.invm[i] = __drcp_rn(c.m[i]);
     } else if (i < c.n_pad) {
         write_padding(c, i);
     }

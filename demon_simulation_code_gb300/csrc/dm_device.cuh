@@ -72,7 +72,7 @@ struct CloudDev {
     int n, n_pad;
     double *x, *y, *vx, *vy, *q, *m;
     double *k1[2], *k2[2];
-    double *invm;                  // 1/m, left by pass 0 for pass 1
+    double *invm;                  // 1/m, kept with m (a reciprocal is 9 FP64 instructions)
     double *px[4], *py[4];
     float4 *pa[4], *pb[4];
     float4 *gbox[4];               // [n_pad/32] FP32 box (x0, y0, x1, y1) of each 32-particle group
@@ -403,6 +403,9 @@ __device__ __forceinline__ void write_stage_position(const CloudDev &c, int b, i
     write_stage_position(c, b, i, xs, ys, c.rc2_up);
 }
 
+// Neither infinite nor NaN, by the exponent bits (a comparison holds the FP64 unit).
+__device__ __forceinline__ bool finite64(double v) { return ((uint32_t)__double2hiint(v) & 0x7FF00000u) != 0x7FF00000u; }
+
 // base + inc/2: the product is exact, so one fma is the reference's two operations.
 __device__ __forceinline__ double half_step(double base, double inc) { return fma(0.5, inc, base); }
 
@@ -469,19 +472,14 @@ struct ParticleAt {
     double x, y, vx, vy, q, m;
 };
 
-// ConfinementForce::force (ConfinementForce.cpp:48-54)
-__device__ __forceinline__ void add_confinement(const ForceParams &f, const ParticleAt &s, double &Fx,
-                                                double &Fy) {
-    const double cq = __dmul_rn(s.q, f.confine);
-    Fx = __dadd_rn(Fx, __dmul_rn(cq, s.x));
-    Fy = __dadd_rn(Fy, __dmul_rn(cq, s.y));
+// ConfinementForce::force (ConfinementForce.cpp:48-54), one axis
+__device__ __forceinline__ double add_confinement(const ForceParams &f, double q, double p, double F) {
+    return __dadd_rn(F, __dmul_rn(__dmul_rn(q, f.confine), p));
 }
 
-// DragForce::force (DragForce.cpp:49-55) with dragConst
-__device__ __forceinline__ void add_drag(double dragConst, const ParticleAt &s, double &Fx, double &Fy) {
-    const double d = __dmul_rn(s.m, dragConst);
-    Fx = __dadd_rn(Fx, __dmul_rn(d, s.vx));
-    Fy = __dadd_rn(Fy, __dmul_rn(d, s.vy));
+// DragForce::force (DragForce.cpp:49-55) with dragConst, one axis
+__device__ __forceinline__ double add_drag(double dragConst, double m, double v, double F) {
+    return __dadd_rn(F, __dmul_rn(__dmul_rn(m, dragConst), v));
 }
 
 // sqrt(x*x + y*y) without contraction (length_pd, VectorCompatibility.h:290-292)
@@ -500,106 +498,92 @@ __device__ __forceinline__ double radius_of(const ParticleAt &s) {
 struct PositionTerms {
     double voidx, voidy, drive, rotx, roty, elecx, elecy, vert;
 };
-__device__ __forceinline__ PositionTerms position_terms(const ForceParams &f, double x, double y, double q, double t) {
+// Part `part` of kTermParts of them (fields of T); the parts are about equally
+// long chains of FP64 operations, for as many warps.
+constexpr int kTermParts = 4;
+__device__ __forceinline__ void position_terms(PositionTerms &T, int part, const ForceParams &f, double x, double y,
+                                               double q, double t) {
     const long long fl = f.flags;
-    PositionTerms T{};
-    double r = 0.0;
-    if (fl & (kConfinementVoid | kRotational | kElectric))  // length_pd (VectorCompatibility.h:290-292)
-        r = __dsqrt_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)));
-    if (fl & kConfinementVoid) {
+    auto radius = [&] { return __dsqrt_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y))); };  // length_pd (VectorCompatibility.h:290-292)
+    if (part == 0 && (fl & kConfinementVoid)) {
+        const double r = radius();
         const double decayV = __dmul_rn(q, -f.void_decay);
         const double expR = __ddiv_rn(exp(__dmul_rn(r, -f.void_decay)), r);
         T.voidx = __dmul_rn(__dmul_rn(decayV, expR), x);
         T.voidy = __dmul_rn(__dmul_rn(decayV, expR), y);
     }
-    if (fl & kDriving) {
+    if (part == 1 && (fl & kDriving)) {
         // the stored driveConst is -drive_const (DrivingForce.h:17-18)
         const double distV = __dsub_rn(x, f.drive_shift);
         const double sinArg = __dsub_rn(__dmul_rn(x, kWaveNum), __dmul_rn(t, kAngFreq));
         const double expArg = __ddiv_rn(__dsub_rn(distV, distV), f.drive_const);
         T.drive = __dmul_rn(__dmul_rn(sin(sinArg), exp(expArg)), f.drive_amplitude);
     }
-    if ((fl & kRotational) && r > f.rot_rmin && r < f.rot_rmax) {
-        T.rotx = __ddiv_rn(__dmul_rn(f.rot_const, y), r);
-        T.roty = __ddiv_rn(__dmul_rn(f.rot_const, x), r);
+    if (part == 2) {
+        if (fl & kRotational) {
+            const double r = radius();
+            const bool in = r > f.rot_rmin && r < f.rot_rmax;
+            T.rotx = in ? __ddiv_rn(__dmul_rn(f.rot_const, y), r) : 0.0;
+            T.roty = in ? __ddiv_rn(__dmul_rn(f.rot_const, x), r) : 0.0;
+        }
+        if (fl & kVertElectric) T.vert = __dmul_rn(__dmul_rn(q, f.vert_electric), exp(__ddiv_rn(y, f.vert_decay)));
     }
-    if (fl & kElectric) {
-        const double eV = __dmul_rn(__dmul_rn(q, f.electric), exp(__ddiv_rn(r, -f.electric_radius)));
+    if (part == 3 && (fl & kElectric)) {
+        const double eV = __dmul_rn(__dmul_rn(q, f.electric), exp(__ddiv_rn(radius(), -f.electric_radius)));
         T.elecx = __dmul_rn(eV, x);
         T.elecy = __dmul_rn(eV, y);
     }
-    if (fl & kVertElectric) T.vert = __dmul_rn(__dmul_rn(q, f.vert_electric), exp(__ddiv_rn(y, f.vert_decay)));
-    return T;
 }
 
-// The total force on a particle at set e of the running pass, every enabled
+// Axis ax of the total force on a particle at set e of the running pass, every enabled
 // force added in the reference driver's order (driver.cpp:372-402):
 // Confinement, ConfinementVoid, Drag, Driving, Magnetic (MagneticForce.cpp:
 // 48-54), RectConfinement (RectConfinementForce.cpp:50-59), Rotational,
-// ShieldedCoulomb (the pair sum fpx, fpy), Thermal, ThermalLocalized
+// ShieldedCoulomb (the pair sum fp), Thermal, ThermalLocalized
 // (ThermalForceLocalized.cpp:124-133), TimeVaryingDrag
 // (TimeVaryingDragForce.cpp:11-40), TimeVaryingThermal
 // (TimeVaryingThermalForce.cpp:14-42), Electric, Gravitational
 // (GravitationalForce.cpp:46-50), VertElectric.  T: position_terms at (s.x, s.y).
-__device__ __forceinline__ void total_force(const StageParams &P, const ForceParams &f, int i, int e,
-                                            const ParticleAt &s, const PositionTerms &T, double fpx, double fpy,
-                                            double &Fx, double &Fy) {
+__device__ __forceinline__ double total_force(const StageParams &P, const ForceParams &f, int i, int e, int ax,
+                                              const ParticleAt &s, const PositionTerms &T, double fp) {
     const long long fl = f.flags;
-    Fx = Fy = 0.0;
-    if (fl & kConfinement) add_confinement(f, s, Fx, Fy);
-    if (fl & kConfinementVoid) {
-        add_confinement(f, s, Fx, Fy);
-        Fx = __dadd_rn(Fx, T.voidx);
-        Fy = __dadd_rn(Fy, T.voidy);
-    }
-    if (fl & kDrag) add_drag(-f.gamma, s, Fx, Fy);  // dragConst = -gamma (DragForce.h:16-17)
-    if (fl & kDriving) Fx = __dadd_rn(Fx, T.drive);
+    const double p = ax ? s.y : s.x, v = ax ? s.vy : s.vx;
+    double F = 0.0;
+    if (fl & kConfinement) F = add_confinement(f, s.q, p, F);
+    if (fl & kConfinementVoid) F = __dadd_rn(add_confinement(f, s.q, p, F), ax ? T.voidy : T.voidx);
+    if (fl & kDrag) F = add_drag(-f.gamma, s.m, v, F);  // dragConst = -gamma (DragForce.h:16-17)
+    if ((fl & kDriving) && ax == 0) F = __dadd_rn(F, T.drive);
     if (fl & kMagnetic) {
         const double qB = __dmul_rn(s.q, f.magnetic);
-        Fx = __dadd_rn(Fx, __dmul_rn(qB, s.vy));
-        Fy = __dsub_rn(Fy, __dmul_rn(qB, s.vx));
+        F = ax ? __dsub_rn(F, __dmul_rn(qB, s.vx)) : __dadd_rn(F, __dmul_rn(qB, s.vy));
     }
-    if (fl & kRectConfinement) {
-        Fx = __dadd_rn(Fx, __dmul_rn(__dmul_rn(s.q, f.confine_x), s.x));
-        Fy = __dadd_rn(Fy, __dmul_rn(__dmul_rn(s.q, f.confine_y), s.y));
-    }
-    if (fl & kRotational) {
-        Fx = __dsub_rn(Fx, T.rotx);
-        Fy = __dadd_rn(Fy, T.roty);
-    }
-    if (fl & kShieldedCoulomb) {
-        Fx = __dadd_rn(Fx, fpx);
-        Fy = __dadd_rn(Fy, fpy);
-    }
+    if (fl & kRectConfinement) F = __dadd_rn(F, __dmul_rn(__dmul_rn(s.q, ax ? f.confine_y : f.confine_x), p));
+    if (fl & kRotational) F = ax ? __dadd_rn(F, T.roty) : __dsub_rn(F, T.rotx);
+    if (fl & kShieldedCoulomb) F = __dadd_rn(F, fp);
     if (fl & kThermal) {
         const double2 k = stage_thermal(P, f, i, e);
-        Fx = __dadd_rn(Fx, k.x);
-        Fy = __dadd_rn(Fy, k.y);
+        F = __dadd_rn(F, ax ? k.y : k.x);
     }
     if (fl & kThermalLocalized) {
         const double heat = (radius_of(s) < f.heat_radius) ? f.heat_in : f.heat_out;
         double tx, ty;
         thermal_draw(f, (uint32_t)P.c.orig[i], pass_step_index(P), thermal_stage(P, e) + 16, heat, tx, ty);
-        Fx = __dadd_rn(Fx, tx);
-        Fy = __dadd_rn(Fy, ty);
+        F = __dadd_rn(F, ax ? ty : tx);
     }
     if (fl & (kTimeVaryingDrag | kTimeVaryingThermal)) {
         const double t = stage_time(P, e);
-        if (fl & kTimeVaryingDrag) add_drag(-__dadd_rn(__dmul_rn(f.drag_scale, t), f.drag_offset), s, Fx, Fy);
+        if (fl & kTimeVaryingDrag) F = add_drag(-__dadd_rn(__dmul_rn(f.drag_scale, t), f.drag_offset), s.m, v, F);
         if (fl & kTimeVaryingThermal) {
             double tx, ty;
             thermal_draw(f, (uint32_t)P.c.orig[i], pass_step_index(P), thermal_stage(P, e) + 32,
                          __dadd_rn(__dmul_rn(f.heat_scale, t), f.heat_offset), tx, ty);
-            Fx = __dadd_rn(Fx, tx);
-            Fy = __dadd_rn(Fy, ty);
+            F = __dadd_rn(F, ax ? ty : tx);
         }
     }
-    if (fl & kElectric) {
-        Fx = __dadd_rn(Fx, T.elecx);
-        Fy = __dadd_rn(Fy, T.elecy);
-    }
-    if (fl & kGravitational) Fy = __dadd_rn(Fy, __dmul_rn(s.m, f.gravity));
-    if (fl & kVertElectric) Fy = __dadd_rn(Fy, T.vert);
+    if (fl & kElectric) F = __dadd_rn(F, ax ? T.elecy : T.elecx);
+    if ((fl & kGravitational) && ax) F = __dadd_rn(F, __dmul_rn(s.m, f.gravity));
+    if ((fl & kVertElectric) && ax) F = __dadd_rn(F, T.vert);
+    return F;
 }
 
 // The same for one axis of the forces in kBasicForces (their axes are

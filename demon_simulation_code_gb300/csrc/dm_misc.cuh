@@ -7,13 +7,14 @@
 
 namespace dm {
 
-// Writes position set 0 (two-float copies and filter bounds) from the state,
-// and the padding particles of every set.
+// Writes position set 0 (two-float copies and filter bounds) and 1/m from the
+// state, and the padding particles of every set.
 static __global__ void init_positions(CloudDev c) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n_pad) return;
     if (i < c.n) {
         write_stage_position(c, 0, i, c.x[i], c.y[i]);
+        c.invm[i] = __drcp_rn(c.m[i]);
     } else {
         write_padding(c, i);
         c.q[i] = 0.0;

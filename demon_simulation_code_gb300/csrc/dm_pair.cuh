@@ -764,6 +764,7 @@ __device__ __forceinline__ double pair_scale(const StageParams &P, int i) {
 // ---------------------------------------------------------------------------
 
 struct EpilogueShared {
+    double v[2][32];  // [axis][particle]: the velocities of the second set's force
     union {
         struct {
             float hi[2][2][32], lo[2][2][32];  // [set][axis][particle]
@@ -787,6 +788,7 @@ __device__ __forceinline__ void epilogue_prefetch(const StageParams &P, int i, i
     prefetch_l1((ax ? c.vy : c.vx) + i);
     prefetch_l1(c.q + i);
     prefetch_l1(c.m + i);
+    prefetch_l1(c.invm + i);
     prefetch_l1(c.orig + i);
     if (P.mode == kModeForceOnly) return;
     if (P.pass == 0) {
@@ -796,30 +798,21 @@ __device__ __forceinline__ void epilogue_prefetch(const StageParams &P, int i, i
         prefetch_l1((ax ? c.py : c.px)[3] + i);
         prefetch_l1(c.k1[ax] + i);
         prefetch_l1(c.k2[ax] + i);
-        prefetch_l1(c.invm + i);
     }
-}
-
-// 1/m of particle i: computed by a step's first pass, which leaves it for the second.
-__device__ __forceinline__ double pass_reciprocal(const StageParams &P, int i, double m, bool store) {
-    if (P.pass == 1) return P.c.invm[i];
-    const double inv = __drcp_rn(m);
-    if (store && P.order == 4) P.c.invm[i] = inv;
-    return inv;
 }
 
 // One axis of particle i's part of the pass, the total force at set e and
 // axis velocity v given by force(e, x, v): the new positions of both sets
 // (out[0], out[1]), stored but for their packed words; returns whether the
-// positions are finite.
+// positions are finite.  Lanes that are not live (i any particle) store nothing.
 template <class Force>
-__device__ __forceinline__ bool advance_axis(const StageParams &P, int i, int ax, double inv, double (&out)[2],
+__device__ __forceinline__ bool advance_axis(const StageParams &P, int i, int ax, bool live, double (&out)[2],
                                              Force force) {
     const CloudDev &c = P.c;
     double *X = ax ? c.y : c.x, *V = ax ? c.vy : c.vx;
     double *const *p = ax ? c.py : c.px;
     const double dt = stage_dt(P), m = c.m[i];
-    const double x = X[i], v = V[i];
+    const double x = X[i], v = V[i], inv = c.invm[i];
     auto increment = [&](double F) { return div_by(__dmul_rn(dt, F), m, inv); };
     bool fine = true;
     double k1, k2, v2;
@@ -828,7 +821,7 @@ __device__ __forceinline__ bool advance_axis(const StageParams &P, int i, int ax
         k1 = increment(force(0, x, v));
         v2 = half_step(v, k1);
         k2 = increment(force(1, x2, v2));
-        fine = isfinite(x2);
+        fine = finite64(x2);
     } else {
         k1 = c.k1[ax][i];
         k2 = c.k2[ax][i];
@@ -839,46 +832,53 @@ __device__ __forceinline__ bool advance_axis(const StageParams &P, int i, int ax
         const double vn = __dadd_rn(v, k2);
         out[0] = __dadd_rn(x, l2);
         out[1] = half_step(out[0], __dmul_rn(dt, vn));
-        V[i] = vn;
-        p[2][i] = out[0];
-        p[3][i] = out[1];
-        return fine && isfinite(out[0]);
+        if (live) {
+            V[i] = vn;
+            p[2][i] = out[0];
+            p[3][i] = out[1];
+        }
+        return fine && finite64(out[0]);
     }
     const double v3 = half_step(v, k2), l3 = __dmul_rn(dt, v3);
     if (P.pass == 0) {
-        c.k1[ax][i] = k1;
-        c.k2[ax][i] = k2;
         out[0] = half_step(x, l2);
         out[1] = __dadd_rn(x, l3);
-        p[2][i] = out[0];
-        p[3][i] = out[1];
-        return fine && isfinite(out[0]) && isfinite(out[1]);
+        if (live) {
+            c.k1[ax][i] = k1;
+            c.k2[ax][i] = k2;
+            p[2][i] = out[0];
+            p[3][i] = out[1];
+        }
+        return fine && finite64(out[0]) && finite64(out[1]);
     }
     const double k3 = increment(force(0, p[2][i], v3));
     const double v4 = __dadd_rn(v, k3);
     const double k4 = increment(force(1, p[3][i], v4));
     const double xn = rk4_sum(x, __dmul_rn(dt, v), l2, l3, __dmul_rn(dt, v4));
     const double vn = rk4_sum(v, k1, k2, k3, k4);
-    X[i] = xn;
-    V[i] = vn;
     out[0] = xn;
     out[1] = half_step(xn, __dmul_rn(dt, vn));  // the next step's x2, for the same dt
-    p[1][i] = out[1];
-    return isfinite(xn);
+    if (live) {
+        X[i] = xn;
+        V[i] = vn;
+        p[1][i] = out[1];
+    }
+    return finite64(xn);
 }
 
-// The pass's epilogue for one 32-particle group: lane = particle i, `half` =
-// 0 or 1, the calling warp of the two (they meet at named barrier `bar`);
-// fs0, fs1 the pair forces (x, y) at the two sets, C q_i included.  Sums the
+// The pass's epilogue for one 32-particle group: lane = particle i, warp ax =
+// 0 or 1 of the two computes that axis (they meet at named barrier `bar`);
+// fs0, fs1 the pair forces along it at the two sets, C q_i included.  Sums the
 // forces, advances the particles, writes the next pass's position sets and
 // their group boxes (force-only: the forces, in the caller's order).
 //
-// With the forces of kBasicForces each warp takes one axis (the epilogue is a
-// chain of dependent FP64 operations at 64 cycles each; two axes are two
-// chains).  The other forces couple the axes: the warps compute the terms of
-// the position sets, one each, and warp 0 advances both axes.
-__device__ __forceinline__ void pass_epilogue(const StageParams &P, const EpilogueCloud &E, int i, int half, int bar,
-                                              double2 fs0, double2 fs1, EpilogueShared &S) {
+// The epilogue is a chain of dependent FP64 operations at 64 cycles each; two
+// axes are two chains.  The forces outside kBasicForces couple the axes: their
+// position terms are computed first (TERMS: the caller has done so), a set per
+// warp, and before the second set's force the warps exchange their velocities.
+template <bool TERMS = false>
+__device__ __forceinline__ void pass_epilogue(const StageParams &P, const EpilogueCloud &E, int i, int ax, int bar,
+                                              double fs0, double fs1, EpilogueShared &S) {
     const int lane = threadIdx.x & 31;
     const CloudDev &c = P.c;
     const ForceParams &f = E.f;
@@ -887,136 +887,65 @@ __device__ __forceinline__ void pass_epilogue(const StageParams &P, const Epilog
     const bool basic = !(f.flags & ~kBasicForces);
     auto meet = [&] { bar_sync(bar, 64); };
     const int ob = (P.pass == 0) ? 2 : 0;  // first buffer written
-    if (basic) {
-        const int ax = half;
-        double out[2] = {0.0, 0.0};
-        if (live) {
-            const double q = c.q[i], m = c.m[i];
-            auto force = [&](int e, double x, double v) {
-                double therm = 0.0;
-                if (f.flags & kThermal) {
-                    const double2 t = stage_thermal(P, f, i, e);
-                    therm = ax ? t.y : t.x;
-                }
-                const double2 fp = e ? fs1 : fs0;
-                return axis_force(f, ax, x, v, q, m, ax ? fp.y : fp.x, therm);
-            };
-            if (fo) {
-                const int b = P.buf[0];
-                (ax ? P.fy_out : P.fx_out)[c.orig[i]] = force(0, (ax ? c.py : c.px)[b][i], (ax ? c.vy : c.vx)[i]);
-            } else if (!advance_axis(P, i, ax, pass_reciprocal(P, i, m, ax == 0), out, force)) {
-                atomicOr(c.err, 1);
-            }
-        }
-        if (fo) return;  // uniform over the launch
+    if (!basic && !TERMS) {
+        if (live && ax < P.nsets) {
+            const int b = P.buf[ax];
 #pragma unroll
-        for (int e = 0; e < 2; e++) {
-            float h = 0.0f, lo = 0.0f;
-            if (live) split2(out[e], h, lo);
-            S.hi[e][ax][lane] = h;
-            S.lo[e][ax][lane] = lo;
+            for (int part = 0; part < kTermParts; part++)
+                position_terms(S.terms[ax][lane], part, f, c.px[b][i], c.py[b][i], c.q[i],
+                               (f.flags & kDriving) ? stage_time(P, ax) : 0.0);
         }
         meet();
-        // write_stage_position's packed words and the group's box, one set per warp
-        const int e = half;
-        const float xh = S.hi[e][0][lane], yh = S.hi[e][1][lane];
-        if (live) {
-            c.pa[ob + e][i] = make_float4(xh, yh, fmaf(yh, yh, xh * xh), c.pa[P.buf[0]][i].w);
-            c.pb[ob + e][i] = make_float4(S.lo[e][0][lane], S.lo[e][1][lane], -filter_threshold(xh, yh, E.rc2_up), 0.0f);
-        }
-        store_group_box(c.gbox[ob + e] + E.group, live, xh, yh, true);
-        return;
     }
-    // the terms of set `half`
-    if (live && (half == 0 || P.nsets > 1)) {
-        const int b = P.buf[half];
-        S.terms[half][lane] = position_terms(f, c.px[b][i], c.py[b][i], c.q[i],
-                                             (f.flags & kDriving) ? stage_time(P, half) : 0.0);
+    double out[2] = {0.0, 0.0};
+    const int j = live ? i : 0;  // lanes without a particle take part in the meetings
+    const double q = c.q[j], m = c.m[j];
+    auto force = [&](int e, double x, double v) {
+        const double fp = e ? fs1 : fs0;
+        if (basic) {
+            double therm = 0.0;
+            if (f.flags & kThermal) {
+                const double2 t = stage_thermal(P, f, j, e);
+                therm = ax ? t.y : t.x;
+            }
+            return axis_force(f, ax, x, v, q, m, fp, therm);
+        }
+        double vo;  // the other axis's velocity
+        if (e == 0) {
+            vo = (ax ? c.vx : c.vy)[j];
+            if (!fo && P.pass == 1) vo = half_step(vo, c.k2[1 - ax][j]);
+        } else {
+            S.v[ax][lane] = v;
+            meet();
+            vo = S.v[1 - ax][lane];
+        }
+        const int b = P.buf[e];
+        const ParticleAt s{c.px[b][j], c.py[b][j], ax ? vo : v, ax ? v : vo, q, m};
+        return total_force(P, f, j, e, ax, s, S.terms[e][lane], fp);
+    };
+    if (fo) {
+        const double F = force(0, (ax ? c.py : c.px)[P.buf[0]][j], (ax ? c.vy : c.vx)[j]);
+        if (live) (ax ? P.fy_out : P.fx_out)[c.orig[i]] = F;
+        return;  // uniform over the launch
+    }
+    if (!advance_axis(P, j, ax, live, out, force) && live) atomicOr(c.err, 1);
+    if (!basic) meet();  // the terms' memory is used again
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        float h = 0.0f, lo = 0.0f;
+        if (live) split2(out[e], h, lo);
+        S.hi[e][ax][lane] = h;
+        S.lo[e][ax][lane] = lo;
     }
     meet();
-    if (half != 0) return;
-    const double q = live ? c.q[i] : 0.0, m = live ? c.m[i] : 1.0;
-    if (fo) {
-        if (live) {
-            const int b = P.buf[0];
-            const ParticleAt s{c.px[b][i], c.py[b][i], c.vx[i], c.vy[i], q, m};
-            double Fx, Fy;
-            total_force(P, f, i, 0, s, S.terms[0][lane], fs0.x, fs0.y, Fx, Fy);
-            P.fx_out[c.orig[i]] = Fx;
-            P.fy_out[c.orig[i]] = Fy;
-        }
-        return;
-    }
-    float h[2][2] = {};
+    // write_stage_position's packed words and the group's box, one set per warp
+    const int e = ax;
+    const float xh = S.hi[e][0][lane], yh = S.hi[e][1][lane];
     if (live) {
-        // the axes in step: stage by stage, both components
-        const double dt = stage_dt(P), inv = pass_reciprocal(P, i, m, true);
-        const double x = c.x[i], y = c.y[i], vx = c.vx[i], vy = c.vy[i];
-        const int b1 = P.buf[1], b0 = P.buf[0];
-        auto increments = [&](int e, double vxs, double vys, double &kx, double &ky) {
-            const int b = e ? b1 : b0;
-            const double2 fp = e ? fs1 : fs0;
-            const ParticleAt s{c.px[b][i], c.py[b][i], vxs, vys, q, m};
-            double Fx, Fy;
-            total_force(P, f, i, e, s, S.terms[e][lane], fp.x, fp.y, Fx, Fy);
-            kx = div_by(__dmul_rn(dt, Fx), m, inv);
-            ky = div_by(__dmul_rn(dt, Fy), m, inv);
-        };
-        double k1x, k1y, k2x, k2y, n0x, n0y, n1x, n1y;
-        if (P.pass == 0) {
-            increments(0, vx, vy, k1x, k1y);
-            increments(1, half_step(vx, k1x), half_step(vy, k1y), k2x, k2y);
-        } else {
-            k1x = c.k1[0][i]; k1y = c.k1[1][i];
-            k2x = c.k2[0][i]; k2y = c.k2[1][i];
-        }
-        const double l2x = __dmul_rn(dt, half_step(vx, k1x)), l2y = __dmul_rn(dt, half_step(vy, k1y));
-        double vnx = vx, vny = vy;
-        bool fine = true;
-        if (P.order == 2) {
-            n0x = __dadd_rn(x, l2x);
-            n0y = __dadd_rn(y, l2y);
-            vnx = __dadd_rn(vx, k2x);
-            vny = __dadd_rn(vy, k2y);
-            fine = isfinite(c.px[1][i]) && isfinite(c.py[1][i]);
-        } else {
-            const double v3x = half_step(vx, k2x), v3y = half_step(vy, k2y);
-            const double l3x = __dmul_rn(dt, v3x), l3y = __dmul_rn(dt, v3y);
-            if (P.pass == 0) {
-                c.k1[0][i] = k1x; c.k1[1][i] = k1y;
-                c.k2[0][i] = k2x; c.k2[1][i] = k2y;
-                n0x = half_step(x, l2x);
-                n0y = half_step(y, l2y);
-                n1x = __dadd_rn(x, l3x);
-                n1y = __dadd_rn(y, l3y);
-                fine = isfinite(c.px[1][i]) && isfinite(c.py[1][i]) && isfinite(n1x) && isfinite(n1y);
-            } else {
-                double k3x, k3y, k4x, k4y;
-                increments(0, v3x, v3y, k3x, k3y);
-                const double v4x = __dadd_rn(vx, k3x), v4y = __dadd_rn(vy, k3y);
-                increments(1, v4x, v4y, k4x, k4y);
-                n0x = rk4_sum(x, __dmul_rn(dt, vx), l2x, l3x, __dmul_rn(dt, v4x));
-                n0y = rk4_sum(y, __dmul_rn(dt, vy), l2y, l3y, __dmul_rn(dt, v4y));
-                vnx = rk4_sum(vx, k1x, k2x, k3x, k4x);
-                vny = rk4_sum(vy, k1y, k2y, k3y, k4y);
-            }
-        }
-        if (P.order == 2 || P.pass == 1) {  // the step ends (set 0 is the state: x, y)
-            c.vx[i] = vnx;
-            c.vy[i] = vny;
-            n1x = half_step(n0x, __dmul_rn(dt, vnx));
-            n1y = half_step(n0y, __dmul_rn(dt, vny));
-        }
-        write_stage_position(c, ob, i, n0x, n0y, E.rc2_up);
-        write_stage_position(c, ob + 1, i, n1x, n1y, E.rc2_up);
-        if (!(fine && isfinite(n0x) && isfinite(n0y))) atomicOr(c.err, 1);
-        h[0][0] = __double2float_rn(n0x);
-        h[0][1] = __double2float_rn(n0y);
-        h[1][0] = __double2float_rn(n1x);
-        h[1][1] = __double2float_rn(n1y);
+        c.pa[ob + e][i] = make_float4(xh, yh, fmaf(yh, yh, xh * xh), c.pa[P.buf[0]][i].w);
+        c.pb[ob + e][i] = make_float4(S.lo[e][0][lane], S.lo[e][1][lane], -filter_threshold(xh, yh, E.rc2_up), 0.0f);
     }
-#pragma unroll
-    for (int e = 0; e < 2; e++) store_group_box(c.gbox[ob + e] + E.group, live, h[e][0], h[e][1], true);
+    store_group_box(c.gbox[ob + e] + E.group, live, xh, yh, true);
 }
 
 // ---------------------------------------------------------------------------
@@ -1046,30 +975,26 @@ __device__ __forceinline__ void tile_epilogue(const StageParams &P, float4 *s_re
                                               EpilogueShared *shared) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int npairs = blockDim.x >> 6, pair = ((warp >> 1) + tile) % npairs;
-    const bool both = (P.f.flags & ~kBasicForces) != 0;  // else a warp needs its own axis only
+    const int ax = warp & 1;
 #pragma unroll 1
     for (int g = pair; g < ILP; g += npairs) {
         const int e = g * 32 + lane, i = tile * 32 * ILP + e;
-        double2 f[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+        double f[2] = {0.0, 0.0};
         const double cq = (i < P.c.n) ? pair_scale(P, i) : 0.0;
         for (int set = 0; set < P.nsets; set++) {
             float4 *mine = s_red + set * stride + e;
             float4 v = *mine;
-            TwoFloatSum sx, sy;
-            sx.add(v.x);
-            sy.add(v.y);
-            float cx = v.z, cy = v.w;
+            TwoFloatSum sum;
+            sum.add(ax ? v.y : v.x);
+            float lost = ax ? v.w : v.z;
             for (int r = 1; r < S; r++) {
                 v = *cg::this_cluster().map_shared_rank(mine, r);
-                sx.add(v.x);
-                sy.add(v.y);
-                cx += v.z;
-                cy += v.w;
+                sum.add(ax ? v.y : v.x);
+                lost += ax ? v.w : v.z;
             }
-            if (both || (warp & 1) == 0) f[set].x = __dmul_rn(cq, widen(sx.hi) + widen(sx.lo - cx));
-            if (both || (warp & 1) == 1) f[set].y = __dmul_rn(cq, widen(sy.hi) + widen(sy.lo - cy));
+            f[set] = __dmul_rn(cq, widen(sum.hi) + widen(sum.lo - lost));
         }
-        pass_epilogue(P, EpilogueCloud{P.f, P.c.rc2_up, i < P.c.n, i >> 5}, i, warp & 1, kBarEpilogue + (warp >> 1), f[0],
+        pass_epilogue(P, EpilogueCloud{P.f, P.c.rc2_up, i < P.c.n, i >> 5}, i, ax, kBarEpilogue + (warp >> 1), f[0],
                       f[1], shared[g]);
     }
 }
@@ -1151,8 +1076,13 @@ __device__ __forceinline__ double finish_rank_sum(const StageParams &P, int i, i
 
 // Completes a pass after a non-cluster pair launch: one block per
 // 32-particle group, warp w < 2 nsets sums set w/2, axis w%2 over the ranks,
-// then the first two warps run the epilogue.
-static __global__ void __launch_bounds__(128) stage_finish(const StageParams P) {
+// then the first two warps run the epilogue.  ALL (forces outside
+// kBasicForces): a block of 2 kTermParts warps, which first compute the
+// position terms, a part of one set each (a chain of ~200 FP64 instructions on
+// two warps otherwise; with one warp advancing both axes too, 4095 particles
+// under every force took 17.2 us instead of 11.4).
+template <bool ALL>
+static __global__ void __launch_bounds__(ALL ? 64 * kTermParts : 128) stage_finish(const StageParams P) {
     pdl_wait();
     __shared__ EpilogueShared S;
     __shared__ double s_f[2][2][32];
@@ -1160,12 +1090,17 @@ static __global__ void __launch_bounds__(128) stage_finish(const StageParams P) 
     const int i = blockIdx.x * 32 + lane;
     if (i < P.c.n) {
         if (warp < 2) epilogue_prefetch(P, i, warp);  // the operands' round trip overlaps the partials'
+        if (ALL && warp / kTermParts < P.nsets) {
+            const int e = warp / kTermParts, b = P.buf[e];
+            position_terms(S.terms[e][lane], warp % kTermParts, P.f, P.c.px[b][i], P.c.py[b][i], P.c.q[i],
+                           (P.f.flags & kDriving) ? stage_time(P, e) : 0.0);
+        }
         if (warp < 2 * P.nsets) s_f[warp >> 1][warp & 1][lane] = finish_rank_sum(P, i, warp >> 1, warp & 1);
     }
     __syncthreads();
     if (warp < 2)
-        pass_epilogue(P, EpilogueCloud{P.f, P.c.rc2_up, i < P.c.n, i >> 5}, i, warp, kBarEpilogue, make_double2(s_f[0][0][lane], s_f[0][1][lane]),
-                      make_double2(s_f[1][0][lane], s_f[1][1][lane]), S);
+        pass_epilogue<ALL>(P, EpilogueCloud{P.f, P.c.rc2_up, i < P.c.n, i >> 5}, i, warp, kBarEpilogue, s_f[0][warp][lane],
+                           s_f[1][warp][lane], S);
     pass_step_advance(P);
 }
 
@@ -1297,21 +1232,17 @@ __global__ void __launch_bounds__(2 * NW * 32, 10 / NW) pair_group_fp64(const St
         __syncthreads();
     }
     if (mine) {
-        const bool basic = !(P.f.flags & ~kBasicForces);
         const int ax = wib & 1;
         const double cq = (i < n) ? __dmul_rn(P.coulomb, qa[i]) : 0.0;
-        double2 f[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+        double f[2] = {0.0, 0.0};
         for (int e = 0; e < P.nsets; e++) {
-            // one axis per warp where the axes are independent
-            double2 t = make_double2(0.0, 0.0);
+            double t = 0.0;
             const int terms = (S > 1) ? S : NW;
             for (int k = 0; k < terms; k++) {
                 const double2 v = (S > 1) ? *cl.map_shared_rank(&sh.set[e].red[lane], k) : sh.set[e].acc[k][lane];
-                if (!basic || ax == 0) t.x = __dadd_rn(t.x, v.x);
-                if (!basic || ax == 1) t.y = __dadd_rn(t.y, v.y);
+                t = __dadd_rn(t, ax ? v.y : v.x);
             }
-            if (!basic || ax == 0) f[e].x = __dmul_rn(cq, t.x);
-            if (!basic || ax == 1) f[e].y = __dmul_rn(cq, t.y);
+            f[e] = __dmul_rn(cq, t);
         }
         pass_epilogue(P, EpilogueCloud{P.f, P.c.rc2_up, i < n, tile}, i, ax, kBarEpilogue, f[0], f[1], sh.epi);
     }

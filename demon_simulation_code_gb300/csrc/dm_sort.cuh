@@ -692,14 +692,14 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
         }
         src[k] = o;
     }
-    const double *in[6] = {c.x, c.y, c.vx, c.vy, c.q, c.m};
-    double val[6][kSortClusterRounds];
+    const double *in[7] = {c.x, c.y, c.vx, c.vy, c.q, c.m, c.invm};
+    double val[7][kSortClusterRounds];
     int ov[kSortClusterRounds];
 #pragma unroll
     for (int k = 0; k < kSortClusterRounds; k++) {
         const bool ok = e0 + k * kSortClusterThreads + tid < n;
 #pragma unroll
-        for (int a = 0; a < 6; a++) val[a][k] = ok ? in[a][src[k]] : 0.0;
+        for (int a = 0; a < 7; a++) val[a][k] = ok ? in[a][src[k]] : 0.0;
         ov[k] = ok ? c.orig[src[k]] : 0;
     }
     // Every block of the cluster holds its sources in registers, and the
@@ -719,6 +719,7 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
             c.vy[s] = val[3][k];
             c.q[s] = val[4][k];
             c.m[s] = val[5][k];
+            c.invm[s] = val[6][k];
             c.orig[s] = ov[k];
             write_stage_position(c, 0, s, x, y);  // set 0 is the state: x, y
             h[0] = make_float2(__double2float_rn(x), __double2float_rn(y));
@@ -776,6 +777,7 @@ static __global__ void __launch_bounds__(256) permute_commit(CloudDev c, SortScr
             c.vy[s] = z.stage[3][s];
             c.q[s] = z.stage[4][s];
             c.m[s] = z.stage[5][s];
+            c.invm[s] = __drcp_rn(z.stage[5][s]);
             c.orig[s] = z.orig_stage[s];
             write_stage_position(c, 0, s, z.stage[0][s], z.stage[1][s]);  // set 0 is the state: x, y
             const float4 A = c.pa[0][s];
