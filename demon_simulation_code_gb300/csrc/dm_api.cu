@@ -56,6 +56,7 @@ struct dm_ctx {
     double prof_pairs = 0.0;
     long long prof_launches = 0;
     int *h_err = nullptr;  // pinned word for the device error flags (read with each download)
+    AdaptiveResult *h_adapt = nullptr;  // page-locked: the adaptive time step's result
     int sort_ctas = 0;     // blocks of the one-cluster sort (0: not chosen yet)
 
     int fail(int code, const char *fmt, ...) {
@@ -92,8 +93,7 @@ struct dm_cloud {
     double *d_fx = nullptr, *d_fy = nullptr;
     double *d_dt = nullptr;
     double *d_diag = nullptr;    // diagnostics: [kDiagBlocks][5] partial sums, then the 5 results
-    unsigned int *d_min = nullptr;
-    float *d_dmin = nullptr;
+    unsigned int *d_min = nullptr;  // adaptive time step: least checked r^2, finished blocks
     int order = 4;               // integrator: 4 = Runge_Kutta4, 2 = Runge_Kutta2
     int eval_thermal_stage = 1;  // substep of the thermal kicks in force-only evaluations
     bool boxes_valid[4] = {false, false, false, false};  // group boxes (culling) match position set b
@@ -151,13 +151,6 @@ int device_error_status(dm_ctx *ctx, dm_cloud *c, int h) {
         return ctx->fail(DM_ERR_NUMERIC, "non-finite particle position after a stage (error bits 0x%x)", h);
     }
     return DM_OK;
-}
-
-int check_device_errors(dm_ctx *ctx, dm_cloud *c) {
-    int h = 0;
-    DM_CUDA(ctx, cudaMemcpyAsync(&h, c->d.err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    DM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return device_error_status(ctx, c, h);
 }
 
 // The autotuners' weights of a candidate's time on the cloud as it is and on
@@ -934,6 +927,7 @@ int dm_ctx_destroy(dm_ctx *ctx) {
     }
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     if (ctx->h_err) cudaFreeHost(ctx->h_err);
+    if (ctx->h_adapt) cudaFreeHost(ctx->h_adapt);
     delete ctx;
     return DM_OK;
 }
@@ -1090,7 +1084,7 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     c->d.time = (double *)(c->d.step_ctr + 4);  // same 256-byte slot, bytes 32-47
     c->d.err = (int *)p; p += 256;
     c->d_dt = (double *)p; p += 256;
-    c->d_min = (unsigned int *)p; c->d_dmin = (float *)(p + 64); p += 256;
+    c->d_min = (unsigned int *)p; p += 256;
     auto takeI = [&]() { int *r = (int *)p; p += ni; return r; };
     c->d.orig = takeI();
     c->sort.keys[0] = (uint32_t *)takeI();
@@ -1322,23 +1316,21 @@ int dm_cloud_modify_timestep(dm_cloud *c, double init_dt, float *min_dist, doubl
     if (c->n % 4 != 0 || c->n < 4)
         return ctx->fail(DM_ERR_ARG, "adaptive time step needs n %% 4 == 0 (Integrator.cpp:87-107)");
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
-    DM_CUDA(ctx, cudaMemsetAsync(c->d_min, 0x7f, sizeof(unsigned int), ctx->stream));
-    const int nb = c->n / 4;
-    const long long total = (long long)nb * (nb + 1) / 2;
-    const int blocks = (int)std::min<long long>((total + 255) / 256, (long long)ctx->num_sms * 16);
-    // the checked pair pattern is defined on the caller's order
-    double **st = c->sort.stage;
-    scatter_to_caller<<<(c->n + 255) / 256, 256, 0, ctx->stream>>>(
-        c->d.orig, c->n, c->d.x, c->d.y, nullptr, nullptr, st[0], st[1], nullptr, nullptr);
-    DM_CUDA(ctx, cudaGetLastError());
-    checked_min_dist2<<<std::max(blocks, 1), 256, 0, ctx->stream>>>(st[0], st[1], nb, c->d_min);
-    DM_CUDA(ctx, cudaGetLastError());
-    adaptive_dt<<<1, 1, 0, ctx->stream>>>(c->d_min, init_dt, c->d_dt, c->d_dmin, c->d.err);
-    DM_CUDA(ctx, cudaGetLastError());
-    if (min_dist) DM_CUDA(ctx, cudaMemcpyAsync(min_dist, c->d_dmin, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-    if (dt_out) DM_CUDA(ctx, cudaMemcpyAsync(dt_out, c->d_dt, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    if (!ctx->h_adapt) DM_CUDA(ctx, cudaMallocHost((void **)&ctx->h_adapt, sizeof(AdaptiveResult)));
+    AdaptiveResult *host = nullptr;
+    DM_CUDA(ctx, cudaHostGetDevicePointer((void **)&host, ctx->h_adapt, 0));
+    const int nb = c->n / 4, nt = (nb + kAdaptTile - 1) / kAdaptTile;
+    const int blocks = (int)std::min<long long>((long long)nt * (nt + 1) / 2, (long long)ctx->num_sms * 8);
+    float2 *pos = (float2 *)c->sort.stage[0];
+    DM_CUDA(ctx, launch_pdl(adaptive_positions, dim3((c->n + 255) / 256), dim3(256), 0, ctx->stream, c->d, pos,
+                            c->d_min));
+    DM_CUDA(ctx, launch_pdl(checked_min_dist2, dim3(blocks), dim3(256), 0, ctx->stream, (const float2 *)pos, nb,
+                            init_dt, c->d_min, c->d_dt, c->d.err, host));
+    ctx->launches += 2;
     DM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return check_device_errors(ctx, c);
+    if (min_dist) *min_dist = ctx->h_adapt->dmin;
+    if (dt_out) *dt_out = ctx->h_adapt->dt;
+    return device_error_status(ctx, c, ctx->h_adapt->err);
 }
 
 int dm_cloud_move_particles(dm_cloud *c, double end_time, double dt, int precision, int adaptive,
