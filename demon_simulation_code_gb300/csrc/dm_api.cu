@@ -38,6 +38,11 @@ std::string g_create_error;
 // group pairs costs ~3 us a stage, the re-sort ~18 us a step).
 constexpr int kFp64UnsortedMax = 4096;
 constexpr int kGraphSteps = 16;
+// States of at most this many particles in pageable memory cross through the
+// context's page-locked staging (256 KiB) and a copy kernel; larger ones by
+// DMA (eight pageable copies cost 35 us of host time a round trip, whatever the
+// size: 64 grains, one step 96 -> 58 us).
+constexpr int kStagedCopyMax = 4096;
 
 }  // namespace
 
@@ -56,6 +61,8 @@ struct dm_ctx {
     double prof_pairs = 0.0;
     long long prof_launches = 0;
     int *h_err = nullptr;  // pinned word for the device error flags (read with each download)
+    double *h_stage = nullptr, *h_stage_dev = nullptr;  // page-locked [2][4][kStagedCopyMax]: uploads, downloads
+    cudaEvent_t stage_read = nullptr;                   // the last staged upload has been read
     AdaptiveResult *h_adapt = nullptr;  // page-locked: the adaptive time step's result
     int sort_ctas = 0;     // blocks of the one-cluster sort (0: not chosen yet)
 
@@ -870,6 +877,31 @@ const void *device_view(const void *p) {
     return (a.type == cudaMemoryTypeHost && a.devicePointer) ? a.devicePointer : nullptr;
 }
 
+// Whether states of n particles are staged (see kStagedCopyMax); not under
+// stream capture, where a replay has to read the caller's memory again.
+bool staged_copies(dm_ctx *ctx, int n) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (n > kStagedCopyMax || cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess ||
+        cs != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    if (ctx->h_stage) return true;
+    void *h = nullptr, *d = nullptr;
+    cudaEvent_t ev = nullptr;
+    if (cudaMallocHost(&h, 8 * (size_t)kStagedCopyMax * sizeof(double)) == cudaSuccess &&
+        cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess &&
+        cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess) {
+        ctx->h_stage = (double *)h;
+        ctx->h_stage_dev = (double *)d;
+        ctx->stage_read = ev;
+        return true;
+    }
+    cudaGetLastError();  // no page-locked memory to be had: by DMA
+    if (h) cudaFreeHost(h);
+    return false;
+}
+
 }  // namespace
 
 // ===========================================================================
@@ -928,6 +960,8 @@ int dm_ctx_destroy(dm_ctx *ctx) {
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     if (ctx->h_err) cudaFreeHost(ctx->h_err);
     if (ctx->h_adapt) cudaFreeHost(ctx->h_adapt);
+    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+    if (ctx->stage_read) cudaEventDestroy(ctx->stage_read);
     delete ctx;
     return DM_OK;
 }
@@ -1158,6 +1192,16 @@ int dm_cloud_upload(dm_cloud *c, const double *x, const double *y, const double 
                                                            st[1], st[2], st[3], nullptr, nullptr);
         DM_CUDA(ctx, cudaGetLastError());
         ctx->launches += 1;
+    } else if (staged_copies(ctx, c->n)) {
+        const size_t n = (size_t)c->n;
+        const double *in[4] = {x, y, vx, vy}, *d = ctx->h_stage_dev;
+        DM_CUDA(ctx, cudaEventSynchronize(ctx->stage_read));
+        for (int k = 0; k < 4; k++) std::memcpy(ctx->h_stage + k * n, in[k], bytes);
+        copy4<<<(c->n + 255) / 256, 256, 0, ctx->stream>>>(c->n, d, d + n, d + 2 * n, d + 3 * n, st[0], st[1], st[2],
+                                                           st[3], nullptr, nullptr);
+        DM_CUDA(ctx, cudaGetLastError());
+        DM_CUDA(ctx, cudaEventRecord(ctx->stage_read, ctx->stream));
+        ctx->launches += 1;
     } else {
         DM_CUDA(ctx, cudaMemcpyAsync(st[0], x, bytes, cudaMemcpyHostToDevice, ctx->stream));
         DM_CUDA(ctx, cudaMemcpyAsync(st[1], y, bytes, cudaMemcpyHostToDevice, ctx->stream));
@@ -1192,6 +1236,18 @@ int dm_cloud_download(dm_cloud *c, double *x, double *y, double *vx, double *vy)
                                                            c->d.err, err_dv);
         DM_CUDA(ctx, cudaGetLastError());
         ctx->launches++;
+    } else if (err_dv && staged_copies(ctx, c->n)) {
+        const size_t n = (size_t)c->n;
+        const double *h = ctx->h_stage + 4 * (size_t)kStagedCopyMax;
+        double *d = ctx->h_stage_dev + 4 * (size_t)kStagedCopyMax, *out[4] = {x, y, vx, vy};
+        copy4<<<(c->n + 255) / 256, 256, 0, ctx->stream>>>(c->n, st[0], st[1], st[2], st[3], d, d + n, d + 2 * n,
+                                                           d + 3 * n, c->d.err, err_dv);
+        DM_CUDA(ctx, cudaGetLastError());
+        ctx->launches++;
+        DM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        for (int k = 0; k < 4; k++)
+            if (out[k]) std::memcpy(out[k], h + k * n, bytes);
+        return device_error_status(ctx, c, *ctx->h_err);
     } else {
         if (x) DM_CUDA(ctx, cudaMemcpyAsync(x, st[0], bytes, cudaMemcpyDeviceToHost, ctx->stream));
         if (y) DM_CUDA(ctx, cudaMemcpyAsync(y, st[1], bytes, cudaMemcpyDeviceToHost, ctx->stream));
