@@ -39,10 +39,10 @@ std::string g_create_error;
 constexpr int kFp64UnsortedMax = 4096;
 constexpr int kGraphSteps = 16;
 // States of at most this many particles in pageable memory cross through the
-// context's page-locked staging (256 KiB) and a copy kernel; larger ones by
+// context's page-locked staging (1 MiB) and a copy kernel; larger ones by
 // DMA (eight pageable copies cost 35 us of host time a round trip, whatever the
-// size: 64 grains, one step 96 -> 58 us).
-constexpr int kStagedCopyMax = 4096;
+// size: 64 grains, one step 96 -> 58 us; 16,384 FP64, one step 242 -> 220 us).
+constexpr int kStagedCopyMax = 16384;
 
 }  // namespace
 
@@ -115,7 +115,9 @@ struct dm_cloud {
     SortScratch sort{};
     int sort_blocks = 0;
     int reorder_interval = 1;   // steps between Morton re-sorts (0 = never)
-    bool order_dirty = true;    // re-sort before the next step
+    bool order_dirty = true;    // re-sort before the next step ...
+    int dirty_upload = 0;       // ... if upload of this number changed the state (0: in any case)
+    int uploads = 0;
     unsigned long long host_steps = 0;  // RK4 steps enqueued so far
     long long graph_launches = 0;       // kernels in one replay of the step graph
     std::map<GraphKey, cudaGraphExec_t> graphs;
@@ -743,12 +745,13 @@ int reorder(dm_cloud *c, double dt, bool mid, bool force) {
         const float4 *pa0 = c->d.pa[0];
         const bool mid_ready = c->mid_valid && c->mid_dt == dt && c->boxes_valid[1];
         force = force || !c->boxes_valid[0];
+        const int upload = c->order_dirty ? c->dirty_upload : 0;
         if (ctx->sort_ctas == 16) {
             const cudaLaunchConfig_t cfg = sort_cluster_cfg<16>(s, attr);
-            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<16>, pa0, c->d, z, dt, mid, mid_ready, force));
+            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<16>, pa0, c->d, z, dt, mid, mid_ready, force, upload));
         } else {
             const cudaLaunchConfig_t cfg = sort_cluster_cfg<8>(s, attr);
-            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<8>, pa0, c->d, z, dt, mid, mid_ready, force));
+            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<8>, pa0, c->d, z, dt, mid, mid_ready, force, upload));
         }
         c->state_changed(true);
         c->boxes_valid[1] = c->mid_valid = mid;
@@ -764,7 +767,8 @@ int reorder(dm_cloud *c, double dt, bool mid, bool force) {
     const bool mid_ready = c->mid_valid && c->mid_dt == dt && c->boxes_valid[1];
     const int *keep = (force || !c->boxes_valid[0]) ? nullptr : z.keep;
     if (keep) {
-        DM_CUDA(ctx, launch_pdl(order_check, dim3(1), dim3(1024), 0, s, c->d, z, cblocks));
+        DM_CUDA(ctx, launch_pdl(order_check, dim3(1), dim3(1024), 0, s, c->d, z, cblocks,
+                                c->order_dirty ? c->dirty_upload : 0));
         ctx->launches++;
     }
     DM_CUDA(ctx, launch_pdl(sort_moments, dim3(mblocks), dim3(256), 0, s, pa0, n, z.moments, keep));
@@ -786,7 +790,8 @@ int reorder_if_due(dm_cloud *c, int precision, double dt, bool mid) {
     if (!wants_order(c->n, precision)) return DM_OK;
     if (c->order_dirty || (c->reorder_interval > 0 && c->host_steps % (unsigned)c->reorder_interval == 0))
         return reorder(c, dt, mid,
-                       c->order_dirty || c->reorder_interval != 1 || c->host_steps % (unsigned)kOrderKeep == 0);
+                       (c->order_dirty && c->dirty_upload == 0) || c->reorder_interval != 1 ||
+                           c->host_steps % (unsigned)kOrderKeep == 0);
     return DM_OK;
 }
 
@@ -1128,7 +1133,8 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     c->sort.orig_stage = takeI();
     for (int k = 0; k < 6; k++) c->sort.stage[k] = takeD();
     c->sort.hist = (uint32_t *)p; p += nh;
-    c->sort.box = (double *)p; c->sort.keep = (int *)(p + 64); p += 256;
+    c->sort.box = (double *)p; c->sort.keep = (int *)(p + 64);
+    c->sort.changed = (int *)(p + 68); p += 256;
     c->sort.cost = (float *)p; p += nco;
     c->sort.moments = (float *)p; p += align256(sizeof(float) * kMomentBlocks * kMomentFields);
     c->d_diag = (double *)p; p += align256(sizeof(double) * 5 * (kDiagBlocks + 1));
@@ -1208,11 +1214,13 @@ int dm_cloud_upload(dm_cloud *c, const double *x, const double *y, const double 
         DM_CUDA(ctx, cudaMemcpyAsync(st[2], vx, bytes, cudaMemcpyHostToDevice, ctx->stream));
         DM_CUDA(ctx, cudaMemcpyAsync(st[3], vy, bytes, cudaMemcpyHostToDevice, ctx->stream));
     }
-    upload_internal_order<<<(c->n_pad + 255) / 256, 256, 0, ctx->stream>>>(c->d, c->sort);
+    // the uploaded positions may be far from the old order
+    if (!c->order_dirty) c->dirty_upload = ++c->uploads;
+    c->order_dirty = true;
+    upload_internal_order<<<(c->n_pad + 255) / 256, 256, 0, ctx->stream>>>(c->d, c->sort, c->dirty_upload);
     c->state_changed(true);
     DM_CUDA(ctx, cudaGetLastError());
     ctx->launches += 1;
-    c->order_dirty = true;  // the uploaded positions may be far from the old order
     return DM_OK;
 }
 

@@ -62,6 +62,7 @@ struct SortScratch {
     double *box;               // [8]: key box x0, y0, extent; -; bounding box min x, min y, max x, max y
     float *cost;               // order_cost of the cloud as last sorted, per block of the kernel that wrote it
     int *keep;                 // set by order_check: the order is still good
+    int *changed;              // number of the last upload that changed the state
     uint32_t *keys[2];
     int *vals[2];
     uint32_t *hist;            // [kSortBuckets * nblocks], then [kSortBuckets] totals
@@ -303,7 +304,7 @@ __device__ __forceinline__ void write_midpoint_group(const CloudDev &c, int s, b
 __device__ __forceinline__ bool order_is_kept(const int *keep) { return keep && *keep; }
 
 // One block: whether the cloud's order is still good.
-static __global__ void __launch_bounds__(1024) order_check(CloudDev c, SortScratch z, int ncost) {
+static __global__ void __launch_bounds__(1024) order_check(CloudDev c, SortScratch z, int ncost, int upload) {
     pdl_wait();
     __shared__ float s[32][2];
     const float rc = sqrtf(c.rc2_up);
@@ -311,7 +312,7 @@ static __global__ void __launch_bounds__(1024) order_check(CloudDev c, SortScrat
     for (int g = threadIdx.x; g < (c.n + 31) / 32; g += 1024) now += order_cost(c.gbox[0][g], rc);
     for (int b = threadIdx.x; b < ncost; b += 1024) was += z.cost[b];
     const bool kept = block_order_kept<32>(now, was, s);
-    if (threadIdx.x == 0) *z.keep = kept;
+    if (threadIdx.x == 0) *z.keep = kept && (upload == 0 || *z.changed != upload);
 }
 
 // Per-block moments of the cloud's positions (origin: its first particle).
@@ -523,13 +524,14 @@ constexpr size_t sort_cluster_smem() { return sizeof(SortClusterSmem<CTAS>); }
 // pa0: the FP32 hi parts of the current positions (position set 0 holds them
 // at every step boundary).  The cloud's x, y, vx, vy, q, m and orig end up in
 // the new order, with position set 0, set 1 for time step dt (if mid) and
-// their group boxes rewritten.  Without `force` a cloud in good order (see
-// kOrderKeep) is left as it is; if `mid` and not `mid_ready` its set 1 is
+// their group boxes rewritten.  Without `force` (or an upload of number
+// `upload` that changed the state) a cloud in good order (see kOrderKeep) is
+// left as it is; if `mid` and not `mid_ready` its set 1 is
 // written.  Launched as one cluster of CTAS blocks.
 template <int CTAS>
 static __global__ void __launch_bounds__(kSortClusterThreads, 1)
     sort_cluster(const float4 *__restrict__ pa0, CloudDev c, SortScratch z, double dt, bool mid, bool mid_ready,
-                 bool force) {
+                 bool force, int upload) {
     constexpr int kSortClusterCtas = CTAS;
     constexpr int kSortClusterPer = SortClusterShape<CTAS>::per;
     constexpr int kSortClusterRounds = SortClusterShape<CTAS>::rounds;
@@ -543,7 +545,7 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
     const int e0 = r * kSortClusterPer;
     const float rc = sqrtf(c.rc2_up);
 
-    if (!force) {  // every block comes to the same decision, from the same sums
+    if (!force && (upload == 0 || *z.changed != upload)) {  // every block comes to the same decision
         float now = 0.0f;
         for (int g = tid; g < (n + 31) / 32; g += kSortClusterThreads) now += order_cost(c.gbox[0][g], rc);
         const float was = (tid < kSortClusterCtas) ? z.cost[tid] : 0.0f;
@@ -805,16 +807,20 @@ static __global__ void __launch_bounds__(256) permute_commit(CloudDev c, SortScr
 // An upload in the caller's order (staging arrays 0..3: x, y, vx, vy) put
 // straight into the cloud's current internal order, with position set 0 and
 // the boxes of its 32-particle groups: charges, masses and the order itself
-// stay where they are (the next re-sort starts from them).
-static __global__ void upload_internal_order(CloudDev c, SortScratch z) {
+// stay where they are (the next re-sort starts from them).  An upload that
+// changes the state leaves its number: a program that downloads and uploads
+// the same state between steps keeps the order (and the bits) of one that
+// only steps.
+static __global__ void upload_internal_order(CloudDev c, SortScratch z, int upload) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= c.n_pad) return;  // whole warps: n_pad is a multiple of 64
     float xh = 0.0f, yh = 0.0f;
     if (s < c.n) {
         const int o = c.orig[s];
-        const double x = z.stage[0][o], y = z.stage[1][o];
-        c.vx[s] = z.stage[2][o];
-        c.vy[s] = z.stage[3][o];
+        const double x = z.stage[0][o], y = z.stage[1][o], vx = z.stage[2][o], vy = z.stage[3][o];
+        if (!(x == c.x[s] && y == c.y[s] && vx == c.vx[s] && vy == c.vy[s])) *z.changed = upload;
+        c.vx[s] = vx;
+        c.vy[s] = vy;
         write_stage_position(c, 0, s, x, y);  // set 0 is the state: x, y
         const float4 A = c.pa[0][s];
         xh = A.x;

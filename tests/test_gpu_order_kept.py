@@ -54,3 +54,21 @@ def test_batch_trajectory_with_skipped_sorts(gpu_ctx, oracle_lib, speed):
     for k, c0 in enumerate(clouds):
         for comp, ref in enumerate(oracle_run(oracle_lib, c0)):
             assert np.array_equal(parts[comp][k], ref)
+
+
+@pytest.mark.parametrize("n", [16384, 20000])
+def test_round_trips_between_steps_keep_the_bits(gpu_ctx, n):
+    """Uploading the state just downloaded changes nothing: the order, and
+    with it every bit of the FP32C sums, stays that of a run without."""
+    c0 = W.disk_cloud(n, 2e-2, 11)
+    a, b = DeviceCloud.from_cloud(gpu_ctx, c0), DeviceCloud.from_cloud(gpu_ctx, c0)
+    for c in (a, b):
+        c.set_kernel("fp32c<4,2,128,false,cull>", 8)
+    for _ in range(10):
+        a.step(1, 1e-5, "fp32c")
+        b.upload(*b.download())
+        b.step(1, 1e-5, "fp32c")
+    for u, v in zip(a.download(), b.download()):
+        assert np.array_equal(u, v)
+    a.close()
+    b.close()
