@@ -1,8 +1,8 @@
 #!/usr/bin/env python
 """Benchmark of the DEMON RK4 / shielded-Coulomb hot path on GB300.
 
-One "step" is one RK4 step (four fused pair-force + stage launches) of the
-workload's cloud.  Metric: pair-interactions/s = 4 * N(N-1) * steps / time
+One "step" is one RK4 step (two passes, each the pair sums of two force
+evaluations and their epilogues) of the workload's cloud.  Metric: pair-interactions/s = 4 * N(N-1) * steps / time
 (ordered pairs i != j, four force evaluations per RK4 step), whole job.
 
     python bench.py [--steps K] [--warmup W] [--workload disk16k]
@@ -448,7 +448,7 @@ def run_gb300(args, world, rank, local):
         if e - prev > dense_sw:
             dense_k, dense_state, dense_sw = k, st, e - prev
         prev = e
-    pair_ms, launches, _ = ctx.profile_read()
+    pair_ms, launches, launch_pairs = ctx.profile_read()
     ctx.profile(False)
     keep32[K] = B.download()
     replay_identical = all(np.array_equal(a, b) for a, b in zip(keep32[K], end_state))
@@ -534,7 +534,7 @@ def run_gb300(args, world, rank, local):
         traj.append({"step": k, "rms_over_R": float(np.sqrt(np.mean(d ** 2))), "max_over_R": float(d.max())})
     parity["trajectory_fp32c_vs_fp64"] = traj
 
-    # batched workload (256 clouds of uneven N, one persistent launch per stage)
+    # batched workload (256 clouds of uneven N, two launches per pass)
     batch = None
     if args.batch_steps > 0:
         from demon_simulation_code_gb300 import DeviceBatch
@@ -674,8 +674,8 @@ def run_gb300(args, world, rank, local):
     # roofline of the dominant kernel (the pair launch; FP32 pipe bound)
     peak = ctx.probe_peak("fp32")
     avg_launch_s = pair_ms / 1e3 / max(launches, 1)
-    achieved = FLOPS_PER_PAIR * n * (n - 1) / avg_launch_s / 1e12
-    kname = "pair_stage_fp32c" if prec == "fp32c" else "pair_stage_fp64"
+    achieved = FLOPS_PER_PAIR * launch_pairs / max(pair_ms / 1e3, 1e-12) / 1e12  # a launch covers two evaluations
+    kname = "pair_stage_fp32c" if prec == "fp32c" else "pair_group_fp64"
     swept_frac = swept / (pairs_step * K) if swept > 0 else 1.0
     traffic = traffic_from_profiles(kname + ("_cull" if "cull" in tuned[0] else ""), w.name)
 
