@@ -1588,12 +1588,12 @@ struct BatchVariant {
     int nt, tile;
     size_t smem;
     const void *fn;
-    cudaError_t (*launch)(const cudaLaunchConfig_t *, const StageParams &, const BatchCloud *, const int2 *);
+    cudaError_t (*launch)(const cudaLaunchConfig_t *, const StageParams &, const BatchCloud *, const BatchItem *);
 };
 
 template <int NW, int ILP, int TC, bool CULL>
 cudaError_t launch_batch(const cudaLaunchConfig_t *cfg, const StageParams &P, const BatchCloud *desc,
-                         const int2 *items) {
+                         const BatchItem *items) {
     return cudaLaunchKernelEx(cfg, batch_stage_fp32c<NW, ILP, TC, CULL>, P, desc, items);
 }
 
@@ -1624,7 +1624,7 @@ struct dm_batch {
     std::vector<int> hn;
     BatchCloud *ddesc = nullptr;
     int *dseg = nullptr;
-    int2 *ditems[kNumBatchVariants] = {nullptr};
+    BatchItem *ditems[kNumBatchVariants] = {nullptr};
     int nitems[kNumBatchVariants] = {0};
     double *dbox = nullptr;  // [nclouds][8] key box and bounding box (batch_boxes)
     SortScratch sort{};
@@ -1794,18 +1794,18 @@ int batch_tune(dm_batch *B) {
         const BatchVariant &k = kBatchVariants[v];
         DM_CUDA(ctx, cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem));
         // work items (cloud, tile), largest clouds first
-        std::vector<int2> items;
+        std::vector<BatchItem> items;
         std::vector<int> order(B->nclouds);
         for (int c = 0; c < B->nclouds; c++) order[c] = c;
         std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return B->hn[a] > B->hn[b]; });
         for (int c : order)
-            for (int t = 0; t * k.tile < B->hn[c]; t++) items.push_back(make_int2(c, t));
+            for (int t = 0; t * k.tile < B->hn[c]; t++) items.push_back({c, t, B->hdesc[c].off, B->hn[c]});
         B->nitems[v] = (int)items.size();
         if (!B->ditems[v]) {
-            DM_CUDA(ctx, cudaMalloc((void **)&B->ditems[v], items.size() * sizeof(int2)));
+            DM_CUDA(ctx, cudaMalloc((void **)&B->ditems[v], items.size() * sizeof(BatchItem)));
             B->extra.push_back(B->ditems[v]);
         }
-        DM_CUDA(ctx, cudaMemcpyAsync(B->ditems[v], items.data(), items.size() * sizeof(int2),
+        DM_CUDA(ctx, cudaMemcpyAsync(B->ditems[v], items.data(), items.size() * sizeof(BatchItem),
                                      cudaMemcpyHostToDevice, ctx->stream));
     }
     int best = 0;

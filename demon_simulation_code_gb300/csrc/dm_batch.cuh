@@ -31,56 +31,67 @@ struct BatchCloud {
     float nkl2e;    // -kappa*log2(e)
 };
 
-// The StageParams of one cloud in shared memory: a copy of the batch's with
-// pointers offset to the cloud's particles.  Every thread of the block.
-__device__ __forceinline__ void batch_view(StageParams &V, const StageParams &P0, const BatchCloud *desc) {
-    static_assert(sizeof(StageParams) % 4 == 0, "copied by words");
-    for (int k = threadIdx.x; k < (int)(sizeof(StageParams) / 4); k += blockDim.x)
-        reinterpret_cast<uint32_t *>(&V)[k] = reinterpret_cast<const uint32_t *>(&P0)[k];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int o = desc->off, n = desc->n, goff = desc->goff;
-        CloudDev &c = V.c;
-        c.x += o; c.y += o; c.vx += o; c.vy += o; c.q += o; c.m += o;
-        for (int k = 0; k < 2; k++) { c.k1[k] += o; c.k2[k] += o; }
-        c.invm += o;
-        for (int b = 0; b < 4; b++) {
-            c.px[b] += o; c.py[b] += o; c.pa[b] += o; c.pb[b] += o;
-            c.gbox[b] += goff;  // group boxes numbered within the cloud
-        }
-        c.orig += o;  // values stay global caller indices (thermal counter, outputs)
-        c.n = n;
-        c.n_pad = n;
-        c.rc2 = desc->rc2;
-        c.rc2_up = desc->rc2_up;
-        V.rc2 = desc->rc2;
-        V.rc2_lo = desc->rc2_lo;
-        V.rc2_hi = desc->rc2_hi;
-        V.kappa_f = desc->kappa_f;
-        V.nkl2e = desc->nkl2e;
-    }
-    for (int k = threadIdx.x; k < (int)(sizeof(ForceParams) / 4); k += blockDim.x)
-        reinterpret_cast<uint32_t *>(&V.f)[k] = reinterpret_cast<const uint32_t *>(&desc->f)[k];
-    __syncthreads();
-}
+// A work item: a tile of a cloud, the cloud's first particle and size.
+struct BatchItem {
+    int cloud, tile, off, n;
+};
 
+// ... of a batch's cloud by value, in shared memory (see StageView).
+struct SweepView {
+    const float4 *pa_, *pb_;
+    const double *px_, *py_;
+    const float4 *gbox_;
+    unsigned long long *eval_pairs_;
+    double kappa_;
+    int n_;
+    float rc2_lo_, rc2_hi_, kappa_f_, nkl2e_;
+    int direct_min_;
+    float near_direct_f2_;
+    __device__ __forceinline__ int n() const { return n_; }
+    __device__ __forceinline__ const float4 *pa() const { return pa_; }
+    __device__ __forceinline__ const float4 *pb() const { return pb_; }
+    __device__ __forceinline__ const double *px() const { return px_; }
+    __device__ __forceinline__ const double *py() const { return py_; }
+    __device__ __forceinline__ const float4 *gbox() const { return gbox_; }
+    __device__ __forceinline__ const float4 *gsuper() const { return nullptr; }
+    __device__ __forceinline__ unsigned long long *eval_pairs() const { return eval_pairs_; }
+    __device__ __forceinline__ double kappa() const { return kappa_; }
+    __device__ __forceinline__ float rc2_lo() const { return rc2_lo_; }
+    __device__ __forceinline__ float rc2_hi() const { return rc2_hi_; }
+    __device__ __forceinline__ float kappa_f() const { return kappa_f_; }
+    __device__ __forceinline__ float nkl2e() const { return nkl2e_; }
+    __device__ __forceinline__ int direct_min() const { return direct_min_; }
+    __device__ __forceinline__ float near_direct_f2() const { return near_direct_f2_; }
+};
+
+// Only what the sweep reads is fetched of a cloud's record, by one thread, and
+// the item itself holds the cloud's place (256 clouds: 221 us a launch; with a
+// copy of all the launch's parameters per block 242 us).
 template <int NW, int ILP, int TC, bool CULL = false>
 __global__ void __launch_bounds__(NW * 32, fp32c_min_blocks<NW, ILP>())
-    batch_stage_fp32c(const StageParams P0, const BatchCloud *__restrict__ desc, const int2 *__restrict__ items) {
+    batch_stage_fp32c(const StageParams P, const BatchCloud *__restrict__ desc, const BatchItem *__restrict__ items) {
     constexpr int TILE = 32 * ILP;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ StageParams sV;
+    __shared__ SweepView V;
     const float4 *s_red = reinterpret_cast<const float4 *>(smem_raw) + Fp32cSmem<NW, ILP, TC>::red_offset;
     pdl_wait();
-    const int set = blockIdx.x % P0.nsets;
-    const int2 w = items[blockIdx.x / P0.nsets];
-    batch_view(sV, P0, desc + w.x);
-    fp32c_sweep<NW, ILP, TC, CULL>(sV, sV.buf[set], w.y, 0, 1, threadIdx.x, [] { __syncthreads(); }, smem_raw);
-    const int first = (int)(sV.c.x - P0.c.x) + w.y * TILE, n = min(TILE, sV.c.n - w.y * TILE);
+    const int set = blockIdx.x % P.nsets;
+    const BatchItem w = items[blockIdx.x / P.nsets];
+    if (threadIdx.x == 0) {
+        const BatchCloud &d = desc[w.cloud];
+        const CloudDev &c = P.c;
+        const int b = P.buf[set];
+        V = {c.pa[b] + w.off, c.pb[b] + w.off, c.px[b] + w.off, c.py[b] + w.off, c.gbox[b] + d.goff,
+             c.eval_pairs,    d.f.shielding,   w.n,             d.rc2_lo,        d.rc2_hi,           d.kappa_f,
+             d.nkl2e,         P.direct_min,    P.near_direct_f2};
+    }
+    __syncthreads();
+    fp32c_sweep<NW, ILP, TC, CULL>(V, w.tile, 0, 1, threadIdx.x, [] { __syncthreads(); }, smem_raw);
+    const int first = w.off + w.tile * TILE, n = min(TILE, w.n - w.tile * TILE);
     for (int e = threadIdx.x; e < n; e += NW * 32) {
         const float4 v = s_red[e];
-        P0.partial[(size_t)(2 * set) * P0.c.n_pad + first + e] = make_float2(v.x, v.z);
-        P0.partial[(size_t)(2 * set + 1) * P0.c.n_pad + first + e] = make_float2(v.y, v.w);
+        P.partial[(size_t)(2 * set) * P.c.n_pad + first + e] = make_float2(v.x, v.z);
+        P.partial[(size_t)(2 * set + 1) * P.c.n_pad + first + e] = make_float2(v.y, v.w);
     }
 }
 

@@ -129,17 +129,41 @@ __device__ __forceinline__ void pair2_terms(const PairI &I, float2 nxh, float2 n
     w = mul2(mul2(q, ex), mul2(mul2(y, y), add2(y, kap)));
 }
 
+// What a sweep reads of its cloud and position set b: of a launch's parameters
+// as they are needed (they are constants; held as values they cost the sweep
+// registers, 3% on 262,144 particles) ...
+struct StageView {
+    const StageParams &P;
+    int b;
+    __device__ __forceinline__ int n() const { return P.c.n; }
+    __device__ __forceinline__ const float4 *pa() const { return P.c.pa[b]; }  // packed positions
+    __device__ __forceinline__ const float4 *pb() const { return P.c.pb[b]; }
+    __device__ __forceinline__ const double *px() const { return P.c.px[b]; }
+    __device__ __forceinline__ const double *py() const { return P.c.py[b]; }
+    __device__ __forceinline__ const float4 *gbox() const { return P.c.gbox[b]; }
+    __device__ __forceinline__ const float4 *gsuper() const { return P.c.gsuper[b]; }
+    __device__ __forceinline__ unsigned long long *eval_pairs() const { return P.c.eval_pairs; }
+    __device__ __forceinline__ double kappa() const { return P.f.shielding; }
+    __device__ __forceinline__ float rc2_lo() const { return P.rc2_lo; }  // these bracket r_c^2: r^2 between
+    __device__ __forceinline__ float rc2_hi() const { return P.rc2_hi; }  // them needs the reference's decision
+    __device__ __forceinline__ float kappa_f() const { return P.kappa_f; }
+    __device__ __forceinline__ float nkl2e() const { return P.nkl2e; }  // -kappa log2(e)
+    __device__ __forceinline__ int direct_min() const { return P.direct_min; }
+    __device__ __forceinline__ float near_direct_f2() const { return P.near_direct_f2; }
+};
+
 // The scalar form of one pair for the slow path (pairs within 4e-6 of the
 // cutoff in r^2, decided exactly as the reference decides): w as in
 // pair2_terms, 0 for a pair outside the cutoff.  j values negated.
-__device__ __forceinline__ float border_pair(const StageParams &P, int b, const PairI &I, int ii, float nxh,
+template <class View>
+__device__ __forceinline__ float border_pair(const View &P, const PairI &I, int ii, float nxh,
                                              float nyh, float nxl, float nyl, float q, int jg, float &dx,
                                              float &dy) {
     dx = (I.xh.x + nxh) + (I.xl.x + nxl);
     dy = (I.yh.x + nyh) + (I.yl.x + nyl);
     double r, a;
     if (jg == ii || jg < 0 ||
-        !ref_in_cutoff(P.c.px[b][ii] - P.c.px[b][jg], P.c.py[b][ii] - P.c.py[b][jg], P.f.shielding, r, a))
+        !ref_in_cutoff(P.px()[ii] - P.px()[jg], P.py()[ii] - P.py()[jg], P.kappa(), r, a))
         return 0.0f;
     const float r2 = fmaf(dx, dx, dy * dy);
     float y = rsqrt_approx(r2);
@@ -147,8 +171,8 @@ __device__ __forceinline__ float border_pair(const StageParams &P, int b, const 
     const float h = -0.5f * fmaf(u, y, -1.0f);
     y = fmaf(h, y, y);
     const float rr = fmaf(h, u, u);
-    const float ex = ex2_approx(rr * P.nkl2e);
-    return (q * ex) * ((y * y) * (y + P.kappa_f));
+    const float ex = ex2_approx(rr * P.nkl2e());
+    return (q * ex) * ((y * y) * (y + P.kappa_f()));
 }
 
 // Conservative FP32 test: can any point of box a come within the cutoff of
@@ -347,14 +371,14 @@ struct Fp32cSmem {
 };
 
 // The FP32C sweep of one i tile against rank `rank` of S of the j chunks:
-// of position set buffer b: i-side setup, the classified j loop, and the combine of the NW warps'
+// of the view's position set: i-side setup, the classified j loop, and the combine of the NW warps'
 // Kahan sums into s_red[TILE] = (sx, sy, cx, cy) (force / (C q_i) = s - c).
 // By NW warps (`tid` the thread's index among them, sync() their barrier); ends
 // with them synchronised.  `P` may live in shared memory (batched
-// kernel).  Particles are those of P.c (n = P.c.n); j at or beyond n read as
+// kernel).  j at or beyond n read as
 // padding, so a cloud needs no padding of its own.
-template <int NW, int ILP, int TC, bool CULL, class Sync>
-__device__ __forceinline__ void fp32c_sweep(const StageParams &P, int b, int tile, int rank, int S, int tid, Sync sync,
+template <int NW, int ILP, int TC, bool CULL, class View, class Sync>
+__device__ __forceinline__ void fp32c_sweep(const View &P, int tile, int rank, int S, int tid, Sync sync,
                                             unsigned char *smem_raw) {
     constexpr int NT = NW * 32;
     constexpr int TILE = 32 * ILP;  // particles per i tile
@@ -371,12 +395,12 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int b, int til
     float4 *s_red = s_acc + NW * ILP * 32;                 // [TILE]
 
     const int lane = tid & 31, warp = tid >> 5;
-    const int n = P.c.n;
-    const float4 *__restrict__ pa = P.c.pa[b];
-    const float4 *__restrict__ pb = P.c.pb[b];
+    const int n = P.n();
+    const float4 *__restrict__ pa = P.pa();
+    const float4 *__restrict__ pb = P.pb();
     float4 *my_acc = s_acc + warp * ILP * 32;
-    const float2 kap = dup2(P.kappa_f), nkl2e = dup2(P.nkl2e);
-    const float rc2_lo = P.rc2_lo, rc2_hi = P.rc2_hi;
+    const float2 kap = dup2(P.kappa_f()), nkl2e = dup2(P.nkl2e());
+    const float rc2_lo = P.rc2_lo(), rc2_hi = P.rc2_hi();
 
     // every warp owns the same TILE particles: lane l, slot k -> i = tile*TILE + k*32 + l.
     // i side duplicated into both halves of a packed pair: the packed FMAs
@@ -471,11 +495,11 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int b, int til
             w.y = (r2.y < rc2_lo && g1 != ii && two) ? w.y : 0.0f;
             if (!(r2.x < rc2_lo) && r2.x < rc2_hi) {
                 float bx, by;
-                w.x = border_pair(P, b, I, ii, s_xf[j0], s_yf[j0], s_xlf[j0], s_ylf[j0], s_qf[j0], g0, bx, by);
+                w.x = border_pair(P, I, ii, s_xf[j0], s_yf[j0], s_xlf[j0], s_ylf[j0], s_qf[j0], g0, bx, by);
             }
             if (two && !(r2.y < rc2_lo) && r2.y < rc2_hi) {
                 float bx, by;
-                w.y = border_pair(P, b, I, ii, s_xf[j1], s_yf[j1], s_xlf[j1], s_ylf[j1], s_qf[j1], g1, bx, by);
+                w.y = border_pair(P, I, ii, s_xf[j1], s_yf[j1], s_xlf[j1], s_ylf[j1], s_qf[j1], g1, bx, by);
             }
             const float2 fx = mul2(w, dx), fy = mul2(w, dy);
             kahan_add(acc.x, acc.z, fx.x + fx.y);
@@ -521,7 +545,7 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int b, int til
                 if (rr < rc2_lo || !(rr < rc2_hi)) continue;
                 const int jj = 4 * c + u;
                 float bx, by;
-                const float wb = border_pair(P, b, I, ii, s_xf[jj], s_yf[jj], s_xlf[jj], s_ylf[jj], s_qf[jj],
+                const float wb = border_pair(P, I, ii, s_xf[jj], s_yf[jj], s_xlf[jj], s_ylf[jj], s_qf[jj],
                                              s_jf[jj], bx, by);
                 fx.x = fmaf(wb, bx, fx.x);
                 fy.x = fmaf(wb, by, fy.x);
@@ -662,7 +686,7 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int b, int til
 #pragma unroll
                 for (int k = 0; k < ILP; k++) {
                     if (gn < 8) m[k] <<= 32 - 4 * gn;
-                    if ((int)__reduce_add_sync(0xffffffffu, __popc(m[k])) >= 8 * P.direct_min) {
+                    if ((int)__reduce_add_sync(0xffffffffu, __popc(m[k])) >= 8 * P.direct_min()) {
 #pragma unroll 1
                         for (int g = 0; g < gn; g++) direct_chunk(c0 + g * NW, k);
                         m[k] = 0u;
@@ -697,7 +721,7 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int b, int til
         // the 32-particle groups whose box is within the cutoff of the tile's
         // box (the others hold no pair the reference counts), dealt
         // round-robin to the ranks, class by class
-        const float4 *__restrict__ gb = P.c.gbox[b];
+        const float4 *__restrict__ gb = P.gbox();
         NearLists<NW, 3> &L = *reinterpret_cast<NearLists<NW, 3> *>(s_red + TILE);
         const int ngroups = (n + 31) >> 5;
         float4 tb = gb[tile * ILP];
@@ -709,16 +733,16 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int b, int til
             }
         }
         unsigned long long swept = 0ull;
-        const float rc2_mostly = P.rc2_lo * P.near_direct_f2;  // 0: no such class
-        const float4 *gs = P.c.gsuper[b];
+        const float rc2_mostly = P.rc2_lo() * P.near_direct_f2();  // 0: no such class
+        const float4 *gs = P.gsuper();
         // the ranks share the tests (rank r takes every S-th group), or, with
         // super groups, the groups found
         const int deal = gs ? S : 1, mine_of = gs ? rank : 0;
         for_near_groups(
-            L, gb, gs, ngroups, gs ? 0 : rank, gs ? 1 : S, tb, P.rc2_hi, tid, sync,
+            L, gb, gs, ngroups, gs ? 0 : rank, gs ? 1 : S, tb, P.rc2_hi(), tid, sync,
             [&](int g, const float4 &gbox) {
                 // the tile's own groups hold the pairs j == i: not "inside"
-                if (g / ILP != tile && boxes_inside(tb, gbox, P.rc2_lo)) return 1;
+                if (g / ILP != tile && boxes_inside(tb, gbox, P.rc2_lo())) return 1;
                 // farthest separation within sqrt(near_direct_f2) r_c: most
                 // pairs pass the filter, so it is skipped
                 return (rc2_mostly > 0.0f && boxes_inside(tb, gbox, rc2_mostly)) ? 2 : 0;
@@ -732,7 +756,7 @@ __device__ __forceinline__ void fp32c_sweep(const StageParams &P, int b, int til
                 swept += (unsigned long long)(total[0] + total[1] + total[2]);
             });
         if (tid == 0 && (rank == 0 || !gs) && swept)
-            atomicAdd(P.c.eval_pairs, swept * 32ull * (unsigned long long)TILE);
+            atomicAdd(P.eval_pairs(), swept * 32ull * (unsigned long long)TILE);
     }
 
     // combine the NW warps in fixed order with a compensated FP32 sum (each
@@ -1011,7 +1035,7 @@ __global__ void __launch_bounds__((CL ? 2 : 1) * NW * 32, fp32c_min_blocks<(CL ?
     if constexpr (!CL) {
         const int S = P.split, r = (int)(blockIdx.x % (S * P.nsets)), set = r / S, rank = r % S;
         const int tile = blockIdx.x / (S * P.nsets), tid = threadIdx.x;
-        fp32c_sweep<NW, ILP, TC, CULL>(P, P.buf[set], tile, rank, S, tid, [] { __syncthreads(); }, smem_raw);
+        fp32c_sweep<NW, ILP, TC, CULL>(StageView{P, P.buf[set]}, tile, rank, S, tid, [] { __syncthreads(); }, smem_raw);
         for (int e = tid; e < TILE; e += NW * 32)
             if (tile * TILE + e < n) {
                 const float4 v = s_red[e];
@@ -1022,7 +1046,7 @@ __global__ void __launch_bounds__((CL ? 2 : 1) * NW * 32, fp32c_min_blocks<(CL ?
         static_assert(sizeof(EpilogueShared) * ILP <= Fp32cSmem<NW, ILP, TC>::tile, "epilogue over the j tile");
         const int S = (int)cg::this_cluster().num_blocks(), rank = (int)cg::this_cluster().block_rank();
         const int tile = blockIdx.x / S, set = threadIdx.x / (NW * 32), tid = threadIdx.x % (NW * 32);
-        fp32c_sweep<NW, ILP, TC, CULL>(P, P.buf[set], tile, rank, S, tid, [&] { bar_sync(kBarSet + set, NW * 32); },
+        fp32c_sweep<NW, ILP, TC, CULL>(StageView{P, P.buf[set]}, tile, rank, S, tid, [&] { bar_sync(kBarSet + set, NW * 32); },
                                        smem_raw + set * kBytes);
         if (S > 1) cg::this_cluster().sync();
         else __syncthreads();
