@@ -189,14 +189,14 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_kernel(const AdjCloud *__
 // ===========================================================================
 // Fused RK4 step and its adjoint for the differentiable rollout.
 //
-// One launch per RK4 stage.  Forward (adj_step_forces): the pair force at
+// One launch per RK4 stage.  Forward (adj_step_fp64, adj_step_fp32c): the pair force at
 // the stage's input state, the per-particle forces, and the stage algebra
 // of the rollout's RK4 step in FP64 (for s = (x, y, vx, vy) and f(s) =
 // (vx, vy, Fx/m, Fy/m)):
 //     k_s = dt f(s_s),  s_2 = S + k_1/2, s_3 = S + k_2/2, s_4 = S + k_3,
 //     S' = S + (k_1 + ((k_2 + k_3) 2 + k_4)) / 6,
 // with the operations in that order (each rounded, nothing contracted).
-// Backward (adj_step_vjp, stages 4, 3, 2, 1): given lam = dL/dS', the stage
+// Backward (adj_vjp_fp64, adj_vjp_fp32c, stages 4, 3, 2, 1): given lam = dL/dS', the stage
 // weights dk_4 = lam/6, dk_3 = lam/3 + mu_4, dk_2 = lam/3 + mu_3/2,
 // dk_1 = lam/6 + mu_2/2 with mu_s = J(s_s)^T (dt dk_s), and finally
 // dL/dS = lam + mu_1 + mu_2 + mu_3 + mu_4; the parameter gradients

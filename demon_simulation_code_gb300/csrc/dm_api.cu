@@ -2,7 +2,7 @@
 //
 // One dm_ctx = one GPU + one stream.  One dm_cloud = one device-resident
 // particle cloud (layout in dm_device.cuh).  Per RK4 step the library issues
-// four launches of the fused pair+stage kernel (dm_pair.cuh); fixed-dt step
+// two passes of two force evaluations each (dm_pair.cuh); fixed-dt step
 // sequences are captured once into a CUDA graph and replayed.
 #include <cuda_runtime.h>
 
@@ -108,6 +108,8 @@ struct dm_cloud {
     bool mid_valid = false;      // position set 1 is the midpoint for time step mid_dt
     double mid_dt = 0.0;
     int slot = 0;                // current step counter / force time slot (RK2 steps alternate it)
+    bool capturing = false;      // the running call is recorded by the caller's stream capture
+    bool captured = false;       // some call was: replays change the state unseen
     int split[2] = {0, 0};  // cluster size per precision (0 = not chosen yet)
     int tuned_variant[2] = {-1, -1};  // per precision: index into kVariants
     float2 *partial = nullptr;         // [2 partial_cap][2][n_pad] non-cluster partial sums (per set and rank, axis)
@@ -529,8 +531,12 @@ int launch_variant(dm_cloud *c, int vi, int S, StageParams P) {
     c->boxes_valid[ob] = c->boxes_valid[ob + 1] = true;
     c->supers_valid[ob / 2] = false;
     if (P.order == 2) {
-        DM_CUDA(ctx, launch_pdl(adopt_sets, dim3((c->n + 255) / 256), dim3(256), 0, ctx->stream, c->d, ngroups));
-        ctx->launches++;
+        if (c->captured) {
+            DM_CUDA(ctx, launch_pdl(adopt_sets, dim3((c->n + 255) / 256), dim3(256), 0, ctx->stream, c->d, ngroups));
+            ctx->launches++;
+        } else {
+            swap_sets(c->d);
+        }
         c->boxes_valid[0] = c->boxes_valid[1] = true;
         c->supers_valid[0] = false;
     }
@@ -656,6 +662,7 @@ int tune_precision(dm_cloud *c, int precision) {
             cands.erase(std::unique(cands.begin(), cands.end()), cands.end());
             for (int S : cands) {
                 if (S > 1 && c->n_pad / S < k.min_j) continue;
+                if (S > 1 && k.cull && 32 * S > c->n_pad) continue;  // j is dealt in groups of 32: idle ranks
                 if (k.cluster) {
                     int nc = 0;
                     cudaLaunchAttribute attr[2];
@@ -808,7 +815,7 @@ int enqueue_steps(dm_cloud *c, int nsteps, double dt, int precision) {
 
 int run_steps(dm_cloud *c, int nsteps, double dt, int precision) {
     dm_ctx *ctx = c->ctx;
-    if (ctx->prof || nsteps < kGraphSteps) return enqueue_steps(c, nsteps, dt, precision);
+    if (ctx->prof || c->capturing || nsteps < kGraphSteps) return enqueue_steps(c, nsteps, dt, precision);
     if (c->graph_stream != ctx->stream) {
         c->drop_graphs();
         c->graph_stream = ctx->stream;
@@ -905,6 +912,39 @@ bool staged_copies(dm_ctx *ctx, int n) {
     cudaGetLastError();  // no page-locked memory to be had: by DMA
     if (h) cudaFreeHost(h);
     return false;
+}
+
+bool stream_capturing(dm_ctx *ctx) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess) cudaGetLastError();
+    return cs == cudaStreamCaptureStatusActive;
+}
+
+// First in every call that uses or changes the state.  What the host knows of
+// the device (valid midpoint, boxes, order) holds neither for a call that is
+// being captured, which runs when it is replayed, nor after one.  From the
+// first such call on the position sets and the slot of the step counter stay
+// where the recorded launches expect them (adopt_sets, cloud_leave).
+void cloud_enter(dm_cloud *c) {
+    c->capturing = stream_capturing(c->ctx);
+    if (c->capturing && !c->captured) {
+        c->drop_graphs();
+        c->captured = true;
+    }
+    if (!c->captured) return;
+    c->state_changed(false);
+    c->order_dirty = true;
+    c->dirty_upload = 0;
+}
+
+// Last in a call that steps: `slot` was current when it began.
+template <class Owner>
+int leave_slot(Owner *c, int slot) {
+    if (c->captured && c->slot != slot) {
+        DM_CUDA(c->ctx, launch_pdl(copy_slot, dim3(1), dim3(1), 0, c->ctx->stream, c->d, c->slot, slot));
+        c->slot = slot;
+    }
+    return DM_OK;
 }
 
 }  // namespace
@@ -1187,6 +1227,7 @@ int dm_cloud_upload(dm_cloud *c, const double *x, const double *y, const double 
     dm_ctx *ctx = c->ctx;
     if (!x || !y || !vx || !vy) return ctx->fail(DM_ERR_ARG, "dm_cloud_upload: NULL array");
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
+    cloud_enter(c);
     const size_t bytes = (size_t)c->n * sizeof(double);
     // caller order -> staging -> the cloud's current internal order (charges,
     // masses and the order stay; position set 0 and its boxes are rewritten)
@@ -1271,6 +1312,7 @@ int dm_cloud_set_charge_mass(dm_cloud *c, const double *q, const double *m) {
     if (!c) return DM_ERR_ARG;
     dm_ctx *ctx = c->ctx;
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
+    cloud_enter(c);
     const size_t bytes = (size_t)c->n * sizeof(double);
     double **st = c->sort.stage;
     // caller order -> staging -> internal order
@@ -1311,6 +1353,7 @@ int dm_cloud_eval_forces_device(dm_cloud *c, int precision, double *d_fx, double
     if (precision != DM_FP64 && precision != DM_FP32C)
         return ctx->fail(DM_ERR_ARG, "bad precision %d", precision);
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
+    cloud_enter(c);
     if (c->order_dirty && wants_order(c->n, precision)) {  // spatial order first (internal only: outputs are in the caller's order)
         const int rc = reorder(c);
         if (rc) return rc;
@@ -1363,12 +1406,15 @@ int dm_cloud_step(dm_cloud *c, int nsteps, double dt, int precision, double *t_i
     if (precision != DM_FP64 && precision != DM_FP32C)
         return ctx->fail(DM_ERR_ARG, "bad precision %d", precision);
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
+    cloud_enter(c);
     if (t_inout) {  // the force time of the first step is the caller's time
         set_time_slots<<<1, 1, 0, ctx->stream>>>(c->d.time, *t_inout);
         DM_CUDA(ctx, cudaGetLastError());
     }
+    const int slot = c->slot;
     int rc = run_steps(c, nsteps, dt, precision);
-    if (rc) return rc;
+    const int left = leave_slot(c, slot);
+    if (rc || left) return rc ? rc : left;
     if (t_inout)
         for (int s = 0; s < nsteps; s++) *t_inout += dt;
     return DM_OK;
@@ -1406,6 +1452,7 @@ int dm_cloud_move_particles(dm_cloud *c, double end_time, double dt, int precisi
     int count = 0;
     // the force time of the first step is the caller's time
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
+    cloud_enter(c);
     set_time_slots<<<1, 1, 0, ctx->stream>>>(c->d.time, t);
     DM_CUDA(ctx, cudaGetLastError());
     if (!adaptive) {
@@ -1417,17 +1464,20 @@ int dm_cloud_move_particles(dm_cloud *c, double end_time, double dt, int precisi
         int rc = dm_cloud_step(c, count, dt, precision, nullptr);
         if (rc) return rc;
     } else {
+        const int slot = c->slot;
+        int rc = DM_OK;
         while (t < end_time) {
             double step_dt = 0.0;
-            int rc = reorder_if_due(c, precision, 0.0, false);
+            rc = reorder_if_due(c, precision, 0.0, false);
             if (!rc) rc = dm_cloud_modify_timestep(c, dt, nullptr, &step_dt);
-            if (rc) return rc;
-            rc = launch_step(c, precision, 0.0, c->d_dt);
-            if (rc) return rc;
+            if (!rc) rc = launch_step(c, precision, 0.0, c->d_dt);
+            if (rc) break;
             c->host_steps++;
             t += step_dt;
             count++;
         }
+        const int left = leave_slot(c, slot);
+        if (rc || left) return rc ? rc : left;
     }
     *t_inout = t;
     if (steps) *steps = count;
@@ -1643,6 +1693,7 @@ struct dm_batch {
     bool mid_valid = false;
     double mid_dt = 0.0;
     int slot = 0;
+    bool capturing = false, captured = false;  // as dm_cloud's
     unsigned long long host_steps = 0;
     std::map<GraphKey, cudaGraphExec_t> graphs;
     cudaStream_t graph_stream = nullptr;
@@ -1711,9 +1762,13 @@ int batch_launch_pass(dm_batch *B, int pass, int mode, double dt, int buf = 0, i
     const int ob = (pass == 0) ? 2 : 0;
     B->boxes_valid[ob] = B->boxes_valid[ob + 1] = true;
     if (P.order == 2) {
-        DM_CUDA(ctx, launch_pdl(adopt_sets, dim3((B->total + 255) / 256), dim3(256), 0, ctx->stream, B->d,
-                                B->ngroups));
-        ctx->launches++;
+        if (B->captured) {
+            DM_CUDA(ctx, launch_pdl(adopt_sets, dim3((B->total + 255) / 256), dim3(256), 0, ctx->stream, B->d,
+                                    B->ngroups));
+            ctx->launches++;
+        } else {
+            swap_sets(B->d);
+        }
         B->boxes_valid[0] = B->boxes_valid[1] = true;
     }
     if (P.order == 2 || pass == 1) {
@@ -1859,6 +1914,61 @@ int batch_tune(dm_batch *B) {
     }
     B->variant = best;
     return DM_OK;
+}
+
+// nsteps of every cloud, in captured blocks where there are enough (see run_steps).
+int batch_run_steps(dm_batch *B, int nsteps, double dt) {
+    dm_ctx *ctx = B->ctx;
+    if (ctx->prof || B->capturing || nsteps < kGraphSteps) return batch_enqueue_steps(B, nsteps, dt);
+    if (B->graph_stream != ctx->stream) {
+        B->drop_graphs();
+        B->graph_stream = ctx->stream;
+    }
+    while (nsteps > 0 && (B->order_dirty || (B->reorder_interval > 0 && B->host_steps % kGraphSteps != 0))) {
+        int rc = batch_enqueue_steps(B, 1, dt);
+        if (rc) return rc;
+        nsteps--;
+    }
+    if (nsteps < kGraphSteps) return batch_enqueue_steps(B, nsteps, dt);
+    const bool sorts = B->reorder_interval > 0 && B->max_n <= kBatchSortMax;
+    if (!sorts && !(B->mid_valid && B->mid_dt == dt)) {  // the captured steps start from a midpoint (see run_steps)
+        int rc = batch_enqueue_steps(B, 1, dt);
+        return rc ? rc : batch_run_steps(B, nsteps - 1, dt);
+    }
+    const GraphKey key{DM_FP32C, kGraphSteps, dt, B->slot};
+    auto it = B->graphs.find(key);
+    static long long graph_launches_cache = 0;
+    if (it == B->graphs.end()) {
+        cudaGraph_t g = nullptr;
+        const unsigned long long saved = B->host_steps;
+        const long long sl = ctx->launches;
+        DM_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+        int rc = batch_enqueue_steps(B, kGraphSteps, dt);
+        cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
+        B->host_steps = saved;
+        graph_launches_cache = ctx->launches - sl;
+        ctx->launches = sl;
+        if (rc) {
+            if (g) cudaGraphDestroy(g);
+            return rc;
+        }
+        if (ec != cudaSuccess) return ctx->fail(DM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(ec));
+        cudaGraphExec_t ge = nullptr;
+        ec = cudaGraphInstantiate(&ge, g, 0);
+        cudaGraphDestroy(g);
+        if (ec != cudaSuccess) return ctx->fail(DM_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(ec));
+        it = B->graphs.emplace(key, ge).first;
+    }
+    const int reps = nsteps / kGraphSteps;
+    for (int r = 0; r < reps; r++) {
+        DM_CUDA(ctx, cudaGraphLaunch(it->second, ctx->stream));
+        B->host_steps += kGraphSteps;
+        ctx->launches += graph_launches_cache;
+        B->mid_valid = true;
+        B->mid_dt = dt;
+        for (bool &v : B->boxes_valid) v = true;
+    }
+    return batch_enqueue_steps(B, nsteps - reps * kGraphSteps, dt);
 }
 
 }  // namespace
@@ -2027,56 +2137,18 @@ int dm_batch_step(dm_batch *B, int nsteps, double dt, int precision) {
         return ctx->fail(DM_ERR_UNSUPPORTED, "batched clouds run the FP32C kernel; step FP64 clouds singly");
     if (nsteps < 0 || !std::isfinite(dt)) return ctx->fail(DM_ERR_ARG, "dm_batch_step: bad nsteps/dt");
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
-    if (ctx->prof || nsteps < kGraphSteps) return batch_enqueue_steps(B, nsteps, dt);
-    if (B->graph_stream != ctx->stream) {
+    B->capturing = stream_capturing(ctx);
+    if (B->capturing && !B->captured) {
         B->drop_graphs();
-        B->graph_stream = ctx->stream;
+        B->captured = true;
     }
-    while (nsteps > 0 && (B->order_dirty || (B->reorder_interval > 0 && B->host_steps % kGraphSteps != 0))) {
-        int rc = batch_enqueue_steps(B, 1, dt);
-        if (rc) return rc;
-        nsteps--;
+    if (B->captured) {  // see cloud_enter
+        B->boxes_valid[0] = B->boxes_valid[1] = B->mid_valid = false;
+        B->order_dirty = true;
     }
-    if (nsteps < kGraphSteps) return batch_enqueue_steps(B, nsteps, dt);
-    const bool sorts = B->reorder_interval > 0 && B->max_n <= kBatchSortMax;
-    if (!sorts && !(B->mid_valid && B->mid_dt == dt)) {  // the captured steps start from a midpoint (see run_steps)
-        int rc = batch_enqueue_steps(B, 1, dt);
-        return rc ? rc : dm_batch_step(B, nsteps - 1, dt, precision);
-    }
-    const GraphKey key{DM_FP32C, kGraphSteps, dt, B->slot};
-    auto it = B->graphs.find(key);
-    static long long graph_launches_cache = 0;
-    if (it == B->graphs.end()) {
-        cudaGraph_t g = nullptr;
-        const unsigned long long saved = B->host_steps;
-        const long long sl = ctx->launches;
-        DM_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        int rc = batch_enqueue_steps(B, kGraphSteps, dt);
-        cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
-        B->host_steps = saved;
-        graph_launches_cache = ctx->launches - sl;
-        ctx->launches = sl;
-        if (rc) {
-            if (g) cudaGraphDestroy(g);
-            return rc;
-        }
-        if (ec != cudaSuccess) return ctx->fail(DM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(ec));
-        cudaGraphExec_t ge = nullptr;
-        ec = cudaGraphInstantiate(&ge, g, 0);
-        cudaGraphDestroy(g);
-        if (ec != cudaSuccess) return ctx->fail(DM_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(ec));
-        it = B->graphs.emplace(key, ge).first;
-    }
-    const int reps = nsteps / kGraphSteps;
-    for (int r = 0; r < reps; r++) {
-        DM_CUDA(ctx, cudaGraphLaunch(it->second, ctx->stream));
-        B->host_steps += kGraphSteps;
-        ctx->launches += graph_launches_cache;
-        B->mid_valid = true;
-        B->mid_dt = dt;
-        for (bool &v : B->boxes_valid) v = true;
-    }
-    return batch_enqueue_steps(B, nsteps - reps * kGraphSteps, dt);
+    const int slot = B->slot;
+    const int rc = batch_run_steps(B, nsteps, dt), left = leave_slot(B, slot);
+    return rc ? rc : left;
 }
 
 int dm_batch_eval_forces(dm_batch *B, int precision, double *fx, double *fy) {

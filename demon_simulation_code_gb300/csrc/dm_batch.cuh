@@ -184,7 +184,7 @@ static __global__ void batch_keys(const double *__restrict__ x, const double *__
 // the whole cloud), rewrites the cloud's arrays in place with position sets 0
 // and 1 and their group boxes.  One launch replaces the batch-wide path
 // (per-cloud boxes, keys with the cloud index in the high bits, four radix
-// passes over every particle of every cloud, gather: fifteen dependent
+// passes over every particle of every cloud, gather: a dozen dependent
 // launches).  As in sort_cluster the key box and keys are FP32 functions of
 // the positions' hi parts (set 0), lanes with equal digits are found by
 // match_digit8, and the element order (warp, round, lane) makes every pass

@@ -30,6 +30,7 @@
 #include <cfloat>
 #include <cmath>
 #include <cstdint>
+#include <utility>
 #include <cuda_runtime.h>
 
 namespace dm {
@@ -86,6 +87,20 @@ struct CloudDev {
     double coulomb;                // 1/(4 pi eps0)
     int *orig;                     // caller's index of internal slot s (Morton order)
 };
+
+// An RK2 step's results (sets 2 and 3) become the state and its midpoint (host).
+inline void swap_sets(CloudDev &c) {
+    for (int b = 0; b < 2; b++) {
+        std::swap(c.px[b], c.px[b + 2]);
+        std::swap(c.py[b], c.py[b + 2]);
+        std::swap(c.pa[b], c.pa[b + 2]);
+        std::swap(c.pb[b], c.pb[b + 2]);
+        std::swap(c.gbox[b], c.gbox[b + 2]);
+        std::swap(c.gsuper[b], c.gsuper[b + 2]);
+    }
+    c.x = c.px[0];
+    c.y = c.py[0];
+}
 
 // Host-side check of a force parameter set, shared by every entry point that
 // takes one: DM_OK (0), or a status with *why set to a static message.

@@ -479,8 +479,8 @@ static __global__ void __launch_bounds__(kSortThreads) radix_scatter(
 // launch: per pass each block counts its digits per warp, the blocks'
 // digit totals meet through distributed shared memory, and every element is
 // stored straight into the shared memory of the block owning its new
-// position.  The multi-kernel path above needs fifteen dependent launches
-// (~0.1 ms at n = 16384); a single block was no better (one SM's issue rate).
+// position.  The multi-kernel path above needs twelve dependent launches
+// for it; a single block was no better (one SM's issue rate).
 //
 // Element order: block r, warp w, round k, lane l is element
 // r*P + w*32*R + k*32 + l (R = P / threads).  Digits are ranked in that order
