@@ -300,9 +300,9 @@ int dm_cloud_get_time(dm_cloud *cloud, double *t);
 
 /* A batch of independent clouds of uneven size, each with its own force
  * parameters (params[c]).  Arrays are concatenated in cloud order (cloud 0's
- * n[0] particles, then cloud 1's, ...).  Each RK4 stage of the whole batch is
- * one persistent FP32C launch handing out (cloud, i-tile) work items, largest
- * clouds first; kernel variants are autotuned at creation.  The reference
+ * n[0] particles, then cloud 1's, ...).  A pass (two force evaluations) of the
+ * whole batch is one FP32C launch over (cloud, i-tile, position set) work
+ * items, largest clouds first, and one launch of the epilogues; kernel variants are autotuned at creation.  The reference
  * runs one cloud per process; this has no reference counterpart beyond
  * dm_cloud_* applied to each cloud. */
 int dm_batch_create(dm_ctx *ctx, int nclouds, const int *n, const double *x,
@@ -322,7 +322,8 @@ int dm_batch_set_kernel(dm_batch *batch, const char *variant);
 /* Ordered pairs the batch's culling kernel variants swept so far (see
  * dm_cloud_evaluated_pairs). */
 int dm_batch_evaluated_pairs(dm_batch *batch, unsigned long long *pairs);
-/* The autotuned kernel variant, work-item count and persistent grid size. */
+/* The autotuned kernel variant, its (cloud, i-tile) count and the pair launch's
+ * grid size (a block per tile and position set). */
 int dm_batch_info(dm_batch *batch, char *variant, size_t len, int *nitems, int *grid);
 int dm_batch_set_step_counter(dm_batch *batch, uint64_t step);
 /* Integrator of dm_batch_step (see dm_cloud_set_integrator). */
