@@ -681,9 +681,11 @@ int tune_precision(dm_cloud *c, int precision) {
                 for (int st = 0; st < nstates && ms < 1.3f * best_ms; st++) {
                     // both sets on the same buffer: a pass's work
                     const StageParams P = make_stage_params(c, 0, kModeForceOnly, 0.0, nullptr, st, 2);
-                    // one launch, then the timed ones; up to 4096 particles without
-                    // looking at the first (a synchronisation costs as much as the launches)
-                    const bool look = c->n > 4096;
+                    // one launch, then the timed ones; up to 1024 particles without
+                    // looking at the first (a synchronisation costs as much as the launches:
+                    // 151 particles 1.9 -> 1.6 ms of tuning; 4095, where the first launch
+                    // of a poor candidate tells, 27 -> 32 ms)
+                    const bool look = c->n > 1024;
                     int warm = DM_OK;
                     if (!look) warm = launch_variant(c, vi, S, P);
                     if (warm) return warm;
@@ -782,7 +784,7 @@ int reorder(dm_cloud *c, double dt, bool mid, bool force) {
     const bool mid_ready = c->mid_valid && c->mid_dt == dt && c->boxes_valid[1];
     const int *keep = (force || !c->boxes_valid[0]) ? nullptr : z.keep;
     if (keep) {
-        DM_CUDA(ctx, launch_pdl(order_check, dim3(1), dim3(1024), 0, s, c->d, z, cblocks,
+        DM_CUDA(ctx, launch_pdl(order_check, dim3(1), dim3(1024), 0, s, c->d, z,
                                 c->order_dirty ? c->dirty_upload : 0));
         ctx->launches++;
     }
@@ -792,6 +794,8 @@ int reorder(dm_cloud *c, double dt, bool mid, bool force) {
     if (rc) return rc;
     DM_CUDA(ctx, launch_pdl(permute_gather, dim3(grid), dim3(256), 0, s, c->d, (const int *)z.vals[cur], z, keep));
     DM_CUDA(ctx, launch_pdl(permute_commit, dim3(cblocks), dim3(256), 0, s, c->d, z, dt, mid, mid_ready, keep));
+    DM_CUDA(ctx, launch_pdl(order_record, dim3(1), dim3(1024), 0, s, c->d, z, keep));
+    ctx->launches++;
     c->state_changed(true);
     c->boxes_valid[1] = c->mid_valid = mid;
     c->mid_dt = dt;
@@ -1140,10 +1144,9 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     const size_t ni = align256((size_t)c->n_pad * sizeof(int));
     c->sort_blocks = (n + kSortPerBlock - 1) / kSortPerBlock;
     const size_t nh = align256((size_t)kSortBuckets * (c->sort_blocks + 1) * sizeof(uint32_t));
-    const size_t nco = align256((size_t)((c->n_pad + 255) / 256 + 16) * sizeof(float));
     const size_t ngb = align256((size_t)(c->n_pad / 32) * sizeof(float4));
     const size_t nsp = align256((size_t)(c->n_pad / 1024 + 1) * sizeof(float4));
-    const size_t total = nd * (6 + 5 + 6 + 2 + 6) + nf4 * 8 + (ngb + nsp) * 4 + ni * 6 + nh + nco + 1024 + 512 +
+    const size_t total = nd * (6 + 5 + 6 + 2 + 6) + nf4 * 8 + (ngb + nsp) * 4 + ni * 6 + nh + 1024 + 512 +
                          align256(sizeof(double) * 5 * (kDiagBlocks + 1)) +
                          align256(sizeof(float) * kMomentBlocks * kMomentFields);
     cudaError_t e = cudaMalloc(&c->block, total);
@@ -1187,8 +1190,9 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     for (int k = 0; k < 6; k++) c->sort.stage[k] = takeD();
     c->sort.hist = (uint32_t *)p; p += nh;
     c->sort.box = (double *)p; c->sort.keep = (int *)(p + 64);
-    c->sort.changed = (int *)(p + 68); p += 256;
-    c->sort.cost = (float *)p; p += nco;
+    c->sort.changed = (int *)(p + 68);
+    c->sort.cost = (float *)(p + 128); p += 256;
+
     c->sort.moments = (float *)p; p += align256(sizeof(float) * kMomentBlocks * kMomentFields);
     c->d_diag = (double *)p; p += align256(sizeof(double) * 5 * (kDiagBlocks + 1));
     cudaStream_t s = ctx->stream;

@@ -222,11 +222,12 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
     const int off = d.off, n = d.n;
     const float4 *__restrict__ pa0 = c.pa[0] + off;
     const float rc = sqrtf(d.rc2_up);
+    const int groups = (n + 31) / 32;
 
     if (!force) {
-        const float now = (tid < (n + 31) / 32) ? order_cost(c.gbox[0][d.goff + tid], rc) : 0.0f;
+        const float now = (tid < groups) ? order_cost(c.gbox[0] + d.goff, tid, groups, rc) : 0.0f;
         const float was = (tid == 0) ? (float)box_out[8 * blockIdx.x + 3] : 0.0f;
-        if (block_order_kept<kBatchSortWarps>(now, was, S.wmom)) {
+        if (block_order_kept<kBatchSortWarps>(now, was, groups, S.wmom)) {
             if (mid && !mid_ready) {
                 CloudDev v = c;
                 v.rc2_up = d.rc2_up;
@@ -353,7 +354,6 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
     __syncthreads();  // every source is in registers: the cloud is rewritten in place
     CloudDev v = c;
     v.rc2_up = d.rc2_up;
-    float cost = 0.0f;
 #pragma unroll
     for (int k = 0; k < kBatchSortRounds; k++) {
         const int li = k * kBatchSortThreads + tid, s = off + li;  // a warp holds 32 consecutive slots
@@ -373,11 +373,13 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
                 h[1] = make_float2(A.x, A.y);
             }
         }
-        const float4 box =
-            store_group_box(c.gbox[0] + d.goff + (li >> 5), li < n, h[0].x, h[0].y, (li & ~31) < n);
+        store_group_box(c.gbox[0] + d.goff + (li >> 5), li < n, h[0].x, h[0].y, (li & ~31) < n);
         if (mid) store_group_box(c.gbox[1] + d.goff + (li >> 5), li < n, h[1].x, h[1].y, (li & ~31) < n);
-        cost += order_cost(box, rc);
     }
+    __syncthreads();  // the boxes are written
+    float cost = (tid < groups) ? order_cost(c.gbox[0] + d.goff, tid, groups, rc) : 0.0f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, o);
     if (lane == 0) S.wmom[warp][0] = cost;
     __syncthreads();
     if (tid == 0) {

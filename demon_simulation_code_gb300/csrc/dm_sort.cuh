@@ -36,22 +36,27 @@ constexpr int kSortBits = 24;
 constexpr int kSortDigitBits = 8;  // 24-bit keys: 3 passes
 constexpr int kSortBuckets = 1 << kSortDigitBits;
 
-// A one-launch sort that is due but not required (same trajectory since a sort
-// or an upload, at most kOrderKeep steps ago) leaves a cloud alone whose order
-// is still good: the area within the cutoff of its 32-particle groups' boxes,
-// which decides how many groups a tile of the sweep has to filter, has grown
-// by less than kOrderSlack since the sort.  The check costs 3 us of a 22-26 us
-// sort (one cluster, latency bound): 4095 particles, 10 RK2 steps 594 -> 437
-// us, 16,384 and 4 RK4 steps 415 -> 345 us, 3 steps through a focus 1396 ->
-// 1358 us, 256 clouds and 16 steps 12.94 -> 12.6 ms.  A required sort at least
-// every kOrderKeep steps, so that a cloud that shrinks while its order decays
-// is put right too.
+// A sort that is due but not required (the cloud was sorted at most kOrderKeep
+// steps ago and no upload has changed it) leaves a cloud alone whose order is
+// still good: compared with the distances between the centres of consecutive
+// 32-particle groups, the groups' boxes (each grown by a cutoff, for what a
+// sweep has to look at) have grown by less than kOrderSlack in area, in the
+// geometric mean over the groups, since the sort.  So neither a cloud that
+// contracts or expands as a whole nor a few particles thrown far out count,
+// and one that mixes does.  (Plain areas summed: a collapsing and re-expanding
+// cloud of 16,384 with particles thrown metres out kept orders that swept half
+// of all pairs over 10,000 steps instead of a quarter.)  The check costs 3 us of a
+// 22-26 us sort (one cluster, latency bound): 4095 particles, 10 RK2 steps 594
+// -> 437 us, 16,384 and 4 RK4 steps 415 -> 345 us.
 constexpr int kOrderKeep = 8;
-constexpr float kOrderSlack = 1.1f;
+constexpr float kOrderSlack = 0.1375f;  // log2(1.1)
 
-// A group's share of that area: its box grown by half a cutoff on each side.
-__device__ __forceinline__ float order_cost(const float4 &b, float rc) {
-    return (b.z >= b.x) ? (b.z - b.x + rc) * (b.w - b.y + rc) : 0.0f;
+// Group g's share of that measure (log2), among `groups` groups with boxes gb.
+__device__ __forceinline__ float order_cost(const float4 *gb, int g, int groups, float rc) {
+    if (g + 1 >= groups) return 0.0f;
+    const float4 a = __ldcg(gb + g), b = __ldcg(gb + g + 1);
+    const float dx = 0.5f * ((a.x + a.z) - (b.x + b.z)), dy = 0.5f * ((a.y + a.w) - (b.y + b.w));
+    return __log2f((a.z - a.x + rc) * (a.w - a.y + rc)) - __log2f(fmaf(dx, dx, fmaf(dy, dy, rc * rc)));
 }
 
 constexpr int kMomentBlocks = 128;  // fixed partition of the moment reduction
@@ -60,7 +65,7 @@ constexpr int kMomentFields = 9;   // count, sum dx, sum dy, sum dx^2, sum dy^2,
 struct SortScratch {
     float *moments;            // [kMomentBlocks][kMomentFields] per-block partials
     double *box;               // [8]: key box x0, y0, extent; -; bounding box min x, min y, max x, max y
-    float *cost;               // order_cost of the cloud as last sorted, per block of the kernel that wrote it
+    float *cost;               // [16]: order_cost of the cloud as last sorted, per block of the kernel that wrote it
     int *keep;                 // set by order_check: the order is still good
     int *changed;              // number of the last upload that changed the state
     uint32_t *keys[2];
@@ -254,10 +259,10 @@ __device__ __forceinline__ uint32_t morton_key_f32(float x, float y, const float
     return spread_bits12(qx) | (spread_bits12(qy) << 1);
 }
 
-// Whether the block's threads' costs `now` together are within kOrderSlack of
-// their `was`.  Every thread of the block; scratch: a row per warp.
+// Whether the block's threads' costs `now` together exceed their `was` by at most
+// kOrderSlack a group.  Every thread of the block; scratch: a row per warp.
 template <int WARPS, int FIELDS>
-__device__ __forceinline__ bool block_order_kept(float now, float was, float (&scratch)[WARPS][FIELDS]) {
+__device__ __forceinline__ bool block_order_kept(float now, float was, int groups, float (&scratch)[WARPS][FIELDS]) {
     static_assert(FIELDS >= 2, "two sums");
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -275,7 +280,7 @@ __device__ __forceinline__ bool block_order_kept(float now, float was, float (&s
         was += scratch[w][1];
     }
     __syncthreads();  // scratch is reused
-    return now <= kOrderSlack * was;  // false for NaN
+    return now - was <= kOrderSlack * (float)groups;  // false for NaN
 }
 
 // Position set 1 (see write_midpoint) of slot s and its group's box; whole warps.
@@ -292,8 +297,8 @@ __device__ __forceinline__ void write_midpoint_group(const CloudDev &c, int s, b
 // ---------------------------------------------------------------------------
 // The sort of clouds larger than one cluster holds: order_check, sort_moments,
 // sort_keys (with the first digit's histogram), per 8-bit digit radix_scan and
-// radix_scatter (and radix_hist before the next), permute_gather and
-// permute_commit.  Where order_check found the order still good the others
+// radix_scatter (and radix_hist before the next), permute_gather,
+// permute_commit and order_record.  Where order_check found the order still good the others
 // return at once (`keep`; null: always sort).  Bound by launch latency and by
 // a pass over the keys each (262,144 particles: ~60 us sorted, 17 us kept;
 // with FP64 moments and keys, one block scanning all the counts and separate
@@ -303,16 +308,37 @@ __device__ __forceinline__ void write_midpoint_group(const CloudDev &c, int s, b
 
 __device__ __forceinline__ bool order_is_kept(const int *keep) { return keep && *keep; }
 
-// One block: whether the cloud's order is still good.
-static __global__ void __launch_bounds__(1024) order_check(CloudDev c, SortScratch z, int ncost, int upload) {
+// One block: whether the cloud's order is still good ...
+static __global__ void __launch_bounds__(1024) order_check(CloudDev c, SortScratch z, int upload) {
     pdl_wait();
     __shared__ float s[32][2];
     const float rc = sqrtf(c.rc2_up);
-    float now = 0.0f, was = 0.0f;
-    for (int g = threadIdx.x; g < (c.n + 31) / 32; g += 1024) now += order_cost(c.gbox[0][g], rc);
-    for (int b = threadIdx.x; b < ncost; b += 1024) was += z.cost[b];
-    const bool kept = block_order_kept<32>(now, was, s);
+    const int groups = (c.n + 31) / 32;
+    float now = 0.0f;
+#pragma unroll 4
+    for (int g = threadIdx.x; g < groups; g += 1024) now += order_cost(c.gbox[0], g, groups, rc);
+    const bool kept = block_order_kept<32>(now, (threadIdx.x == 0) ? z.cost[0] : 0.0f, groups, s);
     if (threadIdx.x == 0) *z.keep = kept && (upload == 0 || *z.changed != upload);
+}
+
+// ... and, after a sort, how good it is.
+static __global__ void __launch_bounds__(1024) order_record(CloudDev c, SortScratch z, const int *keep) {
+    pdl_wait();
+    if (order_is_kept(keep)) return;
+    __shared__ float s[32];
+    const float rc = sqrtf(c.rc2_up);
+    const int groups = (c.n + 31) / 32;
+    float now = 0.0f;
+#pragma unroll 4
+    for (int g = threadIdx.x; g < groups; g += 1024) now += order_cost(c.gbox[0], g, groups, rc);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) now += __shfl_xor_sync(0xffffffffu, now, o);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = now;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 32; w++) now += s[w];
+        z.cost[0] = now;
+    }
 }
 
 // Per-block moments of the cloud's positions (origin: its first particle).
@@ -543,13 +569,14 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = c.n;
     const int e0 = r * kSortClusterPer;
+    const int groups = (n + 31) / 32;
     const float rc = sqrtf(c.rc2_up);
 
     if (!force && (upload == 0 || *z.changed != upload)) {  // every block comes to the same decision
         float now = 0.0f;
-        for (int g = tid; g < (n + 31) / 32; g += kSortClusterThreads) now += order_cost(c.gbox[0][g], rc);
+        for (int g = tid; g < groups; g += kSortClusterThreads) now += order_cost(c.gbox[0], g, groups, rc);
         const float was = (tid < kSortClusterCtas) ? z.cost[tid] : 0.0f;
-        if (block_order_kept<kSortClusterWarps>(now, was, S.wmom)) {
+        if (block_order_kept<kSortClusterWarps>(now, was, groups, S.wmom)) {
             if (mid && !mid_ready)
                 for (int k = 0; k < kSortClusterRounds; k++) {
                     const int s = e0 + k * kSortClusterThreads + tid;
@@ -710,7 +737,6 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
     // rewritten in place in the new order, with position sets 0 and 1 (the
     // next pass's inputs), the padding slots and the 32-particle group boxes.
     cl.sync();
-    float cost = 0.0f;
 #pragma unroll
     for (int k = 0; k < kSortClusterRounds; k++) {
         const int s = e0 + k * kSortClusterThreads + tid;  // a warp holds 32 consecutive slots
@@ -735,15 +761,17 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
             c.q[s] = 0.0;
             c.m[s] = 1.0;
         }
-        const float4 box = store_group_box(c.gbox[0] + (s >> 5), s < n, h[0].x, h[0].y, (s & ~31) < c.n_pad);
+        store_group_box(c.gbox[0] + (s >> 5), s < n, h[0].x, h[0].y, (s & ~31) < c.n_pad);
         if (mid) store_group_box(c.gbox[1] + (s >> 5), s < n, h[1].x, h[1].y, (s & ~31) < c.n_pad);
-        cost += order_cost(box, rc);
     }
-    if (lane == 0) S.wmom[warp][0] = cost;
-    __syncthreads();
-    if (tid == 0) {
-        for (int w = 1; w < kSortClusterWarps; w++) cost += S.wmom[w][0];
-        z.cost[r] = cost;
+    cl.sync();  // the boxes are written (ordered at cluster scope)
+    if (warp == 0) {
+        float cost = 0.0f;
+        for (int g = e0 / 32 + lane; g < (e0 + kSortClusterPer) / 32; g += 32)
+            cost += order_cost(c.gbox[0], g, groups, rc);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, o);
+        if (lane == 0) z.cost[r] = cost;
     }
 }
 
@@ -769,7 +797,6 @@ static __global__ void permute_gather(CloudDev c, const int *__restrict__ perm, 
 static __global__ void __launch_bounds__(256) permute_commit(CloudDev c, SortScratch z, double dt, bool mid,
                                                              bool mid_ready, const int *keep) {
     pdl_wait();
-    __shared__ float s_cost[8];
     const int s = blockIdx.x * 256 + threadIdx.x;  // n_pad: whole warps
     const bool live = s < c.n, store = s < c.n_pad;
     if (!order_is_kept(keep)) {
@@ -790,14 +817,7 @@ static __global__ void __launch_bounds__(256) permute_commit(CloudDev c, SortScr
             c.q[s] = 0.0;
             c.m[s] = 1.0;
         }
-        const float4 box = store_group_box(c.gbox[0] + (s >> 5), live, xh, yh, store);
-        if ((threadIdx.x & 31) == 0) s_cost[threadIdx.x >> 5] = order_cost(box, sqrtf(c.rc2_up));
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float cost = 0.0f;
-            for (int w = 0; w < 8; w++) cost += s_cost[w];
-            z.cost[blockIdx.x] = cost;
-        }
+        store_group_box(c.gbox[0] + (s >> 5), live, xh, yh, store);
     } else if (mid_ready) {
         return;
     }
