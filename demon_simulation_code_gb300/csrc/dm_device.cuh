@@ -459,10 +459,15 @@ __device__ __forceinline__ void write_padding(const CloudDev &c, int i) {
 // Reference cutoff decision for one pair, bit for bit:
 // r = sqrt(dx*dx + dy*dy) (no fused multiply-add, SSE4.2 has none),
 // kappa*r < 10 (ShieldedCoulombForce.cpp:144-147, 175-178).
-__device__ __forceinline__ bool ref_in_cutoff(double dx, double dy, double kappa, double &r,
-                                              double &a) {
+__host__ __device__ __forceinline__ bool ref_in_cutoff(double dx, double dy, double kappa, double &r,
+                                                       double &a) {
+#ifdef __CUDA_ARCH__
     r = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
     a = __dmul_rn(r, kappa);
+#else
+    r = std::sqrt(dx * dx + dy * dy);
+    a = r * kappa;
+#endif
     return a < 10.0;
 }
 

@@ -152,6 +152,18 @@ struct StageView {
     __device__ __forceinline__ float near_direct_f2() const { return P.near_direct_f2; }
 };
 
+// The reference's cutoff decision for particle ii and j = jg; false for j == i
+// and where either index is -1 (a lane past the cloud's last particle, which
+// sits at the origin and takes part in the direct chunks with the others; a
+// padding j).
+#pragma nv_exec_check_disable
+template <class View>
+__host__ __device__ __forceinline__ bool border_in(const View &P, int ii, int jg) {
+    if (jg == ii || jg < 0 || ii < 0) return false;
+    double r, a;
+    return ref_in_cutoff(P.px()[ii] - P.px()[jg], P.py()[ii] - P.py()[jg], P.kappa(), r, a);
+}
+
 // The scalar form of one pair for the slow path (pairs within 4e-6 of the
 // cutoff in r^2, decided exactly as the reference decides): w as in
 // pair2_terms, 0 for a pair outside the cutoff.  j values negated.
@@ -161,10 +173,7 @@ __device__ __forceinline__ float border_pair(const View &P, const PairI &I, int 
                                              float &dy) {
     dx = (I.xh.x + nxh) + (I.xl.x + nxl);
     dy = (I.yh.x + nyh) + (I.yl.x + nyl);
-    double r, a;
-    if (jg == ii || jg < 0 ||
-        !ref_in_cutoff(P.px()[ii] - P.px()[jg], P.py()[ii] - P.py()[jg], P.kappa(), r, a))
-        return 0.0f;
+    if (!border_in(P, ii, jg)) return 0.0f;
     const float r2 = fmaf(dx, dx, dy * dy);
     float y = rsqrt_approx(r2);
     const float u = r2 * y;
