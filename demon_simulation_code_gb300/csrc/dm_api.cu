@@ -857,6 +857,10 @@ int run_steps(dm_cloud *c, int nsteps, double dt, int precision) {
         cudaGraph_t g = nullptr;
         const unsigned long long saved = c->host_steps;
         const long long saved_launches = ctx->launches;
+        // a replay meets particles that the block before it has moved: the
+        // block forms the super group boxes it reads (set 0's may be valid now,
+        // after a force evaluation)
+        c->supers_valid[0] = c->supers_valid[1] = false;
         DM_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         int rc = enqueue_steps(c, kGraphSteps, dt, precision);
         cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
