@@ -1937,6 +1937,18 @@ int batch_tune(dm_batch *B) {
     return DM_OK;
 }
 
+// First in every call that uses the state: as cloud_enter.
+void batch_enter(dm_batch *B) {
+    B->capturing = stream_capturing(B->ctx);
+    if (B->capturing && !B->captured) {
+        B->drop_graphs();
+        B->captured = true;
+    }
+    if (!B->captured) return;
+    B->boxes_valid[0] = B->boxes_valid[1] = B->mid_valid = false;
+    B->order_dirty = true;
+}
+
 // nsteps of every cloud, in captured blocks where there are enough (see run_steps).
 int batch_run_steps(dm_batch *B, int nsteps, double dt) {
     dm_ctx *ctx = B->ctx;
@@ -2158,15 +2170,7 @@ int dm_batch_step(dm_batch *B, int nsteps, double dt, int precision) {
         return ctx->fail(DM_ERR_UNSUPPORTED, "batched clouds run the FP32C kernel; step FP64 clouds singly");
     if (nsteps < 0 || !std::isfinite(dt)) return ctx->fail(DM_ERR_ARG, "dm_batch_step: bad nsteps/dt");
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
-    B->capturing = stream_capturing(ctx);
-    if (B->capturing && !B->captured) {
-        B->drop_graphs();
-        B->captured = true;
-    }
-    if (B->captured) {  // see cloud_enter
-        B->boxes_valid[0] = B->boxes_valid[1] = B->mid_valid = false;
-        B->order_dirty = true;
-    }
+    batch_enter(B);
     const int slot = B->slot;
     const int rc = batch_run_steps(B, nsteps, dt), left = leave_slot(B, slot);
     return rc ? rc : left;
@@ -2178,6 +2182,7 @@ int dm_batch_eval_forces(dm_batch *B, int precision, double *fx, double *fy) {
     if (precision != DM_FP32C)
         return ctx->fail(DM_ERR_UNSUPPORTED, "batched clouds run the FP32C kernel");
     DM_CUDA(ctx, cudaSetDevice(ctx->device));
+    batch_enter(B);
     int rc = batch_launch_pass(B, 0, kModeForceOnly, 0.0);
     if (rc) return rc;
     const size_t bt = (size_t)B->total * sizeof(double);
