@@ -111,6 +111,7 @@ struct dm_cloud {
     int slot = 0;                // current step counter / force time slot (RK2 steps alternate it)
     bool capturing = false;      // the running call is recorded by the caller's stream capture
     bool captured = false;       // some call was: replays change the state unseen
+    bool split_stale = false;    // ... and may leave set 0's filter bounds of other force parameters
     int split[2] = {0, 0};  // cluster size per precision (0 = not chosen yet)
     int tuned_variant[2] = {-1, -1};  // per precision: index into kVariants
     float2 *partial = nullptr;         // [2 partial_cap][2][n_pad] non-cluster partial sums (per set and rank, axis)
@@ -478,6 +479,12 @@ int launch_variant(dm_cloud *c, int vi, int S, StageParams P) {
     P.split = S;
     P.partial = c->partial;
     const int ngroups = (c->n + 31) / 32;
+    if (c->split_stale) {
+        init_positions<<<(c->n_pad + 255) / 256, 256, 0, ctx->stream>>>(c->d);
+        DM_CUDA(ctx, cudaGetLastError());
+        ctx->launches++;
+        c->split_stale = false;
+    }
     cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t cfg = make_cfg(ctx, k, (c->n + k.tile - 1) / k.tile, S, P.nsets, attr);
     if (k.cull) {
@@ -773,6 +780,7 @@ int reorder(dm_cloud *c, double dt, bool mid, bool force) {
         c->state_changed(true);
         c->boxes_valid[1] = c->mid_valid = mid;
         c->mid_dt = dt;
+        c->split_stale = false;  // (stale: the sort was a forced one, which rewrites set 0)
         DM_CUDA(ctx, cudaGetLastError());
         ctx->launches += 1;
         c->order_dirty = false;
@@ -799,6 +807,7 @@ int reorder(dm_cloud *c, double dt, bool mid, bool force) {
     c->state_changed(true);
     c->boxes_valid[1] = c->mid_valid = mid;
     c->mid_dt = dt;
+    c->split_stale = false;
     ctx->launches += 4;
     c->order_dirty = false;
     return DM_OK;
@@ -942,10 +951,10 @@ bool stream_capturing(dm_ctx *ctx) {
 }
 
 // First in every call that uses or changes the state.  What the host knows of
-// the device (valid midpoint, boxes, order) holds neither for a call that is
+// the device (valid midpoint, boxes, filter bounds, order) holds neither for a call that is
 // being captured, which runs when it is replayed, nor after one.  From the
 // first such call on the position sets and the slot of the step counter stay
-// where the recorded launches expect them (adopt_sets, cloud_leave).
+// where the recorded launches expect them (adopt_sets, leave_slot).
 void cloud_enter(dm_cloud *c) {
     c->capturing = stream_capturing(c->ctx);
     if (c->capturing && !c->captured) {
@@ -954,6 +963,7 @@ void cloud_enter(dm_cloud *c) {
     }
     if (!c->captured) return;
     c->state_changed(false);
+    c->split_stale = true;
     c->order_dirty = true;
     c->dirty_upload = 0;
 }
@@ -1356,6 +1366,7 @@ int dm_cloud_set_forces(dm_cloud *c, const dm_force_params *p) {
     const char *why = nullptr;
     if (const int st = check_force_params(fp, &why))
         return ctx->fail(st, "dm_cloud_set_forces: %s (flags 0x%llx)", why, (unsigned long long)p->flags);
+    cloud_enter(c);
     c->f = fp;
     c->d.rc2 = (p->shielding > 0.0) ? (10.0 / p->shielding) * (10.0 / p->shielding) : 0.0;
     c->d.rc2_up = round_up_f32(c->d.rc2);
