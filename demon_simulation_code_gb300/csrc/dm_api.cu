@@ -900,24 +900,40 @@ int run_steps(dm_cloud *c, int nsteps, double dt, int precision) {
     return enqueue_steps(c, nsteps - reps * kGraphSteps, dt, precision);
 }
 
-// The device's own address of a caller's host buffer when the device may
-// dereference it (page-locked host memory: cudaHostAlloc, cudaMallocHost,
-// cudaHostRegister, torch's pin_memory), else nullptr: then the buffer is
-// copied by DMA.  On GB300 such buffers are read and written over
-// NVLink-C2C by the copy kernel, one launch for all four arrays.
-const void *device_view(const void *p) {
-    cudaPointerAttributes a;
-    if (!p || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
+// What a caller's buffer is.  view: the device's own address of it when the
+// device may dereference it (page-locked host memory: cudaHostAlloc,
+// cudaMallocHost, cudaHostRegister, torch's pin_memory): on GB300 such buffers
+// are read and written over NVLink-C2C by the copy kernel, one launch for all
+// four arrays.  pageable: plain memory (or no buffer at all), which the host
+// may read and write at once.  Page-locked, managed and device memory may be in
+// use by work queued on the stream: copies of it stay in stream order.
+struct Buffer {
+    const void *view = nullptr;
+    bool pageable = true;
+    explicit Buffer(const void *p) {
+        cudaPointerAttributes a;
+        if (!p) return;
+        pageable = false;
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) cudaGetLastError();
+        else if (a.type == cudaMemoryTypeHost) view = a.devicePointer;
+        else pageable = a.type == cudaMemoryTypeUnregistered;
     }
-    return (a.type == cudaMemoryTypeHost && a.devicePointer) ? a.devicePointer : nullptr;
-}
+};
+// The four arrays of a state.
+struct StateBuffers {
+    Buffer b[4];
+    StateBuffers(const void *x, const void *y, const void *vx, const void *vy)
+        : b{Buffer(x), Buffer(y), Buffer(vx), Buffer(vy)} {}
+    bool viewed() const { return b[0].view && b[1].view && b[2].view && b[3].view; }
+    bool pageable() const { return b[0].pageable && b[1].pageable && b[2].pageable && b[3].pageable; }
+    double *view(int k) const { return (double *)b[k].view; }
+};
 
-// Whether states of n particles are staged (see kStagedCopyMax); not under
+// Whether a state of n particles is staged (see kStagedCopyMax); not under
 // stream capture, where a replay has to read the caller's memory again.
-bool staged_copies(dm_ctx *ctx, int n) {
+bool staged_copies(dm_ctx *ctx, int n, const StateBuffers &B) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (!B.pageable()) return false;
     if (n > kStagedCopyMax || cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess ||
         cs != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
@@ -1263,14 +1279,13 @@ int dm_cloud_upload(dm_cloud *c, const double *x, const double *y, const double 
     // caller order -> staging -> the cloud's current internal order (charges,
     // masses and the order stay; position set 0 and its boxes are rewritten)
     double **st = c->sort.stage;
-    const void *dv[4] = {device_view(x), device_view(y), device_view(vx), device_view(vy)};
-    if (dv[0] && dv[1] && dv[2] && dv[3]) {
-        copy4<<<(c->n + 255) / 256, 256, 0, ctx->stream>>>(c->n, (const double *)dv[0], (const double *)dv[1],
-                                                           (const double *)dv[2], (const double *)dv[3], st[0],
+    const StateBuffers B(x, y, vx, vy);
+    if (B.viewed()) {
+        copy4<<<(c->n + 255) / 256, 256, 0, ctx->stream>>>(c->n, B.view(0), B.view(1), B.view(2), B.view(3), st[0],
                                                            st[1], st[2], st[3], nullptr, nullptr);
         DM_CUDA(ctx, cudaGetLastError());
         ctx->launches += 1;
-    } else if (staged_copies(ctx, c->n)) {
+    } else if (staged_copies(ctx, c->n, B)) {
         const size_t n = (size_t)c->n;
         const double *in[4] = {x, y, vx, vy}, *d = ctx->h_stage_dev;
         DM_CUDA(ctx, cudaEventSynchronize(ctx->stage_read));
@@ -1308,15 +1323,14 @@ int dm_cloud_download(dm_cloud *c, double *x, double *y, double *vx, double *vy)
     ctx->launches++;
     // the error flags come back with the state: one synchronisation
     if (!ctx->h_err) DM_CUDA(ctx, cudaMallocHost((void **)&ctx->h_err, sizeof(int)));
-    const void *dv[4] = {device_view(x), device_view(y), device_view(vx), device_view(vy)};
-    int *err_dv = (int *)device_view(ctx->h_err);
-    if (dv[0] && dv[1] && dv[2] && dv[3] && err_dv) {
-        copy4<<<(c->n + 255) / 256, 256, 0, ctx->stream>>>(c->n, st[0], st[1], st[2], st[3], (double *)dv[0],
-                                                           (double *)dv[1], (double *)dv[2], (double *)dv[3],
-                                                           c->d.err, err_dv);
+    const StateBuffers B(x, y, vx, vy);
+    int *err_dv = (int *)Buffer(ctx->h_err).view;
+    if (B.viewed() && err_dv) {
+        copy4<<<(c->n + 255) / 256, 256, 0, ctx->stream>>>(c->n, st[0], st[1], st[2], st[3], B.view(0), B.view(1),
+                                                           B.view(2), B.view(3), c->d.err, err_dv);
         DM_CUDA(ctx, cudaGetLastError());
         ctx->launches++;
-    } else if (err_dv && staged_copies(ctx, c->n)) {
+    } else if (err_dv && staged_copies(ctx, c->n, B)) {
         const size_t n = (size_t)c->n;
         const double *h = ctx->h_stage + 4 * (size_t)ctx->stage_n;
         double *d = ctx->h_stage_dev + 4 * (size_t)ctx->stage_n, *out[4] = {x, y, vx, vy};
