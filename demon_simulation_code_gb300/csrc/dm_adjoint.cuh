@@ -261,13 +261,31 @@ struct AdjVjpIO {
     int stage;
 };
 
+__device__ __forceinline__ float4 adj_split_hi(float xh, float yh, float rc2_up) {
+    return make_float4(xh, yh, fmaf(yh, yh, xh * xh), -filter_threshold(xh, yh, rc2_up));
+}
 __device__ __forceinline__ void adj_store_split(const AdjSplit &o, int i, double x, double y, float rc2_up) {
     float xh, xl, yh, yl;
     split2(x, xh, xl);
     split2(y, yh, yl);
-    o.p[i] = make_float4(xh, yh, fmaf(yh, yh, xh * xh), -filter_threshold(xh, yh, rc2_up));
+    o.p[i] = adj_split_hi(xh, yh, rc2_up);
     o.l[i] = make_float2(xl, yl);
 }
+
+// AdjSplit::p of particle i: as stored, or formed where it is read (calls of
+// their own, which keep no scratch; the same values; for a j the bound's
+// arithmetic falls away).
+struct AdjStoredSplit {
+    const float4 *p;
+    __device__ __forceinline__ float4 operator()(int i) const { return p[i]; }
+};
+struct AdjFormedSplit {
+    const double *x, *y;
+    float rc2_up;
+    __device__ __forceinline__ float4 operator()(int i) const {
+        return adj_split_hi(__double2float_rn(x[i]), __double2float_rn(y[i]), rc2_up);
+    }
+};
 
 // Splits positions (x, y); invm (if given) = 1/m; backward (lam given): dk_4 =
 // lam/6 and the force adjoint a = dt dk_v / m of stage 4.
@@ -682,9 +700,9 @@ __device__ __forceinline__ void adj_pair64(const Yukawa64 &K, const double *tab,
     }
 }
 
-template <int MODE>
+template <int MODE, class Split>
 __device__ __forceinline__ void adj_group_sums(const AdjCloud &d, int tile, const double *x, const double *y,
-                                               const double *q, const double *ax, const double *ay, const AdjSplit &in,
+                                               const double *q, const double *ax, const double *ay, Split in,
                                                AdjGroupSmem<MODE == 0 ? 2 : 4> &sm) {
     constexpr int NS = MODE == 0 ? 2 : 4;
     cg::cluster_group cl = cg::this_cluster();
@@ -700,11 +718,11 @@ __device__ __forceinline__ void adj_group_sums(const AdjCloud &d, int tile, cons
         y += d.off;
         q += d.off;
         if (MODE == 1) ax += d.off, ay += d.off;
-        const float4 *pa = in.p + d.off;
+        auto pa = [&](int k) { return in(d.off + k); };
         float px2 = 0.0f, py2 = 0.0f, nu = INFINITY;
         double xi = 0.0, yi = 0.0, aix = 0.0, aiy = 0.0;
         if (valid) {
-            const float4 A = pa[li];
+            const float4 A = pa(li);
             px2 = 2.0f * A.x;
             py2 = 2.0f * A.y;
             nu = A.w;
@@ -798,7 +816,7 @@ static __global__ void __launch_bounds__(32 * kAdjWarps) adj_step_fp64(const Adj
     const int2 g = groups[blockIdx.x / cl.num_blocks()];
     const AdjCloud &d = desc[g.x];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    adj_group_sums<0>(d, g.y, io.x, io.y, io.q, nullptr, nullptr, io.in, sm);
+    adj_group_sums<0>(d, g.y, io.x, io.y, io.q, nullptr, nullptr, AdjStoredSplit{io.in.p}, sm);
     const int li = 32 * g.y + lane, i = d.off + li;
     if (cl.block_rank() == 0) {
         const bool valid = li < d.n;
@@ -823,7 +841,7 @@ static __global__ void __launch_bounds__(32 * kAdjWarps) adj_vjp_fp64(const AdjC
     const int2 g = groups[blockIdx.x / cl.num_blocks()];
     const AdjCloud &d = desc[g.x];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    adj_group_sums<1>(d, g.y, V.x, V.y, V.q, V.ax, V.ay, V.in, sm);
+    adj_group_sums<1>(d, g.y, V.x, V.y, V.q, V.ax, V.ay, AdjStoredSplit{V.in.p}, sm);
     const int li = 32 * g.y + lane, i = d.off + li;
     if (cl.block_rank() == 0 && li < d.n) {
         double S[4];
@@ -841,13 +859,13 @@ static __global__ void __launch_bounds__(32 * kAdjWarps) adj_vjp_fp64(const AdjC
 template <int MODE>
 __global__ void __launch_bounds__(32 * kAdjWarps) adj_once_fp64(const AdjCloud *__restrict__ desc,
                                                                 const int2 *__restrict__ groups, const AdjOnce A,
-                                                                const AdjSplit in, double coulomb) {
+                                                                double coulomb) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     auto &sm = *reinterpret_cast<AdjGroupSmem<MODE == 0 ? 2 : 4> *>(smem_raw);
     cg::cluster_group cl = cg::this_cluster();
     const int2 g = groups[blockIdx.x / cl.num_blocks()];
     const AdjCloud &d = desc[g.x];
-    adj_group_sums<MODE>(d, g.y, A.x, A.y, A.q, A.ax, A.ay, in, sm);
+    adj_group_sums<MODE>(d, g.y, A.x, A.y, A.q, A.ax, A.ay, AdjFormedSplit{A.x, A.y, d.rc2_up}, sm);
     const int li = 32 * g.y + (int)(threadIdx.x & 31);
     if (cl.block_rank() == 0 && threadIdx.x < 32 && li < d.n) {
         double S[4];

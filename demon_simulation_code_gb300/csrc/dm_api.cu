@@ -2405,24 +2405,9 @@ cudaError_t adj_launch_once(dm_adjoint *A, int precision, const AdjOnce &O) {
                                                                              A->coulomb);
         return cudaGetLastError();
     }
-    // stream-ordered scratch of its own: such calls may be queued on several
-    // streams at once, and share nothing
-    AdjSplit split{};
-    const size_t n = (size_t)A->total;
-    cudaStream_t st = A->ctx->stream;
-    cudaError_t e = cudaMallocAsync((void **)&split.p, n * (sizeof(float4) + sizeof(float2)), st);
-    if (e != cudaSuccess) return e;
-    split.l = (float2 *)(split.p + n);
-    AdjPrepareIO R{};
-    R.x = O.x;
-    R.y = O.y;
-    R.out = split;
-    e = adj_launch_prepare(A, R);
-    if (e == cudaSuccess)
-        e = adj_launch64<(MODE == 0 ? 2 : 4)>(A, adj_once_fp64<MODE>, (const AdjCloud *)A->ddesc,
-                                              (const int2 *)A->dgroups, O, split, A->coulomb);
-    const cudaError_t ef = cudaFreeAsync(split.p, st);
-    return e != cudaSuccess ? e : ef;
+    // no scratch: such calls may be queued on several streams at once
+    return adj_launch64<(MODE == 0 ? 2 : 4)>(A, adj_once_fp64<MODE>, (const AdjCloud *)A->ddesc,
+                                             (const int2 *)A->dgroups, O, A->coulomb);
 }
 }  // namespace
 

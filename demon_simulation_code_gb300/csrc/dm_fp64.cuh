@@ -201,17 +201,17 @@ struct alignas(16) HitWarp {
     uint16_t code[kHitPerLane * 32];  // (k << 10) | (jl << 5) | il
 };
 
-// Filters j group g (FP32 positions pa, n particles) against this lane's i
+// Filters j group g (FP32 position of j: load(j) = (xh, yh, |p|^2, -); n particles) against this lane's i
 // (px2 = 2 xh_i, py2 = 2 yh_i, nu = -bound_i; nu = INFINITY: no particle) and
 // stores the lane's mask as entry k.  A pair is out if bound_i - |p_j|^2 + 2
 // p_i.p_j is negative (two j per packed instruction, 3 instructions per pair);
 // NaN passes: such a pair is decided later.  Returns the lane's number of hits.
-template <class Result>
-__device__ __forceinline__ int hit_filter(HitWarp<Result> &W, int k, int g, int self, const float4 *__restrict__ pa,
-                                          int n, float px2, float py2, float nu) {
+template <class Result, class Load>
+__device__ __forceinline__ int hit_filter(HitWarp<Result> &W, int k, int g, int self, Load load, int n, float px2,
+                                          float py2, float nu) {
     const int lane = threadIdx.x & 31;
     const int j = 32 * g + lane;
-    const float4 A = (j < n) ? pa[j] : make_float4(0.0f, 0.0f, INFINITY, 0.0f);
+    const float4 A = (j < n) ? load(j) : make_float4(0.0f, 0.0f, INFINITY, 0.0f);
     __syncwarp();
     W.fx[lane] = A.x;
     W.fy[lane] = A.y;

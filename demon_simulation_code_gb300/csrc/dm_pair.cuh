@@ -1225,7 +1225,7 @@ __global__ void __launch_bounds__(2 * NW * 32, 10 / NW) pair_group_fp64(const St
                 prefetch_l1(py + j);
                 prefetch_l1(qa + j);
             }
-            hits += hit_filter(W, nk, g, tile, pa, n, px2, py2, nu);
+            hits += hit_filter(W, nk, g, tile, [&](int k) { return pa[k]; }, n, px2, py2, nu);
             if (++nk == kHitGroups || __reduce_add_sync(0xffffffffu, hits) >= 7 * 32) {
                 __syncwarp();
                 hit_flush(W, nk, sum, eval);
