@@ -119,6 +119,7 @@ struct dm_cloud {
     SortScratch sort{};
     int sort_blocks = 0;
     int reorder_interval = 1;   // steps between Morton re-sorts (0 = never)
+    bool keep_orders = true;    // a due sort leaves an order that is still good (no interval was asked for)
     bool order_dirty = true;    // re-sort before the next step ...
     int dirty_upload = 0;       // ... if upload of this number changed the state (0: in any case)
     int uploads = 0;
@@ -818,7 +819,7 @@ int reorder_if_due(dm_cloud *c, int precision, double dt, bool mid) {
     if (!wants_order(c->n, precision)) return DM_OK;
     if (c->order_dirty || (c->reorder_interval > 0 && c->host_steps % (unsigned)c->reorder_interval == 0))
         return reorder(c, dt, mid,
-                       (c->order_dirty && c->dirty_upload == 0) || c->reorder_interval != 1 ||
+                       (c->order_dirty && c->dirty_upload == 0) || !c->keep_orders ||
                            c->host_steps % (unsigned)kOrderKeep == 0);
     return DM_OK;
 }
@@ -1617,6 +1618,7 @@ int dm_cloud_set_reorder_interval(dm_cloud *c, int steps) {
     if (steps < 0 || steps > kGraphSteps || (steps & (steps - 1)) != 0)
         return c->ctx->fail(DM_ERR_ARG, "reorder interval must be 0 or a power of two <= %d", kGraphSteps);
     c->reorder_interval = steps;
+    c->keep_orders = false;
     c->drop_graphs();
     return DM_OK;
 }

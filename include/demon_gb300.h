@@ -262,9 +262,10 @@ int dm_cloud_set_kernel(dm_cloud *cloud, const char *variant, int split);
  * wakes the precise arithmetic for few j; the order is internal (every
  * array crossing this ABI is in the caller's order).  The cloud is re-sorted
  * every `steps` RK4 steps (0 = only after an upload; otherwise a power of
- * two <= 16).  Default: every step (clouds of up to 16384 particles are
- * sorted by one thread-block cluster in one launch, which seven steps of
- * eight first looks whether the order is still good and then leaves it).
+ * two <= 16).  Default, until this is called: every step looks whether the
+ * order is still good and re-sorts where it is not (clouds of up to 16384
+ * particles in one launch of a thread-block cluster); after
+ * dm_cloud_set_reorder_interval(cloud, 1) every step sorts.
  * FP64 steps of up to 4096 particles run on the caller's order.  No reference
  * counterpart. */
 int dm_cloud_set_reorder_interval(dm_cloud *cloud, int steps);
