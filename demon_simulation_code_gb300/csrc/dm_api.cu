@@ -773,10 +773,12 @@ int reorder(dm_cloud *c, double dt, bool mid, bool force) {
         const int upload = c->order_dirty ? c->dirty_upload : 0;
         if (ctx->sort_ctas == 16) {
             const cudaLaunchConfig_t cfg = sort_cluster_cfg<16>(s, attr);
-            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<16>, pa0, c->d, z, dt, mid, mid_ready, force, upload));
+            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<16>, pa0, c->d, z, dt, mid, mid_ready, force, c->slot,
+                                            upload));
         } else {
             const cudaLaunchConfig_t cfg = sort_cluster_cfg<8>(s, attr);
-            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<8>, pa0, c->d, z, dt, mid, mid_ready, force, upload));
+            DM_CUDA(ctx, cudaLaunchKernelEx(&cfg, sort_cluster<8>, pa0, c->d, z, dt, mid, mid_ready, force, c->slot,
+                                            upload));
         }
         c->state_changed(true);
         c->boxes_valid[1] = c->mid_valid = mid;
@@ -793,7 +795,7 @@ int reorder(dm_cloud *c, double dt, bool mid, bool force) {
     const bool mid_ready = c->mid_valid && c->mid_dt == dt && c->boxes_valid[1];
     const int *keep = (force || !c->boxes_valid[0]) ? nullptr : z.keep;
     if (keep) {
-        DM_CUDA(ctx, launch_pdl(order_check, dim3(1), dim3(1024), 0, s, c->d, z,
+        DM_CUDA(ctx, launch_pdl(order_check, dim3(1), dim3(1024), 0, s, c->d, z, c->slot,
                                 c->order_dirty ? c->dirty_upload : 0));
         ctx->launches++;
     }
@@ -803,7 +805,7 @@ int reorder(dm_cloud *c, double dt, bool mid, bool force) {
     if (rc) return rc;
     DM_CUDA(ctx, launch_pdl(permute_gather, dim3(grid), dim3(256), 0, s, c->d, (const int *)z.vals[cur], z, keep));
     DM_CUDA(ctx, launch_pdl(permute_commit, dim3(cblocks), dim3(256), 0, s, c->d, z, dt, mid, mid_ready, keep));
-    DM_CUDA(ctx, launch_pdl(order_record, dim3(1), dim3(1024), 0, s, c->d, z, keep));
+    DM_CUDA(ctx, launch_pdl(order_record, dim3(1), dim3(1024), 0, s, c->d, z, c->slot, keep));
     ctx->launches++;
     c->state_changed(true);
     c->boxes_valid[1] = c->mid_valid = mid;
@@ -818,9 +820,7 @@ int reorder(dm_cloud *c, double dt, bool mid, bool force) {
 int reorder_if_due(dm_cloud *c, int precision, double dt, bool mid) {
     if (!wants_order(c->n, precision)) return DM_OK;
     if (c->order_dirty || (c->reorder_interval > 0 && c->host_steps % (unsigned)c->reorder_interval == 0))
-        return reorder(c, dt, mid,
-                       (c->order_dirty && c->dirty_upload == 0) || !c->keep_orders ||
-                           c->host_steps % (unsigned)kOrderKeep == 0);
+        return reorder(c, dt, mid, (c->order_dirty && c->dirty_upload == 0) || !c->keep_orders);
     return DM_OK;
 }
 
@@ -852,11 +852,12 @@ int run_steps(dm_cloud *c, int nsteps, double dt, int precision) {
     }
     if (nsteps < kGraphSteps) return enqueue_steps(c, nsteps, dt, precision);
     // the captured steps start from a midpoint left by the step before (or by
-    // the re-sort that begins them): make it so, outside the capture
+    // the re-sort that begins them, which may leave the order, and so needs
+    // valid boxes, but always writes the midpoint): make it so, outside the capture
     int rc0 = ensure_tuned(c, precision);
     if (rc0) return rc0;
     const bool sorts = wants_order(c->n, precision) && c->reorder_interval > 0;
-    if (!sorts && !(c->mid_valid && c->mid_dt == dt)) {
+    if (sorts ? !c->boxes_valid[0] : !(c->mid_valid && c->mid_dt == dt)) {
         rc0 = enqueue_steps(c, 1, dt, precision);
         if (rc0) return rc0;
         return run_steps(c, nsteps - 1, dt, precision);
@@ -871,6 +872,7 @@ int run_steps(dm_cloud *c, int nsteps, double dt, int precision) {
         // block forms the super group boxes it reads (set 0's may be valid now,
         // after a force evaluation)
         c->supers_valid[0] = c->supers_valid[1] = false;
+        if (sorts) c->mid_valid = false;
         DM_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         int rc = enqueue_steps(c, kGraphSteps, dt, precision);
         cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
@@ -1222,7 +1224,8 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     c->sort.hist = (uint32_t *)p; p += nh;
     c->sort.box = (double *)p; c->sort.keep = (int *)(p + 64);
     c->sort.changed = (int *)(p + 68);
-    c->sort.cost = (float *)(p + 128); p += 256;
+    c->sort.cost = (float *)(p + 128);
+    c->sort.sorted_at = (unsigned long long *)(p + 192); p += 256;
 
     c->sort.moments = (float *)p; p += align256(sizeof(float) * kMomentBlocks * kMomentFields);
     c->d_diag = (double *)p; p += align256(sizeof(double) * 5 * (kDiagBlocks + 1));
@@ -1839,7 +1842,8 @@ int batch_reorder(dm_batch *B, double dt = 0.0, bool mid = false, bool force = t
                                           (int)kBatchSortSmem));
         DM_CUDA(ctx, launch_pdl(batch_sort_clouds, dim3(B->nclouds), dim3(kBatchSortThreads), kBatchSortSmem, s,
                                 B->d, (const BatchCloud *)B->ddesc, B->dbox, dt, mid,
-                                B->mid_valid && B->mid_dt == dt && B->boxes_valid[1], force || !B->boxes_valid[0]));
+                                B->mid_valid && B->mid_dt == dt && B->boxes_valid[1], force || !B->boxes_valid[0], B->slot,
+                                B->sort.sorted_at));
         ctx->launches++;
         B->boxes_valid[0] = true;
         B->boxes_valid[1] = B->mid_valid = mid;
@@ -1868,9 +1872,7 @@ int batch_enqueue_steps(dm_batch *B, int nsteps, double dt) {
     dm_ctx *ctx = B->ctx;
     for (int s = 0; s < nsteps; s++) {
         if (B->order_dirty || (B->reorder_interval > 0 && B->host_steps % (unsigned)B->reorder_interval == 0)) {
-            int rc = batch_reorder(B, dt, true,
-                                   B->order_dirty || B->reorder_interval != 1 ||
-                                       B->host_steps % (unsigned)kOrderKeep == 0);
+            int rc = batch_reorder(B, dt, true, B->order_dirty || B->reorder_interval != 1);
             if (rc) return rc;
         }
         if (!B->mid_valid || B->mid_dt != dt) {
@@ -1991,7 +1993,8 @@ int batch_run_steps(dm_batch *B, int nsteps, double dt) {
     }
     if (nsteps < kGraphSteps) return batch_enqueue_steps(B, nsteps, dt);
     const bool sorts = B->reorder_interval > 0 && B->max_n <= kBatchSortMax;
-    if (!sorts && !(B->mid_valid && B->mid_dt == dt)) {  // the captured steps start from a midpoint (see run_steps)
+    // what the captured steps start from: see run_steps
+    if (sorts ? !B->boxes_valid[0] : !(B->mid_valid && B->mid_dt == dt)) {
         int rc = batch_enqueue_steps(B, 1, dt);
         return rc ? rc : batch_run_steps(B, nsteps - 1, dt);
     }
@@ -2002,6 +2005,7 @@ int batch_run_steps(dm_batch *B, int nsteps, double dt) {
         cudaGraph_t g = nullptr;
         const unsigned long long saved = B->host_steps;
         const long long sl = ctx->launches;
+        if (sorts) B->mid_valid = false;
         DM_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         int rc = batch_enqueue_steps(B, kGraphSteps, dt);
         cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
@@ -2075,7 +2079,8 @@ int dm_batch_create(dm_ctx *ctx, int nclouds, const int *n, const double *x, con
     const size_t nh = align256((size_t)kSortBuckets * (B->sort_blocks + 1) * sizeof(uint32_t));
     const size_t ndesc = align256((size_t)nclouds * sizeof(BatchCloud));
     const size_t nbb = align256((size_t)nclouds * 8 * sizeof(double));
-    const size_t bytes_total = nd * (6 + 5 + 6 + 2 + 6) + nf4 * 8 + ni * 7 + nh + ndesc + nbb + 1024;
+    const size_t nat = align256((size_t)nclouds * sizeof(unsigned long long));
+    const size_t bytes_total = nd * (6 + 5 + 6 + 2 + 6) + nf4 * 8 + ni * 7 + nh + ndesc + nbb + nat + 1024;
     cudaError_t e = cudaMalloc(&B->block, bytes_total);
     if (e != cudaSuccess) {
         delete B;
@@ -2109,6 +2114,7 @@ int dm_batch_create(dm_ctx *ctx, int nclouds, const int *n, const double *x, con
     B->sort.hist = (uint32_t *)p; p += nh;
     B->ddesc = (BatchCloud *)p; p += ndesc;
     B->dbox = (double *)p; p += nbb;
+    B->sort.sorted_at = (unsigned long long *)p; p += nat;
     d.step_ctr = (unsigned long long *)p; p += 256;
     d.time = (double *)(d.step_ctr + 4);  // same 256-byte slot, bytes 32-47
     d.err = (int *)p; p += 256;

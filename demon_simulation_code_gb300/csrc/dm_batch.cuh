@@ -210,10 +210,11 @@ constexpr size_t kBatchSortSmem = sizeof(BatchSortSmem);
 // bounding box min x, min y, max x, max y (as batch_boxes writes them; the
 // batch autotuner reads it).  Without `force` a cloud in good order (see
 // kOrderKeep) is left as it is; if `mid` and not `mid_ready` its set 1 is
-// written.
+// written.  sorted_at[cloud]: step index of its last sort; slot: of the step
+// counter.
 static __global__ void __launch_bounds__(kBatchSortThreads, 1)
     batch_sort_clouds(CloudDev c, const BatchCloud *__restrict__ desc, double *box_out, double dt, bool mid,
-                      bool mid_ready, bool force) {
+                      bool mid_ready, bool force, int slot, unsigned long long *sorted_at) {
     pdl_wait();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     BatchSortSmem &S = *reinterpret_cast<BatchSortSmem *>(smem_raw);
@@ -224,7 +225,7 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
     const float rc = sqrtf(d.rc2_up);
     const int groups = (n + 31) / 32;
 
-    if (!force) {
+    if (!force && order_is_recent(c, slot, sorted_at[blockIdx.x])) {
         const float now = (tid < groups) ? order_cost(c.gbox[0] + d.goff, tid, groups, rc) : 0.0f;
         const float was = (tid == 0) ? (float)box_out[8 * blockIdx.x + 3] : 0.0f;
         if (block_order_kept<kBatchSortWarps>(now, was, groups, S.wmom)) {
@@ -385,6 +386,7 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
     if (tid == 0) {
         for (int w = 1; w < kBatchSortWarps; w++) cost += S.wmom[w][0];
         box_out[8 * blockIdx.x + 3] = cost;
+        sorted_at[blockIdx.x] = c.step_ctr[slot];
     }
 }
 

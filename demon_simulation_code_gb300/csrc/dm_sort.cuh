@@ -51,6 +51,13 @@ constexpr int kSortBuckets = 1 << kSortDigitBits;
 constexpr int kOrderKeep = 8;
 constexpr float kOrderSlack = 0.1375f;  // log2(1.1)
 
+// Whether the last sort, at step index `at`, is less than kOrderKeep steps ago.
+// Counted from the sort on the device, so that the same state and the same
+// steps are sorted at the same places whatever the cloud did before.
+__device__ __forceinline__ bool order_is_recent(const CloudDev &c, int slot, unsigned long long at) {
+    return c.step_ctr[slot] - at < (unsigned long long)kOrderKeep;
+}
+
 // Group g's share of that measure (log2), among `groups` groups with boxes gb.
 __device__ __forceinline__ float order_cost(const float4 *gb, int g, int groups, float rc) {
     if (g + 1 >= groups) return 0.0f;
@@ -68,6 +75,7 @@ struct SortScratch {
     float *cost;               // [16]: order_cost of the cloud as last sorted, per block of the kernel that wrote it
     int *keep;                 // set by order_check: the order is still good
     int *changed;              // number of the last upload that changed the state
+    unsigned long long *sorted_at;  // step index of the last sort
     uint32_t *keys[2];
     int *vals[2];
     uint32_t *hist;            // [kSortBuckets * nblocks], then [kSortBuckets] totals
@@ -308,8 +316,8 @@ __device__ __forceinline__ void write_midpoint_group(const CloudDev &c, int s, b
 
 __device__ __forceinline__ bool order_is_kept(const int *keep) { return keep && *keep; }
 
-// One block: whether the cloud's order is still good ...
-static __global__ void __launch_bounds__(1024) order_check(CloudDev c, SortScratch z, int upload) {
+// One block: whether the cloud's order is still good (slot: of the step counter) ...
+static __global__ void __launch_bounds__(1024) order_check(CloudDev c, SortScratch z, int slot, int upload) {
     pdl_wait();
     __shared__ float s[32][2];
     const float rc = sqrtf(c.rc2_up);
@@ -318,11 +326,12 @@ static __global__ void __launch_bounds__(1024) order_check(CloudDev c, SortScrat
 #pragma unroll 4
     for (int g = threadIdx.x; g < groups; g += 1024) now += order_cost(c.gbox[0], g, groups, rc);
     const bool kept = block_order_kept<32>(now, (threadIdx.x == 0) ? z.cost[0] : 0.0f, groups, s);
-    if (threadIdx.x == 0) *z.keep = kept && (upload == 0 || *z.changed != upload);
+    if (threadIdx.x == 0)
+        *z.keep = kept && order_is_recent(c, slot, *z.sorted_at) && (upload == 0 || *z.changed != upload);
 }
 
 // ... and, after a sort, how good it is.
-static __global__ void __launch_bounds__(1024) order_record(CloudDev c, SortScratch z, const int *keep) {
+static __global__ void __launch_bounds__(1024) order_record(CloudDev c, SortScratch z, int slot, const int *keep) {
     pdl_wait();
     if (order_is_kept(keep)) return;
     __shared__ float s[32];
@@ -338,6 +347,7 @@ static __global__ void __launch_bounds__(1024) order_record(CloudDev c, SortScra
     if (threadIdx.x == 0) {
         for (int w = 1; w < 32; w++) now += s[w];
         z.cost[0] = now;
+        *z.sorted_at = c.step_ctr[slot];
     }
 }
 
@@ -553,11 +563,11 @@ constexpr size_t sort_cluster_smem() { return sizeof(SortClusterSmem<CTAS>); }
 // their group boxes rewritten.  Without `force` (or an upload of number
 // `upload` that changed the state) a cloud in good order (see kOrderKeep) is
 // left as it is; if `mid` and not `mid_ready` its set 1 is
-// written.  Launched as one cluster of CTAS blocks.
+// written.  slot: of the step counter.  Launched as one cluster of CTAS blocks.
 template <int CTAS>
 static __global__ void __launch_bounds__(kSortClusterThreads, 1)
     sort_cluster(const float4 *__restrict__ pa0, CloudDev c, SortScratch z, double dt, bool mid, bool mid_ready,
-                 bool force, int upload) {
+                 bool force, int slot, int upload) {
     constexpr int kSortClusterCtas = CTAS;
     constexpr int kSortClusterPer = SortClusterShape<CTAS>::per;
     constexpr int kSortClusterRounds = SortClusterShape<CTAS>::rounds;
@@ -572,7 +582,8 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
     const int groups = (n + 31) / 32;
     const float rc = sqrtf(c.rc2_up);
 
-    if (!force && (upload == 0 || *z.changed != upload)) {  // every block comes to the same decision
+    // every block comes to the same decision
+    if (!force && order_is_recent(c, slot, *z.sorted_at) && (upload == 0 || *z.changed != upload)) {
         float now = 0.0f;
         for (int g = tid; g < groups; g += kSortClusterThreads) now += order_cost(c.gbox[0], g, groups, rc);
         const float was = (tid < kSortClusterCtas) ? z.cost[tid] : 0.0f;
@@ -771,7 +782,10 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
             cost += order_cost(c.gbox[0], g, groups, rc);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, o);
-        if (lane == 0) z.cost[r] = cost;
+        if (lane == 0) {
+            z.cost[r] = cost;
+            if (r == 0) *z.sorted_at = c.step_ctr[slot];
+        }
     }
 }
 
