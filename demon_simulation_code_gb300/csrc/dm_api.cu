@@ -1224,8 +1224,7 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     c->sort.hist = (uint32_t *)p; p += nh;
     c->sort.box = (double *)p; c->sort.keep = (int *)(p + 64);
     c->sort.changed = (int *)(p + 68);
-    c->sort.cost = (float *)(p + 128);
-    c->sort.sorted_at = (unsigned long long *)(p + 192); p += 256;
+    c->sort.order = (OrderRecord *)(p + 128); p += 256;
 
     c->sort.moments = (float *)p; p += align256(sizeof(float) * kMomentBlocks * kMomentFields);
     c->d_diag = (double *)p; p += align256(sizeof(double) * 5 * (kDiagBlocks + 1));
@@ -1843,7 +1842,7 @@ int batch_reorder(dm_batch *B, double dt = 0.0, bool mid = false, bool force = t
         DM_CUDA(ctx, launch_pdl(batch_sort_clouds, dim3(B->nclouds), dim3(kBatchSortThreads), kBatchSortSmem, s,
                                 B->d, (const BatchCloud *)B->ddesc, B->dbox, dt, mid,
                                 B->mid_valid && B->mid_dt == dt && B->boxes_valid[1], force || !B->boxes_valid[0], B->slot,
-                                B->sort.sorted_at));
+                                B->sort.order));
         ctx->launches++;
         B->boxes_valid[0] = true;
         B->boxes_valid[1] = B->mid_valid = mid;
@@ -2079,8 +2078,8 @@ int dm_batch_create(dm_ctx *ctx, int nclouds, const int *n, const double *x, con
     const size_t nh = align256((size_t)kSortBuckets * (B->sort_blocks + 1) * sizeof(uint32_t));
     const size_t ndesc = align256((size_t)nclouds * sizeof(BatchCloud));
     const size_t nbb = align256((size_t)nclouds * 8 * sizeof(double));
-    const size_t nat = align256((size_t)nclouds * sizeof(unsigned long long));
-    const size_t bytes_total = nd * (6 + 5 + 6 + 2 + 6) + nf4 * 8 + ni * 7 + nh + ndesc + nbb + nat + 1024;
+    const size_t nord = align256((size_t)nclouds * sizeof(OrderRecord));
+    const size_t bytes_total = nd * (6 + 5 + 6 + 2 + 6) + nf4 * 8 + ni * 7 + nh + ndesc + nbb + nord + 1024;
     cudaError_t e = cudaMalloc(&B->block, bytes_total);
     if (e != cudaSuccess) {
         delete B;
@@ -2114,7 +2113,7 @@ int dm_batch_create(dm_ctx *ctx, int nclouds, const int *n, const double *x, con
     B->sort.hist = (uint32_t *)p; p += nh;
     B->ddesc = (BatchCloud *)p; p += ndesc;
     B->dbox = (double *)p; p += nbb;
-    B->sort.sorted_at = (unsigned long long *)p; p += nat;
+    B->sort.order = (OrderRecord *)p; p += nord;
     d.step_ctr = (unsigned long long *)p; p += 256;
     d.time = (double *)(d.step_ctr + 4);  // same 256-byte slot, bytes 32-47
     d.err = (int *)p; p += 256;

@@ -206,15 +206,13 @@ struct BatchSortSmem {
 };
 constexpr size_t kBatchSortSmem = sizeof(BatchSortSmem);
 
-// box_out[8 * cloud]: key box x0, y0, extent, order_cost of the sorted cloud,
-// bounding box min x, min y, max x, max y (as batch_boxes writes them; the
-// batch autotuner reads it).  Without `force` a cloud in good order (see
+// box_out[8 * cloud]: key box x0, y0, extent, -, bounding box min x, min y, max
+// x, max y (as batch_boxes writes them; the batch autotuner reads it).  Without `force` a cloud in good order (see
 // kOrderKeep) is left as it is; if `mid` and not `mid_ready` its set 1 is
-// written.  sorted_at[cloud]: step index of its last sort; slot: of the step
-// counter.
+// written.  order[cloud]: its last sort; slot: of the step counter.
 static __global__ void __launch_bounds__(kBatchSortThreads, 1)
     batch_sort_clouds(CloudDev c, const BatchCloud *__restrict__ desc, double *box_out, double dt, bool mid,
-                      bool mid_ready, bool force, int slot, unsigned long long *sorted_at) {
+                      bool mid_ready, bool force, int slot, OrderRecord *order) {
     pdl_wait();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     BatchSortSmem &S = *reinterpret_cast<BatchSortSmem *>(smem_raw);
@@ -222,13 +220,12 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
     const BatchCloud d = desc[blockIdx.x];
     const int off = d.off, n = d.n;
     const float4 *__restrict__ pa0 = c.pa[0] + off;
-    const float rc = sqrtf(d.rc2_up);
     const int groups = (n + 31) / 32;
 
-    if (!force && order_is_recent(c, slot, sorted_at[blockIdx.x])) {
-        const float now = (tid < groups) ? order_cost(c.gbox[0] + d.goff, tid, groups, rc) : 0.0f;
-        const float was = (tid == 0) ? (float)box_out[8 * blockIdx.x + 3] : 0.0f;
-        if (block_order_kept<kBatchSortWarps>(now, was, groups, S.wmom)) {
+    const OrderRecord was = order[blockIdx.x];
+    if (!force && order_is_recent(c, slot, was)) {
+        const OrderRecord now = block_order_record<1>(c.gbox[0] + d.goff, pa0, groups, S.wmom);
+        if (order_is_good(now, was, groups, sqrtf(d.rc2_up))) {
             if (mid && !mid_ready) {
                 CloudDev v = c;
                 v.rc2_up = d.rc2_up;
@@ -378,16 +375,9 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
         if (mid) store_group_box(c.gbox[1] + d.goff + (li >> 5), li < n, h[1].x, h[1].y, (li & ~31) < n);
     }
     __syncthreads();  // the boxes are written
-    float cost = (tid < groups) ? order_cost(c.gbox[0] + d.goff, tid, groups, rc) : 0.0f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, o);
-    if (lane == 0) S.wmom[warp][0] = cost;
-    __syncthreads();
-    if (tid == 0) {
-        for (int w = 1; w < kBatchSortWarps; w++) cost += S.wmom[w][0];
-        box_out[8 * blockIdx.x + 3] = cost;
-        sorted_at[blockIdx.x] = c.step_ctr[slot];
-    }
+    OrderRecord now = block_order_record<1>(c.gbox[0] + d.goff, c.pa[0] + off, groups, S.wmom);
+    now.step = c.step_ctr[slot];
+    if (tid == 0) order[blockIdx.x] = now;
 }
 
 // For the batch autotuner: every cloud squeezed about its own box centre

@@ -38,32 +38,119 @@ constexpr int kSortBuckets = 1 << kSortDigitBits;
 
 // A sort that is due but not required (the cloud was sorted at most kOrderKeep
 // steps ago and no upload has changed it) leaves a cloud alone whose order is
-// still good: compared with the distances between the centres of consecutive
-// 32-particle groups, the groups' boxes (each grown by a cutoff, for what a
-// sweep has to look at) have grown by less than kOrderSlack in area, in the
-// geometric mean over the groups, since the sort.  So neither a cloud that
-// contracts or expands as a whole nor a few particles thrown far out count,
-// and one that mixes does.  (Plain areas summed: a collapsing and re-expanding
-// cloud of 16,384 with particles thrown metres out kept orders that swept half
-// of all pairs over 10,000 steps instead of a quarter.)  The check costs 3 us of a
-// 22-26 us sort (one cluster, latency bound): 4095 particles, 10 RK2 steps 594
-// -> 437 us, 16,384 and 4 RK4 steps 415 -> 345 us.
+// still good: where the sweep is expected to look at less than kOrderSlack times
+// what it would in the order as it was sorted, had the cloud since only grown or
+// shrunk as a whole.  Expected from the boxes of the 32-particle groups: a
+// box of w x h is looked at by the groups in (w + g) x (h + g) about it, g two
+// cutoffs and a typical group's side.  Sides are capped at the cloud's size
+// (a box cannot be looked at by more than all), and the size is one that single
+// particles cannot move (block_order_record), so a particle thrown out counts as
+// what it costs: its group is swept by every other.  Emulated on uniform disks
+// of 4096, 16,384 and 262,144 particles, the ratio follows that of the pairs
+// swept before and after a sort: particles that moved 0.2 mm each way 1.09
+// (pairs 1.07-1.10), 1 mm 2.1 (2.5-3.0), 20 thrown out 2.2-2.5 (1.4-1.8), 400
+// 15-24 (7-13).  Boxes against the distance between consecutive groups' centres,
+// in the geometric mean, fell with every particle thrown: the uniform disk of
+// 16,384, steps 5 to 24, swept 20.6% of all pairs and took 0.196 ms a step, now
+// 16.7% and 0.184 ms; over 1500 steps 0.174 -> 0.164 ms.  A slack of 1 (always
+// sorted) 0.193 and 0.167 ms, 1.05 0.185 and 0.166, 1.2 0.184 and 0.168, 1.4 0.186
+// and 0.174; 262,144 particles 2.44 ms a step up to 1.1, 2.70 at 1.2.
+// The check costs about 3 us of a 22-26 us sort (one cluster, latency bound):
+// calm clouds of 4095 particles, 10 RK2 steps 594 -> 437 us, of 16,384 and 4 RK4
+// steps 415 -> 345 us.
 constexpr int kOrderKeep = 8;
-constexpr float kOrderSlack = 0.1375f;  // log2(1.1)
+constexpr float kOrderSlack = 1.1f;
 
-// Whether the last sort, at step index `at`, is less than kOrderKeep steps ago.
-// Counted from the sort on the device, so that the same state and the same
-// steps are sorted at the same places whatever the cloud did before.
-__device__ __forceinline__ bool order_is_recent(const CloudDev &c, int slot, unsigned long long at) {
-    return c.step_ctr[slot] - at < (unsigned long long)kOrderKeep;
+// The order as last sorted.
+struct OrderRecord {
+    float area, sides;  // sums of w h and of w + h over the groups
+    float scale;        // log2 of the cloud's size
+    unsigned long long step;  // step index of the sort
+};
+
+// Whether the last sort is less than kOrderKeep steps ago.  Counted from the
+// sort on the device, so that the same state and the same steps are sorted at
+// the same places whatever the cloud did before.
+__device__ __forceinline__ bool order_is_recent(const CloudDev &c, int slot, const OrderRecord &was) {
+    return c.step_ctr[slot] - was.step < (unsigned long long)kOrderKeep;
 }
 
-// Group g's share of that measure (log2), among `groups` groups with boxes gb.
-__device__ __forceinline__ float order_cost(const float4 *gb, int g, int groups, float rc) {
-    if (g + 1 >= groups) return 0.0f;
-    const float4 a = __ldcg(gb + g), b = __ldcg(gb + g + 1);
-    const float dx = 0.5f * ((a.x + a.z) - (b.x + b.z)), dy = 0.5f * ((a.y + a.w) - (b.y + b.w));
-    return __log2f((a.z - a.x + rc) * (a.w - a.y + rc)) - __log2f(fmaf(dx, dx, fmaf(dy, dy, rc * rc)));
+// The sums of a and b over the block, in every thread; scratch: a row per warp.
+template <int WARPS, int FIELDS>
+__device__ __forceinline__ float2 block_sum2(float a, float b, float (&scratch)[WARPS][FIELDS]) {
+    static_assert(FIELDS >= 2, "two sums");
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        scratch[threadIdx.x >> 5][0] = a;
+        scratch[threadIdx.x >> 5][1] = b;
+    }
+    __syncthreads();
+    a = b = 0.0f;
+    for (int w = 0; w < WARPS; w++) {
+        a += scratch[w][0];
+        b += scratch[w][1];
+    }
+    __syncthreads();  // scratch is reused
+    return make_float2(a, b);
+}
+
+// The present order's record (but for the step): boxes gb, positions pa0 of
+// `groups` groups; by every thread of the block.  The size is the geometric mean
+// distance between the first particles of groups half the order apart: it does
+// not change when particles mix, and one particle thrown out moves it only if
+// it is such a first one, by its logarithm over their number.  Bound by two
+// round trips to L2 and two block sums; each thread's first HELD boxes are on
+// their way with the positions.
+template <int HELD, int WARPS, int FIELDS>
+__device__ __forceinline__ OrderRecord block_order_record(const float4 *gb, const float4 *pa0, int groups,
+                                                          float (&scratch)[WARPS][FIELDS]) {
+    constexpr int NT = 32 * WARPS;
+    const int tid = threadIdx.x, half = groups >> 1;
+    float4 held[HELD];
+#pragma unroll
+    for (int u = 0; u < HELD; u++)
+        held[u] = (tid + u * NT < groups) ? __ldcg(gb + tid + u * NT) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float lg = 0.0f, cnt = 0.0f;
+    const int g0 = tid * max(1, half / NT);  // a pair per thread is enough of a sample
+    if (g0 < half) {
+        const float4 a = __ldcg(pa0 + 32 * g0), b = __ldcg(pa0 + 32 * (g0 + half));
+        const float dx = a.x - b.x, dy = a.y - b.y, d2 = fmaf(dx, dx, dy * dy);
+        if (d2 > 0.0f && d2 < INFINITY) {  // NaN: neither
+            lg = 0.5f * __log2f(d2);
+            cnt = 1.0f;
+        }
+    }
+    const float2 size = block_sum2(lg, cnt, scratch);
+    OrderRecord R;
+    R.scale = size.x / fmaxf(size.y, 1.0f);
+    const float cap = 2.0f * exp2f(R.scale);
+    float area = 0.0f, sides = 0.0f;
+    auto add = [&](const float4 &box) {
+        const float w = fminf(box.z - box.x, cap), h = fminf(box.w - box.y, cap);  // NaN: cap
+        area = fmaf(w, h, area);
+        sides += w + h;
+    };
+#pragma unroll
+    for (int u = 0; u < HELD; u++)
+        if (tid + u * NT < groups) add(held[u]);
+#pragma unroll HELD
+    for (int g = tid + HELD * NT; g < groups; g += NT) add(__ldcg(gb + g));
+    const float2 sum = block_sum2(area, sides, scratch);
+    R.area = sum.x;
+    R.sides = sum.y;
+    R.step = 0;
+    return R;
+}
+
+// Whether the order `now` is as good as it `was` (see kOrderSlack); false for NaN.
+__device__ __forceinline__ bool order_is_good(const OrderRecord &now, const OrderRecord &was, int groups, float rc) {
+    const float k = exp2f(now.scale - was.scale), G = (float)groups;
+    const float g = 2.0f * rc + k * was.sides / (2.0f * G);
+    return now.area + g * now.sides + G * g * g <= kOrderSlack * (k * k * was.area + k * g * was.sides + G * g * g);
 }
 
 constexpr int kMomentBlocks = 128;  // fixed partition of the moment reduction
@@ -72,10 +159,9 @@ constexpr int kMomentFields = 9;   // count, sum dx, sum dy, sum dx^2, sum dy^2,
 struct SortScratch {
     float *moments;            // [kMomentBlocks][kMomentFields] per-block partials
     double *box;               // [8]: key box x0, y0, extent; -; bounding box min x, min y, max x, max y
-    float *cost;               // [16]: order_cost of the cloud as last sorted, per block of the kernel that wrote it
+    OrderRecord *order;        // the cloud as last sorted (a batch: each cloud)
     int *keep;                 // set by order_check: the order is still good
     int *changed;              // number of the last upload that changed the state
-    unsigned long long *sorted_at;  // step index of the last sort
     uint32_t *keys[2];
     int *vals[2];
     uint32_t *hist;            // [kSortBuckets * nblocks], then [kSortBuckets] totals
@@ -267,30 +353,6 @@ __device__ __forceinline__ uint32_t morton_key_f32(float x, float y, const float
     return spread_bits12(qx) | (spread_bits12(qy) << 1);
 }
 
-// Whether the block's threads' costs `now` together exceed their `was` by at most
-// kOrderSlack a group.  Every thread of the block; scratch: a row per warp.
-template <int WARPS, int FIELDS>
-__device__ __forceinline__ bool block_order_kept(float now, float was, int groups, float (&scratch)[WARPS][FIELDS]) {
-    static_assert(FIELDS >= 2, "two sums");
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        now += __shfl_xor_sync(0xffffffffu, now, o);
-        was += __shfl_xor_sync(0xffffffffu, was, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        scratch[threadIdx.x >> 5][0] = now;
-        scratch[threadIdx.x >> 5][1] = was;
-    }
-    __syncthreads();
-    now = was = 0.0f;
-    for (int w = 0; w < WARPS; w++) {
-        now += scratch[w][0];
-        was += scratch[w][1];
-    }
-    __syncthreads();  // scratch is reused
-    return now - was <= kOrderSlack * (float)groups;  // false for NaN
-}
-
 // Position set 1 (see write_midpoint) of slot s and its group's box; whole warps.
 __device__ __forceinline__ void write_midpoint_group(const CloudDev &c, int s, bool live, float4 *gbox, bool store,
                                                      double dt) {
@@ -320,35 +382,21 @@ __device__ __forceinline__ bool order_is_kept(const int *keep) { return keep && 
 static __global__ void __launch_bounds__(1024) order_check(CloudDev c, SortScratch z, int slot, int upload) {
     pdl_wait();
     __shared__ float s[32][2];
-    const float rc = sqrtf(c.rc2_up);
     const int groups = (c.n + 31) / 32;
-    float now = 0.0f;
-#pragma unroll 4
-    for (int g = threadIdx.x; g < groups; g += 1024) now += order_cost(c.gbox[0], g, groups, rc);
-    const bool kept = block_order_kept<32>(now, (threadIdx.x == 0) ? z.cost[0] : 0.0f, groups, s);
+    const OrderRecord now = block_order_record<8>(c.gbox[0], c.pa[0], groups, s);
     if (threadIdx.x == 0)
-        *z.keep = kept && order_is_recent(c, slot, *z.sorted_at) && (upload == 0 || *z.changed != upload);
+        *z.keep = order_is_good(now, *z.order, groups, sqrtf(c.rc2_up)) && order_is_recent(c, slot, *z.order) &&
+                  (upload == 0 || *z.changed != upload);
 }
 
 // ... and, after a sort, how good it is.
 static __global__ void __launch_bounds__(1024) order_record(CloudDev c, SortScratch z, int slot, const int *keep) {
     pdl_wait();
     if (order_is_kept(keep)) return;
-    __shared__ float s[32];
-    const float rc = sqrtf(c.rc2_up);
-    const int groups = (c.n + 31) / 32;
-    float now = 0.0f;
-#pragma unroll 4
-    for (int g = threadIdx.x; g < groups; g += 1024) now += order_cost(c.gbox[0], g, groups, rc);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) now += __shfl_xor_sync(0xffffffffu, now, o);
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = now;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < 32; w++) now += s[w];
-        z.cost[0] = now;
-        *z.sorted_at = c.step_ctr[slot];
-    }
+    __shared__ float s[32][2];
+    OrderRecord now = block_order_record<8>(c.gbox[0], c.pa[0], (c.n + 31) / 32, s);
+    now.step = c.step_ctr[slot];
+    if (threadIdx.x == 0) *z.order = now;
 }
 
 // Per-block moments of the cloud's positions (origin: its first particle).
@@ -580,14 +628,11 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
     const int n = c.n;
     const int e0 = r * kSortClusterPer;
     const int groups = (n + 31) / 32;
-    const float rc = sqrtf(c.rc2_up);
 
     // every block comes to the same decision
-    if (!force && order_is_recent(c, slot, *z.sorted_at) && (upload == 0 || *z.changed != upload)) {
-        float now = 0.0f;
-        for (int g = tid; g < groups; g += kSortClusterThreads) now += order_cost(c.gbox[0], g, groups, rc);
-        const float was = (tid < kSortClusterCtas) ? z.cost[tid] : 0.0f;
-        if (block_order_kept<kSortClusterWarps>(now, was, groups, S.wmom)) {
+    if (!force && order_is_recent(c, slot, *z.order) && (upload == 0 || *z.changed != upload)) {
+        const OrderRecord now = block_order_record<1>(c.gbox[0], pa0, groups, S.wmom);
+        if (order_is_good(now, *z.order, groups, sqrtf(c.rc2_up))) {
             if (mid && !mid_ready)
                 for (int k = 0; k < kSortClusterRounds; k++) {
                     const int s = e0 + k * kSortClusterThreads + tid;
@@ -776,16 +821,10 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
         if (mid) store_group_box(c.gbox[1] + (s >> 5), s < n, h[1].x, h[1].y, (s & ~31) < c.n_pad);
     }
     cl.sync();  // the boxes are written (ordered at cluster scope)
-    if (warp == 0) {
-        float cost = 0.0f;
-        for (int g = e0 / 32 + lane; g < (e0 + kSortClusterPer) / 32; g += 32)
-            cost += order_cost(c.gbox[0], g, groups, rc);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, o);
-        if (lane == 0) {
-            z.cost[r] = cost;
-            if (r == 0) *z.sorted_at = c.step_ctr[slot];
-        }
+    if (r == 0) {
+        OrderRecord now = block_order_record<1>(c.gbox[0], c.pa[0], groups, S.wmom);
+        now.step = c.step_ctr[slot];
+        if (tid == 0) *z.order = now;
     }
 }
 
