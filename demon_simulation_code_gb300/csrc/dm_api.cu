@@ -116,6 +116,7 @@ struct dm_cloud {
     int tuned_variant[2] = {-1, -1};  // per precision: index into kVariants
     float2 *partial = nullptr;         // [2 partial_cap][2][n_pad] non-cluster partial sums (per set and rank, axis)
     int partial_cap = 0;
+    std::vector<void *> retired;       // outgrown partial-sum buffers that recorded steps may still use
     SortScratch sort{};
     int sort_blocks = 0;
     int reorder_interval = 1;   // steps between Morton re-sorts (0 = never)
@@ -140,6 +141,7 @@ struct dm_cloud {
     }
     ~dm_cloud() {
         if (partial) cudaFree(partial);
+        for (void *p : retired) cudaFree(p);
     }
 };
 
@@ -461,7 +463,8 @@ int ensure_partial(dm_cloud *c, int S) {
     if (S <= c->partial_cap) return DM_OK;
     dm_ctx *ctx = c->ctx;
     DM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (c->partial) cudaFree(c->partial);
+    if (c->partial && c->captured) c->retired.push_back(c->partial);  // the caller's graphs hold its address
+    else if (c->partial) cudaFree(c->partial);
     c->partial = nullptr;
     c->partial_cap = 0;
     cudaError_t e = cudaMalloc((void **)&c->partial, (size_t)S * 4 * c->n_pad * sizeof(float2));
