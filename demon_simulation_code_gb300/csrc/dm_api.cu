@@ -40,8 +40,10 @@ constexpr int kFp64UnsortedMax = 4096;
 constexpr int kGraphSteps = 16;
 // States of at most this many particles in pageable memory cross through the
 // context's page-locked staging (64 bytes each) and a copy kernel; larger ones by
-// DMA (eight pageable copies cost 35 us of host time a round trip, whatever the
-// size: 64 grains, one step 96 -> 58 us; 16,384 FP64, one step 242 -> 220 us).
+// DMA.  Eight pageable copies cost the host a fixed ~70 us a round trip (upload
+// and download), staging ~2.3 us per 1024 particles, two passes of the host over
+// the state: 1024 particles 71 us by DMA, 37 staged; 8192 87 and 59; 16,384 108
+// and 86; 24,576 111 and 120; 65,536 129 and 302.
 constexpr int kStagedCopyMax = 16384;
 
 }  // namespace
