@@ -878,12 +878,19 @@ int run_steps(dm_cloud *c, int nsteps, double dt, int precision) {
         // after a force evaluation)
         c->supers_valid[0] = c->supers_valid[1] = false;
         if (sorts) c->mid_valid = false;
+        const CloudDev state = c->d;
+        const int slot = c->slot;
         DM_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         int rc = enqueue_steps(c, kGraphSteps, dt, precision);
         cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
         c->host_steps = saved;  // capture recorded the steps, it did not run them
         c->graph_launches = ctx->launches - saved_launches;
         ctx->launches = saved_launches;
+        if (rc || ec != cudaSuccess) {  // nothing has run: the state is where it was
+            c->d = state;
+            c->slot = slot;
+            c->state_changed(false);
+        }
         if (rc) {
             if (g) cudaGraphDestroy(g);
             return rc;
@@ -2010,12 +2017,19 @@ int batch_run_steps(dm_batch *B, int nsteps, double dt) {
         const unsigned long long saved = B->host_steps;
         const long long sl = ctx->launches;
         if (sorts) B->mid_valid = false;
+        const CloudDev state = B->d;
+        const int slot = B->slot;
         DM_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         int rc = batch_enqueue_steps(B, kGraphSteps, dt);
         cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
         B->host_steps = saved;
         graph_launches_cache = ctx->launches - sl;
         ctx->launches = sl;
+        if (rc || ec != cudaSuccess) {  // see run_steps
+            B->d = state;
+            B->slot = slot;
+            B->boxes_valid[0] = B->boxes_valid[1] = B->mid_valid = false;
+        }
         if (rc) {
             if (g) cudaGraphDestroy(g);
             return rc;
