@@ -694,16 +694,11 @@ int tune_precision(dm_cloud *c, int precision) {
                 for (int st = 0; st < nstates && ms < 1.3f * best_ms; st++) {
                     // both sets on the same buffer: a pass's work
                     const StageParams P = make_stage_params(c, 0, kModeForceOnly, 0.0, nullptr, st, 2);
-                    // one launch, then the timed ones; up to 1024 particles without
-                    // looking at the first (a synchronisation costs as much as the launches:
-                    // 151 particles 1.9 -> 1.6 ms of tuning; 4095, where the first launch
-                    // of a poor candidate tells, 27 -> 32 ms)
-                    const bool look = c->n > 1024;
-                    int warm = DM_OK;
-                    if (!look) warm = launch_variant(c, vi, S, P);
-                    if (warm) return warm;
-                    for (int runs : {look ? 1 : 0, reps}) {
-                        if (runs == 0) continue;
+                    // one launch, then the timed ones.  (Without a look at the first, which
+                    // saves a synchronisation a candidate but times every poor one in
+                    // full, tuning took 2.9 ms instead of 2.2 at 512 particles, 29
+                    // instead of 19 at 4095; 151 particles 1.6 either way.)
+                    for (int runs : {1, reps}) {
                         int rc = cudaEventRecord(a, ctx->stream) == cudaSuccess ? DM_OK : DM_ERR_CUDA;
                         for (int r = 0; r < runs && !rc; r++) rc = launch_variant(c, vi, S, P);
                         if (!rc) rc = cudaEventRecord(b, ctx->stream) == cudaSuccess ? DM_OK : DM_ERR_CUDA;
