@@ -652,8 +652,8 @@ static __global__ void __launch_bounds__(kAdjThreads) adj_vjp_fp32c(const AdjClo
 // (dm_fp64.cuh), or, where most of the 32 x 32 pairs are hits, lane by lane
 // (every lane its own i, all on the same j: no list, the sums by FMA).  The
 // four warps of the cluster's first block then take one component each of the
-// particles' stage epilogue.  Bound by the FP64 pipe: 22 (forward) and 37
-// (backward) FP64 instructions per pair.
+// particles' stage epilogue.  Bound by the FP64 pipe: 20 (forward) and 35
+// (backward) FP64 instructions per pair, 2 and 4 more to add up a listed hit.
 // ---------------------------------------------------------------------------
 constexpr int kAdjWarps = 4;
 

@@ -1216,7 +1216,7 @@ int dm_cloud_create(dm_ctx *ctx, int n, const double *x, const double *y, const 
     }
     c->d.eval_pairs = (unsigned long long *)p; p += 256;
     c->d.step_ctr = (unsigned long long *)p; p += 256;
-    c->d.time = (double *)(c->d.step_ctr + 4);  // same 256-byte slot, bytes 32-47
+    c->d.time = (double *)(c->d.step_ctr + 4);  // same 256-byte slot, bytes 32-55
     c->d.err = (int *)p; p += 256;
     c->d_dt = (double *)p; p += 256;
     c->d_min = (unsigned int *)p; p += 256;
@@ -2129,7 +2129,7 @@ int dm_batch_create(dm_ctx *ctx, int nclouds, const int *n, const double *x, con
     B->dbox = (double *)p; p += nbb;
     B->sort.order = (OrderRecord *)p; p += nord;
     d.step_ctr = (unsigned long long *)p; p += 256;
-    d.time = (double *)(d.step_ctr + 4);  // same 256-byte slot, bytes 32-47
+    d.time = (double *)(d.step_ctr + 4);  // same 256-byte slot, bytes 32-55
     d.err = (int *)p; p += 256;
     // host descriptors
     B->hdesc.resize(nclouds);

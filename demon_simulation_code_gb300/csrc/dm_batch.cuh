@@ -142,8 +142,6 @@ static __global__ void batch_midpoint(CloudDev c, const BatchCloud *__restrict__
 
 // --- per-cloud Morton order ------------------------------------------------
 
-// bbox rows are (min x, min y, max x, max y) in ordered bits: the min
-// entries start at all-ones (memset), the max entries at zero.
 // One block per cloud: the cloud's key box (the bounding box clipped to
 // mean +- 4 sigma per axis) and bounding box, box[8 * cloud ...] as in
 // moments_to_box.  Deterministic (fixed partition and order).

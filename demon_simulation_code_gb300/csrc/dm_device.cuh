@@ -619,9 +619,13 @@ __device__ __forceinline__ double axis_force(const ForceParams &f, int ax, doubl
     return F;
 }
 
-// a / b correctly rounded, given rb = 1/b correctly rounded: one residual
-// correction of a rb (Markstein), 3 FP64 instructions instead of the ~9 of a
-// division.  Zero, tiny, huge and non-finite values take the division itself.
+// a / b given rb = 1/b correctly rounded: one residual correction of a rb, 3 FP64
+// instructions instead of the ~9 of a division.  Correctly rounded wherever a rb
+// is within one ulp of a/b (Markstein's theorem); the product alone only bounds
+// that by 1.5, but of 1.6e9 quotients tried, the corners next to powers of two
+// among them, every product was within one ulp and every result that of the
+// division (3 and 6 as divisors too).  Zero, tiny, huge and non-finite values
+// take the division itself.
 __device__ __forceinline__ double div_by(double a, double b, double rb) {
     const double q = __dmul_rn(a, rb);
     const uint32_t ea = ((uint32_t)__double2hiint(a) >> 20) & 0x7FFu, eq = ((uint32_t)__double2hiint(q) >> 20) & 0x7FFu;

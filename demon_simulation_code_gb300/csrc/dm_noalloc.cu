@@ -5,13 +5,12 @@
 // must not trigger cudaMalloc's implicit device-wide synchronisation while
 // its other streams run.  They already hold the particle state in their own
 // device buffers and want the FP64 energies and momentum of it without
-// creating a dm_cloud (which allocates ~200 bytes per particle) and without
-// the temporary partial-sum buffer dm_cloud_diagnostics allocates.
+// creating a dm_cloud (which allocates ~350 bytes per particle).
 //
 // This file gives them dm_diagnostics_noalloc: the same diagnostics kernel,
 // with its per-block partial sums in a fixed-size file-scope device array.
-// Every GPU that loads this library holds that array (kMaxBlocks * 5
-// doubles = 160 KiB) until the process exits.  Calls share the array, so
+// Every GPU that loads this library holds that array (kDiagBlocks * 5
+// doubles = 24 KiB) until the process exits.  Calls share the array, so
 // calls that overlap on the GPU (different streams, or different host
 // threads on the same device) race on it and must be serialised by the
 // caller.  Each call overwrites every partial it later reads, so nothing has
@@ -28,12 +27,10 @@ using namespace dm;
 
 namespace {
 
-constexpr int kMaxBlocks = 4096;        // rows of the scratch (kDiagBlocks of them are used)
-constexpr int kMaxParticles = 524288;   // the documented limit
-static_assert(kDiagBlocks <= kMaxBlocks, "one scratch row per block");
+constexpr int kMaxParticles = 524288;  // the interface's limit (the scratch holds the blocks of any size)
 
-// The scratch: one row of 5 partial sums per block.
-static __device__ __align__(256) double g_diag_scratch[kMaxBlocks * 5];
+// The scratch: one row of 5 partial sums per block (diagnostics_blocks: at most kDiagBlocks).
+static __device__ __align__(256) double g_diag_scratch[kDiagBlocks * 5];
 
 // In host code g_diag_scratch names a host-side stand-in, not device memory:
 // the device address is looked up on every call, with the calling device

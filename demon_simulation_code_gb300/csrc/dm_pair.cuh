@@ -1145,9 +1145,9 @@ static __global__ void __launch_bounds__(ALL ? 64 * kTermParts : 128) stage_fini
 // hits in FP64 with full warps (dm_fp64.cuh).  The sums meet in the cluster's
 // first block, which runs the epilogue.
 //
-// Bound by the FP64 pipe on dense clouds (22 FP64 instructions per pair in
-// reach, 64 cycles of a scheduler's FP64 unit per 32 pairs each), by latency
-// on sparse ones.
+// Bound by the FP64 pipe on dense clouds (20 FP64 instructions per pair that
+// passed the filter and 2 to add it up, 64 cycles of a scheduler's FP64 unit per
+// 32 pairs each), by latency on sparse ones.
 // ---------------------------------------------------------------------------
 template <int NW>
 struct Group64Set {  // one position set's half of the block

@@ -128,7 +128,14 @@ int dm_ctx_create(int device, dm_ctx **out);
 int dm_ctx_destroy(dm_ctx *ctx);
 
 /* Use an existing cudaStream_t (passed as void*) for all later work; NULL
- * means the CUDA default (legacy) stream, as in the CUDA runtime. */
+ * means the CUDA default (legacy) stream, as in the CUDA runtime.
+ *
+ * Calls that only queue work (fixed-dt steps, uploads) may be recorded by the
+ * caller's stream capture on that stream and replayed, once the cloud has
+ * taken a step at that precision without a capture (kernels are chosen then).
+ * A replay changes the state unseen by the library, so from its first recorded
+ * call on, every call on that cloud (or batch) sorts and forms the step's
+ * midpoint anew. */
 int dm_ctx_set_stream(dm_ctx *ctx, void *cuda_stream);
 /* Back to the context's own stream. */
 int dm_ctx_reset_stream(dm_ctx *ctx);
@@ -398,7 +405,7 @@ int dm_adjoint_rk4_step_vjp(dm_adjoint *adj, int precision, double dt,
  * `stream` (a cudaStream_t, NULL = the legacy default stream) and the call
  * returns without waiting.  It needs no dm_ctx or dm_cloud and calls no
  * allocating CUDA or library routine: its partial sums live in a fixed
- * file-scope device array of 4096 x 5 doubles (160 KiB, held by every GPU
+ * file-scope device array of 608 x 5 doubles (24 KiB, held by every GPU
  * that loads this library until the process exits).
  *  - n must be in [1, 524288]; larger n returns DM_ERR_ARG without launching.
  *  - params are checked as dm_cloud_set_forces checks them.
