@@ -215,13 +215,14 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     BatchSortSmem &S = *reinterpret_cast<BatchSortSmem *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const OrderRecord was = order[blockIdx.x];
+    const unsigned long long step = c.step_ctr[slot];
     const BatchCloud d = desc[blockIdx.x];
     const int off = d.off, n = d.n;
     const float4 *__restrict__ pa0 = c.pa[0] + off;
     const int groups = (n + 31) / 32;
 
-    const OrderRecord was = order[blockIdx.x];
-    if (!force && order_is_recent(c, slot, was)) {
+    if (!force && order_is_recent(step, was.step)) {
         const OrderRecord now = block_order_record<1>(c.gbox[0] + d.goff, pa0, groups, S.wmom);
         if (order_is_good(now, was, groups, sqrtf(d.rc2_up))) {
             if (mid && !mid_ready) {
@@ -374,7 +375,7 @@ static __global__ void __launch_bounds__(kBatchSortThreads, 1)
     }
     __syncthreads();  // the boxes are written
     OrderRecord now = block_order_record<1>(c.gbox[0] + d.goff, c.pa[0] + off, groups, S.wmom);
-    now.step = c.step_ctr[slot];
+    now.step = step;
     if (tid == 0) order[blockIdx.x] = now;
 }
 

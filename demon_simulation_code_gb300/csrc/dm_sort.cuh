@@ -68,33 +68,34 @@ struct OrderRecord {
     unsigned long long step;  // step index of the sort
 };
 
-// Whether the last sort is less than kOrderKeep steps ago.  Counted from the
-// sort on the device, so that the same state and the same steps are sorted at
-// the same places whatever the cloud did before.
-__device__ __forceinline__ bool order_is_recent(const CloudDev &c, int slot, const OrderRecord &was) {
-    return c.step_ctr[slot] - was.step < (unsigned long long)kOrderKeep;
+// Whether a sort at step index `at` is less than kOrderKeep steps ago.  Counted
+// from the sort on the device, so that the same state and the same steps are
+// sorted at the same places whatever the cloud did before.
+__device__ __forceinline__ bool order_is_recent(unsigned long long step, unsigned long long at) {
+    return step - at < (unsigned long long)kOrderKeep;
 }
 
-// The sums of a and b over the block, in every thread; scratch: a row per warp.
-template <int WARPS, int FIELDS>
+// The sums of a and b over the block, in every thread; columns COL and COL + 1 of
+// scratch (a row per warp) are free again after the block's next barrier.
+template <int COL, int WARPS, int FIELDS>
 __device__ __forceinline__ float2 block_sum2(float a, float b, float (&scratch)[WARPS][FIELDS]) {
-    static_assert(FIELDS >= 2, "two sums");
+    static_assert(FIELDS >= COL + 2, "two sums");
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         a += __shfl_xor_sync(0xffffffffu, a, o);
         b += __shfl_xor_sync(0xffffffffu, b, o);
     }
     if ((threadIdx.x & 31) == 0) {
-        scratch[threadIdx.x >> 5][0] = a;
-        scratch[threadIdx.x >> 5][1] = b;
+        scratch[threadIdx.x >> 5][COL] = a;
+        scratch[threadIdx.x >> 5][COL + 1] = b;
     }
     __syncthreads();
     a = b = 0.0f;
+#pragma unroll
     for (int w = 0; w < WARPS; w++) {
-        a += scratch[w][0];
-        b += scratch[w][1];
+        a += scratch[w][COL];
+        b += scratch[w][COL + 1];
     }
-    __syncthreads();  // scratch is reused
     return make_float2(a, b);
 }
 
@@ -124,7 +125,7 @@ __device__ __forceinline__ OrderRecord block_order_record(const float4 *gb, cons
             cnt = 1.0f;
         }
     }
-    const float2 size = block_sum2(lg, cnt, scratch);
+    const float2 size = block_sum2<0>(lg, cnt, scratch);
     OrderRecord R;
     R.scale = size.x / fmaxf(size.y, 1.0f);
     const float cap = 2.0f * exp2f(R.scale);
@@ -139,7 +140,8 @@ __device__ __forceinline__ OrderRecord block_order_record(const float4 *gb, cons
         if (tid + u * NT < groups) add(held[u]);
 #pragma unroll HELD
     for (int g = tid + HELD * NT; g < groups; g += NT) add(__ldcg(gb + g));
-    const float2 sum = block_sum2(area, sides, scratch);
+    const float2 sum = block_sum2<2>(area, sides, scratch);
+    __syncthreads();  // scratch is reused
     R.area = sum.x;
     R.sides = sum.y;
     R.step = 0;
@@ -381,19 +383,22 @@ __device__ __forceinline__ bool order_is_kept(const int *keep) { return keep && 
 // One block: whether the cloud's order is still good (slot: of the step counter) ...
 static __global__ void __launch_bounds__(1024) order_check(CloudDev c, SortScratch z, int slot, int upload) {
     pdl_wait();
-    __shared__ float s[32][2];
+    __shared__ float s[32][4];
     const int groups = (c.n + 31) / 32;
+    const OrderRecord was = *z.order;  // on their way with the boxes
+    const unsigned long long step = c.step_ctr[slot];
+    const int changed = *z.changed;
     const OrderRecord now = block_order_record<8>(c.gbox[0], c.pa[0], groups, s);
     if (threadIdx.x == 0)
-        *z.keep = order_is_good(now, *z.order, groups, sqrtf(c.rc2_up)) && order_is_recent(c, slot, *z.order) &&
-                  (upload == 0 || *z.changed != upload);
+        *z.keep = order_is_good(now, was, groups, sqrtf(c.rc2_up)) && order_is_recent(step, was.step) &&
+                  (upload == 0 || changed != upload);
 }
 
 // ... and, after a sort, how good it is.
 static __global__ void __launch_bounds__(1024) order_record(CloudDev c, SortScratch z, int slot, const int *keep) {
     pdl_wait();
     if (order_is_kept(keep)) return;
-    __shared__ float s[32][2];
+    __shared__ float s[32][4];
     OrderRecord now = block_order_record<8>(c.gbox[0], c.pa[0], (c.n + 31) / 32, s);
     now.step = c.step_ctr[slot];
     if (threadIdx.x == 0) *z.order = now;
@@ -630,9 +635,11 @@ static __global__ void __launch_bounds__(kSortClusterThreads, 1)
     const int groups = (n + 31) / 32;
 
     // every block comes to the same decision
-    if (!force && order_is_recent(c, slot, *z.order) && (upload == 0 || *z.changed != upload)) {
+    if (!force && (upload == 0 || *z.changed != upload)) {
+        const OrderRecord was = *z.order;  // on their way with the boxes
+        const unsigned long long step = c.step_ctr[slot];
         const OrderRecord now = block_order_record<1>(c.gbox[0], pa0, groups, S.wmom);
-        if (order_is_good(now, *z.order, groups, sqrtf(c.rc2_up))) {
+        if (order_is_good(now, was, groups, sqrtf(c.rc2_up)) && order_is_recent(step, was.step)) {
             if (mid && !mid_ready)
                 for (int k = 0; k < kSortClusterRounds; k++) {
                     const int s = e0 + k * kSortClusterThreads + tid;
