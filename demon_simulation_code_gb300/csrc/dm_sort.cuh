@@ -55,7 +55,7 @@ constexpr int kSortBuckets = 1 << kSortDigitBits;
 // 16.7% and 0.184 ms; over 1500 steps 0.174 -> 0.164 ms.  A slack of 1 (always
 // sorted) 0.193 and 0.167 ms, 1.05 0.185 and 0.166, 1.2 0.184 and 0.168, 1.4 0.186
 // and 0.174; 262,144 particles 2.44 ms a step up to 1.1, 2.70 at 1.2.
-// The check costs about 3 us of a 22-26 us sort (one cluster, latency bound):
+// The check costs about 4 us of a 27 us sort (one cluster, latency bound):
 // calm clouds of 4095 particles, 10 RK2 steps 594 -> 437 us, of 16,384 and 4 RK4
 // steps 415 -> 345 us.
 constexpr int kOrderKeep = 8;
