@@ -93,6 +93,12 @@ struct GraphKey {
     }
 };
 
+// A captured block of steps and the kernels in it.
+struct StepGraph {
+    cudaGraphExec_t exec;
+    long long launches;
+};
+
 struct dm_cloud {
     dm_ctx *ctx = nullptr;
     int n = 0, n_pad = 0;
@@ -127,12 +133,11 @@ struct dm_cloud {
     int dirty_upload = 0;       // ... if upload of this number changed the state (0: in any case)
     int uploads = 0;
     unsigned long long host_steps = 0;  // RK4 steps enqueued so far
-    long long graph_launches = 0;       // kernels in one replay of the step graph
-    std::map<GraphKey, cudaGraphExec_t> graphs;
+    std::map<GraphKey, StepGraph> graphs;
     cudaStream_t graph_stream = nullptr;  // stream the graphs were built for
 
     void drop_graphs() {
-        for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
+        for (auto &kv : graphs) cudaGraphExecDestroy(kv.second.exec);
         graphs.clear();
     }
     // the state (set 0) was rewritten: what was derived from it is stale;
@@ -879,7 +884,7 @@ int run_steps(dm_cloud *c, int nsteps, double dt, int precision) {
         int rc = enqueue_steps(c, kGraphSteps, dt, precision);
         cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
         c->host_steps = saved;  // capture recorded the steps, it did not run them
-        c->graph_launches = ctx->launches - saved_launches;
+        const long long launches = ctx->launches - saved_launches;
         ctx->launches = saved_launches;
         if (rc || ec != cudaSuccess) {  // nothing has run: the state is where it was
             c->d = state;
@@ -895,13 +900,13 @@ int run_steps(dm_cloud *c, int nsteps, double dt, int precision) {
         ec = cudaGraphInstantiate(&ge, g, 0);
         cudaGraphDestroy(g);
         if (ec != cudaSuccess) return ctx->fail(DM_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(ec));
-        it = c->graphs.emplace(key, ge).first;
+        it = c->graphs.emplace(key, StepGraph{ge, launches}).first;
     }
     const int reps = nsteps / kGraphSteps;
     for (int r = 0; r < reps; r++) {
-        DM_CUDA(ctx, cudaGraphLaunch(it->second, ctx->stream));
+        DM_CUDA(ctx, cudaGraphLaunch(it->second.exec, ctx->stream));
         c->host_steps += kGraphSteps;
-        ctx->launches += c->graph_launches;
+        ctx->launches += it->second.launches;
         c->mid_valid = true;  // the replayed steps leave every position set's boxes and the midpoint
         c->mid_dt = dt;
         for (bool &v : c->boxes_valid) v = true;
@@ -1752,12 +1757,12 @@ struct dm_batch {
     int slot = 0;
     bool capturing = false, captured = false;  // as dm_cloud's
     unsigned long long host_steps = 0;
-    std::map<GraphKey, cudaGraphExec_t> graphs;
+    std::map<GraphKey, StepGraph> graphs;
     cudaStream_t graph_stream = nullptr;
     std::vector<void *> extra;
 
     void drop_graphs() {
-        for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
+        for (auto &kv : graphs) cudaGraphExecDestroy(kv.second.exec);
         graphs.clear();
     }
     ~dm_batch() {
@@ -2006,7 +2011,6 @@ int batch_run_steps(dm_batch *B, int nsteps, double dt) {
     }
     const GraphKey key{DM_FP32C, kGraphSteps, dt, B->slot};
     auto it = B->graphs.find(key);
-    static long long graph_launches_cache = 0;
     if (it == B->graphs.end()) {
         cudaGraph_t g = nullptr;
         const unsigned long long saved = B->host_steps;
@@ -2018,7 +2022,7 @@ int batch_run_steps(dm_batch *B, int nsteps, double dt) {
         int rc = batch_enqueue_steps(B, kGraphSteps, dt);
         cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
         B->host_steps = saved;
-        graph_launches_cache = ctx->launches - sl;
+        const long long launches = ctx->launches - sl;
         ctx->launches = sl;
         if (rc || ec != cudaSuccess) {  // see run_steps
             B->d = state;
@@ -2034,13 +2038,13 @@ int batch_run_steps(dm_batch *B, int nsteps, double dt) {
         ec = cudaGraphInstantiate(&ge, g, 0);
         cudaGraphDestroy(g);
         if (ec != cudaSuccess) return ctx->fail(DM_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(ec));
-        it = B->graphs.emplace(key, ge).first;
+        it = B->graphs.emplace(key, StepGraph{ge, launches}).first;
     }
     const int reps = nsteps / kGraphSteps;
     for (int r = 0; r < reps; r++) {
-        DM_CUDA(ctx, cudaGraphLaunch(it->second, ctx->stream));
+        DM_CUDA(ctx, cudaGraphLaunch(it->second.exec, ctx->stream));
         B->host_steps += kGraphSteps;
-        ctx->launches += graph_launches_cache;
+        ctx->launches += it->second.launches;
         B->mid_valid = true;
         B->mid_dt = dt;
         for (bool &v : B->boxes_valid) v = true;
